@@ -34,6 +34,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -137,6 +138,13 @@ __global__ void k_input_layer(int64_t n, const float* __restrict__ x4,
 
 // ---------------------------------------------------------------- E X (warp per row)
 
+// Entries a warp gathers together in the row kernels below.  Each lane loads
+// one entry of the row (column, coupling), the warp takes them from the lanes
+// kEdgeGroup at a time, and a group's 256-byte gathers are in flight together:
+// a row of 15 entries is two rounds of load latency where one entry after
+// another made 45 dependent loads.  Sums stay in entry order.
+constexpr int kEdgeGroup = 8;
+
 // Y = (add + E X) o [maskH > 0]   (add, maskH optional; X, Y, add, maskH n x 64)
 __global__ void __launch_bounds__(kThreads) k_spmm(int64_t n, const int32_t* __restrict__ soff,
                                                    const int32_t* __restrict__ sw,
@@ -152,15 +160,30 @@ __global__ void __launch_bounds__(kThreads) k_spmm(int64_t n, const int32_t* __r
   const int li = int(i & 31);
   const int32_t off = soff[i >> 5], w = sw[i >> 5];
   float2 acc = add ? reinterpret_cast<const float2*>(add + i * H)[lane] : make_float2(0.f, 0.f);
-  for (int k = 0; k < w; ++k) {
-    const int32_t p = off + k * kSlice + li;
-    const int32_t j = __ldg(col + p);
-    if (j < 0) continue;
-    const float e = __ldg(eF + p);
-    if (e == 0.f) continue;
-    const float2 xj = __ldg(reinterpret_cast<const float2*>(X + int64_t(j) * H) + lane);
-    acc.x += e * xj.x;
-    acc.y += e * xj.y;
+  for (int k0 = 0; k0 < w; k0 += kSlice) {
+    // lane k holds entry k0 + k; weight 0 marks what is skipped (padding and
+    // zero couplings)
+    const bool in = k0 + lane < w;
+    const int32_t p = off + (k0 + lane) * kSlice + li;
+    const int32_t jr = in ? __ldg(col + p) : -1;
+    const float er = jr >= 0 ? __ldg(eF + p) : 0.f;
+    const int m = min(w - k0, kSlice);
+    for (int k = 0; k < m; k += kEdgeGroup) {
+      float e[kEdgeGroup];
+      float2 x[kEdgeGroup];
+#pragma unroll
+      for (int u = 0; u < kEdgeGroup; ++u) {
+        const int32_t j = __shfl_sync(0xffffffffu, jr, k + u);
+        e[u] = __shfl_sync(0xffffffffu, er, k + u);
+        x[u] = e[u] != 0.f ? __ldg(reinterpret_cast<const float2*>(X + int64_t(j) * H) + lane)
+                           : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < kEdgeGroup; ++u) {
+        acc.x += e[u] * x[u].x;
+        acc.y += e[u] * x[u].y;
+      }
+    }
   }
   if (maskH) {
     const float2 m = reinterpret_cast<const float2*>(maskH + i * H)[lane];
@@ -376,10 +399,10 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
   __shared__ uint32_t taddr_s;
   const int tid = threadIdx.x, warp = tid >> 5;
   // the weight operand, once per CTA
-  for (int t = tid; t < NOUT * KIN; t += kUmmaThreads) {
-    const int o = t / KIN, k = t % KIN;
-    const float v = FROM_W ? W[k * NOUT + o] : W[o * KIN + k];
-    *reinterpret_cast<uint16_t*>(sB + umma_off(o, k, KIN)) = bf16_bits(v);
+#pragma unroll 8
+  for (int t = tid; t < NOUT * KIN; t += kUmmaThreads) {  // W in memory order
+    const int o = FROM_W ? t % NOUT : t / KIN, k = FROM_W ? t / NOUT : t % KIN;
+    *reinterpret_cast<uint16_t*>(sB + umma_off(o, k, KIN)) = bf16_bits(__ldg(W + t));
   }
   if (tid == 0) mbar_init(&mbar, 1);
   if (warp == 0) tmem_alloc(&taddr_s, NOUT);
@@ -467,6 +490,38 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
   if (warp == 0) tmem_free(tmem, NOUT);
 }
 
+// Rows i0 .. i0 + 127 (zero past n) of [X1 | X2] (NC columns, 64 or 128) as a
+// transposed BF16 operand: element (column c, row r) at umma_off(c, r, 128).
+// A thread takes 8 rows of 4 columns: its lanes read whole 256-byte rows, and
+// each column's 8 values leave as one 16-byte store (one value at a time was
+// 4-byte loads of 32 different rows per warp and 2-byte stores).
+template <int NC>
+__device__ __forceinline__ void fill_transposed(uint8_t* s, const float* __restrict__ X1,
+                                                const float* __restrict__ X2, int64_t i0,
+                                                int64_t n, int tid) {
+  constexpr int NQ = NC / 4;
+#pragma unroll 1
+  for (int item = tid; item < NQ * (kUmmaM / 8); item += kUmmaThreads) {
+    const int c = (item % NQ) * 4, r0 = (item / NQ) * 8;
+    const float* X = (c < H ? X1 + c : X2 + (c - H)) + (i0 + r0) * H;
+    float4 v[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      v[r] = i0 + r0 + r < n ? __ldg(reinterpret_cast<const float4*>(X + r * H))
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t b[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        b[r] = bf16_bits(j == 0 ? v[r].x : j == 1 ? v[r].y : j == 2 ? v[r].z : v[r].w);
+      *reinterpret_cast<uint4*>(s + umma_off(c + j, r0, kUmmaM)) =
+          make_uint4(b[0] | (b[1] << 16), b[2] | (b[3] << 16), b[4] | (b[5] << 16),
+                     b[6] | (b[7] << 16));
+    }
+  }
+}
+
 // Per-CTA partials of dW = X^T dY (KIN x NOUT, KIN = 64 or 128 from X1 | X2)
 // on the tensor cores and, with BIAS, db = sum dY (FP32 on the CUDA cores):
 // the CTA accumulates its 128-row tiles in TMEM (rows as the reduction
@@ -504,22 +559,14 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
   bool ok = true;
   float dbias = 0.f;  // thread tid < NOUT: column tid of dY summed over this CTA's rows
   for (int64_t tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x) {
-    // row tid of the tile: its KIN inputs as column tid of A, its NOUT
-    // output gradients as column tid of B
-    const int64_t i = tile * KR + tid;
-    for (int k = 0; k < KIN; ++k) {
-      const float v = i < n ? (k < H ? X1[i * H + k] : X2[i * H + (k - H)]) : 0.f;
-      *reinterpret_cast<uint16_t*>(sA + umma_off(k, tid, KR)) = bf16_bits(v);
-    }
-    for (int o = 0; o < NOUT; ++o) {
-      const float v = i < n ? (o < H ? dY1[i * H + o] : dY2[i * H + (o - H)]) : 0.f;
-      *reinterpret_cast<uint16_t*>(sB + umma_off(o, tid, KR)) = bf16_bits(v);
-    }
+    // the tile's rows along K: inputs as A, output gradients as B
+    fill_transposed<KIN>(sA, X1, X2, tile * KR, n, tid);
+    fill_transposed<NOUT>(sB, dY1, dY2, tile * KR, n, tid);
     if (BIAS && tid < NOUT) {
-      for (int r = 0; r < KR; ++r) {
-        const int64_t ir = tile * KR + r;
-        if (ir < n) dbias += tid < H ? dY1[ir * H + tid] : dY2[ir * H + (tid - H)];
-      }
+      const float* col = (tid < H ? dY1 + tid : dY2 + (tid - H)) + tile * KR * H;
+      const int nr = static_cast<int>(n - tile * KR < KR ? n - tile * KR : KR);
+#pragma unroll 16
+      for (int r = 0; r < nr; ++r) dbias += __ldg(col + r * H);
     }
     fence_async_smem();
     tc_fence_before();
@@ -626,14 +673,56 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(int64_t n, const float* __re
 
 // grad[dst[k]] += sum over blocks of part[blk][k] (fixed order, FP64).
 // dst maps output k to a parameter index: k < nw -> wofs + k, else bofs + (k - nw).
-__global__ void k_reduce_parts(const float* __restrict__ part, int nblk, int nout, int nw,
-                               int64_t wofs, int64_t bofs, float* __restrict__ grad) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nout) return;
+// A block takes 32 outputs; its 8 warps each sum every 8th row of partials.
+// Latency is the bound: one thread per output over all the rows, a serial
+// chain of loads and FP64 adds, took 2.56 ms of a 5.3 ms gradient on a 49^3
+// system (6 launches, the 14,706 rows of the edge pass most of it); with the
+// two-level sums below and the grouped gathers and operand fills of this file
+// that gradient takes 1.8 ms.
+constexpr int kRedRows = 8;
+template <class T>
+__global__ void __launch_bounds__(32 * kRedRows)
+    k_reduce_parts(const T* __restrict__ part, int nblk, int nout, int nw, int64_t wofs,
+                   int64_t bofs, float* __restrict__ grad) {
+  __shared__ double red[kRedRows][32];
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
   double s = 0.0;
-  for (int b = 0; b < nblk; ++b) s += part[int64_t(b) * nout + k];
+  if (k < nout) {
+#pragma unroll 8
+    for (int b = row; b < nblk; b += kRedRows) s += double(part[int64_t(b) * nout + k]);
+  }
+  red[row][lane] = s;
+  __syncthreads();
+  if (row || k >= nout) return;
+#pragma unroll
+  for (int r = 1; r < kRedRows; ++r) s += red[r][lane];
   const int64_t dst = k < nw ? wofs + k : bofs + (k - nw);
   grad[dst] += float(s);
+}
+
+// fold[c][k] = sum of rows c per .. c per + per - 1 of part[row][k]: the first
+// level of the reduction where there are many rows (one per block of the
+// edge pass: n / 8 of them).  32 outputs and one chunk per block.
+constexpr int kFold = 128;  // chunks at most
+__global__ void __launch_bounds__(32 * kRedRows)
+    k_fold_parts(const float* __restrict__ part, int64_t nblk, int nout, int64_t per,
+                 double* __restrict__ fold) {
+  __shared__ double red[kRedRows][32];
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
+  const int64_t b0 = blockIdx.y * per, b1 = b0 + per < nblk ? b0 + per : nblk;
+  double s = 0.0;
+  if (k < nout) {
+#pragma unroll 8
+    for (int64_t b = b0 + row; b < b1; b += kRedRows) s += double(part[b * nout + k]);
+  }
+  red[row][lane] = s;
+  __syncthreads();
+  if (row || k >= nout) return;
+#pragma unroll
+  for (int r = 1; r < kRedRows; ++r) s += red[r][lane];
+  fold[int64_t(blockIdx.y) * nout + k] = s;
 }
 
 // ---------------------------------------------------------------- edge network
@@ -687,24 +776,46 @@ __global__ void __launch_bounds__(kThreads) k_edge_fwd(int64_t n, const int32_t*
   const float2 ai = reinterpret_cast<const float2*>(A + i * H)[lane];
   const EdgeLane E(P, lane);
   const float ob = *P.ob;
-  for (int k = 0; k < w; ++k) {
-    const int32_t p = off + k * kSlice + li;
-    const int32_t j = __ldg(colL + p);
-    if (j < 0) continue;
-    const float e = __ldg(eL + p);
-    const int32_t pu = tposU[p];
-    const float t = tU[pu];
-    float nv = 0.f, th = 0.f;
-    // e = t = 0 on edges at Dirichlet nodes (N = 0 there); a zero coupling
-    // elsewhere can still carry a second-order term
-    if (e != 0.f || t != 0.f) {
-      const float2 bj = __ldg(reinterpret_cast<const float2*>(B + int64_t(j) * H) + lane);
-      const float2 z = E.z(ai, bj, e, t);
-      const float o = warp_sum(E.w.x * relu(z.x) + E.w.y * relu(z.y)) + ob;
-      th = tanhf(o);
-      nv = (e + t) * (1.f + th);
+  for (int k0 = 0; k0 < w; k0 += kSlice) {
+    // lane k holds entry k0 + k and its outputs
+    const int32_t p = off + (k0 + lane) * kSlice + li;
+    const int32_t jr = k0 + lane < w ? __ldg(colL + p) : -1;
+    int32_t pu = 0;
+    float er = 0.f, tr = 0.f, nv = 0.f, th = 0.f;
+    if (jr >= 0) {
+      er = __ldg(eL + p);
+      pu = __ldg(tposU + p);
+      tr = __ldg(tU + pu);
     }
-    if (lane == 0) {
+    const int m = min(w - k0, kSlice);
+    for (int k = 0; k < m; k += kEdgeGroup) {
+      float e[kEdgeGroup], t[kEdgeGroup];
+      float2 bj[kEdgeGroup];
+#pragma unroll
+      for (int u = 0; u < kEdgeGroup; ++u) {
+        const int32_t j = __shfl_sync(0xffffffffu, jr, k + u);
+        e[u] = __shfl_sync(0xffffffffu, er, k + u);
+        t[u] = __shfl_sync(0xffffffffu, tr, k + u);
+        // e = t = 0 on edges at Dirichlet nodes (N = 0 there); a zero
+        // coupling elsewhere can still carry a second-order term
+        if (e[u] != 0.f || t[u] != 0.f)
+          bj[u] = __ldg(reinterpret_cast<const float2*>(B + int64_t(j) * H) + lane);
+      }
+#pragma unroll
+      for (int u = 0; u < kEdgeGroup; ++u) {
+        if (e[u] != 0.f || t[u] != 0.f) {
+          const float2 z = E.z(ai, bj[u], e[u], t[u]);
+          const float o = warp_sum(E.w.x * relu(z.x) + E.w.y * relu(z.y)) + ob;
+          if (lane == k + u) th = o;
+        }
+      }
+    }
+    // tanh and the stores, one entry per lane
+    if (jr >= 0) {
+      if (er != 0.f || tr != 0.f) {
+        th = tanhf(th);
+        nv = (er + tr) * (1.f + th);
+      }
       nL[p] = nv;
       nU[pu] = nv;
       if (TRAIN) thL[p] = th;
@@ -735,35 +846,54 @@ __global__ void __launch_bounds__(kThreads) k_edge_bwd_lower(
     const int32_t off = soffL[i >> 5], w = swL[i >> 5];
     const float2 ai = reinterpret_cast<const float2*>(A + i * H)[lane];
     const EdgeLane E(P, lane);
-    for (int k = 0; k < w; ++k) {
-      const int32_t p = off + k * kSlice + li;
-      const int32_t j = __ldg(colL + p);
-      if (j < 0) continue;
-      const float e = __ldg(eL + p);
-      const int32_t pu = tposU[p];
-      const float t = tU[pu];
-      if (e == 0.f && t == 0.f) {
-        if (lane == 0) doU[pu] = 0.f;
-        continue;
+    for (int k0 = 0; k0 < w; k0 += kSlice) {
+      // lane k holds entry k0 + k
+      const int32_t p = off + (k0 + lane) * kSlice + li;
+      const int32_t jr = k0 + lane < w ? __ldg(colL + p) : -1;
+      float er = 0.f, tr = 0.f, dr = 0.f;
+      if (jr >= 0) {
+        const int32_t pu = __ldg(tposU + p);
+        er = __ldg(eL + p);
+        tr = __ldg(tU + pu);
+        if (er != 0.f || tr != 0.f) {
+          const float th = __ldg(thL + p);
+          dr = __ldg(dnU + pu) * (er + tr) * (1.f - th * th);
+        }
+        doU[pu] = dr;
       }
-      const float th = thL[p];
-      const float dov = dnU[pu] * (e + t) * (1.f - th * th);
-      const float2 bj = __ldg(reinterpret_cast<const float2*>(B + int64_t(j) * H) + lane);
-      const float2 z = E.z(ai, bj, e, t);
-      const float dz0 = z.x > 0.f ? dov * E.w.x : 0.f;
-      const float dz1 = z.y > 0.f ? dov * E.w.y : 0.f;
-      dai.x += dz0;
-      dai.y += dz1;
-      gw.x += dov * relu(z.x);
-      gw.y += dov * relu(z.y);
-      gc.x += dz0 * e;
-      gc.y += dz1 * e;
-      gc2.x += dz0 * t;
-      gc2.y += dz1 * t;
-      gd.x += dz0;
-      gd.y += dz1;
-      gob += dov;
-      if (lane == 0) doU[pu] = dov;
+      const int m = min(w - k0, kSlice);
+      for (int kk = 0; kk < m; kk += kEdgeGroup) {
+        float e[kEdgeGroup], t[kEdgeGroup], dv[kEdgeGroup];
+        float2 bj[kEdgeGroup];
+#pragma unroll
+        for (int u = 0; u < kEdgeGroup; ++u) {
+          const int32_t j = __shfl_sync(0xffffffffu, jr, kk + u);
+          e[u] = __shfl_sync(0xffffffffu, er, kk + u);
+          t[u] = __shfl_sync(0xffffffffu, tr, kk + u);
+          dv[u] = __shfl_sync(0xffffffffu, dr, kk + u);
+          if (e[u] != 0.f || t[u] != 0.f)
+            bj[u] = __ldg(reinterpret_cast<const float2*>(B + int64_t(j) * H) + lane);
+        }
+#pragma unroll
+        for (int u = 0; u < kEdgeGroup; ++u) {
+          if (e[u] == 0.f && t[u] == 0.f) continue;
+          const float dov = dv[u];
+          const float2 z = E.z(ai, bj[u], e[u], t[u]);
+          const float dz0 = z.x > 0.f ? dov * E.w.x : 0.f;
+          const float dz1 = z.y > 0.f ? dov * E.w.y : 0.f;
+          dai.x += dz0;
+          dai.y += dz1;
+          gw.x += dov * relu(z.x);
+          gw.y += dov * relu(z.y);
+          gc.x += dz0 * e[u];
+          gc.y += dz1 * e[u];
+          gc2.x += dz0 * t[u];
+          gc2.y += dz1 * t[u];
+          gd.x += dz0;
+          gd.y += dz1;
+          gob += dov;
+        }
+      }
     }
     reinterpret_cast<float2*>(da + i * H)[lane] = dai;
   }
@@ -798,17 +928,37 @@ __global__ void __launch_bounds__(kThreads) k_edge_bwd_upper(
   const float2 bj = reinterpret_cast<const float2*>(B + j * H)[lane];
   const EdgeLane E(P, lane);
   float2 acc = make_float2(0.f, 0.f);
-  for (int k = 0; k < w; ++k) {
-    const int32_t p = off + k * kSlice + lj;
-    const int32_t i = __ldg(colU + p);
-    if (i < 0) continue;
-    const float dov = doU[p];
-    if (dov == 0.f) continue;
-    const float e = __ldg(eU + p);
-    const float2 ai = __ldg(reinterpret_cast<const float2*>(A + int64_t(i) * H) + lane);
-    const float2 z = E.z(ai, bj, e, tU[p]);
-    if (z.x > 0.f) acc.x += dov * E.w.x;
-    if (z.y > 0.f) acc.y += dov * E.w.y;
+  for (int k0 = 0; k0 < w; k0 += kSlice) {
+    // lane k holds entry k0 + k
+    const int32_t p = off + (k0 + lane) * kSlice + lj;
+    const int32_t ir = k0 + lane < w ? __ldg(colU + p) : -1;
+    float er = 0.f, tr = 0.f, dr = 0.f;
+    if (ir >= 0) {
+      dr = __ldg(doU + p);
+      er = __ldg(eU + p);
+      tr = __ldg(tU + p);
+    }
+    const int m = min(w - k0, kSlice);
+    for (int k = 0; k < m; k += kEdgeGroup) {
+      float dv[kEdgeGroup];
+      float2 ai[kEdgeGroup];
+#pragma unroll
+      for (int u = 0; u < kEdgeGroup; ++u) {
+        const int32_t i = __shfl_sync(0xffffffffu, ir, k + u);
+        dv[u] = __shfl_sync(0xffffffffu, dr, k + u);
+        if (dv[u] != 0.f)
+          ai[u] = __ldg(reinterpret_cast<const float2*>(A + int64_t(i) * H) + lane);
+      }
+#pragma unroll
+      for (int u = 0; u < kEdgeGroup; ++u) {
+        const float e = __shfl_sync(0xffffffffu, er, k + u);
+        const float t = __shfl_sync(0xffffffffu, tr, k + u);
+        if (dv[u] == 0.f) continue;
+        const float2 z = E.z(ai[u], bj, e, t);
+        if (z.x > 0.f) acc.x += dv[u] * E.w.x;
+        if (z.y > 0.f) acc.y += dv[u] * E.w.y;
+      }
+    }
   }
   reinterpret_cast<float2*>(db + j * H)[lane] = acc;
 }
@@ -928,6 +1078,7 @@ struct xg_lpc {
         *tU = nullptr;
   double* dpart = nullptr;
   float* epart = nullptr;  // edge-parameter partials, one row per block
+  double* efold = nullptr;  // their first-level sums, kFold rows at most
 };
 
 namespace xg {
@@ -978,9 +1129,12 @@ int ensure_work(xg_ctx* c, xg_lpc* m, int64_t n, int64_t nl, int64_t nu) {
 }
 
 // The tensor-core GEMMs: dense layer (forward or backward data) and weight
-// gradient partials, on one CTA per SM at most (each holds up to 128 TMEM
-// columns and 64 KB of operand tiles).
-int umma_grid(int64_t n) {
+// gradient partials.  A CTA takes its tiles one after another (load, MMA,
+// epilogue), so a few CTAs per SM overlap each other's phases: per_sm of them
+// at most (up to 128 TMEM columns and 64 KB of operand tiles each: four dense
+// CTAs fill the SM's 512 columns, two weight-gradient CTAs fit its partials).
+constexpr int kDensePerSm = 4, kWgradPerSm = 2;
+int umma_grid(int64_t n, int per_sm, int most) {
   static int nsm = [] {
     int dev = 0, v = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -988,7 +1142,8 @@ int umma_grid(int64_t n) {
       v = 1;
     return v < 1 ? 1 : v;
   }();
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((n + kUmmaM - 1) / kUmmaM, nsm)));
+  const int64_t cap = std::min<int64_t>(most, int64_t(per_sm) * nsm);
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((n + kUmmaM - 1) / kUmmaM, cap)));
 }
 
 template <int KIN, int NOUT, bool FROM_W>
@@ -998,7 +1153,7 @@ int dense_umma(xg_ctx* c, xg_lpc* m, int64_t n, const float* X1, const float* X2
   static const cudaError_t attr = cudaFuncSetAttribute(
       k_dense_umma<KIN, NOUT, FROM_W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   XG_CUDA(c, attr);
-  k_dense_umma<KIN, NOUT, FROM_W><<<umma_grid(n), kUmmaThreads, smem, c->stream>>>(
+  k_dense_umma<KIN, NOUT, FROM_W><<<umma_grid(n, kDensePerSm, INT_MAX), kUmmaThreads, smem, c->stream>>>(
       n, X1, X2, W, bias, act, maskY, Y1, Y2, m->uerr);
   XG_CHECK_LAUNCH(c);
   return XG_OK;
@@ -1012,11 +1167,11 @@ int wgrad_umma(xg_ctx* c, xg_lpc* m, int64_t n, const float* X1, const float* X2
   static const cudaError_t attr = cudaFuncSetAttribute(
       k_wgrad_umma<KIN, NOUT, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   XG_CUDA(c, attr);
-  const int grid = umma_grid(n);
+  const int grid = umma_grid(n, kWgradPerSm, kWgradBlocks);  // wpart holds kWgradBlocks rows
   k_wgrad_umma<KIN, NOUT, BIAS><<<grid, kUmmaThreads, smem, c->stream>>>(n, X1, X2, dY1, dY2,
                                                                           m->wpart, m->uerr);
-  k_reduce_parts<<<(NOUTP + 255) / 256, 256, 0, c->stream>>>(m->wpart, grid, NOUTP, NW, wofs,
-                                                             bofs, m->grad);
+  k_reduce_parts<<<(NOUTP + 31) / 32, 32 * kRedRows, 0, c->stream>>>(m->wpart, grid, NOUTP, NW,
+                                                                     wofs, bofs, m->grad);
   XG_CHECK_LAUNCH(c);
   return XG_OK;
 }
@@ -1084,8 +1239,8 @@ int wgrad(xg_ctx* c, xg_lpc* m, int64_t n, const float* X1, const float* X2, con
   cudaStream_t s = c->stream;
   constexpr int NOUT = (K1 + K2) * N + (BIAS ? N : 0);
   k_wgrad<K1, K2, N, BIAS><<<kWgradBlocks, kThreads, 0, s>>>(n, X1, X2, dY1, dY2, m->wpart);
-  k_reduce_parts<<<(NOUT + 255) / 256, 256, 0, s>>>(m->wpart, kWgradBlocks, NOUT,
-                                                    (K1 + K2) * N, wofs, bofs, m->grad);
+  k_reduce_parts<<<(NOUT + 31) / 32, 32 * kRedRows, 0, s>>>(m->wpart, kWgradBlocks, NOUT,
+                                                            (K1 + K2) * N, wofs, bofs, m->grad);
   XG_CHECK_LAUNCH(c);
   return XG_OK;
 }
@@ -1138,6 +1293,7 @@ int xg_lpc_create(xg_ctx* c, int precision, xg_lpc** out) {
     P.plan(m->lossv, 4);
     P.plan(m->uerr, 1);
     P.plan(m->wpart, int64_t(kWgradBlocks) * (2 * H * 2 * H + 2 * H));
+    P.plan(m->efold, int64_t(kFold) * kEdgeParts);
     if (pass == 0 && P.reserve() != cudaSuccess) {
       xg_lpc_destroy(m);
       return fail(c, XG_ERR_CUDA, "lpc_create: device allocation failed");
@@ -1248,7 +1404,13 @@ int xg_lpc_grad(xg_lpc* m, xg_ctx* c, double* loss) {
   k_edge_bwd_lower<<<nrb, kThreads, 0, s>>>(n, g.soffL, g.swL, g.colL, g.eL, g.tposU, m->tU,
                                             m->tL, m->A, m->B, P, m->dnU, m->da, m->doU,
                                             m->epart);
-  k_reduce_parts<<<1, 512, 0, s>>>(m->epart, int(nrb), kEdgeParts, kEdgeParts, oc, 0, m->grad);
+  const int64_t per = std::max<int64_t>(64, (int64_t(nrb) + kFold - 1) / kFold);
+  const int nfold = static_cast<int>((int64_t(nrb) + per - 1) / per);
+  const unsigned ncol = (kEdgeParts + 31) / 32;
+  k_fold_parts<<<dim3(ncol, nfold), 32 * kRedRows, 0, s>>>(m->epart, nrb, kEdgeParts, per,
+                                                           m->efold);
+  k_reduce_parts<<<ncol, 32 * kRedRows, 0, s>>>(m->efold, nfold, kEdgeParts, kEdgeParts, oc, 0,
+                                                m->grad);
   k_edge_bwd_upper<<<nrb, kThreads, 0, s>>>(n, g.soffU, g.swU, g.colU, g.eU, m->tU, m->doU, m->A,
                                             m->B, P, m->db);
   XG_CHECK_LAUNCH(c);
