@@ -16,7 +16,10 @@
 // their diagonal), and the right-hand side correction sum_i a_ji * val_i is
 // summed per row in the reference's order (decreasing node id).
 //
-// One PCG iteration (the reference's FP64 algorithm) is three kernels:
+// One PCG iteration (the reference's FP64 algorithm) runs inside k_cg_loop,
+// one cooperative launch for the whole solve, where the rows fit the SMs'
+// shared memory (about 960,000 rows) and no factor is applied.  Otherwise it
+// is three kernels:
 //   k_cg_p: p = z + beta p (beta = rho/rho0)
 //   k_cg_a: q = A p, partial (p, q)
 //   k_cg_b: alpha = rho/(p,q); r -= alpha q; x += alpha p; z = r/d (Jacobi,
@@ -65,6 +68,8 @@ constexpr int32_t kPad = -1;
 constexpr int16_t kPad16 = std::numeric_limits<int16_t>::min();
 constexpr int kBlock = 256;
 constexpr int kBatch = 16;
+constexpr int kLoopThreads = 1024;  // the whole-solve kernel k_cg_loop: one block per SM
+constexpr int kLoopRound = 8;       // its entries in flight per row
 
 struct CGScalars {
   double rho, rho0, pq, alpha, rr, normb, tol, delta, rlast;
@@ -73,7 +78,10 @@ struct CGScalars {
   int32_t done, finished, converged, pc;
   int32_t guard, pad1;  // 0: |(p,q)| < DBL_EPSILON ends the solve; 1: underflow only
   unsigned int ticket[4];
+  int32_t err, pad2;  // k_cg_loop: a wait for the other blocks ran out
 };
+
+
 }  // namespace
 
 struct CGDev {
@@ -96,6 +104,8 @@ struct CGDev {
   float* p32[2] = {nullptr, nullptr};
   double* partial = nullptr;  // 3 * maxgrid
   CGScalars* scal = nullptr;
+  double* lpart = nullptr;         // k_cg_loop: [3 barriers of an iteration][2 sums][SMs]
+  unsigned int* larrive = nullptr;  // and its arrival count
   bool apply = false;
   bool ready = false;
   bool use16 = false;  // every |j - i| fits a 16-bit offset
@@ -296,6 +306,7 @@ __device__ __forceinline__ T sell_row_x(CI ci, const V* __restrict__ val, int32_
 
 // One wave of resident blocks of kernel K for n rows.
 int g_nsm = 0;
+size_t g_smem = 0;  // shared memory a block may ask for; 0: no cooperative launches
 template <auto K>
 unsigned pgrid(int64_t n) {
   static const int per_sm = [] {
@@ -751,6 +762,224 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 6 : 1) k_pc_lower(int
   }
 }
 
+// ---- the FP64 iteration as one kernel
+
+// Polls of the arrival count before a wait gives up (about a second).
+constexpr int kLoopSpin = 1 << 20;
+
+// The blocks' meeting points in k_cg_loop.
+struct LoopSync {
+  double* part;          // [3][2][blocks]
+  unsigned int* arrive;  // arrivals since the launch
+  unsigned int target;   // arrivals when every block has reached this barrier
+  int turn;              // barriers so far, modulo 3
+};
+
+// Barrier of all blocks of k_cg_loop that also sums K values per thread over
+// the grid (K = 0: the barrier alone; the threads from `active` on hold 0);
+// lane 0 of warp k calls fin(k, sum) with the total of value k before the
+// block goes on.  Everything the grid wrote
+// before the barrier is visible after it.
+//
+// An FP64 instruction holds its SM quarter's FP64 unit for 64 cycles on
+// GB300, whatever the number of lanes, so the block's sums are formed with as
+// few warp instructions as a tree allows: through shared memory, one warp of
+// each quarter adds a quarter of the rows, then one warp per value the rest
+// (11 in sequence; shuffles in each of 32 warps would take 40 per quarter).
+// Each value's warp leaves the block's sum in global memory and counts
+// itself in; one counter polled by lane 0 meets in 1.3 us on 152 SMs, where
+// every block polling every block's slot took 4.7 us.  The warp then adds all
+// blocks' sums in block order, so every block holds the same bits.  The sums
+// alternate between three arrays: a block passes a barrier only after every
+// block has arrived, so it may be one barrier ahead of the slowest reader
+// and never overwrites what is still to be read.  False in every thread of the
+// block when a wait ran out.
+template <int K, class F>
+__device__ __forceinline__ bool grid_sum(const double (&v)[K > 0 ? K : 1], int active,
+                                         LoopSync& sync, CGScalars* sc, F fin) {
+  constexpr int KW = K > 0 ? K : 1;          // polling warps
+  constexpr int NW = kLoopThreads / 32 / 4;  // rows of each quarter's warp
+  __shared__ double rows[KW][kLoopThreads];
+  __shared__ double quarter[KW][4][32];
+  __shared__ int okay;
+  const int nb = gridDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (threadIdx.x == 0) okay = 1;
+  if (K > 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) rows[k][threadIdx.x] = v[k];
+    __syncthreads();
+    if (wid < 4 * K) {
+      const int k = wid >> 2, qd = wid & 3;
+      double s = 0.0;
+#pragma unroll
+      for (int j = 0; j < NW; ++j)
+        if (32 * (qd + 4 * j) < active) s += rows[k][lane + 32 * (qd + 4 * j)];
+      quarter[k][qd][lane] = s;
+    }
+  }
+  __syncthreads();
+  sync.target += unsigned(nb) * KW;
+  if (wid < KW) {
+    double* part = sync.part + (sync.turn * 2 + wid) * nb;
+    if (K > 0) {
+      double s = (quarter[wid][0][lane] + quarter[wid][1][lane]) +
+                 (quarter[wid][2][lane] + quarter[wid][3][lane]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) part[blockIdx.x] = s;
+    }
+    if (lane == 0) {
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(sync.arrive) : "memory");
+      unsigned int seen = 0;
+      int spin = 0;
+      do {
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync.arrive) : "memory");
+      } while (int(seen - sync.target) < 0 && ++spin < kLoopSpin);
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      if (spin >= kLoopSpin) {
+        okay = 0;
+        atomicExch(&sc->err, 1);
+      }
+    }
+    __syncwarp();
+    if (K > 0) {
+      double sum = 0.0;
+      for (int b = lane; b < nb; b += 32) sum += __ldcg(part + b);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0) fin(wid, sum);
+    }
+  }
+  sync.turn = sync.turn == 2 ? 0 : sync.turn + 1;
+  __syncthreads();
+  return okay != 0;
+}
+
+// Up to maxits whole iterations of the FP64 PCG without a factor
+// (ConjugateGradients::next/qAp/q/pq/rz/x, ConjugateGradients.cpp:584-823; the
+// same operations in the same order per row as k_cg_p, k_cg_a and k_cg_b) in
+// one cooperative launch, one block per SM, each block holding a contiguous
+// run of `per` rows with its residual, q (then z), direction and inverse
+// diagonal in shared memory; only the direction (gathered by other rows), x
+// and the matrix are in global memory.
+//
+// Three launches per iteration cost their drains, launch gaps and two
+// reduction tails (about 20 us an iteration however small the system), and
+// on GB300 the FP64 pipe is a bound beside memory: 22 FP64 operations a row
+// and iteration take 11 us at 65^3 and 38 us at 97^3 (530 G operations/s).
+// Here an iteration pays three grid barriers (grid_sum): 38 -> 21 us an
+// iteration at 65^3, 65 -> 48 us at 97^3, 17 -> 10 us at 17^3.  1024 threads with
+// rounds of 8 entries and 512 with rounds of 16 measured within 3 % of each
+// other.
+template <class CI>
+__global__ void __launch_bounds__(kLoopThreads, 1)
+    k_cg_loop(int64_t n, int per, int64_t maxits, const int32_t* __restrict__ soff,
+              const int32_t* __restrict__ sw, CI ci, const double* __restrict__ a,
+              const double* __restrict__ d, double* r, double* z, double* p, double* x,
+              double* lpart, unsigned int* larrive, CGScalars* sc) {
+  extern __shared__ double loop_smem[];
+  __shared__ double sh_scale, sh_rho, sh_rho0, sh_rr, sh_pq;  // scale: alpha, then beta
+  __shared__ int sh_fin, sh_end;
+  if (sc->done) return;
+  double* sr = loop_smem;
+  double* sq = sr + per;  // q, then z
+  double* sp = sq + per;
+  double* sd = sp + per;
+  const int64_t r0 = int64_t(blockIdx.x) * per;
+  const int rows = static_cast<int>(n - r0 < per ? n - r0 : per);
+  for (int t = threadIdx.x; t < rows; t += kLoopThreads) {
+    sr[t] = r[r0 + t];
+    sq[t] = z[r0 + t];
+    sp[t] = p[r0 + t];
+    sd[t] = d[r0 + t];
+  }
+  int64_t it = sc->it;
+  const int64_t maxit = sc->maxit;
+  const double nb = sc->normb > 1.0e-14 ? sc->normb : 1.0;
+  const double lim = sc->tol * nb;
+  const double eps = sc->guard == 0 ? DBL_EPSILON : DBL_MIN;
+  if (threadIdx.x == 0) {
+    sh_rho = sc->rho;
+    sh_rho0 = sc->rho0;
+    sh_rr = sc->rr;
+    sh_pq = sc->pq;
+    sh_fin = sc->finished;
+    sh_end = 0;
+    sh_scale = it == 0 ? 0.0 : sc->rho / sc->rho0;
+  }
+  __syncthreads();
+  LoopSync sync{lpart, larrive, 0u, 0};
+  double alpha = sc->alpha;
+  const double none[1] = {0.0};
+  for (int64_t step = 0; step < maxits && !sh_end; ++step) {
+    // p = z + beta p
+    const double beta = sh_scale;
+    for (int t = threadIdx.x; t < rows; t += kLoopThreads) {
+      const double pi = sq[t] + beta * sp[t];
+      sp[t] = pi;
+      p[r0 + t] = pi;
+    }
+    if (!grid_sum<0>(none, 0, sync, sc, [](int, double) {})) return;
+    // q = A p, (p, q)
+    double dot[1] = {0.0};
+    for (int t = threadIdx.x; t < rows; t += kLoopThreads) {
+      const int64_t i = r0 + t;
+      const double s =
+          sell_row_x<double, kLoopRound>(ci, a, soff[i >> 5], sw[i >> 5], int(i & 31), int32_t(i),
+                                         [&](int32_t c) { return p[c]; });
+      sq[t] = s;
+      dot[0] += sp[t] * s;
+    }
+    if (!grid_sum<1>(dot, rows, sync, sc, [&](int, double pq) {
+          sh_pq = pq;
+          sh_fin = fabs(pq) < eps;
+          sh_scale = sh_fin ? 0.0 : sh_rho / pq;
+        }))
+      return;
+    alpha = sh_scale;
+    // r -= alpha q, x += alpha p, z = r d, (r, z), (r, r)
+    double v[2] = {0.0, 0.0};
+    for (int t = threadIdx.x; t < rows; t += kLoopThreads) {
+      const double ri = sr[t] - alpha * sq[t];
+      sr[t] = ri;
+      x[r0 + t] += alpha * sp[t];
+      const double zi = ri * sd[t];
+      sq[t] = zi;
+      v[0] += ri * zi;
+      v[1] += ri * ri;
+    }
+    it += 1;
+    if (!grid_sum<2>(v, rows, sync, sc, [&](int k, double sum) {
+          if (k == 0) {
+            sh_rho0 = sh_rho;
+            sh_rho = sum;
+            sh_scale = sum / sh_rho0;
+          } else {  // the stopping test (ConjugateGradients.cpp:772-823)
+            sh_rr = sum;
+            const double nr = sqrt(sum);
+            sh_end = sh_fin || nr < lim || it >= maxit ? (nr > lim ? 1 : 2) : 0;
+          }
+        }))
+      return;
+  }
+  for (int t = threadIdx.x; t < rows; t += kLoopThreads) {
+    r[r0 + t] = sr[t];
+    z[r0 + t] = sq[t];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->rho = sh_rho;
+    sc->rho0 = sh_rho0;
+    sc->rr = sh_rr;
+    sc->pq = sh_pq;
+    sc->alpha = alpha;
+    sc->it = it;
+    sc->finished = sh_fin;
+    sc->converged = sh_end == 2;
+    sc->done = sh_end != 0;
+  }
+}
+
 // v = S r
 template <class T>
 __global__ void k_scale(int64_t n, const float* __restrict__ srow, const T* __restrict__ r,
@@ -1000,12 +1229,66 @@ void factor_apply32(xg_ctx* c, CGDev* d, CI cu, CI cl) {
       d->bcmask, d->u32, d->r32, d->r32b, d->z32, d->partial, d->scal);
 }
 
+// Rows per block of k_cg_loop and its blocks for n rows: contiguous runs of
+// whole slices, one block per SM, at least kLoopMinRows rows each: a warp for
+// each of the SM's four FP64 units, which take as long for one warp as for
+// none beside it, and fewer blocks' sums to add.
+constexpr int64_t kLoopMinRows = 128;
+constexpr size_t kLoopStatic = 4 * (kLoopThreads + 128) * 8 + 1024;  // its static shared memory, rounded up
+struct LoopShape {
+  int per = 0;
+  unsigned grid = 0;
+  size_t smem = 0;
+};
+bool loop_shape(int64_t n, LoopShape* out) {
+  const int64_t want = (n + g_nsm - 1) / g_nsm;
+  const int64_t per = std::max<int64_t>(kLoopMinRows, (want + kSlice - 1) / kSlice * kSlice);
+  out->smem = size_t(per) * 4 * sizeof(double);
+  if (out->smem + kLoopStatic > g_smem) return false;
+  out->per = static_cast<int>(per);
+  out->grid = static_cast<unsigned>((n + per - 1) / per);
+  return true;
+}
+
+// The FP64 solve by k_cg_loop launches of at most kLoopIts iterations (a
+// launch is bounded in time; the state goes through global memory between
+// launches).
+constexpr int64_t kLoopIts = 8192;
+template <class CI>
+int loop_solve(xg_ctx* c, CGDev* d, const LoopShape& sh, CI ci, CGScalars* h) {
+  cudaStream_t s = c->stream;
+  XG_CUDA(c, cudaFuncSetAttribute(k_cg_loop<CI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(sh.smem)));
+  int64_t n = d->n, its = kLoopIts;
+  int per = sh.per;
+  const double *a = d->a, *dd = d->d;
+  void* args[] = {&n,    &per,  &its,     &d->soff, &d->swidth, &ci,         &a,      &dd,
+                  &d->r, &d->z, &d->p[0], &d->x,    &d->lpart,  &d->larrive, &d->scal};
+  for (;;) {
+    XG_CUDA(c, cudaMemsetAsync(d->larrive, 0, sizeof(unsigned int), s));
+    XG_CUDA(c, cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_cg_loop<CI>),
+                                           dim3(sh.grid), dim3(kLoopThreads), args, sh.smem, s));
+    int rc = read_scal(c, d, h);
+    if (rc) return rc;
+    if (h->err) {
+      h->err = 0;
+      rc = write_scal(c, d, h);
+      return rc ? rc : fail(c, XG_ERR_DEVICE, "cg_solve: a grid barrier timed out");
+    }
+    if (h->done) return XG_OK;
+  }
+}
+
 int cg_iterate(xg_ctx* c, CGDev* d, int64_t maxit, double tol, CGScalars* h) {
   cudaStream_t s = c->stream;
   // tol and maxit into the device scalars without touching the rest
   XG_CUDA(c, cudaMemcpyAsync(&d->scal->tol, &tol, sizeof(double), cudaMemcpyHostToDevice, s));
   XG_CUDA(c, cudaMemcpyAsync(&d->scal->maxit, &maxit, sizeof(int64_t), cudaMemcpyHostToDevice, s));
   const int64_t n = d->n;
+  LoopShape sh;
+  if (d->pc != 2 && loop_shape(n, &sh))
+    return d->use16 ? loop_solve(c, d, sh, Cols16{d->col16}, h)
+                    : loop_solve(c, d, sh, Cols32{d->col}, h);
   for (;;) {
     for (int k = 0; k < kBatch; ++k) {
       double* p0 = d->p[0];
@@ -1216,6 +1499,10 @@ int xg_cg_setup(xg_ctx* c, int64_t nrow, const uint64_t* ia, const uint64_t* ja,
     int dev = 0, nsm = 0;
     XG_CUDA(c, cudaGetDevice(&dev));
     XG_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    int smem = 0, coop = 0;
+    XG_CUDA(c, cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    XG_CUDA(c, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    g_smem = coop ? static_cast<size_t>(smem) : 0;
     g_nsm = nsm > 0 ? nsm : 1;
   }
   const int64_t nslice = (nrow + kSlice - 1) / kSlice;
@@ -1362,6 +1649,8 @@ int xg_cg_setup(xg_ctx* c, int64_t nrow, const uint64_t* ia, const uint64_t* ja,
     A.plan(d->p32[1], nrow);
     A.plan(d->partial, 3 * d->maxgrid);
     A.plan(d->scal, 1);
+    A.plan(d->lpart, size_t(6) * g_nsm);
+    A.plan(d->larrive, 1);
     A.plan(d->soffL, nslice + 1);
     A.plan(d->swL, nslice);
     A.plan(d->colL, colL.size());
