@@ -18,6 +18,9 @@ int xg_create(int device, xg_ctx** out) {
   auto* c = new (std::nothrow) xg_ctx;
   if (!c) return XG_ERR_ARG;
   c->device = device;
+  if (cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+      c->nsm < 1)
+    c->nsm = 1;
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     delete c;

@@ -48,6 +48,20 @@ namespace {
 constexpr int kSlice = 32;
 constexpr int32_t kPad = INT32_MIN;
 constexpr int kBlock = 256;
+// Lanes per boundary node (see bnd_lane): beside the domain pass, and after it.
+// FP32 systems large enough for the separate kernels keep the chip busy with
+// one (k_rhs_bnd at 129^3: 23 us, with four 31 us); in FP64 the serial chain
+// of one lane is the bound (18 us at 33^3 with four, 91 us with one).
+constexpr int kBL = 4;
+template <class F>
+constexpr int bl_after() {
+  return sizeof(F) == 8 ? 4 : 1;
+}
+// Below these node counts the boundary nodes run beside the domain pass.  Whole
+// steps, beside against after it: FP32 57 / 75 us at 19^3, 259 / 271 at 65^3,
+// 744 / 740 at 97^3; FP64 302 / 337 at 19^3, 459 / 474 at 27^3, 636 / 616 at
+// 33^3, 1162 / 1148 at 41^3.
+constexpr int64_t kBeside32 = 600000, kBeside64 = 25000;
 
 struct Scalars {
   double dt;                  // current step size
@@ -87,12 +101,13 @@ struct RieCGDev {
   void* ent1 = nullptr;
   void* fbuf = nullptr;  // F: [nent2][4] components 0-3, then [nent2] component 4
   void* Rp = nullptr;    // F [5][n] first-end partial residuals
+  void* Rb = nullptr;    // F [5][nbn] domain residual of the boundary nodes
   double* ivol = nullptr;
-  float* cbrtv = nullptr;
+  float* cbrtv = nullptr;   // FP32 mode
+  double* cbrtd = nullptr;  // FP64 mode
   // boundary triangles, per boundary node lists of (tri << 2 | position)
   int32_t *bptr = nullptr, *bnode = nullptr;
   int4* bent4 = nullptr;  // per boundary entry: the triangle's 3 nodes, pos | sym flags << 2
-  void* Rb = nullptr;  // F [5][nbn] domain residual of the boundary nodes
   int32_t* bcof = nullptr;  // per boundary node: its BC program entry or -1
   // BC program: one thread per BC node
   int64_t nbc = 0;
@@ -262,6 +277,9 @@ __device__ __forceinline__ void cp_async_wait() {
 // Primitive variables from conserved ones (primitive(),
 // src/Physics/Riemann.cpp:211-227), evaluated in double.
 __device__ __forceinline__ void prim5(const double u[5], double w[5]) {
+  // quotients, not products with 1/rho: a uniform velocity stays exactly
+  // uniform, where its last-bit noise would enter the gradients and decide the
+  // limiter's sign tests (differences of about its 1e-9 regularisation)
   w[0] = u[0];
   w[1] = u[1] / w[0];
   w[2] = u[2] / w[0];
@@ -291,15 +309,15 @@ __device__ __forceinline__ void prim_record(const double u[5], F o[5]) {
   }
 }
 
-// Per-node CFL time step (src/Inciter/RieCG.cpp:827-838), before the CFL factor.
-__device__ __forceinline__ double node_dt(const double u[5], double vol, double g) {
-  double r = u[0];
-  double uu = u[1] / r, vv = u[2] / r, ww = u[3] / r;
-  double pr = (u[4] - 0.5 * r * (uu * uu + vv * vv + ww * ww)) * (g - 1.0);
-  double c = sqrt(g * fmax(pr, 0.0) / r);
-  double L = cbrt(vol);
-  double vel = sqrt(uu * uu + vv * vv + ww * ww);
-  return L / fmax(vel + c, 1.0e-8);
+// Per-node CFL time step (src/Inciter/RieCG.cpp:827-838), before the CFL
+// factor, with L = cbrt(vol) formed at setup and one quotient by the density.
+__device__ __forceinline__ double node_dt(const double u[5], double L, double g) {
+  const double ir = 1.0 / u[0];
+  const double uu = u[1] * ir, vv = u[2] * ir, ww = u[3] * ir;
+  const double k2 = uu * uu + vv * vv + ww * ww;
+  const double pr = (u[4] - 0.5 * u[0] * k2) * (g - 1.0);
+  const double c = sqrt(g * fmax(pr, 0.0) * ir);
+  return L / fmax(sqrt(k2) + c, 1.0e-8);
 }
 
 // Block-wide minimum of positive doubles folded into *dst with one atomic per
@@ -767,11 +785,41 @@ struct Bnd {
   const int4* bent4;     // per entry: triangle nodes N0, N1, N2 and
                          // pos | symN0 << 2 | symN1 << 3 | symN2 << 4
 };
-// Per-node factors of the FP32-mode epilogue: 1/vol and cbrt(vol).
+// Per-node factors formed at setup: 1/vol and cbrt(vol) in the mode's
+// precision.
 struct NodeAux {
   const double* ivol;
   const float* cbrtv;
+  const double* cbrtd;
 };
+
+// Boundary nodes in the node passes k_grad and k_rhs2: BL lanes per node share
+// its triangles and add their sums by shuffles, in one of two ways.
+// * Beside the domain pass (BESIDE): the grid's first blocks take the boundary
+//   nodes whole, edges and triangles, and the domain blocks skip them.  One
+//   launch per pass, for systems that are latency and launches.
+// * After it, in a kernel of their own that adds the triangles to the domain
+//   sums: those were read coalesced, where boundary lanes reading the
+//   edges again take memory bandwidth.
+// A thread per node in the separate kernels was a serial chain on a handful of
+// SMs (in FP64 some 700 instructions of 64 cycles: 69 and 91 us a stage at any
+// size).  Also measured at 129^3, FP32, per stage (separate 297 us): beside
+// 322 us, beside with the boundary blocks spread over the grid 311 us, the
+// triangles by the domain blocks' own threads after a barrier 450 us.
+template <int BL>
+__device__ __forceinline__ bool bnd_lane(int64_t nbn, int64_t& bi, int& l) {
+  const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  bi = t / BL;
+  l = static_cast<int>(t % BL);
+  return bi < nbn;
+}
+template <int BL, class F, int N>
+__device__ __forceinline__ void bnd_add(F (&v)[N]) {
+#pragma unroll
+  for (int o = 1; o < BL; o <<= 1)
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+}
 
 // Nodal gradients of primitive variables (riemann::grad,
 // src/Physics/Riemann.cpp:229-367): sum over the node's edges of
@@ -784,48 +832,166 @@ struct NodeAux {
 // the entry stream runs ahead.  The ring is kept small: shared memory comes
 // out of the L1 capacity that serves the neighbour gathers.
 // Weak gradient to nodal gradient: divide by the nodal volume
-// (RieCG::rhs, src/Inciter/RieCG.cpp:936-939), as 1/vol in FP32 mode.
+// (RieCG::rhs, src/Inciter/RieCG.cpp:936-939), as a product with 1/vol.
 template <class F>
-__device__ __forceinline__ void finish_grad(const F g[15], int divide,
-                                            const double* __restrict__ vol, NodeAux aux,
-                                            int64_t p, F o[16]) {
+__device__ __forceinline__ void finish_grad(F g[16], int divide, NodeAux aux, int64_t p) {
   if (divide) {
-    if constexpr (sizeof(F) == 8) {
-      const double v = vol[p];
+    const F iv = F(aux.ivol[p]);
 #pragma unroll
-      for (int i = 0; i < 15; ++i) o[i] = g[i] / v;
-    } else {
-      const float iv = float(aux.ivol[p]);
+    for (int i = 0; i < 15; ++i) g[i] *= iv;
+  }
+  g[15] = F(0);
+}
+
+// One edge's term of the gradient sum: +/- D (u_p + u_q) per component.
+// Splitting off the node's half (u_p times a per-node sum of its D, 15 FP64
+// instructions an edge instead of 20) took k_grad from 403 to 335 us on an
+// 81^3 cube, but its rounding moves the limiter's sign tests where a field
+// is constant to about 1e-9: one 129^3 step then differs from the reference
+// arithmetic at some 30 nodes by up to 6e-12, beyond what a reversed order of
+// the reference's own sums does.
+template <class F>
+__device__ __forceinline__ void grad_edge(const F d[3], const F wq[5], const F wp[5], F g[16]) {
 #pragma unroll
-      for (int i = 0; i < 15; ++i) o[i] = g[i] * iv;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 15; ++i) o[i] = g[i];
+  for (int c = 0; c < 5; ++c) {
+    const F sum = wq[c] + wp[c];
+    g[c * 3 + 0] += d[0] * sum;
+    g[c * 3 + 1] += d[1] * sum;
+    g[c * 3 + 2] += d[2] * sum;
   }
 }
 
+// FP64 blocks are small: the FP64 units of an SM take its blocks' work one
+// after another, so an SM with one block more than the others holds them all
+// up by that block's time (k_grad<double> at 33^3 33 -> 25 us, 81^3 430 ->
+// 394 us, the latter mostly the 15 products with 1/vol for 15 divisions).
 template <class F>
 struct GradShape {
   static constexpr int GU = 2;                        // entries per group
   static constexpr int RG = 2;                        // ring groups per thread
-  static constexpr int BLOCK = 256;
+  static constexpr int BLOCK = sizeof(F) == 8 ? 64 : 256;
 };
+
+// Boundary-triangle term of riemann::grad (src/Physics/Riemann.cpp:329-364)
+// at boundary node bi, added to g: its triangles j0 + l, j0 + l + step, ...
+// With n the triangle's unscaled normal and s = a + b + c its vertex sum, the
+// reference's ((a + b)/4 + (c + a)/4 + a) n_0 / 12 and so on are
+// (s + 5 a) n_0 / 48, (s + 5 b) n_1 / 48, (s + 5 c) n_2 / 48.
+template <class F>
+__device__ __forceinline__ void grad_bnd_term(const Bnd& bnd, int64_t bi, int l, int step,
+                                              const F* __restrict__ W, F g[16]) {
+  const int32_t j1 = __ldg(bnd.bptr + bi + 1);
+  for (int32_t j = __ldg(bnd.bptr + bi) + l; j < j1; j += step) {
+    const int4 te = __ldg(bnd.bent4 + j);
+    F a[8], b[8], c[8];
+    load8(W + int64_t(te.x) * 8, a);
+    load8(W + int64_t(te.y) * 8, b);
+    load8(W + int64_t(te.z) * 8, c);
+    const F bax = b[5] - a[5], bay = b[6] - a[6], baz = b[7] - a[7];
+    const F cax = c[5] - a[5], cay = c[6] - a[6], caz = c[7] - a[7];
+    const F k = F(1.0) / F(48.0);
+    const F nn[3] = {(bay * caz - cay * baz) * k, (baz * cax - caz * bax) * k,
+                     (bax * cay - cax * bay) * k};
+#pragma unroll
+    for (int cc = 0; cc < 5; ++cc) {
+      const F s = a[cc] + b[cc] + c[cc];
+      g[cc * 3 + 0] += (s + F(5.0) * a[cc]) * nn[0];
+      g[cc * 3 + 1] += (s + F(5.0) * b[cc]) * nn[1];
+      g[cc * 3 + 2] += (s + F(5.0) * c[cc]) * nn[2];
+    }
+  }
+}
+
+// Gradients of the boundary nodes (see bnd_lane), EDGES: with the edge sums,
+// otherwise from the domain sums that k_grad left in G.
+template <class F, bool EDGES, int BL>
+__device__ __forceinline__ void grad_boundary(int64_t nbn, const Adj<F>& adj,
+                                              const F* __restrict__ W, const Bnd& bnd,
+                                              NodeAux aux, int divide, F* G) {
+  int64_t bi;
+  int l;
+  const bool live = bnd_lane<BL>(nbn, bi, l);
+  F g[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) g[i] = F(0);
+  int64_t p = 0;
+  if (live) {
+    p = __ldg(bnd.bnode + bi);
+    if constexpr (EDGES) {
+      const int64_t s = p >> 5;
+      const int32_t w = __ldg(adj.swidth + s);
+      const typename EntOf<F>::type* src = adj.ent + __ldg(adj.soff + s) + (p & (kSlice - 1));
+      F wp[5];
+      load5(W + p * 8, wp);
+#pragma unroll 2
+      for (int k = l; k < w; k += BL) {
+        int32_t q;
+        F d[3];
+        dec_ent(src + k * kSlice, q, d[0], d[1], d[2]);
+        if (q == kPad) continue;
+        if (q >= 0) {  // this node is the first end: G -= f
+          d[0] = -d[0];
+          d[1] = -d[1];
+          d[2] = -d[2];
+        } else {
+          q = ~q;
+        }
+        F wq[5];
+        load5(W + int64_t(q) * 8, wq);
+        grad_edge(d, wq, wp, g);
+      }
+    } else if (l == 0) {
+      F rec[16];
+      load16(G + p * 16, rec);
+      from_rec(rec, g);
+    }
+    grad_bnd_term(bnd, bi, l, BL, W, g);
+  }
+  bnd_add<BL>(g);
+  if (!live) return;
+  finish_grad(g, divide, aux, p);
+  F rec[16];
+  to_rec(g, rec);
+  if constexpr (BL == 1) {
+    store16(G + p * 16, rec);
+    return;
+  }
+  // a quarter of the record per lane
+  static_assert(BL == 1 || BL == 4, "a quarter record per lane");
+  F o[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    o[i] = l == 0 ? rec[i] : l == 1 ? rec[4 + i] : l == 2 ? rec[8 + i] : rec[12 + i];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) G[p * 16 + l * 4 + i] = o[i];
+}
 
 template <class F>
 __global__ void __launch_bounds__(GradShape<F>::BLOCK)
-    k_grad(int64_t n, Adj<F> adj, const F* __restrict__ W, Bnd bnd,
-           const double* __restrict__ vol, NodeAux aux, int divide, F* __restrict__ G) {
+    k_grad_bnd(int64_t nbn, const F* __restrict__ W, Bnd bnd, NodeAux aux, int divide, F* G) {
+  grad_boundary<F, false, bl_after<F>()>(nbn, Adj<F>{}, W, bnd, aux, divide, G);
+}
+
+template <class F, bool BESIDE>
+__global__ void __launch_bounds__(GradShape<F>::BLOCK)
+    k_grad(int64_t n, unsigned nbblk, int64_t nbn, Adj<F> adj, const F* __restrict__ W, Bnd bnd,
+           NodeAux aux, int divide, F* __restrict__ G) {
   using EntT = typename EntOf<F>::type;
   constexpr int GU = GradShape<F>::GU, RG = GradShape<F>::RG, NB = GradShape<F>::BLOCK;
   static_assert((RG & (RG - 1)) == 0 && RG >= 2, "ring of a power-of-two number of groups");
   __shared__ EntT ring[GU * RG][NB];
-  int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (BESIDE && blockIdx.x < nbblk) {
+    grad_boundary<F, true, kBL>(nbn, adj, W, bnd, aux, divide, G);
+    return;
+  }
+  const int64_t p = (blockIdx.x - (BESIDE ? nbblk : 0u)) * int64_t(blockDim.x) + threadIdx.x;
   if (p >= n) return;
   const int tid = threadIdx.x;
   const int lane = static_cast<int>(p & (kSlice - 1));
   const int64_t s = p >> 5;
-  const int32_t off = __ldg(adj.soff + s), w = __ldg(adj.swidth + s);
+  const int32_t bi = __ldg(bnd.bidx + p);
+  const int32_t off = __ldg(adj.soff + s), width = __ldg(adj.swidth + s);
+  const int32_t w = BESIDE && bi >= 0 ? 0 : width;  // boundary nodes: grad_boundary
   const EntT* src = adj.ent + off + lane;
   // group j holds entries GU*j..GU*j+GU-1; groups 0..RG-2 are requested up
   // front, group k+RG-1 while group k is processed, into the slots group k-1
@@ -839,9 +1005,9 @@ __global__ void __launch_bounds__(GradShape<F>::BLOCK)
   }
   F wp[5];
   load5(W + p * 8, wp);
-  F g[15];
+  F g[16];
 #pragma unroll
-  for (int i = 0; i < 15; ++i) g[i] = F(0);
+  for (int i = 0; i < 16; ++i) g[i] = F(0);
   const int ng = (w + GU - 1) / GU;
   for (int kg = 0; kg < ng; ++kg) {
     cp_async_wait<RG - 2>();
@@ -873,77 +1039,15 @@ __global__ void __launch_bounds__(GradShape<F>::BLOCK)
       load5(W + int64_t(q[u]) * 8, wq[u]);
     }
 #pragma unroll
-    for (int u = 0; u < GU; ++u) {
-      if (q[u] == kPad) continue;
-#pragma unroll
-      for (int c = 0; c < 5; ++c) {
-        F sum = wq[u][c] + wp[c];
-        g[c * 3 + 0] += d[u][0] * sum;
-        g[c * 3 + 1] += d[u][1] * sum;
-        g[c * 3 + 2] += d[u][2] * sum;
-      }
-    }
+    for (int u = 0; u < GU; ++u)
+      if (q[u] != kPad) grad_edge(d[u], wq[u], wp, g);
   }
   cp_async_wait<0>();
-  F o[16];
-  if (__ldg(bnd.bidx + p) >= 0) {
-    // boundary node: the domain sum as it stands; k_grad_bnd adds the
-    // boundary integral and divides (the reference's order of summation)
-#pragma unroll
-    for (int i = 0; i < 15; ++i) o[i] = g[i];
-  } else {
-    finish_grad(g, divide, vol, aux, p, o);
-  }
-  o[15] = F(0);
+  if (BESIDE && bi >= 0) return;
+  // a boundary node's domain sum stays as it is for k_grad_bnd
+  finish_grad(g, bi < 0 ? divide : 0, aux, p);
   F rec[16];
-  to_rec(o, rec);
-  store16(G + p * 16, rec);
-}
-
-// Boundary-triangle term of riemann::grad (src/Physics/Riemann.cpp:329-364)
-// at boundary node p, added to g in the node's triangle order.
-template <class F>
-__device__ __forceinline__ void grad_bnd_term(const Bnd& bnd, int32_t bi, const F* __restrict__ W,
-                                              F g[15]) {
-  for (int32_t j = __ldg(bnd.bptr + bi); j < __ldg(bnd.bptr + bi + 1); ++j) {
-    const int4 te = __ldg(bnd.bent4 + j);
-    F a[8], b[8], c[8];
-    load8(W + int64_t(te.x) * 8, a);
-    load8(W + int64_t(te.y) * 8, b);
-    load8(W + int64_t(te.z) * 8, c);
-    F bax = b[5] - a[5], bay = b[6] - a[6], baz = b[7] - a[7];
-    F cax = c[5] - a[5], cay = c[6] - a[6], caz = c[7] - a[7];
-    F nn[3] = {(bay * caz - cay * baz) / F(12.0), (baz * cax - caz * bax) / F(12.0),
-               (bax * cay - cax * bay) / F(12.0)};
-#pragma unroll
-    for (int cc = 0; cc < 5; ++cc) {
-      F uab = (a[cc] + b[cc]) / F(4.0);
-      F ubc = (b[cc] + c[cc]) / F(4.0);
-      F uca = (c[cc] + a[cc]) / F(4.0);
-      F gg[3] = {uab + uca + a[cc], uab + ubc + b[cc], ubc + uca + c[cc]};
-#pragma unroll
-      for (int j2 = 0; j2 < 3; ++j2) g[cc * 3 + j2] += gg[j2] * nn[j2];
-    }
-  }
-}
-
-// Boundary nodes of the gradient pass, one thread per boundary node.
-template <class F>
-__global__ void __launch_bounds__(kBlock) k_grad_bnd(int64_t nbn, Bnd bnd,
-                                                      const F* __restrict__ W,
-                                                      const double* __restrict__ vol,
-                                                      NodeAux aux, int divide, F* G) {
-  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i >= nbn) return;
-  const int64_t p = __ldg(bnd.bnode + i);
-  F rec[16], g[16];
-  load16(G + p * 16, rec);
-  from_rec(rec, g);
-  grad_bnd_term(bnd, static_cast<int32_t>(i), W, g);
-  F o[16];
-  finish_grad(g, divide, vol, aux, p, o);
-  o[15] = F(0);
-  to_rec(o, rec);
+  to_rec(g, rec);
   store16(G + p * 16, rec);
 }
 
@@ -978,14 +1082,19 @@ struct Half {
   int64_t nent2;
 };
 
+// FP64 blocks of 64 threads: see GradShape.
+template <class F>
+constexpr int flux_block() {
+  return sizeof(F) == 8 ? 64 : kBlock;
+}
 template <class F, int FLUX>
-__global__ void __launch_bounds__(kBlock, sizeof(F) == 4 ? 3 : 1)
+__global__ void __launch_bounds__(flux_block<F>(), sizeof(F) == 4 ? 3 : 1)
     k_flux1(int64_t n, Half<F> h, const F* __restrict__ W, const F* __restrict__ G,
             double gamma_d, int stab2, double stab2coef_d, F* __restrict__ fbuf,
             F* __restrict__ Rp) {
   using EntT = typename EntOf<F>::type;
   constexpr int RL = ring_len<EntT>();
-  __shared__ EntT ring[RL][kBlock];
+  __shared__ EntT ring[RL][flux_block<F>()];
   int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (p >= n) return;
   const int tid = threadIdx.x;
@@ -1076,11 +1185,16 @@ __global__ void __launch_bounds__(kBlock, sizeof(F) == 4 ? 3 : 1)
 }
 
 // Boundary integral of riemann::rhs (advbnd, src/Physics/Riemann.cpp:768-878)
-// at the boundary node with index bi, added to R in the node's triangle order.
+// at the boundary node with index bi, added to R: its triangles j0 + l,
+// j0 + l + step, ...  The fluxes f of the three vertices are linear in the
+// triangle's normal; scaled by its 1/48, the reference's own value plus the
+// two pair averages that hold the node, f + (f + g)/4 + (h + f)/4, is
+// (f + g + h) + 5 f.
 template <class F>
-__device__ __forceinline__ void rhs_bnd_term(const Bnd& bnd, int32_t bi, const F* __restrict__ W,
-                                             F gamma, F R[5]) {
-  for (int32_t j = __ldg(bnd.bptr + bi); j < __ldg(bnd.bptr + bi + 1); ++j) {
+__device__ __forceinline__ void rhs_bnd_term(const Bnd& bnd, int64_t bi, int l, int step,
+                                             const F* __restrict__ W, F gamma, F R[5]) {
+  const int32_t j1 = __ldg(bnd.bptr + bi + 1);
+  for (int32_t j = __ldg(bnd.bptr + bi) + l; j < j1; j += step) {
     const int4 te = __ldg(bnd.bent4 + j);
     const int32_t pos = te.w & 3;
     F x[3][8];
@@ -1088,30 +1202,25 @@ __device__ __forceinline__ void rhs_bnd_term(const Bnd& bnd, int32_t bi, const F
     load8(W + int64_t(te.y) * 8, x[1]);
     load8(W + int64_t(te.z) * 8, x[2]);
     const bool sy[3] = {((te.w >> 2) & 1) != 0, ((te.w >> 3) & 1) != 0, ((te.w >> 4) & 1) != 0};
-    F bax = x[1][5] - x[0][5], bay = x[1][6] - x[0][6], baz = x[1][7] - x[0][7];
-    F cax = x[2][5] - x[0][5], cay = x[2][6] - x[0][6], caz = x[2][7] - x[0][7];
-    F nx = (bay * caz - cay * baz) / F(12.0);
-    F ny = (baz * cax - caz * bax) / F(12.0);
-    F nz = (bax * cay - cax * bay) / F(12.0);
-    F fl[3][5];
+    const F bax = x[1][5] - x[0][5], bay = x[1][6] - x[0][6], baz = x[1][7] - x[0][7];
+    const F cax = x[2][5] - x[0][5], cay = x[2][6] - x[0][6], caz = x[2][7] - x[0][7];
+    const F k = F(1.0) / F(48.0);
+    const F nx = (bay * caz - cay * baz) * k;
+    const F ny = (baz * cax - caz * bax) * k;
+    const F nz = (bax * cay - cax * bay) * k;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const F r = x[a][0], u = x[a][1], v = x[a][2], ww = x[a][3], ie = x[a][4];
+      const F wt = pos == a ? F(6.0) : F(1.0);
       const F pr = r * ie * (gamma - F(1.0));
       const F vn = sy[a] ? F(0) : (nx * u + ny * v + nz * ww);
-      const F re = r * (ie + F(0.5) * (u * u + v * v + ww * ww));
-      fl[a][0] = r * vn;
-      fl[a][1] = r * u * vn + pr * nx;
-      fl[a][2] = r * v * vn + pr * ny;
-      fl[a][3] = r * ww * vn + pr * nz;
-      fl[a][4] = (re + pr) * vn;
-    }
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      // own value, plus the two averages of the pairs containing this node
-      F fa = fl[0][c], fb = fl[1][c], fcc = fl[2][c];
-      F fab = (fa + fb) / F(4.0), fbc = (fb + fcc) / F(4.0), fca = (fcc + fa) / F(4.0);
-      R[c] += pos == 0 ? (fab + fca + fa) : (pos == 1 ? (fab + fbc + fb) : (fbc + fca + fcc));
+      const F h = r * (ie + F(0.5) * (u * u + v * v + ww * ww)) + pr;
+      const F m = wt * (r * vn), pw = wt * pr;
+      R[0] += m;
+      R[1] += m * u + pw * nx;
+      R[2] += m * v + pw * ny;
+      R[3] += m * ww + pw * nz;
+      R[4] += h * (wt * vn);
     }
   }
 }
@@ -1190,28 +1299,18 @@ __device__ __forceinline__ void apply_bc(const BCProg& bc, int64_t i, double gam
 // One node's stage state (RieCG::solve, src/Inciter/RieCG.cpp:1010-1021):
 // un = Un - rkcoef*dt*R/vol from uo (U at stage 0, copied to Un, and Un
 // after; in the time loop's lean form uo is U, the state at the start of the
-// step, at every stage and nothing is copied).  The FP64 mode keeps the
-// reference's expression; FP32 mode uses 1/vol (no FP64 division per node).
+// step, at every stage and nothing is copied).  The quotient by the volume is
+// a product with 1/vol (no FP64 division per node).
 template <class F, int STAGE, bool LEAN = false>
 __device__ __forceinline__ void stage_state(int64_t n, int64_t p, const F R[5],
-                                            const double uo[5],
-                                            const double* __restrict__ vol, NodeAux aux,
-                                            double dt, double* Un, double un[5]) {
+                                            const double uo[5], NodeAux aux, double dt,
+                                            double* Un, double un[5]) {
   constexpr double rk = STAGE == 0 ? 1.0 / 3.0 : (STAGE == 1 ? 0.5 : 1.0);
-  if constexpr (sizeof(F) == 8) {
-    const double v = vol[p];
+  const double cf = rk * dt * aux.ivol[p];
 #pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      if (STAGE == 0 && !LEAN) Un[c * n + p] = uo[c];
-      un[c] = uo[c] - rk * dt * double(R[c]) / v;
-    }
-  } else {
-    const double cf = rk * dt * aux.ivol[p];
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      if (STAGE == 0 && !LEAN) Un[c * n + p] = uo[c];
-      un[c] = uo[c] - cf * double(R[c]);
-    }
+  for (int c = 0; c < 5; ++c) {
+    if (STAGE == 0 && !LEAN) Un[c * n + p] = uo[c];
+    un[c] = uo[c] - cf * double(R[c]);
   }
 }
 
@@ -1220,8 +1319,7 @@ __device__ __forceinline__ void stage_state(int64_t n, int64_t p, const F R[5],
 // FP32 estimate in FP32 mode); DBL_MAX otherwise.
 template <class F>
 __device__ __forceinline__ double store_node(int64_t n, int64_t p, const double u[5],
-                                             const F wp[8], bool want_dt,
-                                             const double* __restrict__ vol, NodeAux aux,
+                                             const F wp[8], bool want_dt, NodeAux aux,
                                              double gamma_d, double* U, F* __restrict__ Wout) {
   double dtp = DBL_MAX;
 #pragma unroll
@@ -1230,7 +1328,7 @@ __device__ __forceinline__ double store_node(int64_t n, int64_t p, const double 
   prim_record<F>(u, o);
   store8(Wout + p * 8, o);
   if (want_dt)
-    dtp = sizeof(F) == 8 ? node_dt(u, vol[p], gamma_d)
+    dtp = sizeof(F) == 8 ? node_dt(u, aux.cbrtd[p], gamma_d)
                          : double(node_dt_f(u, aux.cbrtv[p], float(gamma_d)));
   return dtp;
 }
@@ -1244,9 +1342,8 @@ __device__ __forceinline__ double store_node(int64_t n, int64_t p, const double 
 // link) and staged in shared memory.
 template <class F>
 __global__ void __launch_bounds__(kBlock)
-    k_state_in(int64_t n, const double* __restrict__ Ua, const double* __restrict__ vol,
-               NodeAux aux, double gamma_d, double* __restrict__ U, F* __restrict__ W,
-               unsigned long long* dtmin) {
+    k_state_in(int64_t n, const double* __restrict__ Ua, NodeAux aux, double gamma_d,
+               double* __restrict__ U, F* __restrict__ W, unsigned long long* dtmin) {
   __shared__ double su[kBlock * 5];
   const int64_t p0 = blockIdx.x * int64_t(kBlock);
   const int64_t p = p0 + threadIdx.x;
@@ -1263,7 +1360,7 @@ __global__ void __launch_bounds__(kBlock)
     for (int c = 0; c < 5; ++c) u[c] = su[threadIdx.x * 5 + c];
     F o[8];
     load8(W + p * 8, o);  // coordinates
-    dtp = store_node<F>(n, p, u, o, true, vol, aux, gamma_d, U, W);
+    dtp = store_node<F>(n, p, u, o, true, aux, gamma_d, U, W);
   }
   block_min_atomic(dtp, dtmin);
 }
@@ -1274,9 +1371,8 @@ __global__ void __launch_bounds__(kBlock)
 // otherwise as store_node.
 template <class F, int STAGE, bool LEAN>
 __device__ __forceinline__ double store_stage(int64_t n, int64_t p, const double u[5],
-                                              const F wp[8], const double* __restrict__ vol,
-                                              NodeAux aux, double gamma_d, double* U,
-                                              F* __restrict__ Wout) {
+                                              const F wp[8], NodeAux aux, double gamma_d,
+                                              double* U, F* __restrict__ Wout) {
   if (LEAN && STAGE != 2) {
     if constexpr (sizeof(F) == 8) {
       double pw[5];
@@ -1293,7 +1389,7 @@ __device__ __forceinline__ double store_stage(int64_t n, int64_t p, const double
     }
     return DBL_MAX;
   }
-  return store_node<F>(n, p, u, wp, STAGE == 2, vol, aux, gamma_d, U, Wout);
+  return store_node<F>(n, p, u, wp, STAGE == 2, aux, gamma_d, U, Wout);
 }
 
 
@@ -1313,37 +1409,119 @@ __global__ void __launch_bounds__(kBlock)
   for (int c = 0; c < 5; ++c) Sv[c * n + p] = F(o[c] * v);
 }
 
-// Half-edge residual, pass 2: the fluxes of the edges the other end owns and
-// (optionally) the RK update of one stage with the new primitive records and,
-// on the last stage, the CFL minimum.  Boundary nodes only park their domain
-// residual in Rb: k_rhs_bnd adds their boundary integral and updates them,
-// so no warp here waits on the triangle gathers.
+// Half-edge residual, pass 2: the fluxes of the edges the other end owns, the
+// boundary integral and (optionally) the RK update of one stage with the new
+// primitive records and, on the last stage, the CFL minimum.
+
+// The boundary nodes (see bnd_lane), EDGES: with the other ends' fluxes,
+// otherwise from the domain residuals that k_rhs2 left in Rb; the boundary
+// integral after them, the stage update, then the node's nodal BCs
+// (RieCG::BC after RieCG::solve's update, src/Inciter/RieCG.cpp:1010-1030;
+// every BC node lies on a boundary triangle) and, on the last stage, the CFL
+// time step of the final state, which it returns (DBL_MAX otherwise).
+template <class F, int STAGE, bool UPDATE, bool LEAN, bool EDGES, int BL>
+__device__ __forceinline__ double rhs_boundary(
+    int64_t n, int64_t nbn, const Half<F>& h, const F* __restrict__ fbuf,
+    const F* __restrict__ Rp, const F* __restrict__ Rb, const F* __restrict__ W, const Bnd& bnd,
+    const int32_t* __restrict__ bcof, const BCProg& bc, NodeAux aux, double gamma_d,
+    const Scalars* __restrict__ scal, double* U, double* Un, F* __restrict__ Wout,
+    double* __restrict__ Rout, const F* __restrict__ Sv) {
+  int64_t bi;
+  int l;
+  const bool live = bnd_lane<BL>(nbn, bi, l);
+  F R[5] = {F(0), F(0), F(0), F(0), F(0)};
+  int64_t p = 0;
+  if (live) {
+    p = __ldg(bnd.bnode + bi);
+    if (l == 0) {
+#pragma unroll
+      for (int c = 0; c < 5; ++c) R[c] = EDGES ? Rp[c * n + p] : Rb[c * nbn + bi];
+    }
+    if constexpr (EDGES) {
+      const int64_t s = p >> 5;
+      const int32_t w = __ldg(h.sw2 + s);
+      const int64_t e0 = __ldg(h.soff2 + s) + (p & (kSlice - 1));
+      for (int k = l; k < w; k += BL) {
+        const int64_t e = e0 + k * kSlice;
+        F f[4];
+        load_f4(fbuf, e, f);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) R[c] += f[c];
+        R[4] += __ldg(fbuf + 4 * h.nent2 + e);
+      }
+    }
+    rhs_bnd_term(bnd, bi, l, BL, W, F(gamma_d), R);
+  }
+  bnd_add<BL>(R);
+  if (!live || l != 0) return DBL_MAX;
+  // the manufactured source after the domain and boundary sums, as
+  // riemann::rhs adds it last
+  if (Sv) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) R[c] -= Sv[c * n + p];
+  }
+  if constexpr (!UPDATE) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) Rout[p * 5 + c] = double(R[c]);
+    return DBL_MAX;
+  } else {
+    double uo[5], un[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) uo[c] = (STAGE == 0 || LEAN) ? U[c * n + p] : Un[c * n + p];
+    F wp[8];
+    load8(W + p * 8, wp);
+    stage_state<F, STAGE, LEAN>(n, p, R, uo, aux, scal->dt, Un, un);
+    // at the stage's time, t + c dt with c = 1/3, 1/2, 1 (RieCG.cpp:1028)
+    constexpr double rkc = STAGE == 0 ? 1.0 / 3.0 : (STAGE == 1 ? 1.0 / 2.0 : 1.0);
+    const int32_t b = __ldg(bcof + bi);
+    if (b >= 0) apply_bc(bc, b, gamma_d, scal->t + rkc * scal->dt, un);
+    return store_stage<F, STAGE, LEAN>(n, p, un, wp, aux, gamma_d, U, Wout);
+  }
+}
+
 template <class F, int STAGE, bool UPDATE, bool LEAN>
-__global__ void __launch_bounds__(kBlock, sizeof(F) == 4 ? 4 : 1)
-    k_rhs2(int64_t n, Half<F> h, const F* __restrict__ fbuf, const F* __restrict__ Rp,
-           const F* __restrict__ W, Bnd bnd, int64_t nbn, F* __restrict__ Rb,
-           const double* __restrict__ vol, NodeAux aux, double gamma_d,
+__global__ void __launch_bounds__(flux_block<F>())
+    k_rhs_bnd(int64_t n, int64_t nbn, const F* __restrict__ Rb, const F* __restrict__ W, Bnd bnd,
+              const int32_t* __restrict__ bcof, BCProg bc, NodeAux aux, double gamma_d,
+              const Scalars* __restrict__ scal, double* U, double* Un, F* __restrict__ Wout,
+              double* __restrict__ Rout, unsigned long long* dtmin, const F* __restrict__ Sv) {
+  const double dtp = rhs_boundary<F, STAGE, UPDATE, LEAN, false, bl_after<F>()>(
+      n, nbn, Half<F>{}, nullptr, nullptr, Rb, W, bnd, bcof, bc, aux, gamma_d, scal, U, Un, Wout,
+      Rout, Sv);
+  if (UPDATE && STAGE == 2) block_min_atomic(dtp, dtmin);
+}
+
+template <class F, int STAGE, bool UPDATE, bool LEAN, bool BESIDE>
+__global__ void __launch_bounds__(flux_block<F>(), sizeof(F) == 4 ? 4 : 1)
+    k_rhs2(int64_t n, unsigned nbblk, int64_t nbn, Half<F> h, const F* __restrict__ fbuf,
+           const F* __restrict__ Rp, F* __restrict__ Rb, const F* __restrict__ W, Bnd bnd,
+           const int32_t* __restrict__ bcof, BCProg bc, NodeAux aux, double gamma_d,
            const Scalars* __restrict__ scal, double* U, double* Un, F* __restrict__ Wout,
            double* __restrict__ Rout, unsigned long long* dtmin, const F* __restrict__ Sv) {
-  int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  const bool active = p < n;
+  if (BESIDE && blockIdx.x < nbblk) {
+    const double dtp = rhs_boundary<F, STAGE, UPDATE, LEAN, true, kBL>(
+        n, nbn, h, fbuf, Rp, nullptr, W, bnd, bcof, bc, aux, gamma_d, scal, U, Un, Wout, Rout, Sv);
+    if (UPDATE && STAGE == 2) block_min_atomic(dtp, dtmin);
+    return;
+  }
+  const int64_t p = (blockIdx.x - (BESIDE ? nbblk : 0u)) * int64_t(blockDim.x) + threadIdx.x;
   double dtp = DBL_MAX;
-  if (active) {
+  const int32_t bi = p < n ? __ldg(bnd.bidx + p) : -1;
+  if (p < n && !(BESIDE && bi >= 0)) {  // boundary nodes: rhs_boundary
     const int lane = static_cast<int>(p & (kSlice - 1));
     const int64_t s = p >> 5;
     const int32_t off = __ldg(h.soff2 + s), w = __ldg(h.sw2 + s);
-    const int32_t bi = __ldg(bnd.bidx + p);
     // every per-node load is issued before the flux stream is summed
     F R[5];
 #pragma unroll
     for (int c = 0; c < 5; ++c) R[c] = Rp[c * n + p];
     double uo[5];
+    F wp[8];
     if (UPDATE && bi < 0) {
 #pragma unroll
       for (int c = 0; c < 5; ++c) uo[c] = (STAGE == 0 || LEAN) ? U[c * n + p] : Un[c * n + p];
+      load8(W + p * 8, wp);
     }
-    F wp[8];
-    if (UPDATE && bi < 0) load8(W + p * 8, wp);
     // the other ends' contributions, a coalesced stream (padding slots hold
     // 0), four slots per batch with all of a batch's loads in flight
     for (int k0 = 0; k0 < w; k0 += 4) {
@@ -1365,13 +1543,13 @@ __global__ void __launch_bounds__(kBlock, sizeof(F) == 4 ? 4 : 1)
         }
       }
     }
-    // the manufactured source after the domain (and, in k_rhs_bnd, the
-    // boundary) sums, as riemann::rhs adds it last
+    // the manufactured source after the domain (and boundary) sum, as
+    // riemann::rhs adds it last
     if (Sv && bi < 0) {
 #pragma unroll
       for (int c = 0; c < 5; ++c) R[c] -= Sv[c * n + p];
     }
-    if (bi >= 0) {
+    if (!BESIDE && bi >= 0) {
 #pragma unroll
       for (int c = 0; c < 5; ++c) Rb[c * nbn + bi] = R[c];
     } else if (!UPDATE) {
@@ -1379,55 +1557,8 @@ __global__ void __launch_bounds__(kBlock, sizeof(F) == 4 ? 4 : 1)
       for (int c = 0; c < 5; ++c) Rout[p * 5 + c] = double(R[c]);
     } else {
       double un[5];
-      stage_state<F, STAGE, LEAN>(n, p, R, uo, vol, aux, scal->dt, Un, un);
-      dtp = store_stage<F, STAGE, LEAN>(n, p, un, wp, vol, aux, gamma_d, U, Wout);
-    }
-  }
-  if (UPDATE && STAGE == 2) block_min_atomic(dtp, dtmin);
-}
-
-// Boundary nodes of pass 2, one thread per boundary node: the boundary
-// integral after the domain residual (the reference's order), the stage
-// update, then the node's nodal BCs (RieCG::BC after RieCG::solve's update,
-// src/Inciter/RieCG.cpp:1010-1030; every BC node lies on a boundary
-// triangle) and, on the last stage, the CFL time step of the final state.
-template <class F, int STAGE, bool UPDATE, bool LEAN>
-__global__ void __launch_bounds__(kBlock)
-    k_rhs_bnd(int64_t n, int64_t nbn, Bnd bnd, const F* __restrict__ Rb,
-              const F* __restrict__ W, const int32_t* __restrict__ bcof, BCProg bc,
-              const double* __restrict__ vol, NodeAux aux, double gamma_d,
-              const Scalars* __restrict__ scal, double* U, double* Un, F* __restrict__ Wout,
-              double* __restrict__ Rout, unsigned long long* dtmin, const F* __restrict__ Sv) {
-  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  double dtp = DBL_MAX;
-  if (i < nbn) {
-    const int64_t p = __ldg(bnd.bnode + i);
-    F R[5];
-#pragma unroll
-    for (int c = 0; c < 5; ++c) R[c] = Rb[c * nbn + i];
-    double uo[5];
-    if (UPDATE) {
-#pragma unroll
-      for (int c = 0; c < 5; ++c) uo[c] = (STAGE == 0 || LEAN) ? U[c * n + p] : Un[c * n + p];
-    }
-    F wp[8];
-    load8(W + p * 8, wp);
-    const int32_t b = UPDATE ? __ldg(bcof + i) : -1;
-    rhs_bnd_term(bnd, static_cast<int32_t>(i), W, F(gamma_d), R);
-    if (Sv) {
-#pragma unroll
-      for (int c = 0; c < 5; ++c) R[c] -= Sv[c * n + p];
-    }
-    if (!UPDATE) {
-#pragma unroll
-      for (int c = 0; c < 5; ++c) Rout[p * 5 + c] = double(R[c]);
-    } else {
-      double un[5];
-      stage_state<F, STAGE, LEAN>(n, p, R, uo, vol, aux, scal->dt, Un, un);
-      // at the stage's time, t + c dt with c = 1/3, 1/2, 1 (RieCG.cpp:1028)
-      constexpr double rkc = STAGE == 0 ? 1.0 / 3.0 : (STAGE == 1 ? 1.0 / 2.0 : 1.0);
-      if (b >= 0) apply_bc(bc, b, gamma_d, scal->t + rkc * scal->dt, un);
-      dtp = store_stage<F, STAGE, LEAN>(n, p, un, wp, vol, aux, gamma_d, U, Wout);
+      stage_state<F, STAGE, LEAN>(n, p, R, uo, aux, scal->dt, Un, un);
+      dtp = store_stage<F, STAGE, LEAN>(n, p, un, wp, aux, gamma_d, U, Wout);
     }
   }
   if (UPDATE && STAGE == 2) block_min_atomic(dtp, dtmin);
@@ -1489,7 +1620,7 @@ __global__ void __launch_bounds__(kBlock)
   float r[8];
   load8(R + p * 8, r);
   const int32_t bi = __ldg(bnd.bidx + p);
-  if (bi >= 0) rhs_bnd_term(bnd, bi, W, float(gamma), r);
+  if (bi >= 0) rhs_bnd_term(bnd, bi, 0, 1, W, float(gamma), r);
   if (Sv) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) r[c] -= Sv[c * n + p];
@@ -1502,8 +1633,8 @@ __global__ void __launch_bounds__(kBlock)
 // the node's primitive record and, when asked, its CFL dt.
 template <class F>
 __global__ void __launch_bounds__(kBlock) k_bc(int64_t n, BCProg bc, double gamma, double* U,
-                                                F* __restrict__ W, const double* __restrict__ vol,
-                                                NodeAux aux, double t, int want_dt,
+                                                F* __restrict__ W, NodeAux aux, double t,
+                                                int want_dt,
                                                 unsigned long long* dtmin) {
   int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   double dtp = DBL_MAX;
@@ -1515,14 +1646,14 @@ __global__ void __launch_bounds__(kBlock) k_bc(int64_t n, BCProg bc, double gamm
     apply_bc(bc, i, gamma, t, u);
     F o[8];
     load8(W + p * 8, o);
-    dtp = store_node<F>(n, p, u, o, want_dt != 0, vol, aux, gamma, U, W);
+    dtp = store_node<F>(n, p, u, o, want_dt != 0, aux, gamma, U, W);
   }
   if (want_dt) block_min_atomic(dtp, dtmin);
 }
 
 // CFL minimum over all nodes of the current state.
 __global__ void __launch_bounds__(kBlock) k_dt(int64_t n, const double* __restrict__ U,
-                                                const double* __restrict__ vol, double gamma,
+                                                const double* __restrict__ cbrtd, double gamma,
                                                 unsigned long long* dtmin) {
   int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   double dtp = DBL_MAX;
@@ -1530,7 +1661,7 @@ __global__ void __launch_bounds__(kBlock) k_dt(int64_t n, const double* __restri
     double u[5];
 #pragma unroll
     for (int c = 0; c < 5; ++c) u[c] = U[c * n + p];
-    dtp = node_dt(u, vol[p], gamma);
+    dtp = node_dt(u, cbrtd[p], gamma);
   }
   block_min_atomic(dtp, dtmin);
 }
@@ -1550,6 +1681,11 @@ __global__ void __launch_bounds__(kBlock) k_dt_f(int64_t n, const double* __rest
     dtp = double(node_dt_f(u, cbrtv[p], float(gamma)));
   }
   block_min_atomic(dtp, dtmin);
+}
+
+__global__ void k_cbrt(int64_t n, const double* __restrict__ vol, double* __restrict__ L) {
+  const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (p < n) L[p] = cbrt(vol[p]);
 }
 
 // Step prologue (RieCG::dt reduction target + RieCG::advance,
@@ -1652,7 +1788,7 @@ template <class F>
 Adj<F> adj_of(RieCGDev* d) {
   return Adj<F>{d->soff, d->swidth, static_cast<const typename EntOf<F>::type*>(d->ent)};
 }
-NodeAux aux_of(RieCGDev* d) { return NodeAux{d->ivol, d->cbrtv}; }
+NodeAux aux_of(RieCGDev* d) { return NodeAux{d->ivol, d->cbrtv, d->cbrtd}; }
 // s V per node when a manufactured source is on, else null
 template <class F>
 const F* src_of(RieCGDev* d) {
@@ -1688,16 +1824,33 @@ BCProg bcprog_of(RieCGDev* d) {
   return b;
 }
 
+// Whether the boundary nodes run beside the domain pass or after it (see
+// bnd_lane).
+template <class F>
+bool bnd_beside(const RieCGDev* d) {
+  return d->n < (sizeof(F) == 8 ? kBeside64 : kBeside32);
+}
+
 template <class F>
 int launch_grad(xg_ctx* c, RieCGDev* d, const F* W, F* G, int divide) {
+  const int tb = node_block(c, d->n, GradShape<F>::BLOCK);
+  const unsigned nd = blocks_for(d->n, tb);
+  if (bnd_beside<F>(d)) {
+    const unsigned nb = blocks_for(d->nbn * kBL, tb);
+    XG_PROF_LAUNCH(c, d, "riecg_grad",
+                   (k_grad<F, true><<<nb + nd, tb, 0, c->stream>>>(
+                       d->n, nb, d->nbn, adj_of<F>(d), W, bnd_of(d), aux_of(d), divide, G)));
+    return XG_OK;
+  }
   XG_PROF_LAUNCH(c, d, "riecg_grad",
-                 (k_grad<F><<<blocks_for(d->n, GradShape<F>::BLOCK), GradShape<F>::BLOCK, 0,
-                                c->stream>>>(
-                     d->n, adj_of<F>(d), W, bnd_of(d), d->vol, aux_of(d), divide, G)));
-  if (d->nbn > 0)
+                 (k_grad<F, false><<<nd, tb, 0, c->stream>>>(
+                     d->n, 0, d->nbn, adj_of<F>(d), W, bnd_of(d), aux_of(d), divide, G)));
+  const int64_t nl = d->nbn * bl_after<F>();
+  const int tbb = node_block(c, nl, GradShape<F>::BLOCK);
+  if (nl > 0)
     XG_PROF_LAUNCH(c, d, "riecg_grad_bnd",
-                   (k_grad_bnd<F><<<blocks_for(d->nbn, kBlock), kBlock, 0, c->stream>>>(
-                       d->nbn, bnd_of(d), W, d->vol, aux_of(d), divide, G)));
+                   (k_grad_bnd<F><<<blocks_for(nl, tbb), tbb, 0, c->stream>>>(
+                       d->nbn, W, bnd_of(d), aux_of(d), divide, G)));
   return XG_OK;
 }
 
@@ -1711,22 +1864,36 @@ template <class F, int FLUX, int STAGE, bool UPDATE, bool LEAN>
 int launch_rhs_t(xg_ctx* c, RieCGDev* d, const F* W, const F* G, F* Wout, double* Rout) {
   F* fbuf = static_cast<F*>(d->fbuf);
   F* Rp = static_cast<F*>(d->Rp);
+  const int tb = node_block(c, d->n, flux_block<F>());
   XG_PROF_LAUNCH(c, d, "riecg_flux",
-                 (k_flux1<F, FLUX><<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(
+                 (k_flux1<F, FLUX><<<blocks_for(d->n, tb), tb, 0, c->stream>>>(
                      d->n, half_of<F>(d), W, G, d->prm.gamma, d->prm.stab2, d->prm.stab2coef,
                      fbuf, Rp)));
+  F* Rb = static_cast<F*>(d->Rb);
+  const unsigned nd = blocks_for(d->n, tb);
+  if (bnd_beside<F>(d)) {
+    const unsigned nb = blocks_for(d->nbn * kBL, tb);
+    XG_PROF_LAUNCH(c, d, "riecg_rhs_update",
+                   (k_rhs2<F, STAGE, UPDATE, LEAN, true><<<nb + nd, tb, 0, c->stream>>>(
+                       d->n, nb, d->nbn, half_of<F>(d), fbuf, Rp, Rb, W, bnd_of(d), d->bcof,
+                       bcprog_of(d), aux_of(d), d->prm.gamma, d->scal, d->U, d->Un, Wout, Rout,
+                       &d->scal->dtmin, src_of<F>(d))));
+    return XG_OK;
+  }
   XG_PROF_LAUNCH(c, d, "riecg_rhs_update",
-                 (k_rhs2<F, STAGE, UPDATE, LEAN><<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(
-                     d->n, half_of<F>(d), fbuf, Rp, W, bnd_of(d), d->nbn,
-                     static_cast<F*>(d->Rb), d->vol, aux_of(d), d->prm.gamma, d->scal, d->U,
-                     d->Un, Wout, Rout, &d->scal->dtmin, src_of<F>(d))));
-  if (d->nbn > 0)
+                 (k_rhs2<F, STAGE, UPDATE, LEAN, false><<<nd, tb, 0, c->stream>>>(
+                     d->n, 0, d->nbn, half_of<F>(d), fbuf, Rp, Rb, W, bnd_of(d), d->bcof,
+                     bcprog_of(d), aux_of(d), d->prm.gamma, d->scal, d->U, d->Un, Wout, Rout,
+                     &d->scal->dtmin, src_of<F>(d))));
+  const int64_t nl = d->nbn * bl_after<F>();
+  const int tbb = node_block(c, nl, flux_block<F>());
+  if (nl > 0)
     XG_PROF_LAUNCH(c, d, "riecg_rhs_bnd",
-                   (k_rhs_bnd<F, STAGE, UPDATE, LEAN><<<blocks_for(d->nbn, kBlock), kBlock, 0,
+                   (k_rhs_bnd<F, STAGE, UPDATE, LEAN><<<blocks_for(nl, tbb), tbb, 0,
                                                         c->stream>>>(
-                       d->n, d->nbn, bnd_of(d), static_cast<const F*>(d->Rb), W, d->bcof,
-                       bcprog_of(d), d->vol, aux_of(d), d->prm.gamma, d->scal, d->U, d->Un,
-                       Wout, Rout, &d->scal->dtmin, src_of<F>(d))));
+                       d->n, d->nbn, Rb, W, bnd_of(d), d->bcof, bcprog_of(d), aux_of(d),
+                       d->prm.gamma, d->scal, d->U, d->Un, Wout, Rout, &d->scal->dtmin,
+                       src_of<F>(d))));
   return XG_OK;
 }
 
@@ -1759,7 +1926,7 @@ int launch_bc(xg_ctx* c, RieCGDev* d, F* W, int want_dt) {
   if (d->nbc == 0) return XG_OK;
   XG_PROF_LAUNCH(c, d, "riecg_bc",
                  (k_bc<F><<<blocks_for(d->nbc, kBlock), kBlock, 0, c->stream>>>(
-                     d->n, bcprog_of(d), d->prm.gamma, d->U, W, d->vol, aux_of(d), d->t, want_dt,
+                     d->n, bcprog_of(d), d->prm.gamma, d->U, W, aux_of(d), d->t, want_dt,
                      &d->scal->dtmin)));
   return XG_OK;
 }
@@ -1789,7 +1956,7 @@ int refresh_dt(xg_ctx* c, RieCGDev* d) {
     k_dt_f<<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(d->n, d->U, d->cbrtv,
                                                                 d->prm.gamma, &d->scal->dtmin);
   else
-    k_dt<<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(d->n, d->U, d->vol, d->prm.gamma,
+    k_dt<<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(d->n, d->U, d->cbrtd, d->prm.gamma,
                                                               &d->scal->dtmin);
   XG_CHECK_LAUNCH(c);
   d->dt_valid = true;
@@ -1828,7 +1995,8 @@ int alloc_and_upload(xg_ctx* c, RieCGDev* d, const double* coord, const double* 
     A.plan(fbuf, std::max<int64_t>(1, hl.nent2) * 5);
     A.plan(Rp, n * 5);
     A.plan(d->ivol, n);
-    A.plan(d->cbrtv, n);
+    A.plan(d->cbrtv, d->fp32 ? n : 1);
+    A.plan(d->cbrtd, d->fp32 ? 1 : n);
     A.plan(d->bptr, bptr.size());
     A.plan(d->bent4, std::max<size_t>(1, bent4.size()));
     A.plan(d->bcof, std::max<int64_t>(1, d->nbn));
@@ -1837,7 +2005,6 @@ int alloc_and_upload(xg_ctx* c, RieCGDev* d, const double* coord, const double* 
     A.plan(d->scal, 1);
     if (pass == 0) XG_CUDA(c, A.reserve());
   }
-  d->Rb = Rb;
   for (int pass = 0; pass < 2; ++pass) {
     Arena& S = d->scratch;
     S.plan(d->stage_buf, n * 15);
@@ -1856,6 +2023,7 @@ int alloc_and_upload(xg_ctx* c, RieCGDev* d, const double* coord, const double* 
   d->ent1 = ent1;
   d->fbuf = fbuf;
   d->Rp = Rp;
+  d->Rb = Rb;
   d->nent1 = hl.nent1;
   d->nent2 = hl.nent2;
   cudaStream_t s = c->stream;
@@ -1914,13 +2082,16 @@ int alloc_and_upload(xg_ctx* c, RieCGDev* d, const double* coord, const double* 
     XG_CUDA(c, cudaMemsetAsync(fbuf, 0, std::max<int64_t>(1, hl.nent2) * 5 * sizeof(F), s));
     XG_CUDA(c, cudaStreamSynchronize(s));
     std::vector<double> iv(n);
-    std::vector<float> cv(n);
-    for (int64_t i = 0; i < n; ++i) {
-      iv[i] = 1.0 / vol[i];
-      cv[i] = static_cast<float>(std::cbrt(vol[i]));
-    }
+    for (int64_t i = 0; i < n; ++i) iv[i] = 1.0 / vol[i];
     XG_CUDA(c, cudaMemcpy(d->ivol, iv.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-    XG_CUDA(c, cudaMemcpy(d->cbrtv, cv.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+    if constexpr (sizeof(F) == 4) {
+      std::vector<float> cv(n);
+      for (int64_t i = 0; i < n; ++i) cv[i] = static_cast<float>(std::cbrt(vol[i]));
+      XG_CUDA(c, cudaMemcpy(d->cbrtv, cv.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+    } else {
+      k_cbrt<<<blocks_for(n, kBlock), kBlock, 0, s>>>(n, d->vol, d->cbrtd);
+      XG_CHECK_LAUNCH(c);
+    }
   }
   std::vector<int32_t> bnode(std::max<int64_t>(1, d->nbn), 0);
   for (int64_t p = 0; p < n; ++p)
@@ -2325,11 +2496,11 @@ int xg_riecg_set_state(xg_ctx* c, const double* U, double t) {
   XG_CHECK_LAUNCH(c);
   if (d->fp32)
     k_state_in<float><<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(
-        d->n, src, d->vol, aux_of(d), d->prm.gamma, d->U, static_cast<float*>(d->W[d->cur]),
+        d->n, src, aux_of(d), d->prm.gamma, d->U, static_cast<float*>(d->W[d->cur]),
         &d->scal->dtmin);
   else
     k_state_in<double><<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(
-        d->n, src, d->vol, aux_of(d), d->prm.gamma, d->U, static_cast<double*>(d->W[d->cur]),
+        d->n, src, aux_of(d), d->prm.gamma, d->U, static_cast<double*>(d->W[d->cur]),
         &d->scal->dtmin);
   XG_CHECK_LAUNCH(c);
   d->t = t;
