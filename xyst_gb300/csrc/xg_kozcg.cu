@@ -18,12 +18,15 @@
 // reference's order, the same bits on every run), in FP32 as vector atomic
 // adds into node records.  The allowed limits Q+/- (extremes over
 // the elements holding a node) are taken per node over the node adjacency,
-// which holds the same nodes, and kept as order-preserving keys.  Node
+// which holds the same nodes, and compared as order-preserving keys.  Node
 // kernels (one thread per node) do the per-node algebra between the element
 // passes.  One step is:
-//   step_begin -> node_prim -> elem_rhs_aec -> [gather] -> bc_p -> node_lo -> node_alw ->
-//   node_lim -> elem_lim -> [gather] -> node_solve -> bc (+ CFL minimum for the next step)
-// ([gather]: FP64; FP32 zeroes its records first instead)
+//   step_begin -> node_prim -> elem_rhs -> node_low -> node_limit -> elem_lim -> node_update
+// node_low sums the element terms (FP64: from the slots), projects the
+// boundary nodes' sums and forms the low-order solution; node_limit takes the
+// allowed limits and the limit coefficients; node_update sums the limited
+// terms, updates, applies the BCs and forms the CFL minimum for the next step.
+// (FP32 zeroes its records first.)
 //
 // FP32-element mode: the element passes read an FP32 copy of the state (made
 // by node_prim) and FP32 element geometry (made at setup), and add into FP32
@@ -63,16 +66,20 @@ struct KozCGDev {
   int64_t n = 0, ne = 0;
   xg_kozcg_params prm{};
   int32_t* inpoel = nullptr;
-  double *xyz = nullptr, *vol = nullptr;
+  double *xyz = nullptr, *ivol = nullptr;  // coordinates, 1/vol
+  double* cbrtv = nullptr;                 // cbrt(vol)
   double *U = nullptr, *R = nullptr, *P = nullptr, *A = nullptr;
-  unsigned long long* Q = nullptr;
+  double* Q = nullptr;              // FP64 mode: limit coefficients C+/- [n][kC64]
+  unsigned long long* K = nullptr;  // and the keys of each node's extremes [n][kC64]
   double* stage = nullptr;
-  double* V = nullptr;  // [n][4] velocity and pressure per node (FP32 packed in the first half)
-  // FP32-element mode: element sums, the FP32 state, the low-order solution
-  // as the allowed-limit pass reads it, 32-bit limit keys, element geometry
-  float *R32 = nullptr, *A32 = nullptr, *U32 = nullptr, *lo32 = nullptr;
-  unsigned int* Q32 = nullptr;
+  double* V = nullptr;  // node records of the element passes (see k_node_prim)
+  // FP32-element mode: element sums, limit coefficients and 32-bit keys
+  // [n][kC32]
+  float *R32 = nullptr, *A32 = nullptr, *Q32 = nullptr;
+  unsigned int* K32 = nullptr;
+  // element geometry in the mode's precision (see k_geo)
   float* geo32 = nullptr;
+  double* geo64 = nullptr;
   // FP64 mode: residual and limited slot records (10 and 6 doubles per
   // (element, local node) slot) and each node's slots in element order,
   // SELL-32 like the adjacency
@@ -86,7 +93,7 @@ struct KozCGDev {
   int64_t nbc = 0;
   int32_t *bcnode = nullptr, *bcdir = nullptr, *bcsymp = nullptr, *dirmask = nullptr;
   double *symn = nullptr, *dirval = nullptr;
-  uint8_t* isbc = nullptr;  // per node
+  int32_t* bcof = nullptr;  // per node: its BC program entry or -1
   KScalars* scal = nullptr;
   double* dthist = nullptr;
   int64_t dthist_cap = 0;
@@ -120,14 +127,17 @@ __device__ __forceinline__ double dval(unsigned long long k) {
   return __longlong_as_double(b);
 }
 
-__device__ __forceinline__ double node_dt(const double u[5], double vol, double g) {
-  double r = u[0];
-  double uu = u[1] / r, vv = u[2] / r, ww = u[3] / r;
-  double pr = (u[4] - 0.5 * r * (uu * uu + vv * vv + ww * ww)) * (g - 1.0);
-  double c = sqrt(g * fmax(pr, 0.0) / r);
-  double L = cbrt(vol);
-  double vel = sqrt(uu * uu + vv * vv + ww * ww);
-  return L / fmax(vel + c, 1.0e-8);
+// A node's CFL time step before the CFL factor (KozCG.cpp:613-688), L =
+// cbrt(vol) formed at setup, with one quotient by the density: an FP64
+// division is about ten instructions, each of which holds an SM quarter's FP64
+// unit for 64 cycles on GB300.
+__device__ __forceinline__ double node_dt(const double u[5], double L, double g) {
+  const double ir = 1.0 / u[0];
+  const double uu = u[1] * ir, vv = u[2] * ir, ww = u[3] * ir;
+  const double k2 = uu * uu + vv * vv + ww * ww;
+  const double pr = (u[4] - 0.5 * u[0] * k2) * (g - 1.0);
+  const double c = sqrt(g * fmax(pr, 0.0) * ir);
+  return L / fmax(sqrt(k2) + c, 1.0e-8);
 }
 
 __device__ __forceinline__ void block_min_atomic(double v, unsigned long long* dst) {
@@ -208,30 +218,66 @@ __device__ __forceinline__ double oval(unsigned long long k) { return dval(k); }
 __device__ __forceinline__ float oval(unsigned int k) {
   return __uint_as_float((k >> 31) ? (k & 0x7fffffffu) : ~k);
 }
-__device__ __forceinline__ double kbits(unsigned long long k) { return __longlong_as_double(k); }
-__device__ __forceinline__ float kbits(unsigned int k) { return __uint_as_float(k); }
-__device__ __forceinline__ unsigned long long tobits(double v) { return __double_as_longlong(v); }
-__device__ __forceinline__ unsigned int tobits(float v) { return __float_as_uint(v); }
 
-// Where component c of node i lives in the element sums: FP64 mode SoA
-// [5][n] (R, A) and [10][n] (P), written whole by k_node_gather from the
-// slot records; FP32 mode node records, so that one element
-// adds a node's contribution with 16-byte vector atomics
-// (red.global.add.v4.f32) instead of one atomic per component: R and P share
-// a [n][16] record (R at 0..4, P+/- at 5..14, P addressed from R + 5), A has
-// [n][8].
+// FP32 element sums are node records, so that one element adds a node's
+// contribution with 16-byte vector atomics (red.global.add.v4.f32) instead of
+// one atomic per component: R and P share a [n][16] record (R at 0..4, P+/- at
+// 5..14), A has [n][8].
 constexpr int kRP = 16;   // FP32 R+P record
 constexpr int kAR = 8;    // FP32 A record
 constexpr int kGB = 4;    // FP64 node gather: slots loaded together
-template <class F, int S>
-__device__ __forceinline__ int64_t ridx(int64_t n, int c, int64_t i) {
-  return sizeof(F) == 4 ? i * S + c : c * n + i;
+// Records of ten values per node (extremes' keys, limit coefficients, + and -
+// per component interleaved), padded to whole 16-byte accesses.
+constexpr int kC64 = 10, kC32 = 12;
+template <class T>
+constexpr int rec10() {
+  return sizeof(T) == 8 ? kC64 : kC32;
 }
-template <class F>
-__device__ __forceinline__ int64_t pidx(int64_t n, int cs, int64_t i) {
-  return sizeof(F) == 4 ? i * kRP + cs : cs * n + i;
+__device__ __forceinline__ void load10(const double* p, double o[10]) {
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const double2 t = __ldg(reinterpret_cast<const double2*>(p) + k);
+    o[2 * k] = t.x;
+    o[2 * k + 1] = t.y;
+  }
 }
-
+__device__ __forceinline__ void load10(const unsigned long long* p, unsigned long long o[10]) {
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const ulonglong2 t = __ldg(reinterpret_cast<const ulonglong2*>(p) + k);
+    o[2 * k] = t.x;
+    o[2 * k + 1] = t.y;
+  }
+}
+__device__ __forceinline__ void load10(const unsigned int* p, unsigned int o[10]) {
+  const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+  const uint2 c = __ldg(reinterpret_cast<const uint2*>(p + 8));
+  o[0] = a.x, o[1] = a.y, o[2] = a.z, o[3] = a.w;
+  o[4] = b.x, o[5] = b.y, o[6] = b.z, o[7] = b.w;
+  o[8] = c.x, o[9] = c.y;
+}
+__device__ __forceinline__ void load10(const float* p, float o[10]) {
+  unsigned int t[10];
+  load10(reinterpret_cast<const unsigned int*>(p), t);
+#pragma unroll
+  for (int k = 0; k < 10; ++k) o[k] = __uint_as_float(t[k]);
+}
+template <class T>
+__device__ __forceinline__ void store10(T* p, const T o[10]) {
+  if constexpr (sizeof(T) == 8) {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const longlong2 t = make_longlong2(reinterpret_cast<const long long*>(o)[2 * k],
+                                         reinterpret_cast<const long long*>(o)[2 * k + 1]);
+      reinterpret_cast<longlong2*>(p)[k] = t;
+    }
+  } else {
+    const int* q = reinterpret_cast<const int*>(o);
+    reinterpret_cast<int4*>(p)[0] = make_int4(q[0], q[1], q[2], q[3]);
+    reinterpret_cast<int4*>(p)[1] = make_int4(q[4], q[5], q[6], q[7]);
+    reinterpret_cast<int2*>(p + 8)[0] = make_int2(q[8], q[9]);
+  }
+}
 // FP32 mode: r[5] added to node i's record of R (S = kRP) or A (S = kAR).
 template <int S>
 __device__ __forceinline__ void add5(float* R, int64_t, int64_t i, const float r[5]) {
@@ -239,177 +285,180 @@ __device__ __forceinline__ void add5(float* R, int64_t, int64_t i, const float r
   atomicAdd(R + i * S + 4, r[4]);
 }
 
-// Per-node velocity and pressure (the node-wise quotients kozak::rhs forms
-// for every element holding the node, Kozak.cpp:93-118): computed once per
-// node, the same expressions, so the element pass gathers bit-identical
-// values instead of repeating the FP64 divisions per element.  In FP32 mode
-// the state itself is also stored in FP32 (Uf), so that the element passes
-// read it without conversions.
+// What the element passes read of a node, one record of eight values (density,
+// momenta, total energy, pressure, 1/density, pad): 32 or 64 bytes in one or two
+// accesses, where component arrays take a sector each.  The node-wise
+// quotients kozak::rhs forms for every element holding the node
+// (Kozak.cpp:93-118) are formed once.
 template <class F>
 __global__ void __launch_bounds__(kBlock) k_node_prim(int64_t n, const double* __restrict__ U,
-                                                       double gamma_d, F* __restrict__ V,
-                                                       F* __restrict__ Uf) {
+                                                       double gamma_d, F* __restrict__ V) {
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   const F gamma = F(gamma_d);
   F u[5];
 #pragma unroll
   for (int c = 0; c < 5; ++c) u[c] = F(U[c * n + i]);
-  F o[4];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) o[j] = u[j + 1] / u[0];
-  o[3] = (gamma - F(1.0)) * (u[4] - F(0.5) * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) / u[0]);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) V[i * 4 + k] = o[k];
-  if (Uf) {
-#pragma unroll
-    for (int c = 0; c < 5; ++c) Uf[c * n + i] = u[c];
+  const F ir = F(1.0) / u[0];
+  const F p =
+      (gamma - F(1.0)) * (u[4] - F(0.5) * (u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) * ir);
+  if constexpr (sizeof(F) == 8) {
+    double2* o = reinterpret_cast<double2*>(V + i * 8);
+    o[0] = make_double2(u[0], u[1]);
+    o[1] = make_double2(u[2], u[3]);
+    o[2] = make_double2(u[4], p);
+    o[3] = make_double2(ir, 0.0);
+  } else {
+    float4* o = reinterpret_cast<float4*>(V + i * 8);
+    o[0] = make_float4(u[0], u[1], u[2], u[3]);
+    o[1] = make_float4(u[4], p, ir, 0.f);
   }
 }
+__device__ __forceinline__ void load_node(const float* V, int32_t i, float o[8]) {
+  asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]),
+                 "=f"(o[6]), "=f"(o[7])
+               : "l"(V + int64_t(i) * 8));
+}
+__device__ __forceinline__ void load_node(const double* V, int32_t i, double o[8]) {
+  const double* p = V + int64_t(i) * 8;
+  asm volatile("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+               : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
+               : "l"(p));
+  asm volatile("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+               : "=d"(o[4]), "=d"(o[5]), "=d"(o[6]), "=d"(o[7])
+               : "l"(p + 4));
+}
 
-// Element geometry in FP32 for the FP32 mode, formed once at setup from the
-// FP64 coordinates (tetgeo<double>, then rounded): J and g1, g2, g3 as
-// [10][T] (g0 = -g1 - g2 - g3 is re-formed in the element passes).
-__global__ void k_geo32(int64_t n, int64_t ne, const int32_t* __restrict__ inpoel,
-                        const double* __restrict__ xyz, float* __restrict__ geo) {
+// Element geometry in the mode's precision, formed once at setup from the
+// FP64 coordinates: J/120, 1/(2J), g1, g2, g3 as [kGeo][T] (g0 = -g1 - g2 - g3
+// is re-formed in the element passes).  In FP64 the 88 bytes a tet replace
+// some 60 FP64 instructions a step (the cross products and two divisions),
+// about 0.18 ms of arithmetic for 0.02 ms of memory traffic at 65^3.
+constexpr int kGeo = 11;
+template <class F>
+__global__ void k_geo(int64_t n, int64_t ne, const int32_t* __restrict__ inpoel,
+                      const double* __restrict__ xyz, F* __restrict__ geo) {
   const int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (e >= ne) return;
   int32_t N[4];
   for (int a = 0; a < 4; ++a) N[a] = inpoel[e * 4 + a];
   const Geo<double> t = tetgeo<double>(xyz, n, N);
-  geo[e] = float(t.J);
+  geo[e] = F(t.J / 120.0);
+  geo[ne + e] = F(0.5 / t.J);
   for (int a = 1; a < 4; ++a)
-    for (int j = 0; j < 3; ++j) geo[(1 + (a - 1) * 3 + j) * ne + e] = float(t.g[a][j]);
+    for (int j = 0; j < 3; ++j) geo[(2 + (a - 1) * 3 + j) * ne + e] = F(t.g[a][j]);
 }
 
 template <class F>
-__device__ __forceinline__ Geo<F> elem_geo(const double* __restrict__ xyz,
-                                           const float* __restrict__ geo, int64_t n, int64_t ne,
-                                           int64_t e, const int32_t N[4]) {
-  if constexpr (sizeof(F) == 8) {
-    return tetgeo<double>(xyz, n, N);
-  } else {
-    Geo<float> t;
-    t.J = __ldg(geo + e);
-    for (int a = 1; a < 4; ++a)
-      for (int j = 0; j < 3; ++j) t.g[a][j] = __ldg(geo + (1 + (a - 1) * 3 + j) * ne + e);
-    for (int j = 0; j < 3; ++j) t.g[0][j] = -t.g[1][j] - t.g[2][j] - t.g[3][j];
-    return t;
-  }
-}
-
-// Component c of the state at a node, as the element arithmetic reads it.
+struct ElemGeo {
+  F j120, ij2;  // J/120, 1/(2J)
+  F g[4][3];
+};
 template <class F>
-__device__ __forceinline__ F ust(const double* __restrict__ U, const F* __restrict__ Uf, int64_t n,
-                                 int c, int32_t node) {
-  if constexpr (sizeof(F) == 8)
-    return U[c * n + node];
-  else
-    return __ldg(Uf + c * n + node);
-}
-
-// kozak::rhs for one tet (Kozak.cpp:73-173) plus the antidiffusive element
-// contributions of KozCG::aec (KozCG.cpp:794-814), scattered to the nodes.
-// V holds each node's velocity and pressure (k_node_prim).
-template <class F>
-__device__ __forceinline__ void load_v4(const F* V, int64_t i, F o[4]) {
-  if constexpr (sizeof(F) == 8) {
-    const double2* q = reinterpret_cast<const double2*>(V + i * 4);
-    const double2 a = __ldg(q), b = __ldg(q + 1);
-    o[0] = a.x;
-    o[1] = a.y;
-    o[2] = b.x;
-    o[3] = b.y;
-  } else {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(V + i * 4));
-    o[0] = a.x;
-    o[1] = a.y;
-    o[2] = a.z;
-    o[3] = a.w;
-  }
+__device__ __forceinline__ ElemGeo<F> elem_geo(const F* __restrict__ geo, int64_t ne, int64_t e) {
+  ElemGeo<F> t;
+  t.j120 = __ldg(geo + e);
+  t.ij2 = __ldg(geo + ne + e);
+#pragma unroll
+  for (int a = 1; a < 4; ++a)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) t.g[a][j] = __ldg(geo + (2 + (a - 1) * 3 + j) * ne + e);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) t.g[0][j] = -t.g[1][j] - t.g[2][j] - t.g[3][j];
+  return t;
 }
 
 // kozak::rhs for one tet (Kozak.cpp:73-173): the residual r[a][c] of its
 // four nodes, and with fct the antidiffusive element contributions of
-// KozCG::aec (KozCG.cpp:794-814) aec[a][c] (zero without).  V holds each
-// node's velocity and pressure (k_node_prim).
+// KozCG::aec (KozCG.cpp:794-814) aec[a][c], from the node records V.
+//
+// In FP64 the operation count is the bound (12.6 M tets of a 129^3 cube at 530
+// G operations/s), so each flux is contracted with its gradient vector as
+// F.g = (v.g) (rho, m, E + p) + p (0, g, 0), 12 operations a node where the
+// sum over directions took 36; the fourth node's residual is minus the sum of
+// the others (the gradients add to zero); and aec_a = ctau J/120 (4 u_a -
+// sum_b u_b), which is exactly zero for a uniform component: about 190
+// operations a tet for 480, k_elem_rhs64 1259 -> 548 us at 65^3, its FP64
+// units busy throughout.
 template <class F>
 __device__ __forceinline__ void elem_terms(int64_t n, int64_t ne, int64_t e,
                                            const int32_t* __restrict__ inpoel,
-                                           const double* __restrict__ xyz,
-                                           const float* __restrict__ geo,
-                                           const double* __restrict__ U, const F* __restrict__ Uf,
-                                           const F* __restrict__ V,
+                                           const F* __restrict__ geo, const F* __restrict__ V,
                                            const KScalars* __restrict__ sc, F gamma, F ctau,
                                            int fct, const double* __restrict__ S,
                                            const double* __restrict__ Se, int32_t N[4],
                                            F r[4][5], F aec[4][5]) {
-  for (int a = 0; a < 4; ++a) N[a] = inpoel[e * 4 + a];
-  const Geo<F> t = elem_geo<F>(xyz, geo, n, ne, e, N);
-  F u[4][5], vel[4][3], p[4];
+  const int4 nd = __ldg(reinterpret_cast<const int4*>(inpoel) + e);
+  N[0] = nd.x;
+  N[1] = nd.y;
+  N[2] = nd.z;
+  N[3] = nd.w;
+  const ElemGeo<F> t = elem_geo<F>(geo, ne, e);
+  F u[4][5], sum[5], acc[5];
+#pragma unroll
   for (int a = 0; a < 4; ++a) {
-    for (int c = 0; c < 5; ++c) u[a][c] = ust<F>(U, Uf, n, c, N[a]);
-    F v4[4];
-    load_v4(V, N[a], v4);
-    vel[a][0] = v4[0];
-    vel[a][1] = v4[1];
-    vel[a][2] = v4[2];
-    p[a] = v4[3];
+    F v[8];
+    load_node(V, N[a], v);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) u[a][c] = v[c];
+    const F gv = (t.g[a][0] * v[1] + t.g[a][1] * v[2] + t.g[a][2] * v[3]) * v[6];
+    const F h = v[4] + v[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      sum[c] = a == 0 ? u[a][c] : sum[c] + u[a][c];
+      const F f = gv * (c == 4 ? h : u[a][c]);
+      acc[c] = a == 0 ? f : acc[c] + f;
+      if (c > 0 && c < 4) acc[c] += t.g[a][c - 1] * v[5];
+    }
   }
   const F dt = F(sc->dt);
+  const F coef = dt * t.ij2;
   F ue[5];
-  for (int c = 0; c < 5; ++c) ue[c] = (u[0][c] + u[1][c] + u[2][c] + u[3][c]) / F(4.0);
-  F coef = dt / t.J / F(2.0);
-  for (int j = 0; j < 3; ++j)
-    for (int a = 0; a < 4; ++a) {
-      const F cg = coef * t.g[a][j];
-      const F uj = vel[a][j];
-      ue[0] -= cg * u[a][j + 1];
-      ue[1] -= cg * u[a][1] * uj;
-      ue[2] -= cg * u[a][2] * uj;
-      ue[3] -= cg * u[a][3] * uj;
-      ue[j + 1] -= cg * p[a];
-      ue[4] -= cg * (u[a][4] + p[a]) * uj;
-    }
+#pragma unroll
+  for (int c = 0; c < 5; ++c) ue[c] = F(0.25) * sum[c] - coef * acc[c];
   if (S) {  // the nodes' sources at the step's start time, dt/8 each
     const F c8 = dt / F(8.0);
     for (int a = 0; a < 4; ++a)
       for (int c = 0; c < 5; ++c) ue[c] += c8 * F(__ldg(S + c * n + N[a]));
   }
-  const F pr =
-      (gamma - F(1.0)) * (ue[4] - F(0.5) * (ue[1] * ue[1] + ue[2] * ue[2] + ue[3] * ue[3]) / ue[0]);
-  for (int a = 0; a < 4; ++a)
-    for (int c = 0; c < 5; ++c) r[a][c] = F(0.0);
-  coef = F(1.0) / F(6.0);
-  for (int j = 0; j < 3; ++j) {
-    const F uj = ue[j + 1] / ue[0];
-    for (int a = 0; a < 4; ++a) {
-      const F cg = coef * t.g[a][j];
-      r[a][0] += cg * ue[j + 1];
-      r[a][1] += cg * ue[1] * uj;
-      r[a][2] += cg * ue[2] * uj;
-      r[a][3] += cg * ue[3] * uj;
-      r[a][j + 1] += cg * pr;
-      r[a][4] += cg * (ue[4] + pr) * uj;
+  const F ir = F(1.0) / ue[0];
+  const F vx = ue[1] * ir, vy = ue[2] * ir, vz = ue[3] * ir;
+  const F pr = (gamma - F(1.0)) * (ue[4] - F(0.5) * (ue[1] * vx + ue[2] * vy + ue[3] * vz));
+  ue[4] += pr;
+  const F p6 = pr * (F(1.0) / F(6.0));
+#pragma unroll
+  for (int c = 0; c < 5; ++c) ue[c] *= F(1.0) / F(6.0);
+#pragma unroll
+  for (int a = 1; a < 4; ++a) {
+    const F gv = t.g[a][0] * vx + t.g[a][1] * vy + t.g[a][2] * vz;
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      r[a][c] = gv * ue[c];
+      if (c > 0 && c < 4) r[a][c] += t.g[a][c - 1] * p6;
     }
   }
+#pragma unroll
+  for (int c = 0; c < 5; ++c) r[0][c] = -r[1][c] - r[2][c] - r[3][c];
   if (Se) {  // the centroid's source half a step later, J/24 to each node
-    const F cj = t.J / F(24.0);
-    F se[5];
-    for (int c = 0; c < 5; ++c) se[c] = F(__ldg(Se + e * 5 + c));
-    for (int a = 0; a < 4; ++a)
-      for (int c = 0; c < 5; ++c) r[a][c] += cj * se[c];
-  }
-  for (int c = 0; c < 5; ++c)
-    for (int a = 0; a < 4; ++a) {
-      F s = F(0.0);
-      if (fct)
-        for (int b = 0; b < 4; ++b) {
-          const F m = t.J / F(120.0) * ((a == b) ? F(3.0) : F(-1.0));
-          s += m * ctau * u[b][c];
-        }
-      aec[a][c] = s;
+    const F cj = F(5.0) * t.j120;
+    for (int c = 0; c < 5; ++c) {
+      const F se = cj * F(__ldg(Se + e * 5 + c));
+      for (int a = 0; a < 4; ++a) r[a][c] += se;
     }
+  }
+  if (fct) {
+    const F k = ctau * t.j120;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int c = 0; c < 5; ++c) aec[a][c] = k * (F(4.0) * u[a][c] - sum[c]);
+  } else {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int c = 0; c < 5; ++c) aec[a][c] = F(0.0);
+  }
 }
 
 // FP32 element pass: per node its residual and its ten antidiffusive sums
@@ -419,7 +468,6 @@ __device__ __forceinline__ void elem_terms(int64_t n, int64_t ne, int64_t e,
 __global__ void __launch_bounds__(kBlock) k_elem_rhs_aec32(int64_t n, int64_t ne,
                                                             const int32_t* __restrict__ inpoel,
                                                             const float* __restrict__ geo,
-                                                            const float* __restrict__ Uf,
                                                             const float* __restrict__ V,
                                                             const KScalars* __restrict__ sc,
                                                             double gamma, double ctau, int fct,
@@ -430,8 +478,8 @@ __global__ void __launch_bounds__(kBlock) k_elem_rhs_aec32(int64_t n, int64_t ne
   if (e >= ne) return;
   int32_t N[4];
   float r[4][5], aec[4][5];
-  elem_terms<float>(n, ne, e, inpoel, nullptr, geo, nullptr, Uf, V, sc, float(gamma),
-                    float(ctau), fct, S, Se, N, r, aec);
+  elem_terms<float>(n, ne, e, inpoel, geo, V, sc, float(gamma), float(ctau), fct, S, Se, N, r,
+                    aec);
   if (!fct) {
     for (int a = 0; a < 4; ++a) add5<kRP>(R, n, N[a], r[a]);
     return;
@@ -459,7 +507,7 @@ __global__ void __launch_bounds__(kBlock) k_elem_rhs_aec32(int64_t n, int64_t ne
 // builds its four in shared memory (kStW double2 per lane: 16-byte stores
 // of 8 lanes fall in distinct banks) and the warp moves the run to or from
 // global memory with contiguous 512-byte accesses.
-constexpr int kEB = 128;   // FP64 element-pass block: 4 warps
+constexpr int kEB = 64;    // FP64 element-pass block: small, as an SM's FP64 units take its blocks in turn
 constexpr int kStW = 21;   // staged double2 per lane
 constexpr int kRecD2 = 5;  // residual slot record, double2
 constexpr int kLimD2 = 3;  // limited slot record, double2
@@ -477,8 +525,7 @@ __device__ __forceinline__ void warp_get(const double2* __restrict__ g, double2*
 
 __global__ void __launch_bounds__(kEB) k_elem_rhs64(int64_t n, int64_t ne,
                                                      const int32_t* __restrict__ inpoel,
-                                                     const double* __restrict__ xyz,
-                                                     const double* __restrict__ U,
+                                                     const double* __restrict__ geo,
                                                      const double* __restrict__ V,
                                                      const KScalars* __restrict__ sc,
                                                      double gamma, double ctau, int fct,
@@ -494,8 +541,7 @@ __global__ void __launch_bounds__(kEB) k_elem_rhs64(int64_t n, int64_t ne,
   if (e < ne) {
     int32_t N[4];
     double r[4][5], aec[4][5];
-    elem_terms<double>(n, ne, e, inpoel, xyz, nullptr, U, nullptr, V, sc, gamma, ctau, fct, S, Se,
-                       N, r, aec);
+    elem_terms<double>(n, ne, e, inpoel, geo, V, sc, gamma, ctau, fct, S, Se, N, r, aec);
     for (int a = 0; a < 4; ++a) {
       double2* b = buf + lane * kStW + a * kRecD2;
       b[0] = make_double2(r[a][0], r[a][1]);
@@ -522,161 +568,233 @@ struct KBC {
   const double* xyz;   // [3][n] node coordinates
 };
 
-// Symmetry projection of the momentum antidiffusive sums (KozCG.cpp:816-830).
-template <class F>
-__global__ void k_bc_p(int64_t n, KBC bc, F* P) {
-  int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i >= bc.nbc) return;
-  const int64_t p = bc.node[i];
-  for (int32_t k = bc.symp[i]; k < bc.symp[i + 1]; ++k) {
-    const F nx = F(bc.symn[3 * k]), ny = F(bc.symn[3 * k + 1]), nz = F(bc.symn[3 * k + 2]);
-    F* P2 = P + pidx<F>(n, 2, p);  // comp 1 (+)
-    F* P3 = P + pidx<F>(n, 3, p);  // comp 1 (-)
-    F* P4 = P + pidx<F>(n, 4, p);
-    F* P5 = P + pidx<F>(n, 5, p);
-    F* P6 = P + pidx<F>(n, 6, p);
-    F* P7 = P + pidx<F>(n, 7, p);
-    const F rvnp = *P2 * nx + *P4 * ny + *P6 * nz;
-    const F rvnn = *P3 * nx + *P5 * ny + *P7 * nz;
-    *P2 -= rvnp * nx;
-    *P3 -= rvnn * nx;
-    *P4 -= rvnp * ny;
-    *P5 -= rvnn * ny;
-    *P6 -= rvnp * nz;
-    *P7 -= rvnn * nz;
-  }
-}
+// What the node passes share.
+struct NodeArgs {
+  int64_t n;
+  const double *ivol, *cbrtv;
+  const KScalars* sc;
+  KBC bc;
+  const int32_t* bcof;
+  int fct, clip;
+  double gamma;
+  double *U, *R, *P;  // state, low-order solution, P/vol [10][n]
+  unsigned long long* dtmin;
+};
 
-// KozCG::alw node part (KozCG.cpp:887-912): P /= vol, low-order solution
-// lo = U + dt R/vol - P+ - P-.
-// Without FCT the update of KozCG::solve (KozCG.cpp:1151-1160) goes straight
-// to A.  Racc/Pacc are the element sums (in F); lo and P/vol go to the FP64
-// arrays Rlo/Pout (the same arrays as Racc/Pacc in FP64 mode), and in FP32
-// mode lo also to lo32 for the element pass of the allowed limits.
+// KozCG::alw node part (KozCG.cpp:887-912) at node i from its sums r and p
+// (p[2c] positive, p[2c + 1] negative antidiffusive sums of component c):
+// the symmetry projection of the momentum sums at BC nodes (KozCG.cpp:816-830),
+// P /= vol and the low-order solution lo = U + dt R/vol - P+ - P-, with the
+// keys of the node's extremes (lo, and U unless clip) for the allowed limits.
 template <class F>
-__global__ void k_node_lo(int64_t n, const double* __restrict__ vol, const double* __restrict__ U,
-                          const KScalars* __restrict__ sc, int fct, const F* Racc, const F* Pacc,
-                          double* Rlo, double* Pout, F* lo32, double* A) {
-  int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
-  const double dt = sc->dt;
-  const double v = vol[i];
-  // FP32 mode: one FP64 division per node (GB300's FP64 divisions are slow);
-  // FP64 mode divides as the reference does
-  const double iv = sizeof(F) == 4 ? 1.0 / v : 0.0;
-  auto per_vol = [&](double x) { return sizeof(F) == 4 ? x * iv : x / v; };
-  for (int c = 0; c < 5; ++c) {
-    if (fct) {
-      double pp = per_vol(double(Pacc[pidx<F>(n, c * 2 + 0, i)]));
-      double pn = per_vol(double(Pacc[pidx<F>(n, c * 2 + 1, i)]));
-      Pout[(c * 2 + 0) * n + i] = pp;
-      Pout[(c * 2 + 1) * n + i] = pn;
-      const double lo = U[c * n + i] + per_vol(dt * double(Racc[ridx<F, kRP>(n, c, i)])) - pp - pn;
-      Rlo[c * n + i] = lo;
-      if (lo32) lo32[c * n + i] = F(lo);
-    } else {
-      A[c * n + i] = U[c * n + i] + per_vol(dt * double(Racc[ridx<F, kRP>(n, c, i)]));
+__device__ __forceinline__ void node_low(const NodeArgs& q, int64_t i, const double r[5],
+                                         F p[10], typename KozT<F>::Key* __restrict__ K) {
+  const int32_t b = __ldg(q.bcof + i);
+  if (b >= 0) {
+    for (int32_t k = q.bc.symp[b]; k < q.bc.symp[b + 1]; ++k) {
+      const F nx = F(q.bc.symn[3 * k]), ny = F(q.bc.symn[3 * k + 1]), nz = F(q.bc.symn[3 * k + 2]);
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const F vn = p[2 + s] * nx + p[4 + s] * ny + p[6 + s] * nz;
+        p[2 + s] -= vn * nx;
+        p[4 + s] -= vn * ny;
+        p[6 + s] -= vn * nz;
+      }
     }
   }
+  const double iv = q.ivol[i], dv = q.sc->dt * iv;
+  typename KozT<F>::Key key[10];
+#pragma unroll
+  for (int c = 0; c < 5; ++c) {
+    const double pp = iv * double(p[2 * c]), pn = iv * double(p[2 * c + 1]);
+    q.P[(c * 2 + 0) * q.n + i] = pp;
+    q.P[(c * 2 + 1) * q.n + i] = pn;
+    const double u = q.U[c * q.n + i];
+    const double lo = u + dv * r[c] - pp - pn;
+    q.R[c * q.n + i] = lo;
+    const F l = F(lo), uf = F(u);
+    key[c * 2 + 0] = okey(q.clip ? l : fmax(l, uf));
+    key[c * 2 + 1] = okey(q.clip ? l : fmin(l, uf));
+  }
+  store10(K + i * rec10<F>(), key);
 }
 
-// KozCG::alw element part (KozCG.cpp:914-935): the allowed limits of a node
-// are the maximum / minimum, over the elements holding it, of the element's
-// extremes of the low-order solution lo (and of the state U unless clip).
-// The nodes of those elements are the node and its adjacency, so the same
-// extremes are taken here per node over {i} and its neighbours: max and min
-// are exact, so the bounds are the element loop's, without atomics.  Stored
-// as order-preserving keys (the node pass of the limits reads keys).
+// KozCG::solve's state u of node i (KozCG.cpp:1144-1160), its BCs (Dirichlet
+// then symmetry at the step's end time, KozCG.cpp:590-611, 1167) and its CFL
+// time step.
+__device__ __forceinline__ double node_finish(const NodeArgs& q, int64_t i, double u[5]) {
+  const int32_t b = __ldg(q.bcof + i);
+  if (b >= 0) {
+    const int32_t d = q.bc.dir[b];
+    if (d >= 0)
+      dirichlet(q.bc.prob, q.bc.xyz[i], q.bc.xyz[q.n + i], q.bc.xyz[2 * q.n + i], q.sc->tnext,
+                q.bc.dirmask + d * 5, q.bc.dirval + d * 5, u);
+    for (int32_t k = q.bc.symp[b]; k < q.bc.symp[b + 1]; ++k) {
+      const double* nn = q.bc.symn + 3 * k;
+      const double vn = u[1] * nn[0] + u[2] * nn[1] + u[3] * nn[2];
+      u[1] -= vn * nn[0];
+      u[2] -= vn * nn[1];
+      u[3] -= vn * nn[2];
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 5; ++c) q.U[c * q.n + i] = u[c];
+  return node_dt(u, q.cbrtv[i], q.gamma);
+}
+
+// FP32 mode: the node passes on the element sums in node records.
+__global__ void __launch_bounds__(kBlock) k_node_low32(NodeArgs q, const float* __restrict__ acc,
+                                                        unsigned int* __restrict__ K) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i >= q.n) return;
+  float v[16];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float4 t = __ldg(reinterpret_cast<const float4*>(acc + i * kRP) + k);
+    v[4 * k] = t.x;
+    v[4 * k + 1] = t.y;
+    v[4 * k + 2] = t.z;
+    v[4 * k + 3] = t.w;
+  }
+  double r[5];
+#pragma unroll
+  for (int c = 0; c < 5; ++c) r[c] = double(v[c]);
+  node_low<float>(q, i, r, v + 5, K);
+}
+__global__ void __launch_bounds__(kBlock) k_node_update32(NodeArgs q,
+                                                           const float* __restrict__ acc) {
+  // acc: the limited sums [n][8], or without FCT the residual records [n][16]
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  double dtp = DBL_MAX;
+  if (i < q.n) {
+    const float* a = acc + i * (q.fct ? kAR : kRP);
+    const float4 t = __ldg(reinterpret_cast<const float4*>(a));
+    const float v[5] = {t.x, t.y, t.z, t.w, __ldg(a + 4)};
+    const double iv = q.fct ? q.ivol[i] : q.sc->dt * q.ivol[i];
+    double u[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c)
+      u[c] = (q.fct ? q.R : q.U)[c * q.n + i] + iv * double(v[c]);
+    dtp = node_finish(q, i, u);
+  }
+  block_min_atomic(dtp, q.dtmin);
+}
+
+// Two quotients a/p and b/q from one division (batch inversion); the plain
+// divisions where the product of the denominators leaves the normal range.
+__device__ __forceinline__ void quotients(double a, double p, double b, double q, double& x,
+                                          double& y) {
+  const double d = p * q, m = fabs(d);
+  if (m > 1e-290 && m < 1e290) {
+    const double inv = 1.0 / d;
+    x = a * (q * inv);
+    y = b * (p * inv);
+  } else {
+    x = a / p;
+    y = b / q;
+  }
+}
+__device__ __forceinline__ void quotients(float a, float p, float b, float q, float& x, float& y) {
+  x = a / p;
+  y = b / q;
+}
+
+// KozCG::alw element part and KozCG::lim node part (KozCG.cpp:914-935,
+// 1004-1024).  The allowed limits of a node are the maximum / minimum, over
+// the elements holding it, of the element's extremes; the nodes of those
+// elements are the node and its adjacency, so the same extremes are taken
+// here per node over {i} and its neighbours (max and min are exact, so the
+// bounds are the element loop's, without atomics), as integer comparisons of
+// the keys: FP64 comparisons would hold the FP64 units, 280 a node (with the
+// records and the two passes in one, 249 -> 67 us at 65^3).  Then Q -=
+// low-order solution and the limit coefficients C+/- into Q.
 template <class F>
-__global__ void __launch_bounds__(kBlock) k_node_alw(int64_t n, const int32_t* __restrict__ aoff,
-                                                      const int32_t* __restrict__ aw,
-                                                      const int32_t* __restrict__ nbr,
-                                                      const F* __restrict__ U,
-                                                      const F* __restrict__ lo, int clip,
-                                                      typename KozT<F>::Key* __restrict__ Q) {
+__global__ void __launch_bounds__(kBlock)
+    k_node_limit(int64_t n, const int32_t* __restrict__ aoff, const int32_t* __restrict__ aw,
+                 const int32_t* __restrict__ nbr, const typename KozT<F>::Key* __restrict__ K,
+                 const double* __restrict__ R, const double* __restrict__ P,
+                 F* __restrict__ Q) {
+  using Key = typename KozT<F>::Key;
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   const int lane = static_cast<int>(i & 31);
   const int64_t s = i >> 5;
   const int32_t off = __ldg(aoff + s), w = __ldg(aw + s);
-  F mx[5], mn[5];
+  constexpr int RL = rec10<F>();
+  Key m[10];  // the maximum and minimum of each component, interleaved
+  load10(K + i * RL, m);
+  // two neighbours together: their records are in flight at once
+  for (int k = 0; k < w; k += 2) {
+    int32_t q[2];
+    Key v[2][10];
 #pragma unroll
-  for (int c = 0; c < 5; ++c) {
-    const F l = lo[c * n + i];
-    mx[c] = l;
-    mn[c] = l;
-    if (!clip) {
-      const F u = U[c * n + i];
-      mx[c] = fmax(mx[c], u);
-      mn[c] = fmin(mn[c], u);
+    for (int j = 0; j < 2; ++j) {
+      q[j] = k + j < w ? __ldg(nbr + off + (k + j) * 32 + lane) : -1;
+      if (q[j] < 0) q[j] = static_cast<int32_t>(i);  // padding: the node itself
     }
-  }
-#pragma unroll 4
-  for (int k = 0; k < w; ++k) {
-    const int32_t q = __ldg(nbr + off + k * 32 + lane);
-    if (q < 0) continue;
 #pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      const F l = __ldg(lo + c * n + q);
-      mx[c] = fmax(mx[c], l);
-      mn[c] = fmin(mn[c], l);
-      if (!clip) {
-        const F u = __ldg(U + c * n + q);
-        mx[c] = fmax(mx[c], u);
-        mn[c] = fmin(mn[c], u);
+    for (int j = 0; j < 2; ++j) load10(K + int64_t(q[j]) * RL, v[j]);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int c = 0; c < 5; ++c) {
+        m[2 * c] = v[j][2 * c] > m[2 * c] ? v[j][2 * c] : m[2 * c];
+        m[2 * c + 1] = v[j][2 * c + 1] < m[2 * c + 1] ? v[j][2 * c + 1] : m[2 * c + 1];
       }
-    }
   }
+  const double eps = DBL_EPSILON;
+  F out[10];
 #pragma unroll
   for (int c = 0; c < 5; ++c) {
-    Q[(c * 2 + 0) * n + i] = okey(mx[c]);
-    Q[(c * 2 + 1) * n + i] = okey(mn[c]);
-  }
-}
-
-// KozCG::lim node part (KozCG.cpp:1004-1024): Q -= low-order solution, limit
-// coefficients C+/- stored back into Q as F values (reinterpreted).
-template <class F>
-__global__ void k_node_lim(int64_t n, const double* __restrict__ R, const double* __restrict__ P,
-                           typename KozT<F>::Key* Q) {
-  int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
-  const double eps = DBL_EPSILON;
-  for (int c = 0; c < 5; ++c) {
-    double qp = double(oval(Q[(c * 2 + 0) * n + i])) - R[c * n + i];
-    double qn = double(oval(Q[(c * 2 + 1) * n + i])) - R[c * n + i];
+    const double lo = R[c * n + i];
+    const double qp = double(oval(m[2 * c])) - lo, qn = double(oval(m[2 * c + 1])) - lo;
     const double pp = P[(c * 2 + 0) * n + i], pn = P[(c * 2 + 1) * n + i];
-    // the coefficient's quotient in F (an FP32 division in FP32 mode)
-    const F cp = pp < eps ? F(0) : fmin(F(1), F(qp) / F(pp));
-    const F cn = pn > -eps ? F(0) : fmin(F(1), F(qn) / F(pn));
-    Q[(c * 2 + 0) * n + i] = tobits(cp);
-    Q[(c * 2 + 1) * n + i] = tobits(cn);
+    const bool zp = pp < eps, zn = pn > -eps;
+    F cp, cn;
+    quotients(F(qp), zp ? F(1) : F(pp), F(qn), zn ? F(1) : F(pn), cp, cn);
+    out[c * 2 + 0] = zp ? F(0) : fmin(F(1), cp);
+    out[c * 2 + 1] = zn ? F(0) : fmin(F(1), cn);
   }
+  store10(Q + i * RL, out);
 }
 
 // KozCG::lim element part (KozCG.cpp:1049-1078): limited antidiffusive
 // element contributions, system-limited over the components in sysmask.
 // Limit coefficients of one element from its antidiffusive contributions
-// aec[a][c] and the nodes' C+/- (Q, as F bits); ca = the limited ones.
+// aec[a][c] and the nodes' C+/- (Q); ca = the limited ones.  Signs and minima
+// are taken on the bits of the values: the coefficients lie in [0, 1] (or are
+// -0), which order as signed integers, and FP64 comparisons would hold the
+// FP64 units.
+__device__ __forceinline__ long long sbits(double v) { return __double_as_longlong(v); }
+__device__ __forceinline__ int sbits(float v) { return __float_as_int(v); }
 template <class F>
-__device__ __forceinline__ void elem_limit(int64_t n, const int32_t N[4],
-                                           const typename KozT<F>::Key* __restrict__ Q,
+__device__ __forceinline__ F lesser(F a, F b) {
+  return sbits(a) < sbits(b) ? a : b;
+}
+template <class F>
+__device__ __forceinline__ void elem_limit(const int32_t N[4], const F* __restrict__ Q,
                                            int sysmask, const F aec[4][5], F ca[4][5]) {
   F coef[5];
-  for (int c = 0; c < 5; ++c) {
-    coef[c] = F(1.0);
-    for (int a = 0; a < 4; ++a) {
-      const F s = aec[a][c];
-      const F lim = kbits(Q[(c * 2 + (s > F(0.0) ? 0 : 1)) * n + N[a]]);
-      coef[c] = coef[c] < lim ? coef[c] : lim;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    F q[10];
+    load10(Q + int64_t(N[a]) * rec10<F>(), q);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      const F lim = sbits(aec[a][c]) > 0 ? q[2 * c] : q[2 * c + 1];
+      coef[c] = lesser(a == 0 ? F(1.0) : coef[c], lim);
     }
   }
   F cs = F(1.0);
+#pragma unroll
   for (int c = 0; c < 5; ++c)
-    if (sysmask & (1 << c)) cs = cs < coef[c] ? cs : coef[c];
+    if (sysmask & (1 << c)) cs = lesser(cs, coef[c]);
+#pragma unroll
   for (int c = 0; c < 5; ++c)
     if (sysmask & (1 << c)) coef[c] = cs;
+#pragma unroll
   for (int a = 0; a < 4; ++a)
+#pragma unroll
     for (int c = 0; c < 5; ++c) ca[a][c] = coef[c] * aec[a][c];
 }
 
@@ -685,26 +803,24 @@ __device__ __forceinline__ void elem_limit(int64_t n, const int32_t N[4],
 __global__ void __launch_bounds__(kBlock) k_elem_lim32(int64_t n, int64_t ne,
                                                         const int32_t* __restrict__ inpoel,
                                                         const float* __restrict__ geo,
-                                                        const float* __restrict__ Uf,
-                                                        const unsigned int* __restrict__ Q,
+                                                        const float* __restrict__ V,
+                                                        const float* __restrict__ Q,
                                                         double ctau_d, int sysmask, float* A) {
   const int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (e >= ne) return;
-  const float ctau = float(ctau_d);
-  int32_t N[4];
-  for (int a = 0; a < 4; ++a) N[a] = inpoel[e * 4 + a];
-  const Geo<float> t = elem_geo<float>(nullptr, geo, n, ne, e, N);
-  float aec[4][5], ca[4][5];
-  for (int c = 0; c < 5; ++c)
-    for (int a = 0; a < 4; ++a) {
-      float s = 0.f;
-      for (int b = 0; b < 4; ++b) {
-        const float m = t.J / 120.f * ((a == b) ? 3.f : -1.f);
-        s += m * ctau * ust<float>(nullptr, Uf, n, c, N[b]);
-      }
-      aec[a][c] = s;
-    }
-  elem_limit<float>(n, N, Q, sysmask, aec, ca);
+  const int4 nd = __ldg(reinterpret_cast<const int4*>(inpoel) + e);
+  const int32_t N[4] = {nd.x, nd.y, nd.z, nd.w};
+  const float k = float(ctau_d) * __ldg(geo + e);  // ctau J/120
+  float u[4][8], aec[4][5], ca[4][5];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) load_node(V, N[a], u[a]);
+#pragma unroll
+  for (int c = 0; c < 5; ++c) {
+    const float sum = u[0][c] + u[1][c] + u[2][c] + u[3][c];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) aec[a][c] = k * (4.f * u[a][c] - sum);
+  }
+  elem_limit<float>(N, Q, sysmask, aec, ca);
   for (int a = 0; a < 4; ++a) add5<kAR>(A, n, N[a], ca[a]);
 }
 
@@ -715,7 +831,7 @@ __global__ void __launch_bounds__(kBlock) k_elem_lim32(int64_t n, int64_t ne,
 __global__ void __launch_bounds__(kEB) k_elem_lim64(int64_t n, int64_t ne,
                                                      const int32_t* __restrict__ inpoel,
                                                      const double* __restrict__ E,
-                                                     const unsigned long long* __restrict__ Q,
+                                                     const double* __restrict__ Q,
                                                      int sysmask, double* __restrict__ L) {
   __shared__ double2 st[kEB / 32][32 * kStW];
   const int lane = threadIdx.x & 31;
@@ -736,7 +852,7 @@ __global__ void __launch_bounds__(kEB) k_elem_lim64(int64_t n, int64_t ne,
       const double* rec = reinterpret_cast<const double*>(buf + lane * kStW + a * kRecD2);
       for (int c = 0; c < 5; ++c) aec[a][c] = rec[5 + c];
     }
-    elem_limit<double>(n, N, Q, sysmask, aec, ca);
+    elem_limit<double>(N, Q, sysmask, aec, ca);
   }
   __syncwarp();
   if (live)
@@ -763,23 +879,18 @@ __global__ void __launch_bounds__(kEB) k_elem_lim64(int64_t n, int64_t ne,
 // time, their loads issued together before the adds (in slot order), so
 // that a node's loads overlap.
 template <int RD2, bool WP>
-__global__ void __launch_bounds__(kBlock) k_node_gather(int64_t n,
-                                                         const int32_t* __restrict__ soff,
-                                                         const int32_t* __restrict__ sw,
-                                                         const int32_t* __restrict__ slot,
-                                                         const double* __restrict__ E,
-                                                         double* __restrict__ R,
-                                                         double* __restrict__ P) {
+__device__ __forceinline__ void node_slots(int64_t i, const int32_t* __restrict__ soff,
+                                           const int32_t* __restrict__ sw,
+                                           const int32_t* __restrict__ slot,
+                                           const double* __restrict__ E, double r[5],
+                                           double p[10]) {
   constexpr int LD2 = WP ? 5 : 3;  // double2 read per slot
-  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
   const int lane = static_cast<int>(i & 31);
   const int64_t s = i >> 5;
   const int32_t off = __ldg(soff + s), w = __ldg(sw + s);
   const double2* E2 = reinterpret_cast<const double2*>(E);
-  double r[5], pp[5], pn[5];
 #pragma unroll
-  for (int c = 0; c < 5; ++c) r[c] = pp[c] = pn[c] = 0.0;
+  for (int c = 0; c < 5; ++c) r[c] = p[2 * c] = p[2 * c + 1] = 0.0;
   for (int k0 = 0; k0 < w; k0 += kGB) {
     int32_t q[kGB];
 #pragma unroll
@@ -810,91 +921,95 @@ __global__ void __launch_bounds__(kBlock) k_node_gather(int64_t n,
           const long long mag = b & 0x7fffffffffffffffll;
           if (mag != 0 && mag <= 0x7ff0000000000000ll) {
             if (b > 0)
-              pp[c] += v;
+              p[2 * c] += v;
             else
-              pn[c] += v;
+              p[2 * c + 1] += v;
           }
         }
       }
     }
   }
+}
+
+// The FP64 node passes: the slots' sums, then the node's algebra, in one
+// kernel each (sums, boundary projection and low-order solution in kernels of
+// their own moved 240 bytes a node through memory in between).
+__global__ void __launch_bounds__(kBlock) k_node_low64(NodeArgs q,
+                                                        const int32_t* __restrict__ soff,
+                                                        const int32_t* __restrict__ sw,
+                                                        const int32_t* __restrict__ slot,
+                                                        const double* __restrict__ E,
+                                                        unsigned long long* __restrict__ K) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i >= q.n) return;
+  double r[5], p[10];
+  node_slots<kRecD2, true>(i, soff, sw, slot, E, r, p);
+  node_low<double>(q, i, r, p, K);
+}
+// FCT: E the limited slot records; otherwise the residual ones.
+template <bool FCT>
+__global__ void __launch_bounds__(kBlock) k_node_update64(NodeArgs q,
+                                                           const int32_t* __restrict__ soff,
+                                                           const int32_t* __restrict__ sw,
+                                                           const int32_t* __restrict__ slot,
+                                                           const double* __restrict__ E) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  double dtp = DBL_MAX;
+  if (i < q.n) {
+    double r[5], p[10];
+    node_slots<FCT ? kLimD2 : kRecD2, false>(i, soff, sw, slot, E, r, p);
+    const double iv = FCT ? q.ivol[i] : q.sc->dt * q.ivol[i];
+    double u[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) u[c] = (FCT ? q.R : q.U)[c * q.n + i] + iv * r[c];
+    dtp = node_finish(q, i, u);
+  }
+  block_min_atomic(dtp, q.dtmin);
+}
+// The residual alone (xg_kozcg_rhs).
+__global__ void __launch_bounds__(kBlock) k_node_rhs64(int64_t n,
+                                                        const int32_t* __restrict__ soff,
+                                                        const int32_t* __restrict__ sw,
+                                                        const int32_t* __restrict__ slot,
+                                                        const double* __restrict__ E,
+                                                        double* __restrict__ R) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i >= n) return;
+  double r[5], p[10];
+  node_slots<kRecD2, false>(i, soff, sw, slot, E, r, p);
 #pragma unroll
   for (int c = 0; c < 5; ++c) R[c * n + i] = r[c];
-  if constexpr (WP) {
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      P[(c * 2 + 0) * n + i] = pp[c];
-      P[(c * 2 + 1) * n + i] = pn[c];
-    }
-  }
 }
 
-// KozCG::solve (KozCG.cpp:1144-1150): A = low-order + A/vol, then U = A and
-// the CFL minimum of the new state for nodes without BCs.  Aacc: the limited
-// sums (F, with FCT); A: the update itself (FP64, without FCT).
-template <class F>
-__global__ void __launch_bounds__(kBlock) k_node_solve(int64_t n, const double* __restrict__ vol,
-                                                        const double* __restrict__ R,
-                                                        const F* __restrict__ Aacc,
-                                                        const double* __restrict__ A, int fct,
-                                                        const uint8_t* __restrict__ isbc,
-                                                        double gamma, double* U,
-                                                        unsigned long long* dtmin) {
+// Nodal BCs (KozCG::BC) on the device state at the caller's time t.
+__global__ void __launch_bounds__(kBlock) k_bc(int64_t n, KBC bc, double* U, double t) {
   int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  double dtp = DBL_MAX;
-  if (i < n) {
-    double u[5];
-    const double v = vol[i];
-    const double iv = sizeof(F) == 4 ? 1.0 / v : 0.0;  // FP32 mode: one division
-    for (int c = 0; c < 5; ++c) {
-      const double a = double(Aacc[ridx<F, kAR>(n, c, i)]);
-      u[c] = fct ? R[c * n + i] + (sizeof(F) == 4 ? a * iv : a / v) : A[c * n + i];
-      U[c * n + i] = u[c];
-    }
-    if (!isbc[i]) dtp = node_dt(u, vol[i], gamma);
+  if (i >= bc.nbc) return;
+  const int64_t p = bc.node[i];
+  double u[5];
+  for (int c = 0; c < 5; ++c) u[c] = U[c * n + p];
+  const int32_t d = bc.dir[i];
+  if (d >= 0)
+    dirichlet(bc.prob, bc.xyz[p], bc.xyz[n + p], bc.xyz[2 * n + p], t, bc.dirmask + d * 5,
+              bc.dirval + d * 5, u);
+  for (int32_t k = bc.symp[i]; k < bc.symp[i + 1]; ++k) {
+    const double* nn = bc.symn + 3 * k;
+    double vn = u[1] * nn[0] + u[2] * nn[1] + u[3] * nn[2];
+    u[1] -= vn * nn[0];
+    u[2] -= vn * nn[1];
+    u[3] -= vn * nn[2];
   }
-  block_min_atomic(dtp, dtmin);
+  for (int c = 0; c < 5; ++c) U[c * n + p] = u[c];
 }
 
-// KozCG::BC: Dirichlet then symmetry (physics::dirbc/symbc), one thread per
-// BC node, with the node's CFL dt.
-// Nodal BCs (KozCG::BC) at time t: after a step t + dt (sc->tnext,
-// KozCG.cpp:1167), otherwise the caller's t_host (sc null).
-__global__ void __launch_bounds__(kBlock) k_bc(int64_t n, KBC bc, double gamma, double* U,
-                                                const double* __restrict__ vol, int want_dt,
-                                                unsigned long long* dtmin,
-                                                const KScalars* __restrict__ sc, double t_host) {
-  int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  double dtp = DBL_MAX;
-  if (i < bc.nbc) {
-    const int64_t p = bc.node[i];
-    double u[5];
-    for (int c = 0; c < 5; ++c) u[c] = U[c * n + p];
-    const int32_t d = bc.dir[i];
-    if (d >= 0)
-      dirichlet(bc.prob, bc.xyz[p], bc.xyz[n + p], bc.xyz[2 * n + p], sc ? sc->tnext : t_host,
-                bc.dirmask + d * 5, bc.dirval + d * 5, u);
-    for (int32_t k = bc.symp[i]; k < bc.symp[i + 1]; ++k) {
-      const double* nn = bc.symn + 3 * k;
-      double vn = u[1] * nn[0] + u[2] * nn[1] + u[3] * nn[2];
-      u[1] -= vn * nn[0];
-      u[2] -= vn * nn[1];
-      u[3] -= vn * nn[2];
-    }
-    for (int c = 0; c < 5; ++c) U[c * n + p] = u[c];
-    if (want_dt) dtp = node_dt(u, vol[p], gamma);
-  }
-  if (want_dt) block_min_atomic(dtp, dtmin);
-}
-
-__global__ void k_dt(int64_t n, const double* __restrict__ U, const double* __restrict__ vol,
+__global__ void k_dt(int64_t n, const double* __restrict__ U, const double* __restrict__ cbrtv,
                      double gamma, unsigned long long* dtmin) {
   int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   double dtp = DBL_MAX;
   if (p < n) {
     double u[5];
     for (int c = 0; c < 5; ++c) u[c] = U[c * n + p];
-    dtp = node_dt(u, vol[p], gamma);
+    dtp = node_dt(u, cbrtv[p], gamma);
   }
   block_min_atomic(dtp, dtmin);
 }
@@ -951,6 +1066,15 @@ __global__ void k_src_elems(int64_t n, int64_t ne, SrcPrm q, const KScalars* __r
   for (int c = 0; c < 5; ++c) Se[e * 5 + c] = o[c];
 }
 
+// 1/vol and cbrt(vol).
+__global__ void k_node_factors(int64_t n, const double* __restrict__ vol,
+                               double* __restrict__ ivol, double* __restrict__ cbrtv) {
+  const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (p >= n) return;
+  ivol[p] = 1.0 / vol[p];
+  cbrtv[p] = cbrt(vol[p]);
+}
+
 __global__ void k_reset_min(KScalars* s) { s->dtmin = __double_as_longlong(DBL_MAX); }
 
 __global__ void k_aos_to_soa(int64_t n, int nc, const double* __restrict__ a,
@@ -978,35 +1102,25 @@ KBC kbc_of(KozCGDev* d) {
 int refresh_dt(xg_ctx* c, KozCGDev* d) {
   k_reset_min<<<1, 1, 0, c->stream>>>(d->scal);
   XG_CHECK_LAUNCH(c);
-  k_dt<<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(d->n, d->U, d->vol, d->prm.gamma,
+  k_dt<<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(d->n, d->U, d->cbrtv, d->prm.gamma,
                                                             &d->scal->dtmin);
   XG_CHECK_LAUNCH(c);
   d->dt_valid = true;
   return XG_OK;
 }
 
-// The arrays of precision F: element sums (R, P, A accumulators), the state
-// the element passes read, the per-node primitives, the limit keys.
-template <class F>
-struct KArrays {
-  F *R, *P, *A, *Uf, *V, *lo;
-  typename KozT<F>::Key* Q;
-  const float* geo;
-};
-KArrays<double> arrays64(KozCGDev* d) {
-  return KArrays<double>{d->R, d->P, d->A, nullptr, d->V, d->R, d->Q, nullptr};
-}
-KArrays<float> arrays32(KozCGDev* d) {
-  return KArrays<float>{d->R32, d->R32 + 5, d->A32, d->U32, reinterpret_cast<float*>(d->V),
-                        d->lo32, d->Q32, d->geo32};
+NodeArgs node_args(KozCGDev* d) {
+  return NodeArgs{d->n,  d->ivol,         d->cbrtv,    d->scal,      kbc_of(d),
+                  d->bcof, d->prm.fct,    d->prm.fctclip, d->prm.gamma, d->U,
+                  d->R,  d->P,            &d->scal->dtmin};
 }
 
-// Node primitives and the element Galerkin (+ antidiffusive) pass on state U
-// into the node sums R, P: in FP64 the element pass fills the residual slot
-// records and k_node_gather forms R (and P with FCT) in the FP64 arrays; in
-// FP32 it adds into the zeroed node records k.R directly.
+// Node primitives and the element Galerkin (+ antidiffusive) pass on state U:
+// in FP64 into the residual slot records, in FP32 added into the zeroed node
+// records.
 template <class F>
-void galerkin(cudaStream_t s, KozCGDev* d, const KArrays<F>& k, const double* U, int fct) {
+void galerkin(xg_ctx* c, KozCGDev* d, const double* U, int fct) {
+  cudaStream_t s = c->stream;
   const int64_t n = d->n, ne = d->ne;
   const double *S = nullptr, *Se = nullptr;
   if (d->src.problem != XG_SRC_NONE) {
@@ -1016,82 +1130,68 @@ void galerkin(cudaStream_t s, KozCGDev* d, const KArrays<F>& k, const double* U,
     S = d->S;
     Se = d->Se;
   }
-  k_node_prim<F><<<blocks_for(n, kBlock), kBlock, 0, s>>>(n, U, d->prm.gamma, k.V, k.Uf);
+  const int tb = node_block(c, n, kBlock);
+  F* V = reinterpret_cast<F*>(d->V);
   if constexpr (sizeof(F) == 8) {
-    k_elem_rhs64<<<blocks_for(ne, kEB), kEB, 0, s>>>(n, ne, d->inpoel, d->xyz, U, k.V, d->scal,
+    k_node_prim<double><<<blocks_for(n, tb), tb, 0, s>>>(n, U, d->prm.gamma, V);
+    k_elem_rhs64<<<blocks_for(ne, kEB), kEB, 0, s>>>(n, ne, d->inpoel, d->geo64, V, d->scal,
                                                      d->prm.gamma, d->prm.ctau, fct, S, Se,
                                                      d->E);
-    if (fct)
-      k_node_gather<kRecD2, true><<<blocks_for(n, kBlock), kBlock, 0, s>>>(
-          n, d->soff, d->sw, d->sslot, d->E, d->R, d->P);
-    else
-      k_node_gather<kRecD2, false><<<blocks_for(n, kBlock), kBlock, 0, s>>>(
-          n, d->soff, d->sw, d->sslot, d->E, d->R, nullptr);
   } else {
-    k_elem_rhs_aec32<<<blocks_for(ne, kBlock), kBlock, 0, s>>>(n, ne, d->inpoel, k.geo, k.Uf, k.V,
-                                                                d->scal, d->prm.gamma,
-                                                                d->prm.ctau, fct, S, Se, k.R);
+    k_node_prim<float><<<blocks_for(n, tb), tb, 0, s>>>(n, U, d->prm.gamma, V);
+    const int eb = node_block(c, ne, kBlock);
+    k_elem_rhs_aec32<<<blocks_for(ne, eb), eb, 0, s>>>(n, ne, d->inpoel, d->geo32, V,
+                                                        d->scal, d->prm.gamma, d->prm.ctau, fct,
+                                                        S, Se, d->R32);
   }
 }
 
 // One KozCG step with the dt already in the device scalars, element
 // arithmetic in F.
 template <class F>
-int step_impl(xg_ctx* c, KozCGDev* d, const KArrays<F>& k) {
+int step_impl(xg_ctx* c, KozCGDev* d) {
   cudaStream_t s = c->stream;
   const int64_t n = d->n, ne = d->ne;
   const int fct = d->prm.fct;
-  // FP32: R with P [n][16], A [n][8] accumulate atomically from zero; FP64:
-  // R, A [5][n], P [10][n] are written whole by k_node_gather
+  const int tb = node_block(c, n, kBlock);
+  const unsigned nb = blocks_for(n, tb);
+  const NodeArgs q = node_args(d);
+  // FP32: R with P [n][16], A [n][8] accumulate atomically from zero
   if (sizeof(F) == 4) {
-    XG_CUDA(c, cudaMemsetAsync(k.R, 0, n * kRP * 4, s));
-    if (fct) XG_CUDA(c, cudaMemsetAsync(k.A, 0, n * kAR * 4, s));
+    XG_CUDA(c, cudaMemsetAsync(d->R32, 0, n * kRP * 4, s));
+    if (fct) XG_CUDA(c, cudaMemsetAsync(d->A32, 0, n * kAR * 4, s));
   }
-  galerkin<F>(s, d, k, d->U, fct);
+  galerkin<F>(c, d, d->U, fct);
   XG_CHECK_LAUNCH(c);
-  if (fct && d->nbc) {
-    k_bc_p<F><<<blocks_for(d->nbc, kBlock), kBlock, 0, s>>>(n, kbc_of(d), k.P);
-    XG_CHECK_LAUNCH(c);
-  }
-  const bool f32 = sizeof(F) == 4;
-  k_node_lo<F><<<blocks_for(n, kBlock), kBlock, 0, s>>>(n, d->vol, d->U, d->scal, fct, k.R, k.P,
-                                                         d->R, d->P, f32 ? k.lo : nullptr, d->A);
-  XG_CHECK_LAUNCH(c);
-  if (fct) {
-    const F* Ust = f32 ? k.Uf : reinterpret_cast<const F*>(d->U);
-    k_node_alw<F><<<blocks_for(n, kBlock), kBlock, 0, s>>>(n, d->aoff, d->aw, d->anbr, Ust,
-                                                            k.lo, d->prm.fctclip, k.Q);
-    XG_CHECK_LAUNCH(c);
-    k_node_lim<F><<<blocks_for(n, kBlock), kBlock, 0, s>>>(n, d->R, d->P, k.Q);
-    XG_CHECK_LAUNCH(c);
-    if constexpr (sizeof(F) == 4) {
-      k_elem_lim32<<<blocks_for(ne, kBlock), kBlock, 0, s>>>(n, ne, d->inpoel, k.geo, k.Uf, k.Q,
-                                                              d->prm.ctau, d->prm.fctsys, k.A);
-      XG_CHECK_LAUNCH(c);
-    } else {
-      k_elem_lim64<<<blocks_for(ne, kEB), kEB, 0, s>>>(n, ne, d->inpoel, d->E, k.Q,
+  if constexpr (sizeof(F) == 4) {
+    if (fct) {
+      k_node_low32<<<nb, tb, 0, s>>>(q, d->R32, d->K32);
+      k_node_limit<float><<<nb, tb, 0, s>>>(n, d->aoff, d->aw, d->anbr, d->K32, d->R, d->P,
+                                            d->Q32);
+      const int eb = node_block(c, ne, kBlock);
+      k_elem_lim32<<<blocks_for(ne, eb), eb, 0, s>>>(n, ne, d->inpoel, d->geo32,
+                                                     reinterpret_cast<float*>(d->V), d->Q32,
+                                                     d->prm.ctau, d->prm.fctsys, d->A32);
+    }
+    k_node_update32<<<nb, tb, 0, s>>>(q, fct ? d->A32 : d->R32);
+  } else {
+    if (fct) {
+      k_node_low64<<<nb, tb, 0, s>>>(q, d->soff, d->sw, d->sslot, d->E, d->K);
+      k_node_limit<double><<<nb, tb, 0, s>>>(n, d->aoff, d->aw, d->anbr, d->K, d->R, d->P, d->Q);
+      k_elem_lim64<<<blocks_for(ne, kEB), kEB, 0, s>>>(n, ne, d->inpoel, d->E, d->Q,
                                                        d->prm.fctsys, d->L);
-      XG_CHECK_LAUNCH(c);
-      k_node_gather<kLimD2, false><<<blocks_for(n, kBlock), kBlock, 0, s>>>(
-          n, d->soff, d->sw, d->sslot, d->L, d->A, nullptr);
-      XG_CHECK_LAUNCH(c);
+      k_node_update64<true><<<nb, tb, 0, s>>>(q, d->soff, d->sw, d->sslot, d->L);
+    } else {
+      k_node_update64<false><<<nb, tb, 0, s>>>(q, d->soff, d->sw, d->sslot, d->E);
     }
   }
-  k_node_solve<F><<<blocks_for(n, kBlock), kBlock, 0, s>>>(n, d->vol, d->R, k.A, d->A, fct,
-                                                            d->isbc, d->prm.gamma, d->U,
-                                                            &d->scal->dtmin);
   XG_CHECK_LAUNCH(c);
-  if (d->nbc) {
-    k_bc<<<blocks_for(d->nbc, kBlock), kBlock, 0, s>>>(n, kbc_of(d), d->prm.gamma, d->U, d->vol,
-                                                        1, &d->scal->dtmin, d->scal, 0.0);
-    XG_CHECK_LAUNCH(c);
-  }
   return XG_OK;
 }
 
 int step(xg_ctx* c, KozCGDev* d) {
-  if (d->prm.precision == XG_FP32_FLUX) return step_impl<float>(c, d, arrays32(d));
-  return step_impl<double>(c, d, arrays64(d));
+  if (d->prm.precision == XG_FP32_FLUX) return step_impl<float>(c, d);
+  return step_impl<double>(c, d);
 }
 
 // The residual of FP32 node records [n][16] to FP64 [5][n].
@@ -1239,32 +1339,34 @@ int xg_kozcg_setup(xg_ctx* c, const xg_kozcg_params* prm, int64_t npoin, const d
     Arena& A = d->arena;
     A.plan(d->inpoel, nelem * 4);
     A.plan(d->xyz, npoin * 3);
-    A.plan(d->vol, npoin);
+    A.plan(d->ivol, npoin);
+    A.plan(d->cbrtv, npoin);
     A.plan(d->U, npoin * 5);
     A.plan(d->R, npoin * 5);
     A.plan(d->P, npoin * 10);
-    A.plan(d->Q, npoin * 10);
     A.plan(d->A, npoin * 5);
     A.plan(d->stage, npoin * 5);
-    A.plan(d->V, npoin * 4);
+    A.plan(d->V, f64 ? npoin * 8 : npoin * 4);  // [n][8] of the mode's precision
     A.plan(d->aoff, aoff.size());
     A.plan(d->aw, aw.size());
     A.plan(d->anbr, anbr.size());
     if (prm->precision == XG_FP32_FLUX) {
       A.plan(d->R32, npoin * 16);  // R and P records
       A.plan(d->A32, npoin * 8);
-      A.plan(d->U32, npoin * 5);
-      A.plan(d->lo32, npoin * 5);
-      A.plan(d->Q32, npoin * 10);
-      A.plan(d->geo32, nelem * 10);
+      A.plan(d->Q32, npoin * kC32);
+      A.plan(d->K32, npoin * kC32);
+      A.plan(d->geo32, nelem * kGeo);
     } else {
+      A.plan(d->Q, npoin * kC64);
+      A.plan(d->K, npoin * kC64);
+      A.plan(d->geo64, nelem * kGeo);
       A.plan(d->E, nelem * 4 * kRecD2 * 2);
       if (prm->fct) A.plan(d->L, nelem * 4 * kLimD2 * 2);
       A.plan(d->soff, soff.size());
       A.plan(d->sw, sw.size());
       A.plan(d->sslot, sslot.size());
     }
-    A.plan(d->isbc, npoin);
+    A.plan(d->bcof, npoin);
     A.plan(d->scal, 1);
     if (pass == 0) {
       cudaError_t e = A.reserve();
@@ -1278,7 +1380,10 @@ int xg_kozcg_setup(xg_ctx* c, const xg_kozcg_params* prm, int64_t npoin, const d
   cudaStream_t s = c->stream;
   XG_CUDA(c, cudaMemcpy(d->inpoel, ip.data(), ip.size() * 4, cudaMemcpyHostToDevice));
   XG_CUDA(c, cudaMemcpy(d->xyz, coord, npoin * 3 * 8, cudaMemcpyHostToDevice));
-  XG_CUDA(c, cudaMemcpy(d->vol, vol, npoin * 8, cudaMemcpyHostToDevice));
+  // through the staging buffer
+  XG_CUDA(c, cudaMemcpy(d->stage, vol, npoin * 8, cudaMemcpyHostToDevice));
+  k_node_factors<<<blocks_for(npoin, kBlock), kBlock, 0, s>>>(npoin, d->stage, d->ivol, d->cbrtv);
+  XG_CHECK_LAUNCH(c);
   XG_CUDA(c, cudaMemcpy(d->aoff, aoff.data(), aoff.size() * 4, cudaMemcpyHostToDevice));
   XG_CUDA(c, cudaMemcpy(d->aw, aw.data(), aw.size() * 4, cudaMemcpyHostToDevice));
   XG_CUDA(c, cudaMemcpy(d->anbr, anbr.data(), anbr.size() * 4, cudaMemcpyHostToDevice));
@@ -1288,12 +1393,14 @@ int xg_kozcg_setup(xg_ctx* c, const xg_kozcg_params* prm, int64_t npoin, const d
     XG_CUDA(c, cudaMemcpy(d->sslot, sslot.data(), sslot.size() * 4, cudaMemcpyHostToDevice));
   }
   XG_CUDA(c, cudaMemsetAsync(d->U, 0, npoin * 5 * 8, s));
-  XG_CUDA(c, cudaMemsetAsync(d->isbc, 0, npoin, s));
-  if (d->geo32) {
-    k_geo32<<<blocks_for(nelem, kBlock), kBlock, 0, s>>>(npoin, nelem, d->inpoel, d->xyz,
-                                                          d->geo32);
-    XG_CHECK_LAUNCH(c);
-  }
+  XG_CUDA(c, cudaMemsetAsync(d->bcof, 0xff, npoin * 4, s));  // -1
+  if (f64)
+    k_geo<double><<<blocks_for(nelem, kBlock), kBlock, 0, s>>>(npoin, nelem, d->inpoel, d->xyz,
+                                                               d->geo64);
+  else
+    k_geo<float><<<blocks_for(nelem, kBlock), kBlock, 0, s>>>(npoin, nelem, d->inpoel, d->xyz,
+                                                              d->geo32);
+  XG_CHECK_LAUNCH(c);
   KScalars k0{};  // every member zero
   double big = DBL_MAX;
   std::memcpy(&k0.dtmin, &big, sizeof(double));
@@ -1343,8 +1450,8 @@ int xg_kozcg_set_bc(xg_ctx* c, int64_t nsym, const uint64_t* symnodes, const dou
       for (int a = 0; a < 3; ++a) symn[j * 3 + a] = symnorms[k * 3 + a];
     }
   }
-  std::vector<uint8_t> isbc(n, 0);
-  for (auto p : ids) isbc[p] = 1;
+  std::vector<int32_t> bcof(n, -1);
+  for (int64_t i = 0; i < nbc; ++i) bcof[ids[i]] = static_cast<int32_t>(i);
   XG_CUDA(c, cudaStreamSynchronize(c->stream));
   d->bcarena.release();
   for (int pass = 0; pass < 2; ++pass) {
@@ -1366,7 +1473,7 @@ int xg_kozcg_set_bc(xg_ctx* c, int64_t nsym, const uint64_t* symnodes, const dou
   XG_CUDA(c, up(d->symn, symn.data(), symn.size() * 8));
   XG_CUDA(c, up(d->dirmask, dirmask, ndir * 5 * 4));
   XG_CUDA(c, up(d->dirval, dirvals, ndir * 5 * 8));
-  XG_CUDA(c, up(d->isbc, isbc.data(), n));
+  XG_CUDA(c, up(d->bcof, bcof.data(), n * 4));
   d->nbc = nbc;
   d->dt_valid = false;
   return XG_OK;
@@ -1418,12 +1525,13 @@ int xg_kozcg_rhs(xg_ctx* c, const double* U, double dt, double* R) {
   k_set_step<<<1, 1, 0, s>>>(d->scal, d->t, dt);  // the sources at the context's time
   XG_CHECK_LAUNCH(c);
   if (d->prm.precision == XG_FP32_FLUX) {
-    const KArrays<float> k = arrays32(d);
-    XG_CUDA(c, cudaMemsetAsync(k.R, 0, d->n * kRP * 4, s));
-    galerkin<float>(s, d, k, d->A, 0);
-    k_rec_to_soa<<<blocks_for(d->n * 5, kBlock), kBlock, 0, s>>>(d->n, k.R, d->R);
+    XG_CUDA(c, cudaMemsetAsync(d->R32, 0, d->n * kRP * 4, s));
+    galerkin<float>(c, d, d->A, 0);
+    k_rec_to_soa<<<blocks_for(d->n * 5, kBlock), kBlock, 0, s>>>(d->n, d->R32, d->R);
   } else {
-    galerkin<double>(s, d, arrays64(d), d->A, 0);
+    galerkin<double>(c, d, d->A, 0);
+    k_node_rhs64<<<blocks_for(d->n, kBlock), kBlock, 0, s>>>(d->n, d->soff, d->sw, d->sslot, d->E,
+                                                             d->R);
   }
   XG_CHECK_LAUNCH(c);
   k_soa_to_aos<<<blocks_for(d->n * 5, kBlock), kBlock, 0, s>>>(d->n, 5, d->R, d->stage);
@@ -1460,8 +1568,7 @@ int xg_kozcg_bc(xg_ctx* c) {
   KozCGDev* d = c->kozcg;
   if (!d) return fail(c, XG_ERR_STATE, "kozcg_bc before kozcg_setup");
   if (d->nbc) {
-    k_bc<<<blocks_for(d->nbc, kBlock), kBlock, 0, c->stream>>>(
-        d->n, kbc_of(d), d->prm.gamma, d->U, d->vol, 0, &d->scal->dtmin, nullptr, d->t);
+    k_bc<<<blocks_for(d->nbc, kBlock), kBlock, 0, c->stream>>>(d->n, kbc_of(d), d->U, d->t);
     XG_CHECK_LAUNCH(c);
   }
   rc = refresh_dt(c, d);
