@@ -23,9 +23,13 @@
 //                 dual-face normal and the viscous coefficient of the edge,
 //                 plus |d| / |x_a - x_b| for the pressure damping
 //   bnode, park   boundary-node list and [nb][9] domain sums between passes
-// Every edge term is evaluated in the edge's canonical orientation at both
-// ends, so the two ends see bit-identical values and each node owns its
-// writes (no atomics except the scalar CFL minimum).  A node's neighbours are
+// Each node owns its writes (no atomics except the scalar CFL minimum).  The
+// linear edge terms and the damp2 flux are evaluated from the node outwards
+// (they only change sign with the orientation); the damp4 reconstruction,
+// whose regularisation depends on it, in the edge's canonical orientation.
+// On GB300 an FP64 instruction holds an SM quarter's FP64 unit for 64 cycles,
+// so these passes are written to their FP64 operation count, and signs are
+// flipped on the bits.  A node's neighbours are
 // visited in increasing id, which for an unrenumbered mesh is the order in
 // which the reference's edge loop reaches the node.  Each node kernel runs
 // as a domain pass over all nodes and a pass over the boundary nodes that
@@ -47,6 +51,11 @@ namespace {
 constexpr int kSlice = 32;
 constexpr int32_t kPad = INT32_MIN;
 constexpr int kBlock = 256;
+// FP64 node passes run in small blocks: an SM's FP64 units take its blocks' work
+// in turn, so an SM with one large block more than the others holds them up
+// (and 20 blocks of 256 run a 17^3 system on 20 SMs: damp4 k_crhs 457 us).
+constexpr int kNode = 64;
+constexpr int kBL = 4;  // lanes per boundary node: they share its triangles
 }  // namespace
 
 // The four edge coefficients of an adjacency entry: d0, d1, d2 (dual-face
@@ -66,7 +75,7 @@ struct ChoCGDev {
   int32_t *bidx = nullptr, *bptr = nullptr, *bent = nullptr, *btri = nullptr;
   int32_t* bnode = nullptr;  // boundary index -> node
   double* park = nullptr;    // [nbn][9] domain sums of boundary nodes between passes
-  double *xyz = nullptr, *vol = nullptr;
+  double *xyz = nullptr, *ivol = nullptr, *cbrtv = nullptr;  // coordinates, 1/vol, cbrt(vol)
   double *u = nullptr, *u2 = nullptr, *un = nullptr, *pr = nullptr, *pgrad = nullptr,
          *vgrad = nullptr, *div = nullptr, *flx = nullptr, *stage = nullptr;
   unsigned long long* dtmin = nullptr;
@@ -127,23 +136,39 @@ struct ChoBnd {
 
 // Every node kernel runs as two passes.  The domain pass (one thread per
 // node) sums the edge terms; a boundary node parks that sum and returns.  The
-// boundary pass (one thread per boundary node) adds the boundary-triangle
-// terms in the reference's order and applies the epilogue.  Folded into the
+// boundary pass (kBL lanes per boundary node, lane l of them) adds the
+// boundary-triangle terms after it and applies the epilogue.  Folded into the
 // domain pass, the few boundary nodes of a warp held all 32 lanes for their
-// triangle loops.
-__device__ __forceinline__ bool node_of(bool bnd_pass, int64_t n, const ChoBnd& b, int64_t& p,
-                                        int32_t& bi) {
+// triangle loops; one lane per node was a serial chain of some 36-54 us at
+// any size.  Past the last node bi and p are -1; the boundary pass's lanes
+// all stay for the shuffles.
+__device__ __forceinline__ void node_of(bool bnd_pass, int64_t n, const ChoBnd& b, int64_t& p,
+                                        int32_t& bi, int& l) {
   const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  p = bi = -1;
+  l = 0;
   if (bnd_pass) {
-    if (t >= b.nb) return false;
-    bi = static_cast<int32_t>(t);
-    p = __ldg(b.bnode + t);
-  } else {
-    if (t >= n) return false;
+    l = static_cast<int>(t % kBL);
+    if (t / kBL < b.nb) {
+      bi = static_cast<int32_t>(t / kBL);
+      p = __ldg(b.bnode + bi);
+    }
+  } else if (t < n) {
     p = t;
-    bi = -1;
   }
-  return true;
+}
+// Adds the kBL lanes' values.
+template <int N>
+__device__ __forceinline__ void lane_add(double (&v)[N]) {
+#pragma unroll
+  for (int o = 1; o < kBL; o <<= 1)
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+}
+
+// v, or -v when neg, on the sign bit.
+__device__ __forceinline__ double flip(double v, bool neg) {
+  return __longlong_as_double(__double_as_longlong(v) ^ (neg ? (1ll << 63) : 0ll));
 }
 
 __device__ __forceinline__ Coef4 ldd4(const Coef4* p) {
@@ -152,10 +177,12 @@ __device__ __forceinline__ Coef4 ldd4(const Coef4* p) {
   return Coef4{a.x, a.y, b.x, b.y};
 }
 
-// Boundary-face normal / 6 of triangle t (tk::crossdiv(..., 6.0),
-// src/Base/Vector.hpp:68-77), the same expression at every vertex.
-__device__ __forceinline__ void tri_normal6(const ChoBnd& b, int64_t n, int32_t t, int32_t N[3],
-                                            double nn[3]) {
+// Boundary-face normal / 48 of triangle t (tk::crossdiv(..., 6.0),
+// src/Base/Vector.hpp:68-77, with the 1/8 of the vertex weights
+// (6 f_own + f_other + f_other)/8, Chorin.cpp:183-205, which wavg leaves as
+// (f_a + f_b + f_c) + 5 f_own).
+__device__ __forceinline__ void tri_normal48(const ChoBnd& b, int64_t n, int32_t t, int32_t N[3],
+                                             double nn[3]) {
   N[0] = __ldg(b.btri + 3 * t);
   N[1] = __ldg(b.btri + 3 * t + 1);
   N[2] = __ldg(b.btri + 3 * t + 2);
@@ -164,16 +191,13 @@ __device__ __forceinline__ void tri_normal6(const ChoBnd& b, int64_t n, int32_t 
   const double* z = b.xyz + 2 * n;
   const double bax = x[N[1]] - x[N[0]], bay = y[N[1]] - y[N[0]], baz = z[N[1]] - z[N[0]];
   const double cax = x[N[2]] - x[N[0]], cay = y[N[2]] - y[N[0]], caz = z[N[2]] - z[N[0]];
-  nn[0] = (bay * caz - cay * baz) / 6.0;
-  nn[1] = (baz * cax - caz * bax) / 6.0;
-  nn[2] = (bax * cay - cax * bay) / 6.0;
+  const double k = 1.0 / 48.0;
+  nn[0] = (bay * caz - cay * baz) * k;
+  nn[1] = (baz * cax - caz * bax) * k;
+  nn[2] = (bax * cay - cax * bay) * k;
 }
-
-// (6 f_pos + f_other + f_other)/8 of a triangle's three vertex values, for
-// the vertex at pos (Chorin.cpp:183-205 and the same weights elsewhere).
 __device__ __forceinline__ double wavg(int pos, double a, double b, double c) {
-  return pos == 0 ? (6.0 * a + b + c) / 8.0
-                  : (pos == 1 ? (a + 6.0 * b + c) / 8.0 : (a + b + 6.0 * c) / 8.0);
+  return (a + b + c) + 5.0 * (pos == 0 ? a : (pos == 1 ? b : c));
 }
 
 __device__ __forceinline__ void block_min(double v, unsigned long long* dst) {
@@ -247,38 +271,34 @@ enum GradOut { GRAD_RAW = 0, GRAD_DIVIDE = 1, GRAD_PROJECT = 2 };
 // ChoCG::psolved (src/Inciter/ChoCG.cpp:1204-1216): u -= dt G/vol, and with
 // addp the pressure update pr += increment (src/Inciter/ChoCG.cpp:1246-1250).
 template <int NC, int MODE, bool BND>
-__global__ void __launch_bounds__(kBlock) k_cgrad(int64_t n, ChoAdj adj, const double* U,
-                                                   ChoBnd bnd, const double* __restrict__ vol,
-                                                   double* __restrict__ G, double dt, int addp,
-                                                   double* u, double* pr) {
+__global__ void __launch_bounds__(kNode) k_cgrad(int64_t n, ChoAdj adj, const double* U,
+                                                  ChoBnd bnd, const double* __restrict__ ivol,
+                                                  double* __restrict__ G, double dt, int addp,
+                                                  double* u, double* pr) {
   int64_t p;
   int32_t bi;
-  if (!node_of(BND, n, bnd, p, bi)) return;
-  double up[NC];
-#pragma unroll
-  for (int i = 0; i < NC; ++i) up[i] = U[i * n + p];
+  int l;
+  node_of(BND, n, bnd, p, bi, l);
   double g[3 * NC];
-  if (!BND) {
 #pragma unroll
-    for (int i = 0; i < 3 * NC; ++i) g[i] = 0.0;
+  for (int i = 0; i < 3 * NC; ++i) g[i] = 0.0;
+  if (!BND) {
+    if (p < 0) return;
+    double up[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) up[i] = U[i * n + p];
     const int lane = static_cast<int>(p & (kSlice - 1));
     const int64_t s = p >> 5;
     const int32_t off = __ldg(adj.soff + s), w = __ldg(adj.swidth + s);
     for_adj<NC == 1 ? 16 : 8>(adj, off, w, lane, [&](int32_t e, int32_t q, bool first) {
       const Coef4 d = ldd4(adj.dd + e);
+      const double dx = flip(d.x, first), dy = flip(d.y, first), dz = flip(d.z, first);
 #pragma unroll
       for (int i = 0; i < NC; ++i) {
         const double sum = U[i * n + q] + up[i];
-        const double f0 = d.x * sum, f1 = d.y * sum, f2 = d.z * sum;
-        if (first) {
-          g[i * 3 + 0] -= f0;
-          g[i * 3 + 1] -= f1;
-          g[i * 3 + 2] -= f2;
-        } else {
-          g[i * 3 + 0] += f0;
-          g[i * 3 + 1] += f1;
-          g[i * 3 + 2] += f2;
-        }
+        g[i * 3 + 0] += dx * sum;
+        g[i * 3 + 1] += dy * sum;
+        g[i * 3 + 2] += dz * sum;
       }
     });
     const int32_t b = __ldg(bnd.bidx + p);
@@ -288,34 +308,40 @@ __global__ void __launch_bounds__(kBlock) k_cgrad(int64_t n, ChoAdj adj, const d
       return;
     }
   } else {
+    if (bi >= 0) {
+      if (l == 0) {
 #pragma unroll
-    for (int i = 0; i < 3 * NC; ++i) g[i] = bnd.park[bi * 9 + i];
-    for (int32_t j = __ldg(bnd.bptr + bi); j < __ldg(bnd.bptr + bi + 1); ++j) {
-      const int32_t ent = __ldg(bnd.bent + j);
-      const int pos = ent & 3;
-      int32_t N[3];
-      double nn[3];
-      tri_normal6(bnd, n, ent >> 2, N, nn);
+        for (int i = 0; i < 3 * NC; ++i) g[i] = bnd.park[bi * 9 + i];
+      }
+      for (int32_t j = __ldg(bnd.bptr + bi) + l; j < __ldg(bnd.bptr + bi + 1); j += kBL) {
+        const int32_t ent = __ldg(bnd.bent + j);
+        const int pos = ent & 3;
+        int32_t N[3];
+        double nn[3];
+        tri_normal48(bnd, n, ent >> 2, N, nn);
 #pragma unroll
-      for (int i = 0; i < NC; ++i) {
-        const double f = wavg(pos, U[i * n + N[0]], U[i * n + N[1]], U[i * n + N[2]]);
+        for (int i = 0; i < NC; ++i) {
+          const double f = wavg(pos, U[i * n + N[0]], U[i * n + N[1]], U[i * n + N[2]]);
 #pragma unroll
-        for (int jj = 0; jj < 3; ++jj) g[i * 3 + jj] += f * nn[jj];
+          for (int jj = 0; jj < 3; ++jj) g[i * 3 + jj] += f * nn[jj];
+        }
       }
     }
+    lane_add(g);
+    if (bi < 0 || l != 0) return;
   }
   if (MODE == GRAD_RAW) {
 #pragma unroll
     for (int i = 0; i < 3 * NC; ++i) G[i * n + p] = g[i];
   } else if (MODE == GRAD_DIVIDE) {
-    const double v = vol[p];
+    const double iv = ivol[p];
 #pragma unroll
-    for (int i = 0; i < 3 * NC; ++i) G[i * n + p] = g[i] / v;
+    for (int i = 0; i < 3 * NC; ++i) G[i * n + p] = g[i] * iv;
   } else {
-    const double v = vol[p];
+    const double iv = ivol[p] * dt;
 #pragma unroll
-    for (int jj = 0; jj < 3; ++jj) u[jj * n + p] -= dt * (g[jj] / v);
-    if (addp) pr[p] += up[0];
+    for (int jj = 0; jj < 3; ++jj) u[jj * n + p] -= g[jj] * iv;
+    if (addp) pr[p] += U[p];
   }
 }
 
@@ -323,111 +349,125 @@ __global__ void __launch_bounds__(kBlock) k_cgrad(int64_t n, ChoAdj adj, const d
 // 4th-order pressure damping when stab, optionally divided by dt
 // (ChoCG::pinit, src/Inciter/ChoCG.cpp:1039).
 template <bool BND>
-__global__ void __launch_bounds__(kBlock) k_cdiv(int64_t n, ChoAdj adj, const double* U,
-                                                  const double* __restrict__ P,
-                                                  const double* __restrict__ PG, ChoBnd bnd,
-                                                  double dt, int stab, int bydt,
-                                                  double* __restrict__ D) {
+__global__ void __launch_bounds__(kNode) k_cdiv(int64_t n, ChoAdj adj, const double* U,
+                                                 const double* __restrict__ P,
+                                                 const double* __restrict__ PG, ChoBnd bnd,
+                                                 double dt, int stab, int bydt,
+                                                 double* __restrict__ D) {
   int64_t p;
   int32_t bi;
-  if (!node_of(BND, n, bnd, p, bi)) return;
-  double acc = 0.0;
+  int l;
+  node_of(BND, n, bnd, p, bi, l);
+  double acc[1] = {0.0};
   if (!BND) {
+    if (p < 0) return;
     const int lane = static_cast<int>(p & (kSlice - 1));
     const int64_t s = p >> 5;
     const int32_t off = __ldg(adj.soff + s), w = __ldg(adj.swidth + s);
     const double* x = bnd.xyz;
     const double* y = bnd.xyz + n;
     const double* z = bnd.xyz + 2 * n;
+    const double up = U[p], vp = U[n + p], wp = U[2 * n + p];
+    double xp = 0.0, yp = 0.0, zp = 0.0, pp = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+    if (stab) {
+      xp = x[p], yp = y[p], zp = z[p];
+      pp = P[p];
+      gx = PG[p], gy = PG[n + p], gz = PG[2 * n + p];
+    }
     for_adj<8>(adj, off, w, lane, [&](int32_t e, int32_t q, bool first) {
       const Coef4 d = ldd4(adj.dd + e);
-      const int64_t a = first ? p : q, b = first ? q : p;  // canonical ends
-      double f = d.x * (U[a] + U[b]) + d.y * (U[n + a] + U[n + b]) +
-                 d.z * (U[2 * n + a] + U[2 * n + b]);
+      acc[0] += flip(d.x, first) * (up + U[q]) + flip(d.y, first) * (vp + U[n + q]) +
+                flip(d.z, first) * (wp + U[2 * n + q]);
       if (stab) {
-        // |d| / |x_a - x_b| is geometric: formed once at setup (two FP64
+        // |d| / |x_p - x_q| is geometric: formed once at setup (two FP64
         // square roots and a division per edge and call are expensive on
         // GB300's FP64 pipe)
-        const double dx = x[a] - x[b], dy = y[a] - y[b], dz = z[a] - z[b];
-        const double p2 = P[b] - P[a];
-        const double dpx = PG[a] + PG[b], dpy = PG[n + a] + PG[n + b],
-                     dpz = PG[2 * n + a] + PG[2 * n + b];
-        const double p4 = 0.5 * (dx * dpx + dy * dpy + dz * dpz);
-        f += __ldg(adj.sdl + e) * dt * (p2 + p4);
+        const double p4 = (xp - x[q]) * (gx + PG[q]) + (yp - y[q]) * (gy + PG[n + q]) +
+                          (zp - z[q]) * (gz + PG[2 * n + q]);
+        acc[0] -= (__ldg(adj.sdl + e) * dt) * ((P[q] - pp) + 0.5 * p4);
       }
-      acc = first ? acc - f : acc + f;
     });
     const int32_t b = __ldg(bnd.bidx + p);
     if (b >= 0) {
-      bnd.park[b * 9] = acc;
+      bnd.park[b * 9] = acc[0];
       return;
     }
   } else {
-    acc = bnd.park[bi * 9];
-    for (int32_t j = __ldg(bnd.bptr + bi); j < __ldg(bnd.bptr + bi + 1); ++j) {
-      const int32_t ent = __ldg(bnd.bent + j);
-      const int pos = ent & 3;
-      int32_t N[3];
-      double nn[3];
-      tri_normal6(bnd, n, ent >> 2, N, nn);
-      const double ux = wavg(pos, U[N[0]], U[N[1]], U[N[2]]);
-      const double uy = wavg(pos, U[n + N[0]], U[n + N[1]], U[n + N[2]]);
-      const double uz = wavg(pos, U[2 * n + N[0]], U[2 * n + N[1]], U[2 * n + N[2]]);
-      acc += ux * nn[0] + uy * nn[1] + uz * nn[2];
+    if (bi >= 0) {
+      if (l == 0) acc[0] = bnd.park[bi * 9];
+      for (int32_t j = __ldg(bnd.bptr + bi) + l; j < __ldg(bnd.bptr + bi + 1); j += kBL) {
+        const int32_t ent = __ldg(bnd.bent + j);
+        const int pos = ent & 3;
+        int32_t N[3];
+        double nn[3];
+        tri_normal48(bnd, n, ent >> 2, N, nn);
+        acc[0] += wavg(pos, U[N[0]], U[N[1]], U[N[2]]) * nn[0] +
+                  wavg(pos, U[n + N[0]], U[n + N[1]], U[n + N[2]]) * nn[1] +
+                  wavg(pos, U[2 * n + N[0]], U[2 * n + N[1]], U[2 * n + N[2]]) * nn[2];
+      }
+    }
+    lane_add(acc);
+    if (bi < 0 || l != 0) return;
+  }
+  D[p] = bydt ? acc[0] / dt : acc[0];
+}
+
+// Momentum flux tensor of chorin::flux at every node (Chorin.cpp:451-507):
+// T_ij = mu (G_ij + G_ji - 2/3 d_ij tr G) - u_i u_j, symmetric, stored as
+// xx, yy, zz, xy, xz, yz.  An edge's flux is the sum of its ends' tensors, so
+// forming them per node leaves 15 operations an edge end for about 150.
+__global__ void __launch_bounds__(kNode) k_mflux(int64_t n, const double* __restrict__ U,
+                                                  const double* __restrict__ G, double mu,
+                                                  double* __restrict__ T) {
+  const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (p >= n) return;
+  const double u[3] = {U[p], U[n + p], U[2 * n + p]};
+  constexpr int a[6] = {0, 1, 2, 0, 0, 1}, b[6] = {0, 1, 2, 1, 2, 2};
+  double vis[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  if (!(mu < DBL_EPSILON)) {
+    const double tr = G[0 * n + p] + G[4 * n + p] + G[8 * n + p];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      vis[k] = G[(a[k] * 3 + b[k]) * n + p] + G[(b[k] * 3 + a[k]) * n + p];
+      if (k < 3) vis[k] -= 2.0 / 3.0 * tr;
     }
   }
-  D[p] = bydt ? acc / dt : acc;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) T[k * n + p] = mu * vis[k] - u[a[k]] * u[b[k]];
 }
 
-// Momentum flux of tensor component (i,j) over an edge and in a point
-// (Chorin.cpp:451-507).  The edge form is called with the canonical second
-// end first, as the reference's loops do.
-__device__ __forceinline__ double mflux_e(const double* U, const double* G, int64_t n, int i,
-                                          int j, int64_t p, int64_t q, double mu) {
-  const double inv = U[i * n + p] * U[j * n + p] + U[i * n + q] * U[j * n + q];
-  if (mu < DBL_EPSILON) return -inv;
-  double vis = G[(i * 3 + j) * n + p] + G[(j * 3 + i) * n + p] + G[(i * 3 + j) * n + q] +
-               G[(j * 3 + i) * n + q];
-  if (i == j)
-    vis -= 2.0 / 3.0 * (G[0 * n + p] + G[4 * n + p] + G[8 * n + p] + G[0 * n + q] +
-                        G[4 * n + q] + G[8 * n + q]);
-  return mu * vis - inv;
-}
-__device__ __forceinline__ double mflux_p(const double* U, const double* G, int64_t n, int i,
-                                          int j, int64_t p, double mu) {
-  const double inv = U[i * n + p] * U[j * n + p];
-  if (mu < DBL_EPSILON) return -inv;
-  double vis = G[(i * 3 + j) * n + p] + G[(j * 3 + i) * n + p];
-  if (i == j) vis -= 2.0 / 3.0 * (G[0 * n + p] + G[4 * n + p] + G[8 * n + p]);
-  return mu * vis - inv;
-}
-
-// chorin::flux (Chorin.cpp:509-638): F_i = d[s_ij - u_i u_j]/dx_j, raw or
-// divided by the volume (ChoCG::div at start-up, src/Inciter/ChoCG.cpp:877).
+// chorin::flux (Chorin.cpp:509-638): F_i = d[s_ij - u_i u_j]/dx_j from the node
+// tensors T, raw or divided by the volume (ChoCG::div at start-up,
+// src/Inciter/ChoCG.cpp:877).
 template <bool BND>
-__global__ void __launch_bounds__(kBlock) k_cflux(int64_t n, ChoAdj adj, const double* U,
-                                                   const double* G, ChoBnd bnd,
-                                                   const double* __restrict__ vol, double mu,
-                                                   int divide, double* __restrict__ F) {
+__global__ void __launch_bounds__(kNode) k_cflux(int64_t n, ChoAdj adj,
+                                                  const double* __restrict__ T, ChoBnd bnd,
+                                                  const double* __restrict__ ivol, int divide,
+                                                  double* __restrict__ F) {
   int64_t p;
   int32_t bi;
-  if (!node_of(BND, n, bnd, p, bi)) return;
+  int l;
+  node_of(BND, n, bnd, p, bi, l);
   double acc[3] = {0.0, 0.0, 0.0};
+  auto add = [&](const double t[6], double dx, double dy, double dz) {
+    acc[0] += dx * t[0] + dy * t[3] + dz * t[4];
+    acc[1] += dx * t[3] + dy * t[1] + dz * t[5];
+    acc[2] += dx * t[4] + dy * t[5] + dz * t[2];
+  };
   if (!BND) {
+    if (p < 0) return;
+    double tp[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) tp[k] = T[k * n + p];
     const int lane = static_cast<int>(p & (kSlice - 1));
     const int64_t s = p >> 5;
     const int32_t off = __ldg(adj.soff + s), w = __ldg(adj.swidth + s);
     for_adj<4>(adj, off, w, lane, [&](int32_t e, int32_t q, bool first) {
       const Coef4 d = ldd4(adj.dd + e);
-      const int64_t a = first ? p : q, b = first ? q : p;
-      const double dj[3] = {d.x, d.y, d.z};
+      double t[6];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const double f = dj[j] * mflux_e(U, G, n, i, j, b, a, mu);
-          acc[i] = first ? acc[i] - f : acc[i] + f;
-        }
+      for (int k = 0; k < 6; ++k) t[k] = tp[k] + __ldg(T + k * n + q);
+      add(t, flip(d.x, first), flip(d.y, first), flip(d.z, first));
     });
     const int32_t b = __ldg(bnd.bidx + p);
     if (b >= 0) {
@@ -436,28 +476,29 @@ __global__ void __launch_bounds__(kBlock) k_cflux(int64_t n, ChoAdj adj, const d
       return;
     }
   } else {
+    if (bi >= 0) {
+      if (l == 0) {
 #pragma unroll
-    for (int i = 0; i < 3; ++i) acc[i] = bnd.park[bi * 9 + i];
-    for (int32_t jb = __ldg(bnd.bptr + bi); jb < __ldg(bnd.bptr + bi + 1); ++jb) {
-      const int32_t ent = __ldg(bnd.bent + jb);
-      const int pos = ent & 3;
-      int32_t N[3];
-      double nn[3];
-      tri_normal6(bnd, n, ent >> 2, N, nn);
+        for (int i = 0; i < 3; ++i) acc[i] = bnd.park[bi * 9 + i];
+      }
+      for (int32_t j = __ldg(bnd.bptr + bi) + l; j < __ldg(bnd.bptr + bi + 1); j += kBL) {
+        const int32_t ent = __ldg(bnd.bent + j);
+        const int pos = ent & 3;
+        int32_t N[3];
+        double nn[3], t[6];
+        tri_normal48(bnd, n, ent >> 2, N, nn);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        double fv[3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-          fv[j] = wavg(pos, mflux_p(U, G, n, i, j, N[0], mu), mflux_p(U, G, n, i, j, N[1], mu),
-                       mflux_p(U, G, n, i, j, N[2], mu));
-        acc[i] += fv[0] * nn[0] + fv[1] * nn[1] + fv[2] * nn[2];
+        for (int k = 0; k < 6; ++k)
+          t[k] = wavg(pos, T[k * n + N[0]], T[k * n + N[1]], T[k * n + N[2]]);
+        add(t, nn[0], nn[1], nn[2]);
       }
     }
+    lane_add(acc);
+    if (bi < 0 || l != 0) return;
   }
-  const double v = divide ? vol[p] : 1.0;
+  const double iv = divide ? ivol[p] : 1.0;
 #pragma unroll
-  for (int i = 0; i < 3; ++i) F[i * n + p] = divide ? acc[i] / v : acc[i];
+  for (int i = 0; i < 3; ++i) F[i * n + p] = divide ? acc[i] * iv : acc[i];
 }
 
 struct AdvPrm {
@@ -465,83 +506,142 @@ struct AdvPrm {
   int stab, stab2;
 };
 
-// adv_damp2 / adv_damp4 edge flux of the three velocity components on the
-// canonical edge a -> b (Chorin.cpp:640-829).
-template <bool DAMP4>
-__device__ __forceinline__ void adv_edge(const double* U, const double* G, const double* P,
-                                         const double* xyz, int64_t n, Coef4 d, int64_t a,
-                                         int64_t b, const AdvPrm& ap, double f[3]) {
-  double uL[3] = {U[a], U[n + a], U[2 * n + a]};
-  double uR[3] = {U[b], U[n + b], U[2 * n + b]};
-  if (DAMP4) {
-    const double eps = 1.0e-9, k = 1.0 / 3.0;
-    const double dx = xyz[b] - xyz[a], dy = xyz[n + b] - xyz[n + a],
-                 dz = xyz[2 * n + b] - xyz[2 * n + a];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const double g1 = G[(c * 3 + 0) * n + a] * dx + G[(c * 3 + 1) * n + a] * dy +
-                        G[(c * 3 + 2) * n + a] * dz;
-      const double g2 = G[(c * 3 + 0) * n + b] * dx + G[(c * 3 + 1) * n + b] * dy +
-                        G[(c * 3 + 2) * n + b] * dz;
-      const double delta2 = uR[c] - uL[c];
-      const double delta1 = 2.0 * g1 - delta2;
-      const double delta3 = 2.0 * g2 - delta2;
-      const double rL = (delta2 + eps) / (delta1 + eps);
-      const double rR = (delta2 + eps) / (delta3 + eps);
-      const double rLinv = (delta1 + eps) / (delta2 + eps);
-      const double rRinv = (delta3 + eps) / (delta2 + eps);
-      const double phiL = (fabs(rL) + rL) / (fabs(rL) + 1.0);
-      const double phiR = (fabs(rR) + rR) / (fabs(rR) + 1.0);
-      const double phiLi = (fabs(rLinv) + rLinv) / (fabs(rLinv) + 1.0);
-      const double phiRi = (fabs(rRinv) + rRinv) / (fabs(rRinv) + 1.0);
-      uL[c] += 0.25 * (delta1 * (1.0 - k) * phiL + delta2 * (1.0 + k) * phiLi);
-      uR[c] -= 0.25 * (delta3 * (1.0 - k) * phiR + delta2 * (1.0 + k) * phiRi);
-    }
-  }
-  const double nx = d.x, ny = d.y, nz = d.z;
-  const double vnL = uL[0] * nx + uL[1] * ny + uL[2] * nz;
-  const double vnR = uR[0] * nx + uR[1] * ny + uR[2] * nz;
-  double aw = 0.0;
-  if (ap.stab) aw = fabs(vnL + vnR) / 2.0;
-  if (ap.stab2) aw += ap.stab2coef * fmax(fabs(vnL), fabs(vnR));
-  const double v = d.w * ap.mu;
-  const double pf = P[a] + P[b];
-  const double nv[3] = {nx, ny, nz};
+// van Leer limited reconstruction of the three velocity components on the
+// canonical edge a -> b (Chorin.cpp:711-829): uL, uR the ends' values on entry,
+// the edge states on return.  With a = delta2 + eps, b = delta1 + eps of one
+// sign s, 0.25 ((1-k) delta1 phi(a/b) + (1+k) delta2 phi(b/a)) is, exactly,
+// (a b - s (eps/2) ((1-k)|a| + (1+k)|b|)) / (a + b), and 0 for a b <= 0.  The six
+// quotients come from one division (batch inversion) where the reference
+// takes eight divisions a component; a product of denominators outside
+// [1e-290, 1e290] falls back to six.
+__device__ __forceinline__ void reconstruct(const double g1[3], const double g2[3], double uL[3],
+                                            double uR[3]) {
+  const double eps = 1.0e-9, k = 1.0 / 3.0, h = 0.5e-9;
+  double num[6], den[6], pre[6], q[6];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    if (DAMP4)
-      f[c] = uL[c] * vnL + uR[c] * vnR + pf * nv[c] + aw * (uR[c] - uL[c]) -
-             v * (U[c * n + b] - U[c * n + a]);
-    else
-      f[c] = uL[c] * vnL + uR[c] * vnR + pf * nv[c] + (aw - v) * (uR[c] - uL[c]);
+    const double d2 = uR[c] - uL[c];
+    const double a = d2 + eps, b = (2.0 * g1[c] - d2) + eps, e = (2.0 * g2[c] - d2) + eps;
+    const double pl = a * b, pr = a * e;
+    const double sh = copysign(h, a), ka = (1.0 - k) * fabs(a);
+    const bool ol = __double_as_longlong(pl) > 0, orr = __double_as_longlong(pr) > 0;
+    num[2 * c] = ol ? pl - sh * (ka + (1.0 + k) * fabs(b)) : 0.0;
+    num[2 * c + 1] = orr ? pr - sh * (ka + (1.0 + k) * fabs(e)) : 0.0;
+    den[2 * c] = ol ? a + b : 1.0;
+    den[2 * c + 1] = orr ? a + e : 1.0;
+  }
+  pre[0] = den[0];
+#pragma unroll
+  for (int m = 1; m < 6; ++m) pre[m] = pre[m - 1] * den[m];
+  const double ap = fabs(pre[5]);
+  if (ap > 1e-290 && ap < 1e290) {
+    double inv = 1.0 / pre[5];
+#pragma unroll
+    for (int m = 5; m > 0; --m) {
+      q[m] = inv * pre[m - 1];
+      inv *= den[m];
+    }
+    q[0] = inv;
+  } else {
+#pragma unroll
+    for (int m = 0; m < 6; ++m) q[m] = 1.0 / den[m];
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    uL[c] += num[2 * c] * q[2 * c];
+    uR[c] -= num[2 * c + 1] * q[2 * c + 1];
   }
 }
 
 // chorin::rhs (Chorin.cpp:831-1044) at every node, fused with the explicit
 // stage update of ChoCG::solve (src/Inciter/ChoCG.cpp:1550-1566):
 // u_out = un - dtk R / vol, where un is this stage's input at stage 0.
-// With dtk == 0 and a null u_out only R is written (drop-in).
+// With dtk == 0 and a null u_out only R is written (drop-in).  The edge flux
+// (adv_damp2 / adv_damp4, Chorin.cpp:640-829) is symmetric in its ends but for
+// the sign of d and of the velocity difference: from node p outwards, with d'
+// = -d at the canonical first end and d at the second, the node receives
+// u_p vn_p + u_q vn_q + (P_p + P_q) d' - (aw - v)(u_q - u_p), vn = u.d'.
 template <bool DAMP4, bool BND>
-__global__ void __launch_bounds__(kBlock) k_crhs(int64_t n, ChoAdj adj, const double* U,
-                                                  const double* G, const double* P, ChoBnd bnd,
-                                                  AdvPrm ap, const double* __restrict__ vol,
-                                                  double dtk, int stage0, double* un,
-                                                  double* __restrict__ uout,
-                                                  double* __restrict__ R) {
+__global__ void __launch_bounds__(kNode) k_crhs(int64_t n, ChoAdj adj, const double* U,
+                                                 const double* G, const double* P, ChoBnd bnd,
+                                                 AdvPrm ap, const double* __restrict__ ivol,
+                                                 double dtk, int stage0, double* un,
+                                                 double* __restrict__ uout,
+                                                 double* __restrict__ R) {
   int64_t p;
   int32_t bi;
-  if (!node_of(BND, n, bnd, p, bi)) return;
+  int l;
+  node_of(BND, n, bnd, p, bi, l);
   double acc[3] = {0.0, 0.0, 0.0};
   if (!BND) {
+    if (p < 0) return;
     const int lane = static_cast<int>(p & (kSlice - 1));
     const int64_t s = p >> 5;
     const int32_t off = __ldg(adj.soff + s), w = __ldg(adj.swidth + s);
+    const double* xyz = bnd.xyz;
+    double u0[3], x0[3], g0[DAMP4 ? 9 : 1];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) u0[c] = U[c * n + p];
+    const double p0 = P[p];
+    if (DAMP4) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) x0[c] = xyz[c * n + p];
+#pragma unroll
+      for (int c = 0; c < (DAMP4 ? 9 : 1); ++c) g0[c] = G[c * n + p];
+    }
     for_adj<DAMP4 ? 4 : 8>(adj, off, w, lane, [&](int32_t e, int32_t q, bool first) {
       const Coef4 d = ldd4(adj.dd + e);
-      double f[3];
-      adv_edge<DAMP4>(U, G, P, bnd.xyz, n, d, first ? p : q, first ? q : p, ap, f);
+      const double dx = flip(d.x, first), dy = flip(d.y, first), dz = flip(d.z, first);
+      double uq[3], du[3], a[3], b[3];  // a, b: the edge states at p and at q
 #pragma unroll
-      for (int c = 0; c < 3; ++c) acc[c] = first ? acc[c] - f[c] : acc[c] + f[c];
+      for (int c = 0; c < 3; ++c) {
+        uq[c] = U[c * n + q];
+        du[c] = uq[c] - u0[c];
+        a[c] = u0[c];
+        b[c] = uq[c];
+      }
+      if constexpr (DAMP4) {
+        const double ex = xyz[q] - x0[0], ey = xyz[n + q] - x0[1], ez = xyz[2 * n + q] - x0[2];
+        double gp[3], gq[3];  // G.(x_q - x_p) at p and at q
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          gp[c] = g0[c * 3] * ex + g0[c * 3 + 1] * ey + g0[c * 3 + 2] * ez;
+          gq[c] = G[(c * 3) * n + q] * ex + G[(c * 3 + 1) * n + q] * ey +
+                  G[(c * 3 + 2) * n + q] * ez;
+        }
+        // in the canonical orientation: left the first end, and the
+        // projections change sign with the edge vector
+        double uL[3], uR[3], g1[3], g2[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          uL[c] = first ? a[c] : b[c];
+          uR[c] = first ? b[c] : a[c];
+          g1[c] = first ? gp[c] : flip(gq[c], true);
+          g2[c] = first ? gq[c] : flip(gp[c], true);
+        }
+        reconstruct(g1, g2, uL, uR);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          a[c] = first ? uL[c] : uR[c];
+          b[c] = first ? uR[c] : uL[c];
+        }
+      }
+      const double va = a[0] * dx + a[1] * dy + a[2] * dz;
+      const double vb = b[0] * dx + b[1] * dy + b[2] * dz;
+      double aw = 0.0;
+      if (ap.stab) aw = 0.5 * fabs(va + vb);
+      if (ap.stab2) aw += ap.stab2coef * fmax(fabs(va), fabs(vb));
+      const double v = d.w * ap.mu;
+      const double pf = p0 + P[q];
+      const double dd[3] = {dx, dy, dz};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        acc[c] += a[c] * va + b[c] * vb + pf * dd[c];
+        if (DAMP4)
+          acc[c] -= aw * (b[c] - a[c]) - v * du[c];
+        else
+          acc[c] -= (aw - v) * du[c];
+      }
     });
     const int32_t b = __ldg(bnd.bidx + p);
     if (b >= 0) {
@@ -550,33 +650,37 @@ __global__ void __launch_bounds__(kBlock) k_crhs(int64_t n, ChoAdj adj, const do
       return;
     }
   } else {
+    if (bi >= 0) {
+      if (l == 0) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) acc[c] = bnd.park[bi * 9 + c];
-    for (int32_t j = __ldg(bnd.bptr + bi); j < __ldg(bnd.bptr + bi + 1); ++j) {
-      const int32_t ent = __ldg(bnd.bent + j);
-      const int pos = ent & 3;
-      int32_t N[3];
-      double nn[3];
-      tri_normal6(bnd, n, ent >> 2, N, nn);
-      double fl[3][3];
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const double uu = U[N[a]], vv = U[n + N[a]], ww = U[2 * n + N[a]], pp = P[N[a]];
-        const double vn = nn[0] * uu + nn[1] * vv + nn[2] * ww;
-        fl[0][a] = uu * vn + pp * nn[0];
-        fl[1][a] = vv * vn + pp * nn[1];
-        fl[2][a] = ww * vn + pp * nn[2];
+        for (int c = 0; c < 3; ++c) acc[c] = bnd.park[bi * 9 + c];
       }
+      for (int32_t j = __ldg(bnd.bptr + bi) + l; j < __ldg(bnd.bptr + bi + 1); j += kBL) {
+        const int32_t ent = __ldg(bnd.bent + j);
+        const int pos = ent & 3;
+        int32_t N[3];
+        double nn[3];
+        tri_normal48(bnd, n, ent >> 2, N, nn);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) acc[c] += wavg(pos, fl[c][0], fl[c][1], fl[c][2]);
+        for (int a = 0; a < 3; ++a) {
+          const double uu = U[N[a]], vv = U[n + N[a]], ww = U[2 * n + N[a]];
+          const double wt = pos == a ? 6.0 : 1.0, pw = wt * P[N[a]];
+          const double vn = wt * (nn[0] * uu + nn[1] * vv + nn[2] * ww);
+          acc[0] += uu * vn + pw * nn[0];
+          acc[1] += vv * vn + pw * nn[1];
+          acc[2] += ww * vn + pw * nn[2];
+        }
+      }
     }
+    lane_add(acc);
+    if (bi < 0 || l != 0) return;
   }
   if (R) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) R[c * n + p] = acc[c];
   }
   if (uout) {
-    const double v = vol[p];
+    const double f = dtk * ivol[p];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       double u0;
@@ -586,7 +690,7 @@ __global__ void __launch_bounds__(kBlock) k_crhs(int64_t n, ChoAdj adj, const do
       } else {
         u0 = un[c * n + p];
       }
-      uout[c * n + p] = u0 - dtk * acc[c] / v;
+      uout[c * n + p] = u0 - f * acc[c];
     }
   }
 }
@@ -626,18 +730,27 @@ __global__ void k_cbc(int64_t n, int64_t nbc, const int32_t* __restrict__ node,
 // ChoCG::dt (src/Inciter/ChoCG.cpp:1356-1412): min over nodes of
 // cbrt(V)/max(|u|, 1e-8) and, with viscosity, V^(2/3)/mu.
 __global__ void __launch_bounds__(kBlock) k_cdt(int64_t n, const double* __restrict__ U,
-                                                 const double* __restrict__ vol, double mu,
+                                                 const double* __restrict__ cbrtv, double mu,
                                                  unsigned long long* dtmin) {
   const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   double m = DBL_MAX;
   if (p < n) {
     const double u = U[p], v = U[n + p], w = U[2 * n + p];
     const double vel = sqrt(u * u + v * v + w * w);
-    const double L = cbrt(vol[p]);
+    const double L = cbrtv[p];
     m = fmin(m, L / fmax(vel, 1.0e-8));
     if (mu > DBL_EPSILON) m = fmin(m, L * L / mu);
   }
   block_min(m, dtmin);
+}
+
+// 1/vol and cbrt(vol).
+__global__ void k_node_factors(int64_t n, const double* __restrict__ vol,
+                               double* __restrict__ ivol, double* __restrict__ cbrtv) {
+  const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (p >= n) return;
+  ivol[p] = 1.0 / vol[p];
+  cbrtv[p] = cbrt(vol[p]);
 }
 
 __global__ void k_aos_soa(int64_t n, int nc, const double* __restrict__ a, double* __restrict__ s) {
@@ -666,8 +779,8 @@ ChoBnd bnd_of(ChoCGDev* d) {
 // boundary pass over the boundary nodes), the same arguments to each.
 template <auto KD, auto KB, class... A>
 void two_pass(cudaStream_t s, int64_t n, int64_t nb, A... args) {
-  KD<<<blocks_for(n, kBlock), kBlock, 0, s>>>(args...);
-  if (nb > 0) KB<<<blocks_for(nb, kBlock), kBlock, 0, s>>>(args...);
+  KD<<<blocks_for(n, kNode), kNode, 0, s>>>(args...);
+  if (nb > 0) KB<<<blocks_for(nb * kBL, kNode), kNode, 0, s>>>(args...);
 }
 AdvPrm adv_of(ChoCGDev* d) {
   return AdvPrm{d->prm.mu, d->prm.stab2coef, d->prm.stab != 0, d->prm.stab2 != 0};
@@ -688,7 +801,7 @@ template <int NC, int MODE>
 int launch_grad(xg_ctx* c, ChoCGDev* d, const double* U, double* G, double dt = 0.0,
                 int addp = 0) {
   two_pass<k_cgrad<NC, MODE, false>, k_cgrad<NC, MODE, true>>(
-      c->stream, d->n, d->nbn, d->n, adj_of(d), U, bnd_of(d), d->vol, G, dt, addp, d->u, d->pr);
+      c->stream, d->n, d->nbn, d->n, adj_of(d), U, bnd_of(d), d->ivol, G, dt, addp, d->u, d->pr);
   XG_CHECK_LAUNCH(c);
   return XG_OK;
 }
@@ -714,11 +827,11 @@ int launch_rhs(xg_ctx* c, ChoCGDev* d, const double* U, double dtk, int stage0, 
   const AdvPrm ap = adv_of(d);
   if (d->prm.flux == XG_DAMP4)
     two_pass<k_crhs<true, false>, k_crhs<true, true>>(c->stream, d->n, d->nbn, d->n, adj_of(d), U,
-                                                       d->vgrad, d->pr, bnd_of(d), ap, d->vol,
+                                                       d->vgrad, d->pr, bnd_of(d), ap, d->ivol,
                                                        dtk, stage0, d->un, uout, R);
   else
     two_pass<k_crhs<false, false>, k_crhs<false, true>>(c->stream, d->n, d->nbn, d->n, adj_of(d),
-                                                         U, d->vgrad, d->pr, bnd_of(d), ap, d->vol,
+                                                         U, d->vgrad, d->pr, bnd_of(d), ap, d->ivol,
                                                          dtk, stage0, d->un, uout, R);
   XG_CHECK_LAUNCH(c);
   return XG_OK;
@@ -823,7 +936,7 @@ int step_dt(xg_ctx* c, ChoCGDev* d, double* dt) {
   }
   const unsigned long long big = 0x7fefffffffffffffull;  // DBL_MAX bits
   XG_CUDA(c, cudaMemcpyAsync(d->dtmin, &big, sizeof(big), cudaMemcpyHostToDevice, c->stream));
-  k_cdt<<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(d->n, d->u, d->vol, d->prm.mu,
+  k_cdt<<<blocks_for(d->n, kBlock), kBlock, 0, c->stream>>>(d->n, d->u, d->cbrtv, d->prm.mu,
                                                              d->dtmin);
   XG_CHECK_LAUNCH(c);
   unsigned long long bits = 0;
@@ -1002,7 +1115,8 @@ int xg_chocg_setup(xg_ctx* c, const xg_chocg_params* prm, int64_t npoin, const d
     A.plan(d->bnode, bnode.size());
     A.plan(d->park, bnode.size() * 9);
     A.plan(d->xyz, 3 * n);
-    A.plan(d->vol, n);
+    A.plan(d->ivol, n);
+    A.plan(d->cbrtv, n);
     A.plan(d->u, 3 * n);
     A.plan(d->u2, 3 * n);
     A.plan(d->un, 3 * n);
@@ -1037,7 +1151,11 @@ int xg_chocg_setup(xg_ctx* c, const xg_chocg_params* prm, int64_t npoin, const d
   XG_CUDA(c, up(d->bnode, bnode.data(), bnode.size() * 4));
   XG_CUDA(c, up(d->xyz, coord, 3 * n * 8));
   d->xyz_host.assign(coord, coord + 3 * n);
-  XG_CUDA(c, up(d->vol, vol, n * 8));
+  // through the staging buffer
+  XG_CUDA(c, up(d->stage, vol, n * 8));
+  k_node_factors<<<blocks_for(n, kBlock), kBlock, 0, c->stream>>>(n, d->stage, d->ivol, d->cbrtv);
+  XG_CHECK_LAUNCH(c);
+  XG_CUDA(c, cudaStreamSynchronize(c->stream));
   for (double* z : {d->u, d->u2, d->un, d->pr, d->pgrad, d->vgrad, d->div, d->flx})
     XG_CUDA(c, cudaMemset(z, 0, (z == d->vgrad ? 9 : (z == d->pr || z == d->div ? 1 : 3)) * n * 8));
   return XG_OK;
@@ -1333,8 +1451,11 @@ int xg_chocg_init(xg_ctx* c, int64_t* it) {
   // divergence of the volume-divided momentum flux with symmetry applied
   rc = launch_grad<3, GRAD_DIVIDE>(c, d, d->u, d->vgrad);
   if (rc) return rc;
-  two_pass<k_cflux<false>, k_cflux<true>>(c->stream, d->n, d->nbn, d->n, adj_of(d), d->u,
-                                          d->vgrad, bnd_of(d), d->vol, d->prm.mu, 1, d->flx);
+  // the node tensors in the staging buffer ([9][n])
+  k_mflux<<<blocks_for(d->n, kNode), kNode, 0, c->stream>>>(d->n, d->u, d->vgrad, d->prm.mu,
+                                                            d->stage);
+  two_pass<k_cflux<false>, k_cflux<true>>(c->stream, d->n, d->nbn, d->n, adj_of(d), d->stage,
+                                          bnd_of(d), d->ivol, 1, d->flx);
   XG_CHECK_LAUNCH(c);
   rc = launch_bc(c, d, d->flx, 1);
   if (rc) return rc;
@@ -1504,7 +1625,7 @@ int xg_chorin_grad(xg_ctx* c, const double* S, double* Gout) {
   cudaStream_t s = c->stream;
   XG_CUDA(c, cudaMemcpyAsync(sv, S, n * 8, cudaMemcpyHostToDevice, s));
   two_pass<k_cgrad<1, GRAD_RAW, false>, k_cgrad<1, GRAD_RAW, true>>(
-      s, n, d->nbn, n, adj_of(d), sv, bnd_of(d), d->vol, g, 0.0, 0, nullptr, nullptr);
+      s, n, d->nbn, n, adj_of(d), sv, bnd_of(d), d->ivol, g, 0.0, 0, nullptr, nullptr);
   XG_CHECK_LAUNCH(c);
   k_soa_aos<<<blocks_for(n * 3, kBlock), kBlock, 0, s>>>(n, 3, g, out);
   XG_CUDA(c, cudaMemcpyAsync(Gout, out, n * 24, cudaMemcpyDeviceToHost, s));
@@ -1530,7 +1651,7 @@ int xg_chorin_vgrad(xg_ctx* c, const double* U, double* Gout) {
   XG_CUDA(c, cudaMemcpyAsync(out, U, n * 24, cudaMemcpyHostToDevice, s));
   k_aos_soa<<<blocks_for(n * 3, kBlock), kBlock, 0, s>>>(n, 3, out, u);
   two_pass<k_cgrad<3, GRAD_RAW, false>, k_cgrad<3, GRAD_RAW, true>>(
-      s, n, d->nbn, n, adj_of(d), u, bnd_of(d), d->vol, g, 0.0, 0, nullptr, nullptr);
+      s, n, d->nbn, n, adj_of(d), u, bnd_of(d), d->ivol, g, 0.0, 0, nullptr, nullptr);
   XG_CHECK_LAUNCH(c);
   k_soa_aos<<<blocks_for(n * 9, kBlock), kBlock, 0, s>>>(n, 9, g, out);
   XG_CUDA(c, cudaMemcpyAsync(Gout, out, n * 72, cudaMemcpyDeviceToHost, s));
@@ -1558,8 +1679,9 @@ int xg_chorin_flux(xg_ctx* c, const double* U, const double* G, double* F) {
   k_aos_soa<<<blocks_for(n * 3, kBlock), kBlock, 0, s>>>(n, 3, tmp, u);
   XG_CUDA(c, cudaMemcpyAsync(tmp, G, n * 72, cudaMemcpyHostToDevice, s));
   k_aos_soa<<<blocks_for(n * 9, kBlock), kBlock, 0, s>>>(n, 9, tmp, g);
-  two_pass<k_cflux<false>, k_cflux<true>>(s, n, d->nbn, n, adj_of(d), u, g, bnd_of(d), d->vol,
-                                          d->prm.mu, 0, f);
+  k_mflux<<<blocks_for(n, kNode), kNode, 0, s>>>(n, u, g, d->prm.mu, tmp);
+  two_pass<k_cflux<false>, k_cflux<true>>(s, n, d->nbn, n, adj_of(d), tmp, bnd_of(d), d->ivol, 0,
+                                          f);
   XG_CHECK_LAUNCH(c);
   k_soa_aos<<<blocks_for(n * 3, kBlock), kBlock, 0, s>>>(n, 3, f, tmp);
   XG_CUDA(c, cudaMemcpyAsync(F, tmp, n * 24, cudaMemcpyDeviceToHost, s));
@@ -1592,11 +1714,11 @@ int xg_chorin_rhs(xg_ctx* c, const double* P, const double* U, const double* G, 
   const AdvPrm ap = adv_of(d);
   if (d->prm.flux == XG_DAMP4)
     two_pass<k_crhs<true, false>, k_crhs<true, true>>(s, n, d->nbn, n, adj_of(d), u, g, p,
-                                                       bnd_of(d), ap, d->vol, 0.0, 0, nullptr,
+                                                       bnd_of(d), ap, d->ivol, 0.0, 0, nullptr,
                                                        nullptr, r);
   else
     two_pass<k_crhs<false, false>, k_crhs<false, true>>(s, n, d->nbn, n, adj_of(d), u, g, p,
-                                                         bnd_of(d), ap, d->vol, 0.0, 0, nullptr,
+                                                         bnd_of(d), ap, d->ivol, 0.0, 0, nullptr,
                                                          nullptr, r);
   XG_CHECK_LAUNCH(c);
   k_soa_aos<<<blocks_for(n * 3, kBlock), kBlock, 0, s>>>(n, 3, r, tmp);
