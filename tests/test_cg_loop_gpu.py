@@ -1,7 +1,8 @@
-"""The one-launch FP64 solve (systems whose rows fit the SMs' shared memory)
-against the oracle's PCG at the sizes where its row split changes shape: one
-block with a ragged slice, blocks of the smallest row count with a ragged last
-one, more rows than a block has threads, 32-bit columns (a bandwidth beyond
+"""The one-launch FP64 solves (one cluster for a few thousand rows, all SMs for
+systems whose rows fit their shared memory) against the oracle's PCG at the
+sizes where the row split changes shape: one block with a ragged slice, a
+cluster with empty blocks and with a ragged last one, the largest cluster, blocks
+of the smallest row count, more rows than a block has threads, 32-bit columns (a bandwidth beyond
 16 bits), several launches' worth of limits, and a solve continued after its
 iteration limit.  Tolerances: both sides run the same recurrence in FP64 with
 sums in another order, so counts agree and x to the accuracy of the solve
@@ -30,7 +31,8 @@ def _case(n, seed, numbering):
 
 
 @pytest.mark.parametrize("n,numbering", [(2, "lex"), (3, "lex"), (5, "random"), (6, "rcm"),
-                                         (18, "rcm"), (27, "rcm"), (41, "random"), (55, "rcm")])
+                                         (8, "rcm"), (13, "random"), (18, "rcm"), (24, "rcm"),
+                                         (27, "rcm"), (41, "random"), (55, "rcm")])
 @pytest.mark.parametrize("pc", ["jacobi", "none"])
 def test_loop_solve_matches_oracle(n, numbering, pc):
     ia, ja, a, dn, dv, b = _case(n, n, numbering)

@@ -87,6 +87,7 @@ struct CGScalars {
 struct CGDev {
   Arena arena;
   int64_t n = 0, nslice = 0, nent = 0, maxgrid = 0;
+  int wmax = 0;  // the widest slice
   int32_t *soff = nullptr, *swidth = nullptr, *col = nullptr;
   int16_t* col16 = nullptr;            // column - row, kPad16 for padding
   double* a0 = nullptr;                // original values (SELL order)
@@ -307,6 +308,7 @@ __device__ __forceinline__ T sell_row_x(CI ci, const V* __restrict__ val, int32_
 // One wave of resident blocks of kernel K for n rows.
 int g_nsm = 0;
 size_t g_smem = 0;  // shared memory a block may ask for; 0: no cooperative launches
+bool g_cluster = false;  // clusters of kClusterSize blocks can be resident
 template <auto K>
 unsigned pgrid(int64_t n) {
   static const int per_sm = [] {
@@ -980,6 +982,216 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
   }
 }
 
+// ---- the FP64 iteration of a small system in one thread-block cluster
+//
+// A system of a few thousand rows is barriers: k_cg_loop's cost 1.3 us each
+// through L2, 10 us an iteration at 17^3.  One cluster of 16 SMs meets by the
+// hardware barrier and holds everything, matrix included, in its blocks'
+// shared memory, gathering the direction from its owner's (distributed shared
+// memory).  The FP64 work runs on 16 SMs instead of all, 22 operations a row
+// and iteration: 6.6 against 11.1 us an iteration at 17^3, 9.4 against 11.2 at
+// 21^3, 10.2 against 12.7 at 24^3, about where the shared memory ends (15
+// entries a row; k_cg_loop takes what is larger or does not fit).
+constexpr int kClusterSize = 16;
+constexpr int kClusterThreads = 512;
+constexpr int64_t kClusterRows = 16384;
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::
+                   : "memory");
+}
+// The address of this block's shared-memory location p in block `rank`.
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(a)
+               : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ double ld_cluster(uint32_t a) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+// As grid_sum over the cluster's blocks: lane 0 of warp k calls fin(k, sum).
+// box: [3][2][kClusterSize] in shared memory, turn: barriers with sums so far,
+// modulo 3 (a block may be one barrier ahead of the slowest reader).
+template <int K, class F>
+__device__ __forceinline__ void cluster_sum(const double (&v)[K], int active, double* box,
+                                            int& turn, F fin) {
+  constexpr int NW = kClusterThreads / 32 / 4;
+  __shared__ double rows[K][kClusterThreads];
+  __shared__ double quarter[K][4][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < K; ++k) rows[k][threadIdx.x] = v[k];
+  __syncthreads();
+  if (wid < 4 * K) {
+    const int k = wid >> 2, qd = wid & 3;
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < NW; ++j)
+      if (32 * (qd + 4 * j) < active) s += rows[k][lane + 32 * (qd + 4 * j)];
+    quarter[k][qd][lane] = s;
+  }
+  __syncthreads();
+  double* b = box + turn * 2 * kClusterSize;
+  if (wid < K) {
+    double s = (quarter[wid][0][lane] + quarter[wid][1][lane]) +
+               (quarter[wid][2][lane] + quarter[wid][3][lane]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane < kClusterSize)
+      st_cluster(cluster_addr(b + wid * kClusterSize + blockIdx.x, lane), s);
+  }
+  cluster_sync();
+  if (wid < K) {
+    double s = lane < kClusterSize ? b[wid * kClusterSize + lane] : 0.0;
+#pragma unroll
+    for (int o = kClusterSize / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) fin(wid, s);
+  }
+  turn = turn == 2 ? 0 : turn + 1;
+  __syncthreads();
+}
+
+// The whole solve of a small system: as k_cg_loop, one cluster of kClusterSize
+// blocks (the grid), `per` rows each (whole slices), `ents` matrix entries at
+// most in a block.
+__global__ void __launch_bounds__(kClusterThreads, 1)
+    k_cg_cluster(int64_t n, int per, int ents, int64_t maxits, const int32_t* __restrict__ soff,
+                 const int32_t* __restrict__ sw, const int32_t* __restrict__ col,
+                 const double* __restrict__ a, const double* __restrict__ d, double* r, double* z,
+                 double* p, double* x, CGScalars* sc) {
+  extern __shared__ double loop_smem[];
+  __shared__ double box[3 * 2 * kClusterSize];
+  __shared__ double sh_scale, sh_rho, sh_rho0, sh_rr, sh_pq;
+  __shared__ int sh_fin, sh_end;
+  double* sr = loop_smem;
+  double* sq = sr + per;  // q, then z
+  double* sp = sq + per;
+  double* sd = sp + per;
+  double* sx = sd + per;
+  double* sa = sx + per;                                   // matrix values
+  uint32_t* sc_at = reinterpret_cast<uint32_t*>(sa + ents);  // where each column's p lies
+  const bool already = sc->done != 0;  // the same in every block
+  const int64_t r0 = int64_t(blockIdx.x) * per;
+  const int rows = already || r0 >= n ? 0 : static_cast<int>(n - r0 < per ? n - r0 : per);
+  const int32_t e0 = rows ? soff[r0 >> 5] : 0;
+  const int32_t e1 = rows ? soff[(r0 + rows + kSlice - 1) >> 5] : 0;
+  for (int t = threadIdx.x; t < rows; t += kClusterThreads) {
+    sr[t] = r[r0 + t];
+    sq[t] = z[r0 + t];
+    sp[t] = p[r0 + t];
+    sd[t] = d[r0 + t];
+    sx[t] = x[r0 + t];
+  }
+  for (int t = threadIdx.x; t < e1 - e0; t += kClusterThreads) {
+    // padding reads the block's first p with weight 0
+    const int32_t c = col[e0 + t];
+    const int rank = c < 0 ? int(blockIdx.x) : c / per;
+    sa[t] = c < 0 ? 0.0 : a[e0 + t];
+    sc_at[t] = cluster_addr(sp, rank) + (c < 0 ? 0 : (c - rank * per) * 8);
+  }
+  int64_t it = sc->it;
+  const int64_t maxit = sc->maxit;
+  const double nb = sc->normb > 1.0e-14 ? sc->normb : 1.0;
+  const double lim = sc->tol * nb;
+  const double eps = sc->guard == 0 ? DBL_EPSILON : DBL_MIN;
+  if (threadIdx.x == 0) {
+    sh_rho = sc->rho;
+    sh_rho0 = sc->rho0;
+    sh_rr = sc->rr;
+    sh_pq = sc->pq;
+    sh_fin = sc->finished;
+    sh_end = already ? 1 : 0;
+    sh_scale = it == 0 ? 0.0 : sc->rho / sc->rho0;
+  }
+  double alpha = sc->alpha;
+  // every block runs before another's shared memory is touched, and the loads
+  // of the scalars are done before block 0 writes them back
+  cluster_sync();
+  int turn = 0;
+  for (int64_t step = 0; step < maxits && !sh_end; ++step) {
+    const double beta = sh_scale;
+    for (int t = threadIdx.x; t < rows; t += kClusterThreads) sp[t] = sq[t] + beta * sp[t];
+    cluster_sync();
+    double dot[1] = {0.0};
+    for (int t = threadIdx.x; t < rows; t += kClusterThreads) {
+      const int64_t sl = (r0 + t) >> 5;
+      const int w = sw[sl], o = soff[sl] - e0 + (t & 31);
+      double s = 0.0;
+      for (int k0 = 0; k0 < w; k0 += kLoopRound) {
+        double v[kLoopRound], g[kLoopRound];
+#pragma unroll
+        for (int u = 0; u < kLoopRound; ++u) {
+          const bool in = k0 + u < w;
+          const int e = o + (k0 + u) * kSlice;
+          v[u] = in ? sa[e] : 0.0;
+          g[u] = in ? ld_cluster(sc_at[e]) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kLoopRound; ++u)
+          if (k0 + u < w) s += v[u] * g[u];
+      }
+      sq[t] = s;
+      dot[0] += sp[t] * s;
+    }
+    cluster_sum<1>(dot, rows, box, turn, [&](int, double pq) {
+      sh_pq = pq;
+      sh_fin = fabs(pq) < eps;
+      sh_scale = sh_fin ? 0.0 : sh_rho / pq;
+    });
+    alpha = sh_scale;
+    double v[2] = {0.0, 0.0};
+    for (int t = threadIdx.x; t < rows; t += kClusterThreads) {
+      const double ri = sr[t] - alpha * sq[t];
+      sr[t] = ri;
+      sx[t] += alpha * sp[t];
+      const double zi = ri * sd[t];
+      sq[t] = zi;
+      v[0] += ri * zi;
+      v[1] += ri * ri;
+    }
+    it += 1;
+    cluster_sum<2>(v, rows, box, turn, [&](int k, double sum) {
+      if (k == 0) {
+        sh_rho0 = sh_rho;
+        sh_rho = sum;
+        sh_scale = sum / sh_rho0;
+      } else {  // the stopping test (ConjugateGradients.cpp:772-823)
+        sh_rr = sum;
+        const double nr = sqrt(sum);
+        sh_end = sh_fin || nr < lim || it >= maxit ? (nr > lim ? 1 : 2) : 0;
+      }
+    });
+  }
+  if (!already) {
+    for (int t = threadIdx.x; t < rows; t += kClusterThreads) {
+      r[r0 + t] = sr[t];
+      z[r0 + t] = sq[t];
+      p[r0 + t] = sp[t];
+      x[r0 + t] = sx[t];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      sc->rho = sh_rho;
+      sc->rho0 = sh_rho0;
+      sc->rr = sh_rr;
+      sc->pq = sh_pq;
+      sc->alpha = alpha;
+      sc->it = it;
+      sc->finished = sh_fin;
+      sc->converged = sh_end == 2;
+      sc->done = sh_end != 0;
+    }
+  }
+  cluster_sync();  // no block leaves while another may read its shared memory
+}
+
 // v = S r
 template <class T>
 __global__ void k_scale(int64_t n, const float* __restrict__ srow, const T* __restrict__ r,
@@ -1250,6 +1462,46 @@ bool loop_shape(int64_t n, LoopShape* out) {
   return true;
 }
 
+// The FP64 solve of a small system by k_cg_cluster launches; false where it
+// does not apply (rows, shared memory, or a device without such clusters).
+constexpr int64_t kClusterIts = 65536;
+bool cluster_shape(const CGDev* d, int* per, int* ents, size_t* smem) {
+  if (d->n > kClusterRows || d->n < kClusterSize * kSlice || !g_cluster) return false;
+  *per = static_cast<int>((d->n + kClusterSize * kSlice - 1) / (kClusterSize * kSlice)) * kSlice;
+  *ents = d->wmax * *per;
+  *smem = size_t(*per) * 5 * sizeof(double) + size_t(*ents) * (sizeof(double) + sizeof(uint32_t));
+  return *smem + 32768 <= g_smem;
+}
+int cluster_solve(xg_ctx* c, CGDev* d, int per, int ents, size_t smem, CGScalars* h) {
+  cudaStream_t s = c->stream;
+  XG_CUDA(c, cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(smem)));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kClusterSize);
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kClusterSize;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  for (;;) {
+    XG_CUDA(c, cudaLaunchKernelEx(&cfg, k_cg_cluster, d->n, per, ents, kClusterIts,
+                                  static_cast<const int32_t*>(d->soff),
+                                  static_cast<const int32_t*>(d->swidth),
+                                  static_cast<const int32_t*>(d->col),
+                                  static_cast<const double*>(d->a),
+                                  static_cast<const double*>(d->d), d->r, d->z, d->p[0], d->x,
+                                  d->scal));
+    const int rc = read_scal(c, d, h);
+    if (rc) return rc;
+    if (h->done) return XG_OK;
+  }
+}
+
 // The FP64 solve by k_cg_loop launches of at most kLoopIts iterations (a
 // launch is bounded in time; the state goes through global memory between
 // launches).
@@ -1285,6 +1537,10 @@ int cg_iterate(xg_ctx* c, CGDev* d, int64_t maxit, double tol, CGScalars* h) {
   XG_CUDA(c, cudaMemcpyAsync(&d->scal->tol, &tol, sizeof(double), cudaMemcpyHostToDevice, s));
   XG_CUDA(c, cudaMemcpyAsync(&d->scal->maxit, &maxit, sizeof(int64_t), cudaMemcpyHostToDevice, s));
   const int64_t n = d->n;
+  int per = 0, ents = 0;
+  size_t smem = 0;
+  if (d->pc != 2 && cluster_shape(d, &per, &ents, &smem))
+    return cluster_solve(c, d, per, ents, smem, h);
   LoopShape sh;
   if (d->pc != 2 && loop_shape(n, &sh))
     return d->use16 ? loop_solve(c, d, sh, Cols16{d->col16}, h)
@@ -1356,6 +1612,37 @@ int replace_residual(xg_ctx* c, CGDev* d, int first) {
     XG_CHECK_LAUNCH(c);
   }
   return XG_OK;
+}
+
+
+// Whether a cluster of kClusterSize blocks of k_cg_cluster with the shared
+// memory of its largest system can be resident (a query, nothing runs).
+bool cluster_ok() {
+  if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+      cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  const int most = static_cast<int>(g_smem > 32768 ? g_smem - 32768 : 0);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kClusterSize);
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = most;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kClusterSize;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int num = 0;
+  if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, most) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&num, k_cg_cluster, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return num > 0;
 }
 
 }  // namespace
@@ -1503,6 +1790,7 @@ int xg_cg_setup(xg_ctx* c, int64_t nrow, const uint64_t* ia, const uint64_t* ja,
     XG_CUDA(c, cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     XG_CUDA(c, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     g_smem = coop ? static_cast<size_t>(smem) : 0;
+    g_cluster = cluster_ok();
     g_nsm = nsm > 0 ? nsm : 1;
   }
   const int64_t nslice = (nrow + kSlice - 1) / kSlice;
@@ -1617,6 +1905,7 @@ int xg_cg_setup(xg_ctx* c, int64_t nrow, const uint64_t* ia, const uint64_t* ja,
   d->nslice = nslice;
   d->nent = tot;
   d->use16 = fits16;
+  d->wmax = *std::max_element(sw.begin(), sw.end());
   d->maxgrid = int64_t(g_nsm) * (2048 / kBlock);
   for (int pass = 0; pass < 2; ++pass) {
     Arena& A = d->arena;
