@@ -44,10 +44,12 @@
 // residual b - A x whenever the recursive residual has fallen by the factor
 // `inner_tol` since the last replacement.  The search direction is kept
 // across replacements, so the FP32 iteration follows the FP64 one instead of
-// restarting.  The FP32 iteration is three kernels: k_cg_a forms
-// p' = z + beta p per gathered entry (FP32 arithmetic is cheap; no p pass),
-// k_pc_upper_res updates r and e and applies (I+N)^T S, k_pc_lower applies
-// -S (I+N) and closes the iteration.
+// restarting.
+//
+// Whole solves run in one launch: k_cg_cluster (FP64, systems that fit the
+// shared memory of 16 SMs), k_cg_loop (FP64, up to about 960,000 rows) and
+// k_mixed_loop (the FP32 iterations up to the next residual replacement); the
+// FP64 factored solve and larger FP64 systems take a launch per pass.
 
 #include <cuda_fp16.h>
 
@@ -101,8 +103,8 @@ struct CGDev {
   double* p[2] = {nullptr, nullptr};
   float *r32 = nullptr, *q32 = nullptr, *z32 = nullptr, *d32 = nullptr;
   double* e64 = nullptr;  // the mixed solve's correction sum alpha p', accumulated in FP64
-  float* r32b = nullptr;  // second FP32 residual (factored mixed iteration, alternating)
-  float* p32[2] = {nullptr, nullptr};
+  float* p32 = nullptr;
+  float2 *zp32 = nullptr, *vt32 = nullptr;  // records of the mixed iteration: (z, p), (S r, S q)
   double* partial = nullptr;  // 3 * maxgrid
   CGScalars* scal = nullptr;
   double* lpart = nullptr;         // k_cg_loop: [3 barriers of an iteration][2 sums][SMs]
@@ -122,7 +124,7 @@ struct CGDev {
   int32_t *soffL = nullptr, *swL = nullptr, *colL = nullptr, *posL = nullptr, *tposU = nullptr;
   int32_t *soffU = nullptr, *swU = nullptr, *colU = nullptr;
   int16_t *colL16 = nullptr, *colU16 = nullptr;
-  float *nvL = nullptr, *nvU = nullptr, *srow = nullptr, *eL = nullptr, *eU = nullptr;
+  float *nvL = nullptr, *nvU = nullptr, *srow = nullptr, *msrow = nullptr, *eL = nullptr, *eU = nullptr;
   __half *hvL = nullptr, *hvU = nullptr;
   float* eF = nullptr;  // e_ij in the full layout (0 on the diagonal and at Dirichlet nodes)
   double *v = nullptr, *u = nullptr, *t = nullptr;  // S r, (I+N)^T S r; t: xg_cg_precondition
@@ -214,11 +216,17 @@ __device__ double sum_partials(const double* partial, int k) {
 // the gathered vectors stay in L2; the FP32 solver's narrower stream is read
 // through the non-coherent cache (measured faster for it).
 struct Cols32 {
+  using E = int32_t;
   const int32_t* c;
+  __device__ __forceinline__ static int32_t of(int32_t v, int32_t) { return v; }
   __device__ __forceinline__ int32_t at(int32_t e, int32_t) const { return __ldcs(c + e); }
 };
 struct Cols16 {
+  using E = int16_t;
   const int16_t* c;
+  __device__ __forceinline__ static int32_t of(int16_t v, int32_t i) {
+    return v == kPad16 ? -1 : i + int32_t(v);
+  }
   __device__ __forceinline__ int32_t at(int32_t e, int32_t i) const {
     const int16_t dlt = __ldg(c + e);
     return dlt == kPad16 ? -1 : i + int32_t(dlt);
@@ -515,47 +523,21 @@ __global__ void __launch_bounds__(kBlock) k_cg_p(int64_t n, const T* __restrict_
   griddep_trigger();
 }
 
-// q = A p', (p', q).  PF: p' = z + beta p formed per gathered entry and
-// stored for the row (the FP32 solver: two gathers, no extra pass; p0/p1
-// alternate with the count); otherwise p' = p0 = p1 (k_cg_p).  The FP32
-// solver sums (p', q) per thread in FP32 and widens once, and forms each row
-// as sum_j a_ij (p'_j - p'_i) + rs_i p'_i (rs: the row's exact sum, zero for
-// an interior row of the pressure Laplacian): on a smooth p' the terms
-// a_ij p'_j of the plain sum cancel to a result about 1/kappa(A) of their
-// size, which FP32 cannot hold, while the differences p'_j - p'_i are
-// formed exactly and nothing large cancels.
-template <class T, class V, class CI, bool PF>
+// q = A p, (p, q).
+template <class T, class V, class CI>
 __global__ void __launch_bounds__(kBlock) k_cg_a(int64_t n, const int32_t* __restrict__ soff,
                                                   const int32_t* __restrict__ sw, CI ci,
                                                   const V* __restrict__ a,
-                                                  const T* __restrict__ z, T* p0, T* p1,
-                                                  T* __restrict__ q, double* partial,
-                                                  CGScalars* sc, const float* __restrict__ rs) {
+                                                  const T* __restrict__ p, T* __restrict__ q,
+                                                  double* partial, CGScalars* sc) {
   griddep_wait();
   if (sc->done) return;
-  const int64_t it = sc->it;
-  const T beta = PF ? block_beta<T>(sc) : T(0);
-  const T* __restrict__ pold = (it & 1) ? p1 : p0;
-  T* __restrict__ pnew = (it & 1) ? p0 : p1;
   T dot = T(0);
   XG_ROWS(i, n) {
-    const int lane = int(i & 31);
-    if (PF) {
-      const T pi = z[i] + beta * pold[i];
-      const T s = sell_row_x<T>(ci, a, soff[i >> 5], sw[i >> 5], lane, int32_t(i),
-                                 [&](int32_t c) {
-                                   return (__ldg(z + c) + beta * __ldg(pold + c)) - pi;
-                                 }) +
-                  T(rs[i]) * pi;
-      pnew[i] = pi;
-      q[i] = s;
-      dot += pi * s;
-    } else {
-      const T s = sell_row_x<T>(ci, a, soff[i >> 5], sw[i >> 5], lane, int32_t(i),
-                                 [&](int32_t c) { return __ldg(p0 + c); });
-      q[i] = s;
-      dot += p0[i] * s;
-    }
+    const T s = sell_row_x<T>(ci, a, soff[i >> 5], sw[i >> 5], int(i & 31), int32_t(i),
+                               [&](int32_t c) { return __ldg(p + c); });
+    q[i] = s;
+    dot += p[i] * s;
   }
   griddep_trigger();
   T v[1] = {dot};
@@ -565,9 +547,8 @@ __global__ void __launch_bounds__(kBlock) k_cg_a(int64_t n, const int32_t* __res
       sc->rho0 = sc->rho;
       sc->pq = pq;
       // the reference's breakdown guard is an absolute epsilon
-      // (ConjugateGradients.cpp:681-690); the FP32 solver, and the FP64 one
-      // with guard 1, guard underflow only
-      const double eps = (sizeof(T) == 8 && sc->guard == 0) ? DBL_EPSILON : DBL_MIN;
+      // (ConjugateGradients.cpp:681-690); with guard 1, underflow only
+      const double eps = sc->guard == 0 ? DBL_EPSILON : DBL_MIN;
       if (fabs(pq) < eps) {
         sc->finished = 1;
         sc->alpha = 0.0;
@@ -580,56 +561,40 @@ __global__ void __launch_bounds__(kBlock) k_cg_a(int64_t n, const int32_t* __res
 }
 
 // The end of an iteration, in the last block: (r,r), the count and the
-// stopping test (ConjugateGradients.cpp:772-823):
-//   FP64: ||r|| < tol ||b||, or maxit iterations (the reference's test);
-//   MIXED: ||r|| < max(tol ||b||, delta * rlast) asks for a residual
-//   replacement (rlast: the last true residual norm), as does maxit.
-template <bool MIXED>
+// stopping test: ||r|| < tol ||b||, or maxit iterations
+// (ConjugateGradients.cpp:772-823).
 __device__ __forceinline__ void end_iteration(double rr, CGScalars* sc) {
   sc->rr = rr;
   sc->it += 1;
   const double nr = sqrt(rr);
   const double nb = sc->normb > 1.0e-14 ? sc->normb : 1.0;
-  if (MIXED) {
-    const double lim = fmax(sc->tol * nb, sc->delta * sc->rlast);
-    if (sc->finished || nr < lim || sc->it >= sc->maxit) sc->done = 1;
-  } else {
-    if (sc->finished || nr < sc->tol * nb || sc->it >= sc->maxit) {
-      sc->done = 1;
-      sc->converged = nr > sc->tol * nb ? 0 : 1;
-    }
+  if (sc->finished || nr < sc->tol * nb || sc->it >= sc->maxit) {
+    sc->done = 1;
+    sc->converged = nr > sc->tol * nb ? 0 : 1;
   }
 }
 
 // pq + rz + x (ConjugateGradients.cpp:671-823), fused: r -= alpha q,
-// x += alpha p'; Jacobi z = r d (d the inverse diagonal), rho = (r, z), or
-// (FACTOR) v = S r for
-// the factor passes that follow; (r, r) and the stopping test:
-//   FP64: ||r|| < tol ||b||, or maxit iterations (the reference's test);
-//   MIXED: ||r|| < max(tol ||b||, delta * rlast) asks for a residual
-//   replacement (rlast: the last true residual norm), as does maxit.
-// x is the FP64 solution (FP64 solver) or the mixed solver's FP64 correction
-// e, summed with exact FP64 products alpha p'.
-template <class T, bool FACTOR, bool MIXED>
+// x += alpha p; Jacobi z = r d (d the inverse diagonal), rho = (r, z), (r, r)
+// and the stopping test, or (FACTOR) v = S r for the factor passes that follow.
+template <class T, bool FACTOR>
 __global__ void __launch_bounds__(kBlock) k_cg_b(int64_t n, const T* __restrict__ q,
-                                                  const T* __restrict__ d, const T* p0,
-                                                  const T* p1, const float* __restrict__ srow,
+                                                  const T* __restrict__ d,
+                                                  const T* __restrict__ p,
+                                                  const float* __restrict__ srow,
                                                   T* __restrict__ r, T* __restrict__ z,
-                                                  T* __restrict__ vs, double* __restrict__ x,
+                                                  T* __restrict__ vs, T* __restrict__ x,
                                                   double* partial, CGScalars* sc) {
   griddep_wait();
   if (sc->done) return;
   const T alpha = T(sc->alpha);
-  // the p' of this iteration (k_cg_a wrote it; the count advances below, or
-  // at the end of the factor passes)
-  const T* __restrict__ p = (sc->it & 1) ? p0 : p1;
   if (FACTOR) {
     // no reduction here: (r,z), (r,r) and the stopping test close the
     // iteration in k_pc_lower
     XG_ROWS(i, n) {
       const T ri = r[i] - alpha * q[i];
       r[i] = ri;
-      x[i] += double(alpha) * double(p[i]);
+      x[i] += alpha * p[i];
       vs[i] = T(srow[i]) * ri;
     }
     griddep_trigger();
@@ -639,7 +604,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_b(int64_t n, const T* __restrict_
   XG_ROWS(i, n) {
     const T ri = r[i] - alpha * q[i];
     r[i] = ri;
-    x[i] += double(alpha) * double(p[i]);
+    x[i] += alpha * p[i];
     const T zi = ri * d[i];
     z[i] = zi;
     rz += ri * zi;
@@ -652,7 +617,7 @@ __global__ void __launch_bounds__(kBlock) k_cg_b(int64_t n, const T* __restrict_
     double rr = sum_partials(partial, 1);
     if (threadIdx.x == 0) {
       sc->rho = rz;
-      end_iteration<MIXED>(rr, sc);
+      end_iteration(rr, sc);
       sc->ticket[2] = 0;
     }
   }
@@ -677,44 +642,9 @@ __global__ void __launch_bounds__(kBlock) k_pc_upper(int64_t n, const int32_t* _
   }
 }
 
-// The update of a factored FP32 iteration fused with the first factor pass:
-// r' = r - alpha q, e += alpha p' (in FP64: FP32 rounding noise in the
-// correction would be amplified by A's largest eigenvalues into the residual
-// the outer loop replaces), u = (I+N)^T S r', with the neighbours'
-// S r' formed from their r and q.  The residual alternates between ra and rb
-// with the count (the current one is ra at even counts): the pass reads one
-// and writes the other, so no row reads a residual that another row of the
-// same pass has replaced.
-template <class CI>
-__global__ void __launch_bounds__(kBlock, 5) k_pc_upper_res(
-    int64_t n, const int32_t* __restrict__ soffU, const int32_t* __restrict__ swU, CI ci,
-    const __half* __restrict__ nvU, const float* __restrict__ srow, const float* __restrict__ q,
-    const float* p0, const float* p1, float* ra, float* rb, double* __restrict__ e,
-    float* __restrict__ u, const CGScalars* __restrict__ sc) {
-  griddep_wait();
-  if (sc->done) return;
-  const float alpha = float(sc->alpha);
-  const int64_t it = sc->it;
-  const float* __restrict__ p = (it & 1) ? p0 : p1;
-  const float* __restrict__ rold = (it & 1) ? rb : ra;
-  float* __restrict__ rnew = (it & 1) ? ra : rb;
-  XG_ROWS(i, n) {
-    const int lane = int(i & 31);
-    const float ri = rold[i] - alpha * q[i];
-    rnew[i] = ri;
-    e[i] += double(alpha) * double(p[i]);
-    u[i] = srow[i] * ri +
-           sell_row_x<float, 8>(ci, nvU, soffU[i >> 5], swU[i >> 5], lane, int32_t(i),
-                              [&](int32_t c) {
-                                return __ldg(srow + c) * (__ldg(rold + c) - alpha * __ldg(q + c));
-                              });
-  }
-}
-
 // z = -S (I+N) u (Dirichlet rows: z = r), partial (r,z); the last block
-// stores rho = (r,z).  MODE 0 applies the preconditioner only; MODE 1 (FP64)
-// and MODE 2 (mixed) also close a CG iteration: partial (r,r), the count and
-// the stopping test.
+// stores rho = (r,z).  MODE 0 applies the preconditioner only; MODE 1 also
+// closes a CG iteration: partial (r,r), the count and the stopping test.
 template <class T, class V, class CI, int MODE>
 __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 6 : 1) k_pc_lower(int64_t n, const int32_t* __restrict__ soffL,
                                                       const int32_t* __restrict__ swL, CI ci,
@@ -722,15 +652,11 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 6 : 1) k_pc_lower(int
                                                       const float* __restrict__ srow,
                                                       const uint8_t* __restrict__ mask,
                                                       const T* __restrict__ u,
-                                                      const T* r_even, const T* r_odd,
+                                                      const T* __restrict__ r,
                                                       T* __restrict__ z, double* partial,
                                                       CGScalars* sc) {
   griddep_wait();
   if (sc->done) return;
-  // the residual: r_even unless it alternates (r_odd given), then the one
-  // k_pc_upper_res wrote (MODE 2) or the current one (MODE 0)
-  const bool odd = r_odd && (((sc->it + (MODE == 2 ? 1 : 0)) & 1) != 0);
-  const T* __restrict__ r = odd ? r_odd : r_even;
   T rz = T(0), rr = T(0);  // per thread in T (FP32 for the mixed solver), widened once
   XG_ROWS(i, n) {
     const int lane = int(i & 31);
@@ -758,7 +684,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 6 : 1) k_pc_lower(int
     double rr = sum_partials(partial, 1);
     if (threadIdx.x == 0) {
       sc->rho = rz;
-      end_iteration<MODE == 2>(rr, sc);
+      end_iteration(rr, sc);
       sc->ticket[3] = 0;
     }
   }
@@ -776,6 +702,50 @@ struct LoopSync {
   unsigned int target;   // arrivals when every block has reached this barrier
   int turn;              // barriers so far, modulo 3
 };
+
+// The second half of a barrier: warp k < K (at least warp 0) comes with the
+// block's sum of value k in lane 0 of `s`.
+template <int K, class F>
+__device__ __forceinline__ bool grid_meet(double s, LoopSync& sync, CGScalars* sc, int* okay, F fin) {
+  constexpr int KW = K > 0 ? K : 1;  // polling warps
+  const int nb = gridDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  sync.target += unsigned(nb) * KW;
+  if (wid < KW) {
+    double* part = sync.part + (sync.turn * 2 + wid) * nb;
+    if (K > 0 && lane == 0) part[blockIdx.x] = s;
+    if (lane == 0) {
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(sync.arrive) : "memory");
+      unsigned int seen = 0;
+      int spin = 0;
+      do {
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync.arrive) : "memory");
+      } while (int(seen - sync.target) < 0 && ++spin < kLoopSpin);
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      if (spin >= kLoopSpin) {
+        *okay = 0;
+        atomicExch(&sc->err, 1);
+      }
+    }
+    __syncwarp();
+    if (K > 0) {
+      // up to 256 blocks' sums in one round of loads
+      double sum = 0.0, at[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) at[j] = lane + 32 * j < nb ? __ldcg(part + lane + 32 * j) : 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (32 * j < nb) sum += at[j];
+      for (int b = lane + 256; b < nb; b += 32) sum += __ldcg(part + b);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0) fin(wid, sum);
+    }
+  }
+  sync.turn = sync.turn == 2 ? 0 : sync.turn + 1;
+  __syncthreads();
+  return *okay != 0;
+}
 
 // Barrier of all blocks of k_cg_loop that also sums K values per thread over
 // the grid (K = 0: the barrier alone; the threads from `active` on hold 0);
@@ -799,12 +769,12 @@ struct LoopSync {
 template <int K, class F>
 __device__ __forceinline__ bool grid_sum(const double (&v)[K > 0 ? K : 1], int active,
                                          LoopSync& sync, CGScalars* sc, F fin) {
-  constexpr int KW = K > 0 ? K : 1;          // polling warps
+  constexpr int KW = K > 0 ? K : 1;          // values, at least one
   constexpr int NW = kLoopThreads / 32 / 4;  // rows of each quarter's warp
   __shared__ double rows[KW][kLoopThreads];
   __shared__ double quarter[KW][4][32];
   __shared__ int okay;
-  const int nb = gridDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (threadIdx.x == 0) okay = 1;
   if (K > 0) {
 #pragma unroll
@@ -820,42 +790,39 @@ __device__ __forceinline__ bool grid_sum(const double (&v)[K > 0 ? K : 1], int a
     }
   }
   __syncthreads();
-  sync.target += unsigned(nb) * KW;
-  if (wid < KW) {
-    double* part = sync.part + (sync.turn * 2 + wid) * nb;
-    if (K > 0) {
-      double s = (quarter[wid][0][lane] + quarter[wid][1][lane]) +
-                 (quarter[wid][2][lane] + quarter[wid][3][lane]);
+  double s = 0.0;
+  if (K > 0 && wid < KW) {
+    s = (quarter[wid][0][lane] + quarter[wid][1][lane]) +
+        (quarter[wid][2][lane] + quarter[wid][3][lane]);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) part[blockIdx.x] = s;
-    }
-    if (lane == 0) {
-      asm volatile("fence.acq_rel.gpu;" ::: "memory");
-      asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(sync.arrive) : "memory");
-      unsigned int seen = 0;
-      int spin = 0;
-      do {
-        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync.arrive) : "memory");
-      } while (int(seen - sync.target) < 0 && ++spin < kLoopSpin);
-      asm volatile("fence.acq_rel.gpu;" ::: "memory");
-      if (spin >= kLoopSpin) {
-        okay = 0;
-        atomicExch(&sc->err, 1);
-      }
-    }
-    __syncwarp();
-    if (K > 0) {
-      double sum = 0.0;
-      for (int b = lane; b < nb; b += 32) sum += __ldcg(part + b);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (lane == 0) fin(wid, sum);
-    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   }
-  sync.turn = sync.turn == 2 ? 0 : sync.turn + 1;
+  return grid_meet<K>(s, sync, sc, &okay, fin);
+}
+
+// The barrier with sums of FP32 values: summed over each warp in FP32, the
+// warps' sums and the blocks' in FP64 (as block_partials sums them).
+template <int NT, int K, class F>
+__device__ __forceinline__ bool grid_sum32(const float (&v)[K], LoopSync& sync, CGScalars* sc, F fin) {
+  __shared__ float warps[K][32];
+  __shared__ int okay;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (threadIdx.x == 0) okay = 1;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    float t = v[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) warps[k][wid] = t;
+  }
   __syncthreads();
-  return okay != 0;
+  double s = 0.0;
+  if (wid < K) {
+    s = lane < NT / 32 ? double(warps[wid][lane]) : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  }
+  return grid_meet<K>(s, sync, sc, &okay, fin);
 }
 
 // Up to maxits whole iterations of the FP64 PCG without a factor
@@ -979,6 +946,439 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
     sc->finished = sh_fin;
     sc->converged = sh_end == 2;
     sc->done = sh_end != 0;
+  }
+}
+
+// ---- the mixed solve's FP32 iteration as one kernel
+
+__device__ __forceinline__ unsigned smem_at(const void* p) {
+  return static_cast<unsigned>(__cvta_generic_to_shared(p));
+}
+// `bytes` (a multiple of 16) from global to shared memory (16-byte boundaries
+// both), asynchronously, counted at the barrier `mb`.  The bytes are read once
+// a pass and leave L2 first: at 129^3 the vectors then stay there (A's pass
+// 46 -> 40 us, the lower triangle's 23.5 -> 21.5).
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, uint64_t* mb) {
+  uint64_t once;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once));
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], "
+      "%4;" ::"r"(
+          smem_at(dst)),
+      "l"(src), "r"(bytes), "r"(smem_at(mb)), "l"(once)
+      : "memory");
+}
+// Waits for the phase `parity` of the barrier; false when it does not come
+// (each try waits for a system-dependent time, so this is seconds).
+__device__ __forceinline__ bool bulk_wait(uint64_t* mb, unsigned parity) {
+  for (int k = 0; k < kLoopSpin; ++k) {
+    unsigned ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(smem_at(mb)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+// Threads of k_mixed_loop, one block per SM, and its gathers in flight per
+// row.  Whole rows of 15 entries in one round need 80 registers (768 threads):
+// 153 us an iteration at 129^3 against 132 for 1024 threads and rounds of 8,
+// both with copies of 16 bytes a lane.
+constexpr int kMixThreads = 1024;
+constexpr int kMixRound = 8;
+
+// A warp's walk over the slices first, first + step, ... < end of a SELL-32
+// layout: columns and values of the next slice (up to XM entries a row) are
+// copied into the warp's stage in shared memory while the gathers of the
+// current one are under way, and the next slice's place is read one slice
+// earlier still.  Columns, values and gathers one after another would cost a
+// slice two memory latencies, and the matrix is the larger part of the bytes.
+// The copies are bulk copies, two a slice: as 16-byte asynchronous copies of
+// every lane they held the load path (129^3: 132 us an iteration, 120 so).
+template <class CI, class V, int XM>
+struct SliceWalk {
+  using E = typename CI::E;
+  static constexpr int kBytes = XM * kSlice * int(sizeof(E) + sizeof(V));
+  const int32_t *soff, *sw;
+  CI ci;
+  const V* val;
+  char* stage;
+  int32_t s, end;
+  int32_t off, w, offn, wn;  // the slice in the stage, the next one
+  const int4* places;        // the warp's first two slices, in shared memory
+  uint64_t* mb;              // the warp's barrier
+  int* bad;                  // set when a copy did not arrive
+  static constexpr int step = kMixThreads / 32;
+
+  // (one lane) the slice's columns and values into the stage
+  __device__ __forceinline__ void copy() {
+    const unsigned we = w < XM ? w : XM;
+    if ((threadIdx.x & 31) || !we) return;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_at(mb)),
+                 "r"(we * unsigned(kSlice * (sizeof(E) + sizeof(V))))
+                 : "memory");
+    bulk_copy(stage, val + off, we * unsigned(kSlice * sizeof(V)), mb);
+    bulk_copy(stage + XM * kSlice * sizeof(V), ci.c + off, we * unsigned(kSlice * sizeof(E)), mb);
+  }
+  // the places of the warp's first two slices
+  __device__ __forceinline__ int4 first_two(int32_t first) const {
+    int4 f = make_int4(0, 0, 0, 0);
+    if (first < end) {
+      f.x = __ldg(soff + first);
+      f.y = __ldg(sw + first);
+    }
+    if (first + step < end) {
+      f.z = __ldg(soff + first + step);
+      f.w = __ldg(sw + first + step);
+    }
+    return f;
+  }
+  // the first slice into the stage; whether a copy is under way
+  __device__ __forceinline__ bool start(int32_t first) {
+    s = first;
+    asm volatile("" : "+r"(s));  // keeps the addresses of every pass out of the registers of the others
+    if (s >= end) return false;
+    const int4 f = places[threadIdx.x >> 5];
+    off = f.x;
+    w = f.y;
+    offn = f.z;
+    wn = f.w;
+    __syncwarp();
+    copy();
+    return w > 0;
+  }
+  // the stage has been read: the next slice into it
+  __device__ __forceinline__ void advance() {
+    __syncwarp();
+    s += step;
+    if (s < end) {
+      off = offn;
+      w = wn;
+      copy();
+      if (s + step < end) {
+        offn = __ldg(soff + s + step);
+        wn = __ldg(sw + s + step);
+      }
+    }
+  }
+  // entries k .. k + W - 1 of row i added to t; next() once the stage is read
+  template <int W, class G, class N>
+  __device__ __forceinline__ float fixed(int k, float t, int32_t i, G g, N next) {
+    int32_t cc[W];
+    float vv[W];
+    const int o = k * kSlice + (threadIdx.x & 31);
+    const V* sval = reinterpret_cast<const V*>(stage) + o;
+    const E* scol = reinterpret_cast<const E*>(stage + XM * kSlice * sizeof(V)) + o;
+#pragma unroll
+    for (int u = 0; u < W; ++u) {
+      const int32_t c = CI::of(scol[u * kSlice], i);
+      vv[u] = c < 0 ? 0.0f : float(sval[u * kSlice]);
+      cc[u] = c < 0 ? i : c;
+    }
+    next();
+#pragma unroll
+    for (int u = 0; u < W; ++u) t += vv[u] * g(cc[u]);
+    return t;
+  }
+  template <int W, class G, class N>
+  __device__ __forceinline__ float pick(int r, int k, float t, int32_t i, G g, N next) {
+    if constexpr (W <= kMixRound) {
+      if (r == W) return fixed<W>(k, t, i, g, next);
+      return pick<W + 1>(r, k, t, i, g, next);
+    } else {
+      next();
+      return t;
+    }
+  }
+  // sum_k val[e_k] g(col[e_k]) over row i of the current slice, in entry
+  // order, in rounds of at most kMixRound entries whose gathers are in flight
+  // together; moves on to the next slice and calls `own` before the gathers
+  // of the last staged round (loads of the next slice's own row go there).
+  // The entries beyond XM of a wide slice are read one by one.
+  template <class G, class O>
+  __device__ __forceinline__ float row(int32_t i, G g, O own, unsigned& parity) {
+    const int32_t o = off;
+    int32_t r = w;
+    if (r > 0) {
+      if (!__all_sync(0xffffffffu, bulk_wait(mb, parity))) {
+        *bad = 1;  // no entry is read, and the walk ends
+        r = 0;
+        end = 0;
+      }
+      parity ^= 1u;
+    }
+    const int32_t rs = r < XM ? r : XM;
+    float t = 0.0f;
+    int k = 0;
+    for (; rs - k > kMixRound; k += kMixRound) t = fixed<kMixRound>(k, t, i, g, [] {});
+    t = pick<1>(rs - k, k, t, i, g, [&] {
+      advance();
+      own();
+    });
+    for (k = XM; k < r; ++k) {
+      const int32_t e = o + k * kSlice + int(threadIdx.x & 31);
+      const int32_t c = ci.at(e, i);
+      if (c >= 0) t += float(ldv(val + e)) * g(c);
+    }
+    return t;
+  }
+};
+
+template <class CI>
+struct MixArgs {
+  int64_t n, maxits;
+  const int32_t *soff, *sw, *soffU, *swU, *soffL, *swL;
+  CI ci, cu, cl;
+  const float* a;
+  const __half *nvU, *nvL;
+  const float *rs, *msrow, *d;  // msrow: S, negative at Dirichlet nodes
+  float *z, *p, *q, *r, *v, *u;
+  float2 *zp, *vt;
+  double* e;
+  double* lpart;
+  unsigned int* larrive;
+  CGScalars* sc;
+};
+
+constexpr int kMixFull = 16, kMixTri = 8;  // staged entries per row: whole rows, triangles
+
+// Up to maxits iterations of the mixed solve's FP32 PCG in one cooperative
+// launch, one block per SM, each with a contiguous run of slices.  FACTOR:
+// q = A p' and (p', q); the update with u = (I+N)^T S r'; z = -S (I+N) u
+// (Dirichlet rows: z = r), (r, z), (r, r) and the stopping test.  Jacobi: the
+// last two are one pass over the block's own rows.
+//
+// What a pass gathers is one record per row, 8 bytes, so an entry costs one
+// address and one load: (z, p) for p' = z + beta p, formed per gathered
+// entry, and with v = S r, t = S q the pair (v, t) for v' = v - alpha t, the
+// neighbours' new scaled residuals (in the factored iteration the residual is
+// kept as v; r = v / S where its norm is taken).  (p', q) is summed per thread
+// in FP32 and widened once, and each row formed as
+// sum_j a_ij (p'_j - p'_i) + rs_i p'_i (rs: the row's exact sum, zero for an
+// interior row of the pressure Laplacian): on a smooth p' the terms
+// a_ij p'_j of the plain sum cancel to a result about 1/kappa(A) of their
+// size, which FP32 cannot hold, while the differences p'_j - p'_i are formed
+// exactly and nothing large cancels.  The correction e += alpha p' is summed
+// in FP64 (FP32 rounding noise in it would be amplified by A's largest
+// eigenvalues into the residual the outer loop replaces).
+//
+// The bound is memory: 6 bytes an entry of A, 4 of each triangle and some 90
+// of vectors a row, 0.5 GB an iteration at 129^3; A's pass runs at 7.4 TB/s
+// there (part of the vectors stays in L2), the triangles' at 5, and the three
+// barriers with their sums take 2 to 5 us each.  A launch per pass (three an
+// iteration, every row waiting in turn for its columns, its values and its
+// gathers) took 145 us an iteration at 129^3 where this takes 106 (89 in the kernel), 35.5
+// against 27.9 at 65^3 and 27.1 against 24.3 at 17^3 (the whole solve's time
+// over its iterations).
+template <class CI, bool FACTOR>
+__global__ void __launch_bounds__(kMixThreads, 1)
+    k_mixed_loop(const __grid_constant__ MixArgs<CI> A) {
+  extern __shared__ __align__(16) char mix_smem[];
+  __shared__ double sh_beta, sh_rho, sh_rho0, sh_rr, sh_pq, sh_lim, sh_alpha;
+  __shared__ int64_t sh_maxit;
+  __shared__ int sh_fin, sh_end, sh_bad;
+  __shared__ uint64_t sh_mb[kMixThreads / 32];
+  __shared__ int4 sh_places[3][kMixThreads / 32];
+  CGScalars* sc = A.sc;
+  if (sc->done) return;
+  using WalkA = SliceWalk<CI, float, kMixFull>;
+  using WalkT = SliceWalk<CI, __half, kMixTri>;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  char* stage = mix_smem + wid * WalkA::kBytes;
+  const int32_t ns = int32_t((A.n + kSlice - 1) / kSlice);
+  const int32_t s0 = int32_t(int64_t(ns) * blockIdx.x / gridDim.x);
+  const int32_t s1 = int32_t(int64_t(ns) * (blockIdx.x + 1) / gridDim.x);
+  const int32_t last = int32_t(A.n - 1);
+  const int64_t r0 = int64_t(s0) * kSlice, r1 = min(int64_t(s1) * kSlice, A.n);
+  int64_t it = sc->it;
+  if (threadIdx.x == 0) {
+    const double nb = sc->normb > 1.0e-14 ? sc->normb : 1.0;
+    // a residual replacement is due when ||r|| < max(tol ||b||, delta * rlast)
+    // (rlast: the last true residual norm), or at maxit iterations
+    sh_lim = fmax(sc->tol * nb, sc->delta * sc->rlast);
+    sh_maxit = sc->maxit;
+    sh_alpha = sc->alpha;
+    sh_rho = sc->rho;
+    sh_rho0 = sc->rho0;
+    sh_rr = sc->rr;
+    sh_pq = sc->pq;
+    sh_fin = sc->finished;
+    sh_end = 0;
+    sh_bad = 0;
+    sh_beta = it == 0 ? 0.0 : sc->rho / sc->rho0;
+  }
+  for (int64_t i = r0 + threadIdx.x; i < r1; i += kMixThreads) A.zp[i] = make_float2(A.z[i], A.p[i]);
+  unsigned parity = 0;
+  WalkA wa{A.soff, A.sw, A.ci, A.a, stage, 0, s1, 0, 0, 0, 0, sh_places[0], &sh_mb[wid], &sh_bad};
+  WalkT wu{A.soffU, A.swU, A.cu, A.nvU, stage, 0, s1, 0, 0, 0, 0, sh_places[1], &sh_mb[wid], &sh_bad};
+  WalkT wl{A.soffL, A.swL, A.cl, A.nvL, stage, 0, s1, 0, 0, 0, 0, sh_places[2], &sh_mb[wid], &sh_bad};
+  if (lane == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_at(&sh_mb[wid])) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) {
+    sh_places[0][wid] = wa.first_two(s0 + wid);
+    if (FACTOR) {
+      sh_places[1][wid] = wu.first_two(s0 + wid);
+      sh_places[2][wid] = wl.first_two(s0 + wid);
+    }
+  }
+  __syncwarp();
+  bool pending = wa.start(s0 + wid);
+  LoopSync sync{A.lpart, A.larrive, 0u, 0};
+  const double none[1] = {0.0};
+  bool ok = grid_sum<0>(none, 0, sync, sc, [](int, double) {});
+  float alpha = 0.0f;
+  for (int64_t step = 0; ok && step < A.maxits && !sh_end; ++step) {
+    {  // q = A p', (p', q); the last iteration's alpha p into e
+      const float beta = float(sh_beta);
+      float dot[1] = {0.0f};
+      float2 zp = make_float2(0.0f, 0.0f);
+      float rs = 0.0f, vi = 0.0f, si = 0.0f;
+      double ei = 0.0;
+      auto own = [&] {
+        if (wa.s < s1) {
+          const int32_t j = min(wa.s * kSlice + lane, last);
+          zp = A.zp[j];
+          rs = __ldg(A.rs + j);
+          ei = A.e[j];
+          if (FACTOR) {
+            vi = A.v[j];
+            si = __ldg(A.msrow + j);
+          }
+        }
+      };
+      own();
+      while (wa.s < s1) {
+        const int32_t k = wa.s * kSlice + lane, row = min(k, last);
+        const float p = zp.x + beta * zp.y, rp = rs * p, v = vi, sr = si;
+        if (k <= last) A.e[row] = ei + double(alpha) * double(zp.y);
+        const float q = wa.row(
+                            row,
+                            [&](int32_t c) {
+                              const float2 g = A.zp[c];
+                              return (g.x + beta * g.y) - p;
+                            },
+                            own, parity) +
+                        rp;
+        if (k <= last) {
+          A.p[row] = p;
+          if (FACTOR)
+            A.vt[row] = make_float2(v, fabsf(sr) * q);
+          else
+            A.q[row] = q;
+          dot[0] += p * q;
+        }
+      }
+      if (FACTOR) pending = wu.start(s0 + wid);
+      ok = grid_sum32<kMixThreads, 1>(dot, sync, sc, [&](int, double pq) {
+        sh_pq = pq;
+        sh_rho0 = sh_rho;
+        sh_fin = fabs(pq) < DBL_MIN;
+        sh_alpha = sh_fin ? 0.0 : sh_rho / pq;
+      });
+      ok = ok && !sh_bad;
+      if (!ok) break;
+    }
+    alpha = float(sh_alpha);
+    float v[2] = {0.0f, 0.0f};
+    if (FACTOR) {
+      {  // v' = v - alpha t, u = (I+N)^T v'
+        float2 vt = make_float2(0.0f, 0.0f);
+        auto own = [&] {
+          if (wu.s < s1) {
+            const int32_t j = min(wu.s * kSlice + lane, last);
+            vt = A.vt[j];
+          }
+        };
+        own();
+        while (wu.s < s1) {
+          const int32_t k = wu.s * kSlice + lane, row = min(k, last);
+          const float vi = vt.x - alpha * vt.y;
+          if (k <= last) A.v[row] = vi;
+          const float t = wu.row(
+              row,
+              [&](int32_t c) {
+                const float2 g = A.vt[c];
+                return g.x - alpha * g.y;
+              },
+              own, parity);
+          if (k <= last) A.u[row] = vi + t;
+        }
+      }
+      pending = wl.start(s0 + wid);
+      ok = grid_sum<0>(none, 0, sync, sc, [](int, double) {});
+      ok = ok && !sh_bad;
+      if (!ok) break;
+      {  // z = -S (I+N) u
+        float vi = 0.0f, ui = 0.0f, si = 1.0f, pi = 0.0f;
+        auto own = [&] {
+          if (wl.s < s1) {
+            const int32_t j = min(wl.s * kSlice + lane, last);
+            ui = A.u[j];
+            vi = A.v[j];
+            pi = A.p[j];
+            si = __ldg(A.msrow + j);
+          }
+        };
+        own();
+        while (wl.s < s1) {
+          const int32_t k = wl.s * kSlice + lane, row = min(k, last);
+          const float u = ui, p = pi, sr = si, r = vi * __frcp_rn(fabsf(sr));
+          const float acc = u + wl.row(row, [&](int32_t c) { return A.u[c]; }, own, parity);
+          const float zi = sr < 0.0f ? r : -sr * acc;
+          if (k <= last) {
+            A.zp[row] = make_float2(zi, p);
+            v[0] += r * zi;
+            v[1] += r * r;
+          }
+        }
+      }
+    } else {
+      for (int64_t i = r0 + threadIdx.x; i < r1; i += kMixThreads) {
+        const float r = A.r[i] - alpha * A.q[i], p = A.p[i];
+        A.r[i] = r;
+        const float zi = r * __ldg(A.d + i);
+        A.zp[i] = make_float2(zi, p);
+        v[0] += r * zi;
+        v[1] += r * r;
+      }
+    }
+    pending = wa.start(s0 + wid);
+    it += 1;
+    ok = grid_sum32<kMixThreads, 2>(v, sync, sc, [&](int k, double sum) {
+      if (k == 0) {
+        sh_rho = sum;
+        sh_beta = sum / sh_rho0;
+      } else {
+        sh_rr = sum;
+        sh_end = sh_fin || sqrt(sum) < sh_lim || it >= sh_maxit;
+      }
+    });
+    ok = ok && !sh_bad;
+  }
+  // the next pass's first slice may be on its way
+  if (pending) (void)bulk_wait(&sh_mb[wid], parity);
+  if (!ok) {  // a wait ran out
+    if (threadIdx.x == 0) atomicExch(&sc->err, 1);
+    return;
+  }
+  for (int64_t i = r0 + threadIdx.x; i < r1; i += kMixThreads) {
+    A.z[i] = A.zp[i].x;
+    A.e[i] += double(alpha) * double(A.p[i]);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->rho = sh_rho;
+    sc->rho0 = sh_rho0;
+    sc->rr = sh_rr;
+    sc->pq = sh_pq;
+    sc->alpha = sh_alpha;
+    sc->it = it;
+    sc->finished = sh_fin;
+    sc->done = sh_end;
   }
 }
 
@@ -1214,12 +1614,10 @@ __global__ void __launch_bounds__(kBlock) k_outer_res(int64_t n, const int32_t* 
                                                        const double* __restrict__ b,
                                                        const float* __restrict__ d32,
                                                        const float* __restrict__ srow,
-                                                       float* r32, float* r32b,
+                                                       float* __restrict__ r32,
                                                        float* __restrict__ z32,
                                                        float* __restrict__ v32, int first,
                                                        double* partial, CGScalars* sc) {
-  // the current residual buffer (it alternates in the factored iteration)
-  float* __restrict__ rout = (r32b && !first && (sc->it & 1)) ? r32b : r32;
   double v[2] = {0.0, 0.0};
   XG_ROWS(i, n) {
     const int lane = int(i & 31);
@@ -1227,7 +1625,7 @@ __global__ void __launch_bounds__(kBlock) k_outer_res(int64_t n, const int32_t* 
                                          int32_t(i), [&](int32_t c) { return __ldg(x + c); });
     const double ri = b[i] - s;
     const float rf = float(ri);
-    rout[i] = rf;
+    r32[i] = rf;
     if (srow) {
       v32[i] = srow[i] * rf;
     } else {
@@ -1268,12 +1666,16 @@ __global__ void k_jacobi_apply(int64_t n, const double* __restrict__ r, const do
 
 // ---- factor construction
 
-// Row scales s_i = 1/sqrt|a_ii| of the working matrix.
+// Row scales s_i = 1/sqrt|a_ii| of the working matrix; msrow: the same with the
+// sign set at Dirichlet nodes.
 __global__ void k_factor_geom(int64_t n, const double* __restrict__ a,
-                              const int32_t* __restrict__ diagpos, float* __restrict__ srow) {
+                              const int32_t* __restrict__ diagpos, float* __restrict__ srow,
+                              const uint8_t* __restrict__ mask,
+                              float* __restrict__ msrow) {
   int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   srow[i] = float(1.0 / sqrt(fabs(a[diagpos[i]])));
+  msrow[i] = mask[i] ? -srow[i] : srow[i];
 }
 // e_ij = a_ij s_i s_j (0 when i or j is a Dirichlet node) in the lower and
 // upper layouts.
@@ -1353,7 +1755,7 @@ int write_scal(xg_ctx* c, CGDev* d, const CGScalars* h) {
 int build_geom(xg_ctx* c, CGDev* d) {
   cudaStream_t s = c->stream;
   const unsigned nb = blocks_for(d->n, kBlock);
-  k_factor_geom<<<nb, kBlock, 0, s>>>(d->n, d->a, d->diagpos, d->srow);
+  k_factor_geom<<<nb, kBlock, 0, s>>>(d->n, d->a, d->diagpos, d->srow, d->bcmask, d->msrow);
   XG_CHECK_LAUNCH(c);
   k_factor_e<<<nb, kBlock, 0, s>>>(d->n, d->soffL, d->swL, d->colL, d->posL, d->tposU, d->a,
                                    d->srow, d->bcmask, d->eL, d->eU);
@@ -1424,7 +1826,7 @@ int factor_apply64(xg_ctx* c, CGDev* d, const double* r, double* z) {
   launch_dep<k_pc_upper<double, float, Cols32>>(n, s, n, d->soffU, d->swU, Cols32{d->colU}, d->nvU,
       d->v, d->u, d->scal);
   launch_dep<k_pc_lower<double, float, Cols32, 0>>(n, s, n, d->soffL, d->swL, Cols32{d->colL},
-      d->nvL, d->srow, d->bcmask, d->u, r, nullptr, z, d->partial, d->scal);
+      d->nvL, d->srow, d->bcmask, d->u, r, z, d->partial, d->scal);
   XG_CHECK_LAUNCH(c);
   return XG_OK;
 }
@@ -1438,7 +1840,7 @@ void factor_apply32(xg_ctx* c, CGDev* d, CI cu, CI cl) {
   launch_dep<k_pc_upper<float, __half, CI>>(n, s, n, d->soffU, d->swU, cu, d->hvU, d->v32, d->u32,
       d->scal);
   launch_dep<k_pc_lower<float, __half, CI, 0>>(n, s, n, d->soffL, d->swL, cl, d->hvL, d->srow,
-      d->bcmask, d->u32, d->r32, d->r32b, d->z32, d->partial, d->scal);
+      d->bcmask, d->u32, d->r32, d->z32, d->partial, d->scal);
 }
 
 // Rows per block of k_cg_loop and its blocks for n rows: contiguous runs of
@@ -1549,17 +1951,17 @@ int cg_iterate(xg_ctx* c, CGDev* d, int64_t maxit, double tol, CGScalars* h) {
     for (int k = 0; k < kBatch; ++k) {
       double* p0 = d->p[0];
       launch_dep<k_cg_p<double>>(n, s, n, d->z, p0, d->scal);
-      launch_dep<k_cg_a<double, double, Cols32, false>>(n, s, n, d->soff, d->swidth, Cols32{d->col},
-          d->a, d->z, p0, p0, d->q, d->partial, d->scal, static_cast<const float*>(nullptr));
+      launch_dep<k_cg_a<double, double, Cols32>>(n, s, n, d->soff, d->swidth, Cols32{d->col},
+          d->a, p0, d->q, d->partial, d->scal);
       if (d->pc == 2) {
-        launch_dep<k_cg_b<double, true, false>>(n, s, n, d->q, d->d, p0, p0, d->srow, d->r, d->z,
+        launch_dep<k_cg_b<double, true>>(n, s, n, d->q, d->d, p0, d->srow, d->r, d->z,
             d->v, d->x, d->partial, d->scal);
         launch_dep<k_pc_upper<double, float, Cols32>>(n, s, n, d->soffU, d->swU, Cols32{d->colU},
             d->nvU, d->v, d->u, d->scal);
         launch_dep<k_pc_lower<double, float, Cols32, 1>>(n, s, n, d->soffL, d->swL, Cols32{d->colL},
-            d->nvL, d->srow, d->bcmask, d->u, d->r, nullptr, d->z, d->partial, d->scal);
+            d->nvL, d->srow, d->bcmask, d->u, d->r, d->z, d->partial, d->scal);
       } else {
-        launch_dep<k_cg_b<double, false, false>>(n, s, n, d->q, d->d, p0, p0, d->srow, d->r, d->z,
+        launch_dep<k_cg_b<double, false>>(n, s, n, d->q, d->d, p0, d->srow, d->r, d->z,
             d->v, d->x, d->partial, d->scal);
       }
     }
@@ -1571,29 +1973,43 @@ int cg_iterate(xg_ctx* c, CGDev* d, int64_t maxit, double tol, CGScalars* h) {
   return XG_OK;
 }
 
-// A batch of FP32 iterations with column encoding CI.  Factored: q = A p'
-// (k_cg_a), the update with u = (I+N)^T S r' (k_pc_upper_res), then
-// z = -S (I+N) u closing the iteration (k_pc_lower); Jacobi: k_cg_a, k_cg_b.
-template <class CI>
-int mixed_batch(xg_ctx* c, CGDev* d, CI ca, CI cu, CI cl) {
+// The mixed solve's FP32 iterations up to the next residual replacement, by
+// k_mixed_loop launches of at most kLoopIts iterations.
+constexpr int kMixMinSlices = 4;  // slices per block at least: fewer blocks meet sooner
+template <class CI, bool FACTOR>
+int mixed_loop(xg_ctx* c, CGDev* d, CI ca, CI cu, CI cl, CGScalars* h) {
   cudaStream_t s = c->stream;
-  const int64_t n = d->n;
-  for (int k = 0; k < kBatch; ++k) {
-    float *p0 = d->p32[0], *p1 = d->p32[1];
-    launch_dep<k_cg_a<float, float, CI, true>>(n, s, n, d->soff, d->swidth, ca, d->a32, d->z32, p0,
-        p1, d->q32, d->partial, d->scal, static_cast<const float*>(d->rs32));
-    if (d->pc == 2) {
-      launch_dep<k_pc_upper_res<CI>>(n, s, n, d->soffU, d->swU, cu, d->hvU, d->srow, d->q32, p0, p1,
-          d->r32, d->r32b, d->e64, d->u32, d->scal);
-      launch_dep<k_pc_lower<float, __half, CI, 2>>(n, s, n, d->soffL, d->swL, cl, d->hvL, d->srow,
-          d->bcmask, d->u32, d->r32, d->r32b, d->z32, d->partial, d->scal);
-    } else {
-      launch_dep<k_cg_b<float, false, true>>(n, s, n, d->q32, d->d32, p0, p1, d->srow, d->r32,
-          d->z32, d->v32, d->e64, d->partial, d->scal);
+  MixArgs<CI> A{d->n,     kLoopIts, d->soff, d->swidth, d->soffU, d->swU,  d->soffL,
+                d->swL,   ca,       cu,      cl,        d->a32,   d->hvU,  d->hvL,
+                d->rs32,  d->msrow, d->d32,  d->z32,    d->p32,
+                d->q32,   d->r32,   d->v32,  d->u32,    d->zp32,  d->vt32, d->e64,
+                d->lpart, d->larrive, d->scal};
+  const size_t smem = size_t(kMixThreads / 32) * SliceWalk<CI, float, kMixFull>::kBytes;
+  const auto kernel = k_mixed_loop<CI, FACTOR>;
+  XG_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(smem)));
+  const int64_t ns = (d->n + kSlice - 1) / kSlice;
+  const unsigned grid = static_cast<unsigned>(
+      std::min<int64_t>(g_nsm, (ns + kMixMinSlices - 1) / kMixMinSlices));
+  void* args[] = {&A};
+  for (;;) {
+    XG_CUDA(c, cudaMemsetAsync(d->larrive, 0, sizeof(unsigned int), s));
+    XG_CUDA(c, cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(grid),
+                                           dim3(kMixThreads), args, smem, s));
+    int rc = read_scal(c, d, h);
+    if (rc) return rc;
+    if (h->err) {
+      h->err = 0;
+      rc = write_scal(c, d, h);
+      return rc ? rc : fail(c, XG_ERR_DEVICE, "cg_solve_mixed: a grid barrier timed out");
     }
+    if (h->done) return XG_OK;
   }
-  XG_CHECK_LAUNCH(c);
-  return XG_OK;
+}
+template <class CI>
+int mixed_loop(xg_ctx* c, CGDev* d, CI ca, CI cu, CI cl, CGScalars* h) {
+  return d->pc == 2 ? mixed_loop<CI, true>(c, d, ca, cu, cl, h)
+                    : mixed_loop<CI, false>(c, d, ca, cu, cl, h);
 }
 
 // True residual into the FP32 iteration (and the factor passes for z32).
@@ -1602,7 +2018,7 @@ int replace_residual(xg_ctx* c, CGDev* d, int first) {
   const int64_t n = d->n;
   k_outer_res<<<pgrid<k_outer_res>(n), kBlock, 0, s>>>(
       n, d->soff, d->swidth, d->col, d->a, d->x, d->b, d->d32, d->pc == 2 ? d->srow : nullptr,
-      d->r32, d->pc == 2 ? d->r32b : nullptr, d->z32, d->v32, first, d->partial, d->scal);
+      d->r32, d->z32, d->v32, first, d->partial, d->scal);
   XG_CHECK_LAUNCH(c);
   if (d->pc == 2) {
     if (d->use16)
@@ -1929,13 +2345,13 @@ int xg_cg_setup(xg_ctx* c, int64_t nrow, const uint64_t* ia, const uint64_t* ja,
     A.plan(d->p[0], nrow);
     A.plan(d->p[1], nrow);
     A.plan(d->r32, nrow);
-    A.plan(d->r32b, nrow);
     A.plan(d->q32, nrow);
     A.plan(d->z32, nrow);
     A.plan(d->d32, nrow);
     A.plan(d->e64, nrow);
-    A.plan(d->p32[0], nrow);
-    A.plan(d->p32[1], nrow);
+    A.plan(d->p32, nrow);
+    A.plan(d->zp32, nrow);
+    A.plan(d->vt32, nrow);
     A.plan(d->partial, 3 * d->maxgrid);
     A.plan(d->scal, 1);
     A.plan(d->lpart, size_t(6) * g_nsm);
@@ -1958,6 +2374,7 @@ int xg_cg_setup(xg_ctx* c, int64_t nrow, const uint64_t* ia, const uint64_t* ja,
     A.plan(d->eU, colU.size());
     A.plan(d->eF, tot);
     A.plan(d->srow, nrow);
+    A.plan(d->msrow, nrow);
     A.plan(d->v, nrow);
     A.plan(d->u, nrow);
     A.plan(d->t, nrow);
@@ -2143,8 +2560,7 @@ int xg_cg_solve_mixed(xg_ctx* c, int64_t maxit, double tol, double inner_tol,
   const double nb0 = h.normb > 1.0e-14 ? h.normb : 1.0;
   XG_CUDA(c, cudaMemsetAsync(d->e64, 0, d->n * 8, s));
   // the first FP32 iteration reads p with weight beta = 0: make it finite
-  XG_CUDA(c, cudaMemsetAsync(d->p32[0], 0, d->n * 4, s));
-  XG_CUDA(c, cudaMemsetAsync(d->p32[1], 0, d->n * 4, s));
+  XG_CUDA(c, cudaMemsetAsync(d->p32, 0, d->n * 4, s));
   rc = replace_residual(c, d, 1);
   if (rc) return rc;
   rc = read_scal(c, d, &h);
@@ -2161,15 +2577,9 @@ int xg_cg_solve_mixed(xg_ctx* c, int64_t maxit, double tol, double inner_tol,
     h.done = 0;
     rc = write_scal(c, d, &h);
     if (rc) return rc;
-    for (;;) {
-      rc = d->use16 ? mixed_batch<Cols16>(c, d, Cols16{d->col16}, Cols16{d->colU16},
-                                          Cols16{d->colL16})
-                    : mixed_batch<Cols32>(c, d, Cols32{d->col}, Cols32{d->colU}, Cols32{d->colL});
-      if (rc) return rc;
-      rc = read_scal(c, d, &h);
-      if (rc) return rc;
-      if (h.done) break;
-    }
+    rc = d->use16 ? mixed_loop(c, d, Cols16{d->col16}, Cols16{d->colU16}, Cols16{d->colL16}, &h)
+                  : mixed_loop(c, d, Cols32{d->col}, Cols32{d->colU}, Cols32{d->colL}, &h);
+    if (rc) return rc;
     breakdown = h.finished;
     k_add_correction<<<blocks_for(d->n, kBlock), kBlock, 0, s>>>(d->n, d->e64, d->x);
     XG_CHECK_LAUNCH(c);
