@@ -346,15 +346,50 @@ __device__ __forceinline__ void block_min_atomic(double v, unsigned long long* d
   }
 }
 
+// Comparisons of doubles on their bits: on GB300 an FP64 instruction holds
+// its unit for 64 cycles, a comparison too, and integer ones run beside it.
+// The key orders as the numbers do, with -0 at +0.
+__device__ __forceinline__ long long order_key(double x) {
+  const long long b = __double_as_longlong(x);
+  return b < 0 ? (long long)(0x8000000000000000ull) - b : b;
+}
+__device__ __forceinline__ bool is_nan(double x) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+// a < b, false with a NaN
+__device__ __forceinline__ bool less(double a, double b) {
+  return order_key(a) < order_key(b) && !is_nan(a) && !is_nan(b);
+}
+__device__ __forceinline__ bool less(float a, float b) { return a < b; }
+// The sign of x - y (y not a NaN), 0 for a NaN x.
+__device__ __forceinline__ int side(double x, double y) {
+  const long long kx = order_key(x), ky = order_key(y);
+  return is_nan(x) ? 0 : kx > ky ? 1 : kx < ky ? -1 : 0;
+}
+__device__ __forceinline__ int side(float x, float y) { return x > y ? 1 : x < y ? -1 : 0; }
+// x with its sign flipped if `flip`, on the bits.
+__device__ __forceinline__ double flip_if(double x, bool flip) {
+  return __longlong_as_double(__double_as_longlong(x) ^ ((long long)(flip) << 63));
+}
+// 1/d from the hardware's approximation x (about 20 bits): with e = 1 - d x,
+// 1/d = x / (1 - e), taken to e^2 (the third-order Householder step; the rest
+// is e^3, below 1e-17): three FP64 instructions.
+__device__ __forceinline__ double recip(double d) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+  const double e = fma(-d, x, 1.0);
+  return fma(x, fma(e, e, e), x);
+}
+__device__ __forceinline__ float recip(float d) { return 1.0f / d; }
+
 // MUSCL reconstruction of the five flow variables on edge L->R
 // (muscl(), src/Physics/Riemann.cpp:34-143) from the edge-end primitives and
 // the projections g1 = G_L.(x_R - x_L), g2 = G_R.(x_R - x_L).  The van Leer
 // limiter of a pair, phi(r) = (|r| + r)/(|r| + 1) at r = a/b and at 1/r, is
 // the same pair of numbers as 2|a|/(|a|+|b|), 2|b|/(|a|+|b|) for a b > 0 and
 // 0, 0 otherwise.  Both precisions reduce the limited reconstruction
-// algebraically (below): FP64 exactly, with one division for all ten
-// quotients instead of the reference's four per side (the difference is
-// rounding, a few 1e-16 of the increment); FP32 to the harmonic slope.
+// algebraically (below): FP64 exactly, with one quotient per side and
+// component instead of the reference's four (the difference is rounding, a few 1e-16 of the increment); FP32 to the harmonic slope.
 template <class F>
 __device__ __forceinline__ void muscl(const F wl[5], const F wr[5], const F g1[5],
                                       const F g2[5], F l[5], F r[5]) {
@@ -362,51 +397,28 @@ __device__ __forceinline__ void muscl(const F wl[5], const F wr[5], const F g1[5
   const F k = F(1.0) / F(3.0);
   F d1[5], d3[5];
   if constexpr (sizeof(F) == 8) {
-    // FP64: with a = d2 + eps, b = d1 + eps of one sign s (a b > 0), the
+    // FP64: with a = d2 + eps, b = d1 + eps of one sign (a b > 0), the
     // reconstruction wl + ((1-k) d1 phiL + (1+k) d2 phiLi) / 4 is, exactly,
-    // wl + (a b - s (eps/2) ((1-k)|a| + (1+k)|b|)) / (a + b), and the right
-    // state likewise with e = d3 + eps (the reference's form up to rounding,
-    // a few 1e-16 of the increment).  The ten quotients come from one
-    // division (batch inversion: prefix products, one reciprocal,
-    // back-substitution); an unused denominator (a b <= 0) counts as 1, and
-    // a product outside [1e-290, 1e290] falls back to ten divisions.
-    const F h = F(0.5) * eps;
-    F d2[5], num[10], den[10], pre[10];
+    // wl + (a b - (eps/2) ((1-k) a + (1+k) b)) / (a + b), the numerator
+    // (a - h2)(b - h1) - h1 h2 with h1, h2 = (eps/2) (1 -+ k), and
+    // a + b = 2 (g1 + eps) as d1 + d2 = 2 g1; the right state likewise with
+    // d3, g2 (the reference's form up to rounding, a few 1e-16 of the
+    // increment).  An unused denominator (a b <= 0) counts as 1.  The kernel
+    // is bound by its FP64 instructions, so signs are tested on integer bits
+    // and the quotients take three FP64 instructions each (recip).
+    const F h1 = F(0.5) * eps * (F(1.0) - k), h2 = F(0.5) * eps * (F(1.0) + k);
+    const F A0 = F(0.5) * (eps - h2), B0 = eps - h1, H = F(0.5) * h1 * h2;
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-      d2[c] = wr[c] - wl[c];
-      d1[c] = F(2.0) * g1[c] - d2[c];
-      d3[c] = F(2.0) * g2[c] - d2[c];
-      const F a = d2[c] + eps, b = d1[c] + eps, e3 = d3[c] + eps;
-      const F pl = a * b, pr = a * e3;
-      const F sh = copysign(h, a);
-      const F ka = (F(1.0) - k) * fabs(a);
-      num[2 * c] = pl > F(0) ? pl - sh * (ka + (F(1.0) + k) * fabs(b)) : F(0);
-      num[2 * c + 1] = pr > F(0) ? pr - sh * (ka + (F(1.0) + k) * fabs(e3)) : F(0);
-      den[2 * c] = pl > F(0) ? a + b : F(1);
-      den[2 * c + 1] = pr > F(0) ? a + e3 : F(1);
-    }
-    pre[0] = den[0];
-#pragma unroll
-    for (int m = 1; m < 10; ++m) pre[m] = pre[m - 1] * den[m];
-    F q[10];
-    const F ap = fabs(pre[9]);
-    if (ap > F(1e-290) && ap < F(1e290)) {
-      F inv = F(1.0) / pre[9];
-#pragma unroll
-      for (int m = 9; m > 0; --m) {
-        q[m] = inv * pre[m - 1];
-        inv *= den[m];
-      }
-      q[0] = inv;
-    } else {
-#pragma unroll
-      for (int m = 0; m < 10; ++m) q[m] = F(1.0) / den[m];
-    }
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      l[c] = wl[c] + num[2 * c] * q[2 * c];
-      r[c] = wr[c] - num[2 * c + 1] * q[2 * c + 1];
+      const F d2 = wr[c] - wl[c];
+      d1[c] = F(2.0) * g1[c] - d2;
+      d3[c] = F(2.0) * g2[c] - d2;
+      const int sa = side(d2, -eps), pl = sa * side(d1[c], -eps), pr = sa * side(d3[c], -eps);
+      const F A = F(0.5) * d2 + A0;
+      const F nl = A * (d1[c] + B0) - H, nr = A * (d3[c] + B0) - H;
+      const F ql = recip(pl > 0 ? g1[c] + eps : F(1)), qr = recip(pr > 0 ? g2[c] + eps : F(1));
+      l[c] = wl[c] + (pl > 0 ? nl : F(0)) * ql;
+      r[c] = wr[c] - (pr > 0 ? nr : F(0)) * qr;
     }
   } else {
     // FP32: with a = d2 + eps, b = d1 + eps of one sign s, the limited
@@ -455,18 +467,29 @@ __device__ __forceinline__ void muscl(const F wl[5], const F wr[5], const F g1[5
       r[4] = wr[4] - (pr > 0.f ? __fdividef(pr, a + e3) : 0.f);
     }
   }
-  if (wl[0] < d1[0] || wl[4] < d1[4]) {
+  if (less(wl[0], d1[0]) || less(wl[4], d1[4])) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) l[c] = wl[c];
   }
-  if (wr[0] < -d3[0] || wr[4] < -d3[4]) {
+  if (less(wr[0], -d3[0]) || less(wr[4], -d3[4])) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) r[c] = wr[c];
   }
 }
 
-// sqrt: IEEE in double; x * rsqrt(x) in float (x >= 0).
-__device__ __forceinline__ double xsqrt(double x) { return sqrt(x); }
+// sqrt: in double from the hardware's approximation y of 1/sqrt(x) (about 20
+// bits): with s = x y and e = 1 - x y^2, sqrt(x) = s / sqrt(1 - e) =
+// s (1 + e/2 + 3 e^2/8 + ...), the rest below 1e-17: five FP64 instructions;
+// the library's root for zero, negative, subnormal and very large x.
+// x * rsqrt(x) in float (x >= 0).
+__device__ __forceinline__ double xsqrt(double x) {
+  const int hi = __double2hiint(x);
+  if (hi < 0x01000000 || hi >= 0x7f000000) return sqrt(x);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double s = x * y, e = fma(-s, y, 1.0);
+  return fma(s * e, fma(0.375, e, 0.5), s);
+}
 __device__ __forceinline__ float xsqrt(float x) { return x > 0.f ? x * rsqrtf(x) : 0.f; }
 
 // Rusanov edge flux (rusanov(), src/Physics/Riemann.cpp:369-478).
@@ -498,7 +521,7 @@ __device__ __forceinline__ void rusanov(const F wl[5], const F wr[5], const F g1
   const F gl = gamma * (gamma - F(1.0)) * (nx * nx + ny * ny + nz * nz);
   F sl = fabs(vnL) + xsqrt(gl * cLe);
   F sr = fabs(vnR) + xsqrt(gl * cRe);
-  F fw = sl > sr ? sl : sr;
+  F fw = less(sr, sl) ? sl : sr;
   f[0] = l[0] * vnL + r[0] * vnR + fw * (r[0] - l[0]);
   f[1] = l[1] * vnL + r[1] * vnR + (pL + pR) * nx + fw * (r[1] - l[1]);
   f[2] = l[2] * vnL + r[2] * vnR + (pL + pR) * ny + fw * (r[2] - l[2]);
@@ -1169,11 +1192,10 @@ __global__ void __launch_bounds__(flux_block<F>(), sizeof(F) == 4 ? 3 : 1)
         hllc(wl, wr, g1, g2, d0, d1, d2, gamma, stab2 != 0, stab2coef, f);
       else
         rusanov(wl, wr, g1, g2, d0, d1, d2, gamma, stab2 != 0, stab2coef, f);
-      const F sg = first ? F(-1) : F(1);
 #pragma unroll
       for (int c = 0; c < 5; ++c) {
-        R[c] += sg * f[c];
-        fo[c] = -sg * f[c];
+        fo[c] = flip_if(f[c], !first);
+        R[c] -= fo[c];
       }
     }
     store_f4(fbuf, dst, fo);
