@@ -24,9 +24,9 @@
 //             canonical edge, PAD for padding) and the canonical edge
 //             integral D (16 bytes in FP32 mode, 32 in FP64 mode).
 //   ivol, cbrtv  1/vol (double) and cbrt(vol) (float) for the FP32 epilogue
-// In FP64 mode every edge flux is evaluated with the canonical orientation
-// (left = first end), so the sum is the reference's up to summation order;
-// FP32 mode evaluates it in the owner's orientation.  Each node owns its
+// Every edge flux is evaluated in its owner's orientation; in FP64 mode it is
+// the canonical one's (left = first end) negative up to the order of its sums,
+// so the result is the reference's up to summation order.  Each node owns its
 // writes: no atomics except the scalar CFL minimum.
 
 #include <algorithm>
@@ -354,13 +354,24 @@ __device__ __forceinline__ long long order_key(double x) {
   return b < 0 ? (long long)(0x8000000000000000ull) - b : b;
 }
 __device__ __forceinline__ bool is_nan(double x) {
-  return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+  // by halves: a compiler turns the 64-bit form back into an FP64 comparison
+  return (unsigned(__double2hiint(x)) & 0x7fffffffu) + (__double2loint(x) != 0) > 0x7ff00000u;
 }
 // a < b, false with a NaN
 __device__ __forceinline__ bool less(double a, double b) {
   return order_key(a) < order_key(b) && !is_nan(a) && !is_nan(b);
 }
+// a < -b
+__device__ __forceinline__ bool less_neg(double a, double b) {
+  return order_key(a) < -order_key(b) && !is_nan(a) && !is_nan(b);
+}
+// a <= b
+__device__ __forceinline__ bool at_most(double a, double b) {
+  return order_key(a) <= order_key(b) && !is_nan(a) && !is_nan(b);
+}
+__device__ __forceinline__ bool at_most(float a, float b) { return a <= b; }
 __device__ __forceinline__ bool less(float a, float b) { return a < b; }
+__device__ __forceinline__ bool less_neg(float a, float b) { return a < -b; }
 // The sign of x - y (y not a NaN), 0 for a NaN x.
 __device__ __forceinline__ int side(double x, double y) {
   const long long kx = order_key(x), ky = order_key(y);
@@ -371,16 +382,37 @@ __device__ __forceinline__ int side(float x, float y) { return x > y ? 1 : x < y
 __device__ __forceinline__ double flip_if(double x, bool flip) {
   return __longlong_as_double(__double_as_longlong(x) ^ ((long long)(flip) << 63));
 }
-// 1/d from the hardware's approximation x (about 20 bits): with e = 1 - d x,
+// |x| cut to a float and back, on the bits (conversions are as slow as FP64
+// arithmetic), for 2^-120 <= |x| < 2^120 (in_float).
+__device__ __forceinline__ bool in_float(double x) {
+  return ((unsigned(__double2hiint(x)) >> 20) & 0x7ffu) - 903u < 240u;
+}
+__device__ __forceinline__ float cut_abs(double x) {
+  const unsigned hi = unsigned(__double2hiint(x)) & 0x7fffffffu;
+  return __uint_as_float(((hi - (896u << 20)) << 3) | (unsigned(__double2loint(x)) >> 29));
+}
+__device__ __forceinline__ double widen(float x, unsigned sign) {  // x > 0
+  const unsigned b = __float_as_uint(x);
+  return __hiloint2double(int(((b >> 3) + (896u << 20)) | sign), int(b << 29));
+}
+__device__ __forceinline__ float flip_if(float x, bool flip) {
+  return __uint_as_float(__float_as_uint(x) ^ (unsigned(flip) << 31));
+}
+// 1/d from the FP32 approximation x of 1/d (about 22 bits): with e = 1 - d x,
 // 1/d = x / (1 - e), taken to e^2 (the third-order Householder step; the rest
-// is e^3, below 1e-17): three FP64 instructions.
+// is e^3, below 1e-18): three FP64 instructions.
 __device__ __forceinline__ double recip(double d) {
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+  if (!in_float(d)) return 1.0 / d;
+  float a;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(cut_abs(d)));
+  const double x = widen(a, unsigned(__double2hiint(d)) & 0x80000000u);
   const double e = fma(-d, x, 1.0);
   return fma(x, fma(e, e, e), x);
 }
 __device__ __forceinline__ float recip(float d) { return 1.0f / d; }
+// a / b, in double as a times ib = recip(b)
+__device__ __forceinline__ double over(double a, double, double ib) { return a * ib; }
+__device__ __forceinline__ float over(float a, float b, float) { return a / b; }
 
 // MUSCL reconstruction of the five flow variables on edge L->R
 // (muscl(), src/Physics/Riemann.cpp:34-143) from the edge-end primitives and
@@ -392,11 +424,11 @@ __device__ __forceinline__ float recip(float d) { return 1.0f / d; }
 // component instead of the reference's four (the difference is rounding, a few 1e-16 of the increment); FP32 to the harmonic slope.
 template <class F>
 __device__ __forceinline__ void muscl(const F wl[5], const F wr[5], const F g1[5],
-                                      const F g2[5], F l[5], F r[5]) {
-  const F eps = F(1.0e-9);
+                                      const F g2[5], bool back, F l[5], F r[5]) {
   const F k = F(1.0) / F(3.0);
   F d1[5], d3[5];
   if constexpr (sizeof(F) == 8) {
+    const F eps = flip_if(1.0e-9, back);
     // FP64: with a = d2 + eps, b = d1 + eps of one sign (a b > 0), the
     // reconstruction wl + ((1-k) d1 phiL + (1+k) d2 phiLi) / 4 is, exactly,
     // wl + (a b - (eps/2) ((1-k) a + (1+k) b)) / (a + b), the numerator
@@ -406,14 +438,20 @@ __device__ __forceinline__ void muscl(const F wl[5], const F wr[5], const F g1[5
     // increment).  An unused denominator (a b <= 0) counts as 1.  The kernel
     // is bound by its FP64 instructions, so signs are tested on integer bits
     // and the quotients take three FP64 instructions each (recip).
-    const F h1 = F(0.5) * eps * (F(1.0) - k), h2 = F(0.5) * eps * (F(1.0) + k);
-    const F A0 = F(0.5) * (eps - h2), B0 = eps - h1, H = F(0.5) * h1 * h2;
+    // `back`: the ends are given as R, L, so every difference and slope has
+    // the other sign; with eps negated as well every product, and so each end's
+    // reconstruction, is the same number as with the ends in order.
+    constexpr F h1 = F(0.5e-9) * (F(1.0) - F(1.0) / F(3.0)), h2 = F(0.5e-9) * (F(1.0) + F(1.0) / F(3.0));
+    constexpr F H = F(0.5) * h1 * h2;
+    const F A0 = flip_if(F(0.5) * (F(1.0e-9) - h2), back), B0 = flip_if(F(1.0e-9) - h1, back);
+    const F meps = flip_if(1.0e-9, !back);
+    (void)k;
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
       const F d2 = wr[c] - wl[c];
       d1[c] = F(2.0) * g1[c] - d2;
       d3[c] = F(2.0) * g2[c] - d2;
-      const int sa = side(d2, -eps), pl = sa * side(d1[c], -eps), pr = sa * side(d3[c], -eps);
+      const int sa = side(d2, meps), pl = sa * side(d1[c], meps), pr = sa * side(d3[c], meps);
       const F A = F(0.5) * d2 + A0;
       const F nl = A * (d1[c] + B0) - H, nr = A * (d3[c] + B0) - H;
       const F ql = recip(pl > 0 ? g1[c] + eps : F(1)), qr = recip(pr > 0 ? g2[c] + eps : F(1));
@@ -429,7 +467,9 @@ __device__ __forceinline__ void muscl(const F wl[5], const F wr[5], const F g1[5
     // rounding): one product, one sum and one quotient per side.
     // Components 0-1 and 2-3 go through the packed FP32x2 pipe (two
     // components per instruction, each rounded as its scalar FMA), 4 alone.
+    const F eps = F(1.0e-9);
     (void)k;
+    (void)back;
 #pragma unroll
     for (int c = 0; c < 4; c += 2) {
       const float2 m1 = make_float2(-1.f, -1.f), two = make_float2(2.f, 2.f),
@@ -467,26 +507,28 @@ __device__ __forceinline__ void muscl(const F wl[5], const F wr[5], const F g1[5
       r[4] = wr[4] - (pr > 0.f ? __fdividef(pr, a + e3) : 0.f);
     }
   }
+  // the reconstructed density or energy would pass zero (the same two tests
+  // whichever end is first)
   if (less(wl[0], d1[0]) || less(wl[4], d1[4])) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) l[c] = wl[c];
   }
-  if (less(wr[0], -d3[0]) || less(wr[4], -d3[4])) {
+  if (less_neg(wr[0], d3[0]) || less_neg(wr[4], d3[4])) {
 #pragma unroll
     for (int c = 0; c < 5; ++c) r[c] = wr[c];
   }
 }
 
-// sqrt: in double from the hardware's approximation y of 1/sqrt(x) (about 20
-// bits): with s = x y and e = 1 - x y^2, sqrt(x) = s / sqrt(1 - e) =
-// s (1 + e/2 + 3 e^2/8 + ...), the rest below 1e-17: five FP64 instructions;
-// the library's root for zero, negative, subnormal and very large x.
+// sqrt: in double from the FP32 approximation y of 1/sqrt(x) (about 22 bits):
+// with s = x y and e = 1 - x y^2, sqrt(x) = s / sqrt(1 - e) =
+// s (1 + e/2 + 3 e^2/8 + ...), the rest below 1e-18: five FP64 instructions;
+// the library's root for negative x and outside FP32's range.
 // x * rsqrt(x) in float (x >= 0).
 __device__ __forceinline__ double xsqrt(double x) {
-  const int hi = __double2hiint(x);
-  if (hi < 0x01000000 || hi >= 0x7f000000) return sqrt(x);
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  if (!in_float(x) || __double2hiint(x) < 0) return sqrt(x);
+  float a;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(cut_abs(x)));
+  const double y = widen(a, 0u);
   const double s = x * y, e = fma(-s, y, 1.0);
   return fma(s * e, fma(0.375, e, 0.5), s);
 }
@@ -496,9 +538,9 @@ __device__ __forceinline__ float xsqrt(float x) { return x > 0.f ? x * rsqrtf(x)
 template <class F>
 __device__ __forceinline__ void rusanov(const F wl[5], const F wr[5], const F g1[5],
                                         const F g2[5], F nx, F ny, F nz, F gamma, bool stab2,
-                                        F stab2coef, F f[5]) {
+                                        F stab2coef, bool back, F f[5]) {
   F l[5], r[5];
-  muscl(wl, wr, g1, g2, l, r);
+  muscl(wl, wr, g1, g2, back, l, r);
   F pL = l[0] * l[4] * (gamma - F(1.0));
   F pR = r[0] * r[4] * (gamma - F(1.0));
   const F cLe = l[4], cRe = r[4];
@@ -538,18 +580,23 @@ __device__ __forceinline__ void rusanov(const F wl[5], const F wr[5], const F g1
 template <class F>
 __device__ __forceinline__ void hllc(const F wl[5], const F wr[5], const F g1[5], const F g2[5],
                                      F dx, F dy, F dz, F gamma, bool stab2, F stab2coef,
-                                     F f[5]) {
+                                     bool back, F f[5]) {
   F l[5], r[5];
-  muscl(wl, wr, g1, g2, l, r);
+  muscl(wl, wr, g1, g2, back, l, r);
   F nx = -dx, ny = -dy, nz = -dz;
-  F len = sqrt(nx * nx + ny * ny + nz * nz);
-  nx /= len;
-  ny /= len;
-  nz /= len;
+  // FP64: a root, quotients and comparisons as in rusanov and muscl; c^2 as
+  // there from the internal energy
+  const F len2 = nx * nx + ny * ny + nz * nz;
+  const F len = sizeof(F) == 8 ? F(xsqrt(len2)) : F(sqrt(len2));
+  const F ilen = recip(len);
+  nx = over(nx, len, ilen);
+  ny = over(ny, len, ilen);
+  nz = over(nz, len, ilen);
   F qL = l[1] * nx + l[2] * ny + l[3] * nz;
   F qR = r[1] * nx + r[2] * ny + r[3] * nz;
   F pL = l[0] * l[4] * (gamma - F(1.0));
   F pR = r[0] * r[4] * (gamma - F(1.0));
+  const F cLe = l[4], cRe = r[4], gg = gamma * (gamma - F(1.0));
   l[4] = (l[4] + F(0.5) * (l[1] * l[1] + l[2] * l[2] + l[3] * l[3])) * l[0];
   l[1] *= l[0];
   l[2] *= l[0];
@@ -558,42 +605,44 @@ __device__ __forceinline__ void hllc(const F wl[5], const F wr[5], const F g1[5]
   r[1] *= r[0];
   r[2] *= r[0];
   r[3] *= r[0];
-  F cL = sqrt(gamma * pL / l[0]);
-  F cR = sqrt(gamma * pR / r[0]);
+  F cL = sizeof(F) == 8 ? F(xsqrt(gg * cLe)) : F(sqrt(gamma * pL / l[0]));
+  F cR = sizeof(F) == 8 ? F(xsqrt(gg * cRe)) : F(sqrt(gamma * pR / r[0]));
   F sL = fmin(qL - cL, qR - cR);
   F sR = fmax(qL + cL, qR + cR);
   F tL = sL - qL;
   F tR = sR - qR;
-  F sM = (r[0] * qR * tR - l[0] * qL * tL + pL - pR) / (r[0] * tR - l[0] * tL);
+  const F sMd = r[0] * tR - l[0] * tL;
+  F sM = over(r[0] * qR * tR - l[0] * qL * tL + pL - pR, sMd, recip(sMd));
   F pS = pL - l[0] * tL * (qL - sM);
   F L2 = F(-2.0) * len;
-  if (sL > F(0.0)) {
+  const F o = F(0.0);
+  if (less(o, sL)) {
     F qL2 = qL * L2;
     f[0] = l[0] * qL2;
     f[1] = l[1] * qL2 + pL * (nx * L2);
     f[2] = l[2] * qL2 + pL * (ny * L2);
     f[3] = l[3] * qL2 + pL * (nz * L2);
     f[4] = (l[4] + pL) * qL2;
-  } else if (sL <= F(0.0) && sM > F(0.0)) {
-    F s = sL - sM;
-    F uL0 = tL * l[0] / s;
-    F uL1 = (tL * l[1] + (pS - pL) * nx) / s;
-    F uL2 = (tL * l[2] + (pS - pL) * ny) / s;
-    F uL3 = (tL * l[3] + (pS - pL) * nz) / s;
-    F uL4 = (tL * l[4] - pL * qL + pS * sM) / s;
+  } else if (at_most(sL, o) && less(o, sM)) {
+    const F s = sL - sM, is = recip(s);
+    F uL0 = over(tL * l[0], s, is);
+    F uL1 = over(tL * l[1] + (pS - pL) * nx, s, is);
+    F uL2 = over(tL * l[2] + (pS - pL) * ny, s, is);
+    F uL3 = over(tL * l[3] + (pS - pL) * nz, s, is);
+    F uL4 = over(tL * l[4] - pL * qL + pS * sM, s, is);
     F qL2 = qL * L2, sL2 = sL * L2;
     f[0] = l[0] * qL2 + sL2 * (uL0 - l[0]);
     f[1] = l[1] * qL2 + pL * (nx * L2) + sL2 * (uL1 - l[1]);
     f[2] = l[2] * qL2 + pL * (ny * L2) + sL2 * (uL2 - l[2]);
     f[3] = l[3] * qL2 + pL * (nz * L2) + sL2 * (uL3 - l[3]);
     f[4] = (l[4] + pL) * qL2 + sL2 * (uL4 - l[4]);
-  } else if (sM <= F(0.0) && sR >= F(0.0)) {
-    F s = sR - sM;
-    F uR0 = tR * r[0] / s;
-    F uR1 = (tR * r[1] + (pS - pR) * nx) / s;
-    F uR2 = (tR * r[2] + (pS - pR) * ny) / s;
-    F uR3 = (tR * r[3] + (pS - pR) * nz) / s;
-    F uR4 = (tR * r[4] - pR * qR + pS * sM) / s;
+  } else if (at_most(sM, o) && at_most(o, sR)) {
+    const F s = sR - sM, is = recip(s);
+    F uR0 = over(tR * r[0], s, is);
+    F uR1 = over(tR * r[1] + (pS - pR) * nx, s, is);
+    F uR2 = over(tR * r[2] + (pS - pR) * ny, s, is);
+    F uR3 = over(tR * r[3] + (pS - pR) * nz, s, is);
+    F uR4 = over(tR * r[4] - pR * qR + pS * sM, s, is);
     F qR2 = qR * L2, sR2 = sR * L2;
     f[0] = r[0] * qR2 + sR2 * (uR0 - r[0]);
     f[1] = r[1] * qR2 + pR * (nx * L2) + sR2 * (uR1 - r[1]);
@@ -611,7 +660,7 @@ __device__ __forceinline__ void hllc(const F wl[5], const F wr[5], const F g1[5]
   if (stab2) {
     F sl = fabs(qL) + cL;
     F sr = fabs(qR) + cR;
-    F fws = stab2coef * (sl > sr ? sl : sr) * len;
+    F fws = stab2coef * (less(sr, sl) ? sl : sr) * len;
 #pragma unroll
     for (int c = 0; c < 5; ++c) f[c] -= fws * (l[c] - r[c]);
   }
@@ -1088,12 +1137,15 @@ __device__ __forceinline__ float node_dt_f(const double ud[5], float L, float g)
 }
 
 // Half-edge residual, pass 1: every edge flux once, at the edge's owner end
-// (riemann::rhs advdom, src/Physics/Riemann.cpp:695-759), in the edge's
-// canonical orientation in FP64 mode (-f summed into the owner's partial
-// residual when the owner is the first end, +f otherwise) and in the owner's
-// orientation in FP32 mode; the other end's contribution is stored into
-// that end's list-2 slot (pos1), so the second pass reads its fluxes as a
-// coalesced stream.
+// (riemann::rhs advdom, src/Physics/Riemann.cpp:695-759), in the owner's
+// orientation, subtracted from the owner's partial residual; the other end's
+// contribution is stored into that end's list-2 slot (pos1), so the second
+// pass reads its fluxes as a coalesced stream.
+//
+// In FP64 the bound is the FP64 pipe: 212 instructions an edge, the pipe 89 %
+// busy, 1454 us at 81^3.  With comparisons, negations and selects in FP64, the
+// limiter's products beside its quotients and the library's division and roots
+// it was 298 an edge and 1935 us.
 template <class F>
 struct Half {
   const int32_t* soff1;
@@ -1153,53 +1205,33 @@ __global__ void __launch_bounds__(flux_block<F>(), sizeof(F) == 4 ? 3 : 1)
     load8(W + int64_t(q) * 8, wq);
     load16(G + int64_t(q) * 16, gq);
     const F v0 = wq[5] - wp[5], v1 = wq[6] - wp[6], v2 = wq[7] - wp[7];
-    F f[5], fo[5];
+    // The flux in the owner's orientation (p -> q, the edge integral signed
+    // accordingly), with no selects per component.  In FP64 the limiter's
+    // regularisation keeps the edge's own direction (muscl's `back`), so the
+    // flux is the canonical one up to the order of its sums; in FP32 it
+    // differs through that 1e-9 alone, far below FP32 rounding.
+    F f[5], g1[5], g2[5];
     if constexpr (sizeof(F) == 4) {
-      // FP32: the flux in the owner's orientation (p -> q, the edge integral
-      // signed accordingly), with no per-component orientation selects; it
-      // differs from the canonical-orientation flux only through the
-      // limiter's 1e-9 regularisation, far below FP32 rounding of the sums
-      F g1[5], g2[5];
       proj5(gp, v0, v1, v2, g1);
       proj5(gq, v0, v1, v2, g2);
-      if (!first) {
-        d0 = -d0;
-        d1 = -d1;
-        d2 = -d2;
-      }
-      if (FLUX == XG_HLLC)
-        hllc(wp, wq, g1, g2, d0, d1, d2, gamma, stab2 != 0, stab2coef, f);
-      else
-        rusanov(wp, wq, g1, g2, d0, d1, d2, gamma, stab2 != 0, stab2coef, f);
-#pragma unroll
-      for (int c = 0; c < 5; ++c) {
-        R[c] -= f[c];
-        fo[c] = f[c];
-      }
     } else {
-      // FP64: the canonical orientation (left = first end), as the reference
-      F wl[5], wr[5], g1[5], g2[5];
 #pragma unroll
       for (int c = 0; c < 5; ++c) {
-        const F A = proj(gp + 3 * c, v0, v1, v2);
-        const F B = proj(gq + 3 * c, v0, v1, v2);
-        g1[c] = first ? A : -B;
-        g2[c] = first ? B : -A;
-        wl[c] = first ? wp[c] : wq[c];
-        wr[c] = first ? wq[c] : wp[c];
-      }
-      if (FLUX == XG_HLLC)
-        hllc(wl, wr, g1, g2, d0, d1, d2, gamma, stab2 != 0, stab2coef, f);
-      else
-        rusanov(wl, wr, g1, g2, d0, d1, d2, gamma, stab2 != 0, stab2coef, f);
-#pragma unroll
-      for (int c = 0; c < 5; ++c) {
-        fo[c] = flip_if(f[c], !first);
-        R[c] -= fo[c];
+        g1[c] = proj(gp + 3 * c, v0, v1, v2);
+        g2[c] = proj(gq + 3 * c, v0, v1, v2);
       }
     }
-    store_f4(fbuf, dst, fo);
-    fbuf[4 * h.nent2 + dst] = fo[4];
+    d0 = flip_if(d0, !first);
+    d1 = flip_if(d1, !first);
+    d2 = flip_if(d2, !first);
+    if (FLUX == XG_HLLC)
+      hllc(wp, wq, g1, g2, d0, d1, d2, gamma, stab2 != 0, stab2coef, !first, f);
+    else
+      rusanov(wp, wq, g1, g2, d0, d1, d2, gamma, stab2 != 0, stab2coef, !first, f);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) R[c] -= f[c];
+    store_f4(fbuf, dst, f);
+    fbuf[4 * h.nent2 + dst] = f[4];
   }
   cp_async_wait<0>();
 #pragma unroll
@@ -1615,9 +1647,9 @@ __global__ void __launch_bounds__(kBlock)
   proj5(gp, v0, v1, v2, g1);
   proj5(gq, v0, v1, v2, g2);
   if (FLUX == XG_HLLC)
-    hllc(wp, wq, g1, g2, d.x, d.y, d.z, gamma, stab2 != 0, stab2coef, f);
+    hllc(wp, wq, g1, g2, d.x, d.y, d.z, gamma, stab2 != 0, stab2coef, false, f);
   else
-    rusanov(wp, wq, g1, g2, d.x, d.y, d.z, gamma, stab2 != 0, stab2coef, f);
+    rusanov(wp, wq, g1, g2, d.x, d.y, d.z, gamma, stab2 != 0, stab2coef, false, f);
   // each record is read and written by this thread alone in this launch
   float rp[8], rq[8];
   load8(R + int64_t(ends.x) * 8, rp);
