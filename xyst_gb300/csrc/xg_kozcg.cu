@@ -369,6 +369,24 @@ __device__ __forceinline__ ElemGeo<F> elem_geo(const F* __restrict__ geo, int64_
   return t;
 }
 
+// KozCG::aec (KozCG.cpp:794-814) in FP32, k = ctau J/120: sum_b k (3 or -1)
+// u_b, rounded term by term as the reference's sum.  The rounding it leaves in a
+// nearly uniform component keeps the limiter's quotients bounded; formed as
+// k (4 u_a - sum), exactly zero there, a run's differences from itself (the
+// order of the atomics) grew from 6e-8 to 2e-6 of the state in 40 steps at 97^3.
+template <class U>
+__device__ __forceinline__ void aec32(float k, const U& u, float aec[4][5]) {
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      float s = 0.f;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) s += (k * (a == b ? 3.f : -1.f)) * u[b][c];
+      aec[a][c] = s;
+    }
+}
+
 // kozak::rhs for one tet (Kozak.cpp:73-173): the residual r[a][c] of its
 // four nodes, and with fct the antidiffusive element contributions of
 // KozCG::aec (KozCG.cpp:794-814) aec[a][c], from the node records V.
@@ -378,7 +396,7 @@ __device__ __forceinline__ ElemGeo<F> elem_geo(const F* __restrict__ geo, int64_
 // F.g = (v.g) (rho, m, E + p) + p (0, g, 0), 12 operations a node where the
 // sum over directions took 36; the fourth node's residual is minus the sum of
 // the others (the gradients add to zero); and aec_a = ctau J/120 (4 u_a -
-// sum_b u_b), which is exactly zero for a uniform component: about 190
+// sum_b u_b), which is exactly zero for a uniform component (FP32: aec32): about 190
 // operations a tet for 480, k_elem_rhs64 1259 -> 548 us at 65^3, its FP64
 // units busy throughout.
 template <class F>
@@ -449,10 +467,14 @@ __device__ __forceinline__ void elem_terms(int64_t n, int64_t ne, int64_t e,
   }
   if (fct) {
     const F k = ctau * t.j120;
+    if constexpr (sizeof(F) == 8) {
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int c = 0; c < 5; ++c) aec[a][c] = k * (F(4.0) * u[a][c] - sum[c]);
+        for (int c = 0; c < 5; ++c) aec[a][c] = k * (F(4.0) * u[a][c] - sum[c]);
+    } else {
+      aec32(k, u, aec);
+    }
   } else {
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -814,12 +836,7 @@ __global__ void __launch_bounds__(kBlock) k_elem_lim32(int64_t n, int64_t ne,
   float u[4][8], aec[4][5], ca[4][5];
 #pragma unroll
   for (int a = 0; a < 4; ++a) load_node(V, N[a], u[a]);
-#pragma unroll
-  for (int c = 0; c < 5; ++c) {
-    const float sum = u[0][c] + u[1][c] + u[2][c] + u[3][c];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) aec[a][c] = k * (4.f * u[a][c] - sum);
-  }
+  aec32(k, u, aec);
   elem_limit<float>(N, Q, sysmask, aec, ca);
   for (int a = 0; a < 4; ++a) add5<kAR>(A, n, N[a], ca[a]);
 }
