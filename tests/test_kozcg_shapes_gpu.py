@@ -73,3 +73,23 @@ def test_source_terms(precision):
         s.set_source("taylor_green", source_prm("taylor_green"))
         s.set_state(U, 0.2)
     assert relerr(d.rhs(U, 1e-3), o.rhs(U, 1e-3)) < (1e-12 if precision == "fp64" else 2e-6)
+
+
+@pytest.mark.parametrize("ne", [1, 63, 64, 65, 200])
+@pytest.mark.parametrize("fct", [True, False])
+def test_elements_without_shared_nodes(ne, fct):
+    """The FP32 block sums where every element's nodes are its own (as many
+    distinct nodes as a block can hold) and where the last block is ragged."""
+    rng = np.random.default_rng(ne)
+    corner = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]], float)
+    coord = (corner[None] + 0.1 * rng.random((ne, 4, 3)) +
+             3.0 * np.arange(ne)[:, None, None]).reshape(-1, 3).T.copy()
+    inpoel = rng.permutation(4 * ne).reshape(ne, 4)
+    where = np.empty(4 * ne, np.int64)
+    where[inpoel.reshape(-1)] = np.arange(4 * ne)
+    coord = np.ascontiguousarray(coord[:, where])
+    v = riecg.volumes(coord, inpoel)
+    d = kozcg.KozCG(ctx(), coord, v, inpoel, precision="fp32", fct=fct)
+    o = oracle.KozCG(coord, v, inpoel, fct=fct)
+    U = random_state(v.size, ne)
+    assert relerr(d.rhs(U, 1e-3), o.rhs(U, 1e-3)) < 1e-5

@@ -66,6 +66,10 @@ struct KozCGDev {
   int64_t n = 0, ne = 0;
   xg_kozcg_params prm{};
   int32_t* inpoel = nullptr;
+  // FP32: per block of kFB elements its distinct nodes and their slots
+  int32_t *bptr = nullptr, *bnode = nullptr;
+  uint16_t* bstart = nullptr;
+  uint8_t* bslot = nullptr;
   double *xyz = nullptr, *ivol = nullptr;  // coordinates, 1/vol
   double* cbrtv = nullptr;                 // cbrt(vol)
   double *U = nullptr, *R = nullptr, *P = nullptr, *A = nullptr;
@@ -219,10 +223,10 @@ __device__ __forceinline__ float oval(unsigned int k) {
   return __uint_as_float((k >> 31) ? (k & 0x7fffffffu) : ~k);
 }
 
-// FP32 element sums are node records, so that one element adds a node's
-// contribution with 16-byte vector atomics (red.global.add.v4.f32) instead of
-// one atomic per component: R and P share a [n][16] record (R at 0..4, P+/- at
-// 5..14), A has [n][8].
+// FP32 element sums are node records, so that a node's contribution is added
+// with 16-byte vector atomics (red.global.add.v4.f32) instead of one atomic per
+// component: R and P share a [n][16] record (R at 0..4, P+/- at 5..14), A has
+// [n][8].
 constexpr int kRP = 16;   // FP32 R+P record
 constexpr int kAR = 8;    // FP32 A record
 constexpr int kGB = 4;    // FP64 node gather: slots loaded together
@@ -278,13 +282,6 @@ __device__ __forceinline__ void store10(T* p, const T o[10]) {
     reinterpret_cast<int2*>(p + 8)[0] = make_int2(q[8], q[9]);
   }
 }
-// FP32 mode: r[5] added to node i's record of R (S = kRP) or A (S = kAR).
-template <int S>
-__device__ __forceinline__ void add5(float* R, int64_t, int64_t i, const float r[5]) {
-  atomicAdd(reinterpret_cast<float4*>(R + i * S), make_float4(r[0], r[1], r[2], r[3]));
-  atomicAdd(R + i * S + 4, r[4]);
-}
-
 // What the element passes read of a node, one record of eight values (density,
 // momenta, total energy, pressure, 1/density, pad): 32 or 64 bytes in one or two
 // accesses, where component arrays take a sector each.  The node-wise
@@ -483,42 +480,118 @@ __device__ __forceinline__ void elem_terms(int64_t n, int64_t ne, int64_t e,
   }
 }
 
+// The FP32 residual pass is made of blocks of kFB elements (a slot 4 e + a of a
+// block fits a byte).  Atomics bound it: at about 200 G of 16 bytes a second,
+// four nodes of four each an element took 396 us at 97^3.  Consecutive elements
+// share nodes (those of 64 hold 50 distinct ones of 256 with locality
+// numbering, 71 numbered at random), so a block leaves its elements'
+// contributions in shared memory, adds them per distinct node (lists made once
+// per mesh) and hands one record a node to the atomics: 262 us, with 14 blocks
+// an SM (12: 287).  The limiting pass, whose two atomics a node are not its
+// bound, gained nothing (227 against 223), nor did either pass from the nodes'
+// records staged in shared memory (308 and 269).
+constexpr int kFB = 64;
+constexpr int kFW = kFB / 32;
+constexpr int kNG = 6;  // nodes a warp adds together, a lane per component
+struct BlockLists {
+  const int32_t *ptr, *node;  // the block's distinct nodes, most slots first
+  const uint16_t* start;      // a node's first slot in the block's list
+  const uint32_t* slot;       // the block's 4 kFB slots, four a word
+};
+struct BlockNodes {
+  int32_t node[4 * kFB];
+  uint16_t start[4 * kFB + 1];
+  uint32_t slot[kFB];
+};
+// The block's lists into shared memory; returns its distinct nodes.
+__device__ __forceinline__ int block_nodes(const BlockLists& l, int64_t ne, BlockNodes& s) {
+  const int32_t b0 = __ldg(l.ptr + blockIdx.x), nu = __ldg(l.ptr + blockIdx.x + 1) - b0;
+  for (int j = threadIdx.x; j < nu; j += kFB) {
+    s.node[j] = __ldg(l.node + b0 + j);
+    s.start[j] = __ldg(l.start + b0 + j);
+  }
+  s.slot[threadIdx.x] = __ldg(l.slot + int64_t(blockIdx.x) * kFB + threadIdx.x);
+  const int64_t left = ne - int64_t(blockIdx.x) * kFB;
+  if (threadIdx.x == 0) s.start[nu] = uint16_t(4 * (left < kFB ? left : kFB));
+  return nu;
+}
+// Adds the contributions v[5 a + c][element] of the block, component by
+// component (add(sum, v)), per distinct node and the sums (put(record, c, sum))
+// to the node records acc [n][S], CH 16-byte pieces each.
+template <int S, int CH, class T, class Sum, class A, class P>
+__device__ __forceinline__ void block_add(const BlockNodes& s, int nu, const T (*v)[kFB + 1],
+                                          float (*rec)[kNG][4 * CH], float* acc, Sum zero, A add,
+                                          P put) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint8_t* slot = reinterpret_cast<const uint8_t*>(s.slot);
+  const int g = lane / 5, c = lane - 5 * g;
+  for (int j0 = w * kNG; j0 < nu; j0 += kFW * kNG) {
+    if (g < kNG && j0 + g < nu) {
+      Sum t = zero;
+      const int k1 = s.start[j0 + g + 1];
+#pragma unroll 4
+      for (int k = s.start[j0 + g]; k < k1; ++k) {
+        const int q = slot[k];
+        add(t, v[(q & 3) * 5 + c][q >> 2]);
+      }
+      put(rec[w][g], c, t);
+    }
+    __syncwarp();
+    if (lane < kNG * CH && j0 + lane / CH < nu) {
+      const int h = lane / CH, k = lane % CH;
+      atomicAdd(reinterpret_cast<float4*>(acc + int64_t(s.node[j0 + h]) * S) + k,
+                *reinterpret_cast<const float4*>(&rec[w][h][4 * k]));
+    }
+    __syncwarp();
+  }
+}
+
 // FP32 element pass: per node its residual and its ten antidiffusive sums
 // (+, - per component; the sign that does not apply adds 0) in one [16]
-// record, four vector atomics (one per 4 floats); without FCT the residual
-// alone.
-__global__ void __launch_bounds__(kBlock) k_elem_rhs_aec32(int64_t n, int64_t ne,
-                                                            const int32_t* __restrict__ inpoel,
-                                                            const float* __restrict__ geo,
-                                                            const float* __restrict__ V,
-                                                            const KScalars* __restrict__ sc,
-                                                            double gamma, double ctau, int fct,
-                                                            const double* __restrict__ S,
-                                                            const double* __restrict__ Se,
-                                                            float* R) {
-  const int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (e >= ne) return;
-  int32_t N[4];
-  float r[4][5], aec[4][5];
-  elem_terms<float>(n, ne, e, inpoel, geo, V, sc, float(gamma), float(ctau), fct, S, Se, N, r,
-                    aec);
-  if (!fct) {
-    for (int a = 0; a < 4; ++a) add5<kRP>(R, n, N[a], r[a]);
-    return;
+// record; without FCT the residual alone.
+__global__ void __launch_bounds__(kFB, 14) k_elem_rhs_aec32(int64_t n, int64_t ne,
+                                                         const int32_t* __restrict__ inpoel,
+                                                         const float* __restrict__ geo,
+                                                         const float* __restrict__ V,
+                                                         const KScalars* __restrict__ sc,
+                                                         double gamma, double ctau, int fct,
+                                                         const double* __restrict__ S,
+                                                         const double* __restrict__ Se,
+                                                         BlockLists lists, float* R) {
+  __shared__ float2 v[20][kFB + 1];  // (residual, antidiffusive) per local node and component
+  __shared__ __align__(16) float rec[kFW][kNG][16];
+  __shared__ BlockNodes s;
+  const int64_t e = blockIdx.x * int64_t(kFB) + threadIdx.x;
+  const int nu = block_nodes(lists, ne, s);
+  for (int k = threadIdx.x; k < kFW * kNG * 16; k += kFB) (&rec[0][0][0])[k] = 0.f;
+  if (e < ne) {
+    int32_t N[4];
+    float r[4][5], aec[4][5];
+    elem_terms<float>(n, ne, e, inpoel, geo, V, sc, float(gamma), float(ctau), fct, S, Se, N, r,
+                      aec);
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int c = 0; c < 5; ++c) v[a * 5 + c][threadIdx.x] = make_float2(r[a][c], aec[a][c]);
   }
-  for (int a = 0; a < 4; ++a) {
-    float v[16];
-    for (int c = 0; c < 5; ++c) v[c] = r[a][c];
-    for (int c = 0; c < 5; ++c) {
-      v[5 + c * 2 + 0] = aec[a][c] > 0.f ? aec[a][c] : 0.f;
-      v[5 + c * 2 + 1] = aec[a][c] < 0.f ? aec[a][c] : 0.f;
-    }
-    v[15] = 0.f;
-    float* q = R + int64_t(N[a]) * kRP;
-    for (int k = 0; k < 4; ++k)
-      atomicAdd(reinterpret_cast<float4*>(q + 4 * k),
-                make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]));
-  }
+  __syncthreads();
+  if (fct)
+    block_add<kRP, 4>(
+        s, nu, v, rec, R, make_float3(0.f, 0.f, 0.f),
+        [](float3& t, float2 x) {
+          t.x += x.x;
+          t.y += x.y > 0.f ? x.y : 0.f;
+          t.z += x.y < 0.f ? x.y : 0.f;
+        },
+        [](float* q, int c, float3 t) {
+          q[c] = t.x;
+          q[5 + 2 * c] = t.y;
+          q[6 + 2 * c] = t.z;
+        });
+  else
+    block_add<kRP, 2>(
+        s, nu, v, reinterpret_cast<float(*)[kNG][8]>(rec), R, 0.f,
+        [](float& t, float2 x) { t += x.x; }, [](float* q, int c, float t) { q[c] = t; });
 }
 
 // FP64 element passes hand their node contributions to k_node_gather through
@@ -838,7 +911,11 @@ __global__ void __launch_bounds__(kBlock) k_elem_lim32(int64_t n, int64_t ne,
   for (int a = 0; a < 4; ++a) load_node(V, N[a], u[a]);
   aec32(k, u, aec);
   elem_limit<float>(N, Q, sysmask, aec, ca);
-  for (int a = 0; a < 4; ++a) add5<kAR>(A, n, N[a], ca[a]);
+  for (int a = 0; a < 4; ++a) {
+    float* q = A + int64_t(N[a]) * kAR;
+    atomicAdd(reinterpret_cast<float4*>(q), make_float4(ca[a][0], ca[a][1], ca[a][2], ca[a][3]));
+    atomicAdd(q + 4, ca[a][4]);
+  }
 }
 
 // FP64: the antidiffusive contributions are the ones the residual pass
@@ -1132,6 +1209,10 @@ NodeArgs node_args(KozCGDev* d) {
                   d->R,  d->P,            &d->scal->dtmin};
 }
 
+BlockLists block_lists(const KozCGDev* d) {
+  return BlockLists{d->bptr, d->bnode, d->bstart, reinterpret_cast<const uint32_t*>(d->bslot)};
+}
+
 // Node primitives and the element Galerkin (+ antidiffusive) pass on state U:
 // in FP64 into the residual slot records, in FP32 added into the zeroed node
 // records.
@@ -1156,10 +1237,9 @@ void galerkin(xg_ctx* c, KozCGDev* d, const double* U, int fct) {
                                                      d->E);
   } else {
     k_node_prim<float><<<blocks_for(n, tb), tb, 0, s>>>(n, U, d->prm.gamma, V);
-    const int eb = node_block(c, ne, kBlock);
-    k_elem_rhs_aec32<<<blocks_for(ne, eb), eb, 0, s>>>(n, ne, d->inpoel, d->geo32, V,
-                                                        d->scal, d->prm.gamma, d->prm.ctau, fct,
-                                                        S, Se, d->R32);
+    k_elem_rhs_aec32<<<blocks_for(ne, kFB), kFB, 0, s>>>(n, ne, d->inpoel, d->geo32, V,
+                                                         d->scal, d->prm.gamma, d->prm.ctau, fct,
+                                                         S, Se, block_lists(d), d->R32);
   }
 }
 
@@ -1310,16 +1390,19 @@ int xg_kozcg_setup(xg_ctx* c, const xg_kozcg_params* prm, int64_t npoin, const d
     std::vector<int64_t> nptr(npoin + 1, 0);
     std::vector<int32_t> nb;
     nb.reserve(static_cast<size_t>(npoin) * 16);
-    std::vector<int32_t> tmp;
+    std::vector<int32_t> tmp, met(npoin, -1);  // met: the last node a node was found beside
     for (int64_t i = 0; i < npoin; ++i) {
       tmp.clear();
+      met[i] = static_cast<int32_t>(i);
       for (int64_t k = eptr[i]; k < eptr[i + 1]; ++k)
         for (int a = 0; a < 4; ++a) {
           const int32_t j = ip[int64_t(eln[k]) * 4 + a];
-          if (j != i) tmp.push_back(j);
+          if (met[j] != i) {
+            met[j] = static_cast<int32_t>(i);
+            tmp.push_back(j);
+          }
         }
       std::sort(tmp.begin(), tmp.end());
-      tmp.erase(std::unique(tmp.begin(), tmp.end()), tmp.end());
       nb.insert(nb.end(), tmp.begin(), tmp.end());
       nptr[i + 1] = static_cast<int64_t>(nb.size());
     }
@@ -1339,6 +1422,58 @@ int xg_kozcg_setup(xg_ctx* c, const xg_kozcg_params* prm, int64_t npoin, const d
       const int64_t sl = i / 32, lane = i % 32;
       for (int64_t k = nptr[i]; k < nptr[i + 1]; ++k)
         anbr[aoff[sl] + (k - nptr[i]) * 32 + lane] = nb[k];
+    }
+  }
+  // FP32: the distinct nodes of each block of kFB elements, most slots first
+  // (the lanes that add a block's nodes together then loop alike), and their
+  // slots in ascending order
+  std::vector<int32_t> bptr, bnode;
+  std::vector<uint16_t> bstart;
+  std::vector<uint8_t> bslot;
+  if (!f64) {
+    const int64_t nblk = (nelem + kFB - 1) / kFB;
+    bptr.assign(static_cast<size_t>(nblk + 1), 0);
+    bslot.assign(static_cast<size_t>(nblk * 4 * kFB), 0);
+    bnode.reserve(static_cast<size_t>(nelem));
+    bstart.reserve(static_cast<size_t>(nelem));
+    std::vector<int32_t> seen(npoin, -1);  // the last block that holds a node
+    std::vector<uint8_t> idx(npoin);       // its place there, in order of appearance
+    for (int64_t b = 0; b < nblk; ++b) {
+      const int nq = static_cast<int>(std::min<int64_t>(4 * kFB, nelem * 4 - b * 4 * kFB));
+      const int32_t* q = ip.data() + b * 4 * kFB;
+      int32_t node[4 * kFB];
+      int cnt[4 * kFB], of[4 * kFB], first[4 * kFB + 2] = {}, start[4 * kFB];
+      int nu = 0;
+      for (int k = 0; k < nq; ++k) {
+        if (seen[q[k]] != b) {
+          seen[q[k]] = static_cast<int32_t>(b);
+          idx[q[k]] = static_cast<uint8_t>(nu);
+          node[nu] = q[k];
+          cnt[nu++] = 0;
+        }
+        ++cnt[idx[q[k]]];
+      }
+      for (int j = 0; j < nu; ++j) ++first[4 * kFB - cnt[j] + 1];
+      for (int k = 0; k <= 4 * kFB; ++k) first[k + 1] += first[k];
+      for (int j = 0; j < nu; ++j) of[j] = first[4 * kFB - cnt[j]]++;  // place, most slots first
+      int32_t sorted[4 * kFB];
+      int count[4 * kFB];
+      for (int j = 0; j < nu; ++j) {
+        sorted[of[j]] = node[j];
+        count[of[j]] = cnt[j];
+      }
+      for (int j = 0, k = 0; j < nu; k += count[j++]) {
+        start[j] = k;
+        bnode.push_back(sorted[j]);
+        bstart.push_back(static_cast<uint16_t>(k));
+      }
+      for (int k = 0; k < nq; ++k) {
+        const int j = of[idx[q[k]]];
+        bslot[b * 4 * kFB + start[j]++] = static_cast<uint8_t>(k);
+      }
+      if (bnode.size() >= (size_t(1) << 31))
+        return fail(c, XG_ERR_ARG, "kozcg_setup: too many elements");
+      bptr[b + 1] = static_cast<int32_t>(bnode.size());
     }
   }
   if (c->kozcg) {
@@ -1373,6 +1508,10 @@ int xg_kozcg_setup(xg_ctx* c, const xg_kozcg_params* prm, int64_t npoin, const d
       A.plan(d->Q32, npoin * kC32);
       A.plan(d->K32, npoin * kC32);
       A.plan(d->geo32, nelem * kGeo);
+      A.plan(d->bptr, bptr.size());
+      A.plan(d->bnode, bnode.size());
+      A.plan(d->bstart, bstart.size());
+      A.plan(d->bslot, bslot.size());
     } else {
       A.plan(d->Q, npoin * kC64);
       A.plan(d->K, npoin * kC64);
@@ -1404,6 +1543,12 @@ int xg_kozcg_setup(xg_ctx* c, const xg_kozcg_params* prm, int64_t npoin, const d
   XG_CUDA(c, cudaMemcpy(d->aoff, aoff.data(), aoff.size() * 4, cudaMemcpyHostToDevice));
   XG_CUDA(c, cudaMemcpy(d->aw, aw.data(), aw.size() * 4, cudaMemcpyHostToDevice));
   XG_CUDA(c, cudaMemcpy(d->anbr, anbr.data(), anbr.size() * 4, cudaMemcpyHostToDevice));
+  if (!f64) {
+    XG_CUDA(c, cudaMemcpy(d->bptr, bptr.data(), bptr.size() * 4, cudaMemcpyHostToDevice));
+    XG_CUDA(c, cudaMemcpy(d->bnode, bnode.data(), bnode.size() * 4, cudaMemcpyHostToDevice));
+    XG_CUDA(c, cudaMemcpy(d->bstart, bstart.data(), bstart.size() * 2, cudaMemcpyHostToDevice));
+    XG_CUDA(c, cudaMemcpy(d->bslot, bslot.data(), bslot.size(), cudaMemcpyHostToDevice));
+  }
   if (f64) {
     XG_CUDA(c, cudaMemcpy(d->soff, soff.data(), soff.size() * 4, cudaMemcpyHostToDevice));
     XG_CUDA(c, cudaMemcpy(d->sw, sw.data(), sw.size() * 4, cudaMemcpyHostToDevice));
