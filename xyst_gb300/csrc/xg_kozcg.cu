@@ -1008,17 +1008,16 @@ __device__ __forceinline__ void node_slots(int64_t i, const int32_t* __restrict_
       if constexpr (WP) {
 #pragma unroll
         for (int c = 0; c < 5; ++c) {
-          // v > 0 and v < 0 as integer tests of the bits (NaN and -0 in
-          // neither), off GB300's narrow FP64 pipe
+          // one FP64 addition to the sum of v's sign (a zero changes neither, a
+          // NaN is left out), chosen on the bits: a branch per sign adds in
+          // both where a warp's lanes differ, and a comparison, or a 64-bit NaN
+          // test that the compiler makes one of, holds the FP64 pipe as well
           const double v = x[j][5 + c];
-          const long long b = __double_as_longlong(v);
-          const long long mag = b & 0x7fffffffffffffffll;
-          if (mag != 0 && mag <= 0x7ff0000000000000ll) {
-            if (b > 0)
-              p[2 * c] += v;
-            else
-              p[2 * c + 1] += v;
-          }
+          const int hi = __double2hiint(v);
+          const bool nan = unsigned(hi & 0x7fffffff) + (__double2loint(v) != 0) > 0x7ff00000u;
+          const double t = (hi >= 0 ? p[2 * c] : p[2 * c + 1]) + (nan ? 0.0 : v);
+          p[2 * c] = hi >= 0 ? t : p[2 * c];
+          p[2 * c + 1] = hi >= 0 ? p[2 * c + 1] : t;
         }
       }
     }
