@@ -43,6 +43,7 @@
 #include <string>
 #include <vector>
 
+#include "xg_fp64.cuh"
 #include "xg_internal.hpp"
 
 namespace xg {
@@ -509,47 +510,26 @@ struct AdvPrm {
 // van Leer limited reconstruction of the three velocity components on the
 // canonical edge a -> b (Chorin.cpp:711-829): uL, uR the ends' values on entry,
 // the edge states on return.  With a = delta2 + eps, b = delta1 + eps of one
-// sign s, 0.25 ((1-k) delta1 phi(a/b) + (1+k) delta2 phi(b/a)) is, exactly,
-// (a b - s (eps/2) ((1-k)|a| + (1+k)|b|)) / (a + b), and 0 for a b <= 0.  The six
-// quotients come from one division (batch inversion) where the reference
-// takes eight divisions a component; a product of denominators outside
-// [1e-290, 1e290] falls back to six.
+// sign, 0.25 ((1-k) delta1 phi(a/b) + (1+k) delta2 phi(b/a)) is, exactly,
+// (a b - (eps/2) ((1-k) a + (1+k) b)) / (a + b), and 0 for a b <= 0: the numerator
+// (a - h2)(b - h1) - h1 h2 with h1, h2 = (eps/2)(1 -+ k), and a + b = 2 (g1 + eps)
+// as delta1 + delta2 = 2 g1.  Signs are tested on integer bits and a quotient
+// takes three FP64 instructions (the reference: eight divisions a component).
 __device__ __forceinline__ void reconstruct(const double g1[3], const double g2[3], double uL[3],
                                             double uR[3]) {
-  const double eps = 1.0e-9, k = 1.0 / 3.0, h = 0.5e-9;
-  double num[6], den[6], pre[6], q[6];
+  constexpr double eps = 1.0e-9, k = 1.0 / 3.0;
+  constexpr double h1 = 0.5 * eps * (1.0 - k), h2 = 0.5 * eps * (1.0 + k);
+  constexpr double A0 = 0.5 * (eps - h2), B0 = eps - h1, H = 0.5 * h1 * h2;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const double d2 = uR[c] - uL[c];
-    const double a = d2 + eps, b = (2.0 * g1[c] - d2) + eps, e = (2.0 * g2[c] - d2) + eps;
-    const double pl = a * b, pr = a * e;
-    const double sh = copysign(h, a), ka = (1.0 - k) * fabs(a);
-    const bool ol = __double_as_longlong(pl) > 0, orr = __double_as_longlong(pr) > 0;
-    num[2 * c] = ol ? pl - sh * (ka + (1.0 + k) * fabs(b)) : 0.0;
-    num[2 * c + 1] = orr ? pr - sh * (ka + (1.0 + k) * fabs(e)) : 0.0;
-    den[2 * c] = ol ? a + b : 1.0;
-    den[2 * c + 1] = orr ? a + e : 1.0;
-  }
-  pre[0] = den[0];
-#pragma unroll
-  for (int m = 1; m < 6; ++m) pre[m] = pre[m - 1] * den[m];
-  const double ap = fabs(pre[5]);
-  if (ap > 1e-290 && ap < 1e290) {
-    double inv = 1.0 / pre[5];
-#pragma unroll
-    for (int m = 5; m > 0; --m) {
-      q[m] = inv * pre[m - 1];
-      inv *= den[m];
-    }
-    q[0] = inv;
-  } else {
-#pragma unroll
-    for (int m = 0; m < 6; ++m) q[m] = 1.0 / den[m];
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    uL[c] += num[2 * c] * q[2 * c];
-    uR[c] -= num[2 * c + 1] * q[2 * c + 1];
+    const double d1 = 2.0 * g1[c] - d2, d3 = 2.0 * g2[c] - d2;
+    const int sa = side(d2, -eps), pl = sa * side(d1, -eps), pr = sa * side(d3, -eps);
+    const double A = 0.5 * d2 + A0;
+    const double nl = A * (d1 + B0) - H, nr = A * (d3 + B0) - H;
+    const double ql = recip(pl > 0 ? g1[c] + eps : 1.0), qr = recip(pr > 0 ? g2[c] + eps : 1.0);
+    uL[c] += (pl > 0 ? nl : 0.0) * ql;
+    uR[c] -= (pr > 0 ? nr : 0.0) * qr;
   }
 }
 
@@ -616,8 +596,8 @@ __global__ void __launch_bounds__(kNode) k_crhs(int64_t n, ChoAdj adj, const dou
         for (int c = 0; c < 3; ++c) {
           uL[c] = first ? a[c] : b[c];
           uR[c] = first ? b[c] : a[c];
-          g1[c] = first ? gp[c] : flip(gq[c], true);
-          g2[c] = first ? gq[c] : flip(gp[c], true);
+          g1[c] = flip(first ? gp[c] : gq[c], !first);
+          g2[c] = flip(first ? gq[c] : gp[c], !first);
         }
         reconstruct(g1, g2, uL, uR);
 #pragma unroll
