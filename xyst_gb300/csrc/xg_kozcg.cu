@@ -14,7 +14,7 @@
 // P = antidiffusive sums +/- per component, A = limited contributions),
 // elements as int32 [T][4].  Element kernels (one thread per tet) hand their
 // four nodes' contributions on: in FP64 as plain stores into element-major
-// slots that k_node_gather sums per node in ascending element order (the
+// slots that the node passes sum per node in ascending element order (the
 // reference's order, the same bits on every run), in FP32 as vector atomic
 // adds into node records.  The allowed limits Q+/- (extremes over
 // the elements holding a node) are taken per node over the node adjacency,
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(kFB, 14) k_elem_rhs_aec32(int64_t n, int64_t n
         [](float& t, float2 x) { t += x.x; }, [](float* q, int c, float t) { q[c] = t; });
 }
 
-// FP64 element passes hand their node contributions to k_node_gather through
+// FP64 element passes hand their node contributions to the node passes through
 // slot records, one per (element e, local node a), slot q = 4 e + a: the
 // residual pass writes 10 doubles (the five contributions, then the five
 // antidiffusive ones), the limiting pass 6 (the five limited contributions
@@ -1323,7 +1323,7 @@ int xg_kozcg_setup(xg_ctx* c, const xg_kozcg_params* prm, int64_t npoin, const d
   // Elements in the order of their smallest node id (stable counting sort),
   // so that consecutive elements share nearby nodes: the element passes then
   // read nearby node data, and the elements holding a run of nodes (the
-  // slots one warp of k_node_gather reads) lie in a window of the slot
+  // slots one warp of a node pass reads) lie in a window of the slot
   // records about the mesh's node bandwidth wide, instead of across the
   // whole array.  Results do not depend on the element order beyond the
   // order of each node's sums, which stays fixed.
