@@ -843,11 +843,17 @@ __global__ void __launch_bounds__(kBlock)
 #pragma unroll
   for (int c = 0; c < 5; ++c) {
     const double lo = R[c * n + i];
-    const double qp = double(oval(m[2 * c])) - lo, qn = double(oval(m[2 * c + 1])) - lo;
+    F qp = F(double(oval(m[2 * c])) - lo), qn = F(double(oval(m[2 * c + 1])) - lo);
+    if (sizeof(F) == 4) {
+      // the extremes hold float(lo), which may lie on the wrong side of lo: at a
+      // node that is its own extreme nothing is allowed (FP64: exactly 0)
+      qp = qp < F(0) ? F(0) : qp;
+      qn = qn > F(0) ? F(0) : qn;
+    }
     const double pp = P[(c * 2 + 0) * n + i], pn = P[(c * 2 + 1) * n + i];
     const bool zp = pp < eps, zn = pn > -eps;
     F cp, cn;
-    quotients(F(qp), zp ? F(1) : F(pp), F(qn), zn ? F(1) : F(pn), cp, cn);
+    quotients(qp, zp ? F(1) : F(pp), qn, zn ? F(1) : F(pn), cp, cn);
     out[c * 2 + 0] = zp ? F(0) : fmin(F(1), cp);
     out[c * 2 + 1] = zn ? F(0) : fmin(F(1), cn);
   }
@@ -858,9 +864,9 @@ __global__ void __launch_bounds__(kBlock)
 // element contributions, system-limited over the components in sysmask.
 // Limit coefficients of one element from its antidiffusive contributions
 // aec[a][c] and the nodes' C+/- (Q); ca = the limited ones.  Signs and minima
-// are taken on the bits of the values: the coefficients lie in [0, 1] (or are
-// -0), which order as signed integers, and FP64 comparisons would hold the
-// FP64 units.
+// are taken on the bits of the values: the coefficients lie in [0, 1] or are -0
+// (k_node_limit), which order as signed integers, and FP64 comparisons would
+// hold the FP64 units.
 __device__ __forceinline__ long long sbits(double v) { return __double_as_longlong(v); }
 __device__ __forceinline__ int sbits(float v) { return __float_as_int(v); }
 template <class F>
