@@ -2161,7 +2161,8 @@ int cg_to_sell(xg_ctx* c, const uint64_t* ia, const double* csr, double* dev_out
     for (uint64_t j = ia[i]; j < ia[i + 1]; ++j)
       v[soff[s] + int64_t(j - ia[i]) * kSlice + lane] = csr[j];
   }
-  XG_CUDA(c, cudaMemcpy(dev_out, v.data(), v.size() * 8, cudaMemcpyHostToDevice));
+  XG_CUDA(c, upload(c, dev_out, v.data(), v.size() * 8));
+  XG_CUDA(c, cudaStreamSynchronize(c->stream));
   return XG_OK;
 }
 int64_t cg_nent(xg_ctx* c) { return c->cg ? c->cg->nent : 0; }

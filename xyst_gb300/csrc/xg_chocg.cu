@@ -1116,9 +1116,7 @@ int xg_chocg_setup(xg_ctx* c, const xg_chocg_params* prm, int64_t npoin, const d
       }
     }
   }
-  auto up = [&](void* dst, const void* src, size_t bytes) {
-    return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
-  };
+  auto up = [&](void* dst, const void* src, size_t bytes) { return upload(c, dst, src, bytes); };
   XG_CUDA(c, up(d->soff, soff.data(), soff.size() * 4));
   XG_CUDA(c, up(d->swidth, swidth.data(), swidth.size() * 4));
   XG_CUDA(c, up(d->nbr, nbr.data(), nbr.size() * 4));
@@ -1135,9 +1133,10 @@ int xg_chocg_setup(xg_ctx* c, const xg_chocg_params* prm, int64_t npoin, const d
   XG_CUDA(c, up(d->stage, vol, n * 8));
   k_node_factors<<<blocks_for(n, kBlock), kBlock, 0, c->stream>>>(n, d->stage, d->ivol, d->cbrtv);
   XG_CHECK_LAUNCH(c);
-  XG_CUDA(c, cudaStreamSynchronize(c->stream));
   for (double* z : {d->u, d->u2, d->un, d->pr, d->pgrad, d->vgrad, d->div, d->flx})
-    XG_CUDA(c, cudaMemset(z, 0, (z == d->vgrad ? 9 : (z == d->pr || z == d->div ? 1 : 3)) * n * 8));
+    XG_CUDA(c, cudaMemsetAsync(
+                   z, 0, (z == d->vgrad ? 9 : (z == d->pr || z == d->div ? 1 : 3)) * n * 8, c->stream));
+  XG_CUDA(c, cudaStreamSynchronize(c->stream));
   return XG_OK;
   XG_HOST_CATCH(c)
 }
@@ -1334,9 +1333,7 @@ int xg_chocg_set_bc(xg_ctx* c, int64_t ndir, const uint64_t* dirnodes, const int
     A.plan(d->dirval, std::max<int64_t>(1, ndir * 3));
     if (pass == 0) XG_CUDA(c, A.reserve());
   }
-  auto up = [&](void* dst, const void* src, size_t bytes) {
-    return bytes ? cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
-  };
+  auto up = [&](void* dst, const void* src, size_t bytes) { return upload(c, dst, src, bytes); };
   XG_CUDA(c, up(d->bcnode, node.data(), node.size() * 4));
   XG_CUDA(c, up(d->bcdir, dir.data(), dir.size() * 4));
   XG_CUDA(c, up(d->bcnoslip, nsl.data(), nsl.size() * 4));
@@ -1344,6 +1341,7 @@ int xg_chocg_set_bc(xg_ctx* c, int64_t ndir, const uint64_t* dirnodes, const int
   XG_CUDA(c, up(d->symn, symn.data(), symn.size() * 8));
   XG_CUDA(c, up(d->dirmask, dirmask, ndir * 3 * 4));
   XG_CUDA(c, up(d->dirval, dirvals, ndir * 3 * 8));
+  XG_CUDA(c, cudaStreamSynchronize(c->stream));
   // Dirichlet rows of the theta-implicit momentum system (ChoCG::solve,
   // ChoCG.cpp:1580-1600): the masked velocity components of the Dirichlet
   // nodes and all three of the noslip nodes, increment 0

@@ -170,6 +170,14 @@ inline int node_block(const xg_ctx* c, int64_t n, int most) {
   return b;
 }
 
+// Host to device on the context's stream.  The stream does not wait for the
+// legacy one, where a copy from pageable memory may return before its transfer
+// has ended: everything a kernel reads comes this way.  The source must live
+// until the stream has been synchronised.
+inline cudaError_t upload(const xg_ctx* c, void* dst, const void* src, size_t bytes) {
+  return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream) : cudaSuccess;
+}
+
 // Make the context's device current for the calling thread.
 inline int use(xg_ctx* c) {
   if (!c) return XG_ERR_ARG;

@@ -1540,25 +1540,26 @@ int xg_kozcg_setup(xg_ctx* c, const xg_kozcg_params* prm, int64_t npoin, const d
     }
   }
   cudaStream_t s = c->stream;
-  XG_CUDA(c, cudaMemcpy(d->inpoel, ip.data(), ip.size() * 4, cudaMemcpyHostToDevice));
-  XG_CUDA(c, cudaMemcpy(d->xyz, coord, npoin * 3 * 8, cudaMemcpyHostToDevice));
+  auto up = [&](void* dst, const void* src, size_t bytes) { return upload(c, dst, src, bytes); };
+  XG_CUDA(c, up(d->inpoel, ip.data(), ip.size() * 4));
+  XG_CUDA(c, up(d->xyz, coord, npoin * 3 * 8));
   // through the staging buffer
-  XG_CUDA(c, cudaMemcpy(d->stage, vol, npoin * 8, cudaMemcpyHostToDevice));
+  XG_CUDA(c, up(d->stage, vol, npoin * 8));
   k_node_factors<<<blocks_for(npoin, kBlock), kBlock, 0, s>>>(npoin, d->stage, d->ivol, d->cbrtv);
   XG_CHECK_LAUNCH(c);
-  XG_CUDA(c, cudaMemcpy(d->aoff, aoff.data(), aoff.size() * 4, cudaMemcpyHostToDevice));
-  XG_CUDA(c, cudaMemcpy(d->aw, aw.data(), aw.size() * 4, cudaMemcpyHostToDevice));
-  XG_CUDA(c, cudaMemcpy(d->anbr, anbr.data(), anbr.size() * 4, cudaMemcpyHostToDevice));
+  XG_CUDA(c, up(d->aoff, aoff.data(), aoff.size() * 4));
+  XG_CUDA(c, up(d->aw, aw.data(), aw.size() * 4));
+  XG_CUDA(c, up(d->anbr, anbr.data(), anbr.size() * 4));
   if (!f64) {
-    XG_CUDA(c, cudaMemcpy(d->bptr, bptr.data(), bptr.size() * 4, cudaMemcpyHostToDevice));
-    XG_CUDA(c, cudaMemcpy(d->bnode, bnode.data(), bnode.size() * 4, cudaMemcpyHostToDevice));
-    XG_CUDA(c, cudaMemcpy(d->bstart, bstart.data(), bstart.size() * 2, cudaMemcpyHostToDevice));
-    XG_CUDA(c, cudaMemcpy(d->bslot, bslot.data(), bslot.size(), cudaMemcpyHostToDevice));
+    XG_CUDA(c, up(d->bptr, bptr.data(), bptr.size() * 4));
+    XG_CUDA(c, up(d->bnode, bnode.data(), bnode.size() * 4));
+    XG_CUDA(c, up(d->bstart, bstart.data(), bstart.size() * 2));
+    XG_CUDA(c, up(d->bslot, bslot.data(), bslot.size()));
   }
   if (f64) {
-    XG_CUDA(c, cudaMemcpy(d->soff, soff.data(), soff.size() * 4, cudaMemcpyHostToDevice));
-    XG_CUDA(c, cudaMemcpy(d->sw, sw.data(), sw.size() * 4, cudaMemcpyHostToDevice));
-    XG_CUDA(c, cudaMemcpy(d->sslot, sslot.data(), sslot.size() * 4, cudaMemcpyHostToDevice));
+    XG_CUDA(c, up(d->soff, soff.data(), soff.size() * 4));
+    XG_CUDA(c, up(d->sw, sw.data(), sw.size() * 4));
+    XG_CUDA(c, up(d->sslot, sslot.data(), sslot.size() * 4));
   }
   XG_CUDA(c, cudaMemsetAsync(d->U, 0, npoin * 5 * 8, s));
   XG_CUDA(c, cudaMemsetAsync(d->bcof, 0xff, npoin * 4, s));  // -1
@@ -1632,9 +1633,7 @@ int xg_kozcg_set_bc(xg_ctx* c, int64_t nsym, const uint64_t* symnodes, const dou
     A.plan(d->dirval, std::max<int64_t>(1, ndir) * 5);
     if (pass == 0) XG_CUDA(c, A.reserve());
   }
-  auto up = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
-    return bytes ? cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
-  };
+  auto up = [&](void* dst, const void* src, size_t bytes) { return upload(c, dst, src, bytes); };
   XG_CUDA(c, up(d->bcnode, node.data(), nbc * 4));
   XG_CUDA(c, up(d->bcdir, dir.data(), nbc * 4));
   XG_CUDA(c, up(d->bcsymp, symp.data(), (nbc + 1) * 4));
@@ -1642,6 +1641,7 @@ int xg_kozcg_set_bc(xg_ctx* c, int64_t nsym, const uint64_t* symnodes, const dou
   XG_CUDA(c, up(d->dirmask, dirmask, ndir * 5 * 4));
   XG_CUDA(c, up(d->dirval, dirvals, ndir * 5 * 8));
   XG_CUDA(c, up(d->bcof, bcof.data(), n * 4));
+  XG_CUDA(c, cudaStreamSynchronize(c->stream));
   d->nbc = nbc;
   d->dt_valid = false;
   return XG_OK;

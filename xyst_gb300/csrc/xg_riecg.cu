@@ -1999,9 +1999,7 @@ int alloc_and_upload(xg_ctx* c, RieCGDev* d, const double* coord, const double* 
   d->nent1 = hl.nent1;
   d->nent2 = hl.nent2;
   cudaStream_t s = c->stream;
-  auto up = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
-    return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess;
-  };
+  auto up = [&](void* dst, const void* src, size_t bytes) { return upload(c, dst, src, bytes); };
   XG_CUDA(c, up(d->vol, vol, n * sizeof(double)));
   XG_CUDA(c, up(d->bidx, bidx.data(), n * sizeof(int32_t)));
   XG_CUDA(c, up(d->soff, soff.data(), soff.size() * 4));
@@ -2025,7 +2023,7 @@ int alloc_and_upload(xg_ctx* c, RieCGDev* d, const double* coord, const double* 
         h[i].pad = 0;
       }
     }
-    XG_CUDA(c, cudaMemcpy(ent, h.data(), h.size() * sizeof(EntT), cudaMemcpyHostToDevice));
+    XG_CUDA(c, up(ent, h.data(), h.size() * sizeof(EntT)));
     std::vector<EntT> h1(hl.nent1);
     for (int64_t i = 0; i < hl.nent1; ++i) {
       if constexpr (sizeof(F) == 4) {
@@ -2055,20 +2053,22 @@ int alloc_and_upload(xg_ctx* c, RieCGDev* d, const double* coord, const double* 
     XG_CUDA(c, cudaStreamSynchronize(s));
     std::vector<double> iv(n);
     for (int64_t i = 0; i < n; ++i) iv[i] = 1.0 / vol[i];
-    XG_CUDA(c, cudaMemcpy(d->ivol, iv.data(), n * sizeof(double), cudaMemcpyHostToDevice));
+    XG_CUDA(c, up(d->ivol, iv.data(), n * sizeof(double)));
     if constexpr (sizeof(F) == 4) {
       std::vector<float> cv(n);
       for (int64_t i = 0; i < n; ++i) cv[i] = static_cast<float>(std::cbrt(vol[i]));
-      XG_CUDA(c, cudaMemcpy(d->cbrtv, cv.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+      XG_CUDA(c, up(d->cbrtv, cv.data(), n * sizeof(float)));
+      XG_CUDA(c, cudaStreamSynchronize(s));  // cv ends here
     } else {
       k_cbrt<<<blocks_for(n, kBlock), kBlock, 0, s>>>(n, d->vol, d->cbrtd);
       XG_CHECK_LAUNCH(c);
     }
+    XG_CUDA(c, cudaStreamSynchronize(s));
   }
   std::vector<int32_t> bnode(std::max<int64_t>(1, d->nbn), 0);
   for (int64_t p = 0; p < n; ++p)
     if (bidx[p] >= 0) bnode[bidx[p]] = static_cast<int32_t>(p);
-  XG_CUDA(c, cudaMemcpy(d->bnode, bnode.data(), bnode.size() * 4, cudaMemcpyHostToDevice));
+  XG_CUDA(c, up(d->bnode, bnode.data(), bnode.size() * 4));
   XG_CUDA(c, up(d->bptr, bptr.data(), bptr.size() * 4));
   XG_CUDA(c, up(d->bent4, bent4.data(), bent4.size() * sizeof(int4)));
   XG_CUDA(c, cudaMemsetAsync(d->bcof, 0xff, std::max<int64_t>(1, d->nbn) * 4, s));  // -1
@@ -2083,14 +2083,15 @@ int alloc_and_upload(xg_ctx* c, RieCGDev* d, const double* coord, const double* 
       w[p * 8 + 6] = F(coord[n + p]);
       w[p * 8 + 7] = F(coord[2 * n + p]);
     }
-    XG_CUDA(c, cudaMemcpy(W0, w.data(), w.size() * sizeof(F), cudaMemcpyHostToDevice));
-    XG_CUDA(c, cudaMemcpy(W1, w.data(), w.size() * sizeof(F), cudaMemcpyHostToDevice));
-    XG_CUDA(c, cudaMemcpy(d->stage_W, w.data(), w.size() * sizeof(F), cudaMemcpyHostToDevice));
+    XG_CUDA(c, up(W0, w.data(), w.size() * sizeof(F)));
+    XG_CUDA(c, up(W1, w.data(), w.size() * sizeof(F)));
+    XG_CUDA(c, up(d->stage_W, w.data(), w.size() * sizeof(F)));
+    XG_CUDA(c, cudaStreamSynchronize(s));
   }
   Scalars s0{};  // every member zero
   double big = DBL_MAX;
   std::memcpy(&s0.dtmin, &big, sizeof(double));
-  XG_CUDA(c, cudaMemcpy(d->scal, &s0, sizeof(s0), cudaMemcpyHostToDevice));
+  XG_CUDA(c, up(d->scal, &s0, sizeof(s0)));
   XG_CUDA(c, cudaStreamSynchronize(s));
   return XG_OK;
 }
@@ -2420,9 +2421,7 @@ int xg_riecg_set_bc(xg_ctx* c, int64_t nsym, const uint64_t* symnodes, const dou
     A.plan(d->preval, std::max<int64_t>(1, npre) * 2);
     if (pass == 0) XG_CUDA(c, A.reserve());
   }
-  auto up = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
-    return bytes ? cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
-  };
+  auto up = [&](void* dst, const void* src, size_t bytes) { return upload(c, dst, src, bytes); };
   XG_CUDA(c, up(d->bcnode, node.data(), nbc * 4));
   XG_CUDA(c, up(d->bcdir, dir.data(), nbc * 4));
   XG_CUDA(c, up(d->bcfar, far.data(), nbc * 4));
@@ -2436,10 +2435,12 @@ int xg_riecg_set_bc(xg_ctx* c, int64_t nsym, const uint64_t* symnodes, const dou
     for (int64_t k = 0; k < ndir; ++k)
       for (int j = 0; j < 3; ++j) dx[k * 3 + j] = d->xyz_host[j * d->n + dirnodes[k]];
     XG_CUDA(c, up(d->dirxyz, dx.data(), ndir * 3 * 8));
+    XG_CUDA(c, cudaStreamSynchronize(c->stream));
   }
   XG_CUDA(c, up(d->farn, farnorms, nfar * 3 * 8));
   XG_CUDA(c, up(d->preval, prevals, npre * 2 * 8));
   XG_CUDA(c, up(d->bcof, bcof.data(), bcof.size() * 4));
+  XG_CUDA(c, cudaStreamSynchronize(c->stream));
   if (far5)
     for (int i = 0; i < 5; ++i) d->far5[i] = far5[i];
   d->nbc = nbc;
@@ -2615,8 +2616,9 @@ int build_colours(xg_ctx* c, RieCGDev* d) {
     A.plan(d->cR, n * 8);
     if (pass == 0) XG_CUDA(c, A.reserve());
   }
-  XG_CUDA(c, cudaMemcpy(d->cpq, spq.data(), spq.size() * sizeof(int2), cudaMemcpyHostToDevice));
-  XG_CUDA(c, cudaMemcpy(d->cd, sdd.data(), sdd.size() * sizeof(float4), cudaMemcpyHostToDevice));
+  XG_CUDA(c, upload(c, d->cpq, spq.data(), spq.size() * sizeof(int2)));
+  XG_CUDA(c, upload(c, d->cd, sdd.data(), sdd.size() * sizeof(float4)));
+  XG_CUDA(c, cudaStreamSynchronize(c->stream));
   d->coff = off;
   return XG_OK;
 }
