@@ -313,19 +313,17 @@ __device__ __forceinline__ T sell_row_x(CI ci, const V* __restrict__ val, int32_
   return s;
 }
 
-// One wave of resident blocks of kernel K for n rows.
-int g_nsm = 0;
-size_t g_smem = 0;  // shared memory a block may ask for; 0: no cooperative launches
-bool g_cluster = false;  // clusters of kClusterSize blocks can be resident
+// One wave of resident blocks of kernel K for n rows (blocks per SM: the same on
+// every sm_103a device).
 template <auto K>
-unsigned pgrid(int64_t n) {
+unsigned pgrid(const xg_ctx* c, int64_t n) {
   static const int per_sm = [] {
     int v = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, K, kBlock, 0) != cudaSuccess) v = 1;
     return v < 1 ? 1 : v;
   }();
   const int64_t want = (n + kBlock - 1) / kBlock;
-  return static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(per_sm) * g_nsm)));
+  return static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(per_sm) * c->nsm)));
 }
 
 #define XG_ROWS(i, n) \
@@ -364,8 +362,8 @@ void launch_dep_k(void (*k)(P...), unsigned grid, cudaStream_t s, A&&... args) {
 
 // Kernel K over n rows, one wave of resident blocks, as a dependent launch.
 template <auto K, class... A>
-void launch_dep(int64_t n, cudaStream_t s, A&&... args) {
-  launch_dep_k(K, pgrid<K>(n), s, std::forward<A>(args)...);
+void launch_dep(const xg_ctx* c, int64_t n, A&&... args) {
+  launch_dep_k(K, pgrid<K>(c, n), c->stream, std::forward<A>(args)...);
 }
 
 // ---------------------------------------------------------------- kernels
@@ -1823,9 +1821,9 @@ int factor_apply64(xg_ctx* c, CGDev* d, const double* r, double* z) {
   cudaStream_t s = c->stream;
   const int64_t n = d->n;
   k_scale<double><<<blocks_for(n, kBlock), kBlock, 0, s>>>(n, d->srow, r, d->v);
-  launch_dep<k_pc_upper<double, float, Cols32>>(n, s, n, d->soffU, d->swU, Cols32{d->colU}, d->nvU,
+  launch_dep<k_pc_upper<double, float, Cols32>>(c, n, n, d->soffU, d->swU, Cols32{d->colU}, d->nvU,
       d->v, d->u, d->scal);
-  launch_dep<k_pc_lower<double, float, Cols32, 0>>(n, s, n, d->soffL, d->swL, Cols32{d->colL},
+  launch_dep<k_pc_lower<double, float, Cols32, 0>>(c, n, n, d->soffL, d->swL, Cols32{d->colL},
       d->nvL, d->srow, d->bcmask, d->u, r, z, d->partial, d->scal);
   XG_CHECK_LAUNCH(c);
   return XG_OK;
@@ -1837,9 +1835,9 @@ template <class CI>
 void factor_apply32(xg_ctx* c, CGDev* d, CI cu, CI cl) {
   cudaStream_t s = c->stream;
   const int64_t n = d->n;
-  launch_dep<k_pc_upper<float, __half, CI>>(n, s, n, d->soffU, d->swU, cu, d->hvU, d->v32, d->u32,
+  launch_dep<k_pc_upper<float, __half, CI>>(c, n, n, d->soffU, d->swU, cu, d->hvU, d->v32, d->u32,
       d->scal);
-  launch_dep<k_pc_lower<float, __half, CI, 0>>(n, s, n, d->soffL, d->swL, cl, d->hvL, d->srow,
+  launch_dep<k_pc_lower<float, __half, CI, 0>>(c, n, n, d->soffL, d->swL, cl, d->hvL, d->srow,
       d->bcmask, d->u32, d->r32, d->z32, d->partial, d->scal);
 }
 
@@ -1854,11 +1852,11 @@ struct LoopShape {
   unsigned grid = 0;
   size_t smem = 0;
 };
-bool loop_shape(int64_t n, LoopShape* out) {
-  const int64_t want = (n + g_nsm - 1) / g_nsm;
+bool loop_shape(const xg_ctx* c, int64_t n, LoopShape* out) {
+  const int64_t want = (n + c->nsm - 1) / c->nsm;
   const int64_t per = std::max<int64_t>(kLoopMinRows, (want + kSlice - 1) / kSlice * kSlice);
   out->smem = size_t(per) * 4 * sizeof(double);
-  if (out->smem + kLoopStatic > g_smem) return false;
+  if (out->smem + kLoopStatic > c->smem) return false;
   out->per = static_cast<int>(per);
   out->grid = static_cast<unsigned>((n + per - 1) / per);
   return true;
@@ -1867,12 +1865,12 @@ bool loop_shape(int64_t n, LoopShape* out) {
 // The FP64 solve of a small system by k_cg_cluster launches; false where it
 // does not apply (rows, shared memory, or a device without such clusters).
 constexpr int64_t kClusterIts = 65536;
-bool cluster_shape(const CGDev* d, int* per, int* ents, size_t* smem) {
-  if (d->n > kClusterRows || d->n < kClusterSize * kSlice || !g_cluster) return false;
+bool cluster_shape(const xg_ctx* c, const CGDev* d, int* per, int* ents, size_t* smem) {
+  if (d->n > kClusterRows || d->n < kClusterSize * kSlice || c->cluster != 1) return false;
   *per = static_cast<int>((d->n + kClusterSize * kSlice - 1) / (kClusterSize * kSlice)) * kSlice;
   *ents = d->wmax * *per;
   *smem = size_t(*per) * 5 * sizeof(double) + size_t(*ents) * (sizeof(double) + sizeof(uint32_t));
-  return *smem + 32768 <= g_smem;
+  return *smem + 32768 <= c->smem;
 }
 int cluster_solve(xg_ctx* c, CGDev* d, int per, int ents, size_t smem, CGScalars* h) {
   cudaStream_t s = c->stream;
@@ -1941,27 +1939,27 @@ int cg_iterate(xg_ctx* c, CGDev* d, int64_t maxit, double tol, CGScalars* h) {
   const int64_t n = d->n;
   int per = 0, ents = 0;
   size_t smem = 0;
-  if (d->pc != 2 && cluster_shape(d, &per, &ents, &smem))
+  if (d->pc != 2 && cluster_shape(c, d, &per, &ents, &smem))
     return cluster_solve(c, d, per, ents, smem, h);
   LoopShape sh;
-  if (d->pc != 2 && loop_shape(n, &sh))
+  if (d->pc != 2 && loop_shape(c, n, &sh))
     return d->use16 ? loop_solve(c, d, sh, Cols16{d->col16}, h)
                     : loop_solve(c, d, sh, Cols32{d->col}, h);
   for (;;) {
     for (int k = 0; k < kBatch; ++k) {
       double* p0 = d->p[0];
-      launch_dep<k_cg_p<double>>(n, s, n, d->z, p0, d->scal);
-      launch_dep<k_cg_a<double, double, Cols32>>(n, s, n, d->soff, d->swidth, Cols32{d->col},
+      launch_dep<k_cg_p<double>>(c, n, n, d->z, p0, d->scal);
+      launch_dep<k_cg_a<double, double, Cols32>>(c, n, n, d->soff, d->swidth, Cols32{d->col},
           d->a, p0, d->q, d->partial, d->scal);
       if (d->pc == 2) {
-        launch_dep<k_cg_b<double, true>>(n, s, n, d->q, d->d, p0, d->srow, d->r, d->z,
+        launch_dep<k_cg_b<double, true>>(c, n, n, d->q, d->d, p0, d->srow, d->r, d->z,
             d->v, d->x, d->partial, d->scal);
-        launch_dep<k_pc_upper<double, float, Cols32>>(n, s, n, d->soffU, d->swU, Cols32{d->colU},
+        launch_dep<k_pc_upper<double, float, Cols32>>(c, n, n, d->soffU, d->swU, Cols32{d->colU},
             d->nvU, d->v, d->u, d->scal);
-        launch_dep<k_pc_lower<double, float, Cols32, 1>>(n, s, n, d->soffL, d->swL, Cols32{d->colL},
+        launch_dep<k_pc_lower<double, float, Cols32, 1>>(c, n, n, d->soffL, d->swL, Cols32{d->colL},
             d->nvL, d->srow, d->bcmask, d->u, d->r, d->z, d->partial, d->scal);
       } else {
-        launch_dep<k_cg_b<double, false>>(n, s, n, d->q, d->d, p0, d->srow, d->r, d->z,
+        launch_dep<k_cg_b<double, false>>(c, n, n, d->q, d->d, p0, d->srow, d->r, d->z,
             d->v, d->x, d->partial, d->scal);
       }
     }
@@ -1990,7 +1988,7 @@ int mixed_loop(xg_ctx* c, CGDev* d, CI ca, CI cu, CI cl, CGScalars* h) {
                                   static_cast<int>(smem)));
   const int64_t ns = (d->n + kSlice - 1) / kSlice;
   const unsigned grid = static_cast<unsigned>(
-      std::min<int64_t>(g_nsm, (ns + kMixMinSlices - 1) / kMixMinSlices));
+      std::min<int64_t>(c->nsm, (ns + kMixMinSlices - 1) / kMixMinSlices));
   void* args[] = {&A};
   for (;;) {
     XG_CUDA(c, cudaMemsetAsync(d->larrive, 0, sizeof(unsigned int), s));
@@ -2016,7 +2014,7 @@ int mixed_loop(xg_ctx* c, CGDev* d, CI ca, CI cu, CI cl, CGScalars* h) {
 int replace_residual(xg_ctx* c, CGDev* d, int first) {
   cudaStream_t s = c->stream;
   const int64_t n = d->n;
-  k_outer_res<<<pgrid<k_outer_res>(n), kBlock, 0, s>>>(
+  k_outer_res<<<pgrid<k_outer_res>(c, n), kBlock, 0, s>>>(
       n, d->soff, d->swidth, d->col, d->a, d->x, d->b, d->d32, d->pc == 2 ? d->srow : nullptr,
       d->r32, d->z32, d->v32, first, d->partial, d->scal);
   XG_CHECK_LAUNCH(c);
@@ -2032,14 +2030,16 @@ int replace_residual(xg_ctx* c, CGDev* d, int first) {
 
 
 // Whether a cluster of kClusterSize blocks of k_cg_cluster with the shared
-// memory of its largest system can be resident (a query, nothing runs).
-bool cluster_ok() {
+// memory of its largest system can be resident on the context's device (a query,
+// nothing runs), and the permission for such a cluster there: a kernel's
+// attributes are per device.
+bool cluster_ok(const xg_ctx* c) {
   if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
       cudaSuccess) {
     (void)cudaGetLastError();
     return false;
   }
-  const int most = static_cast<int>(g_smem > 32768 ? g_smem - 32768 : 0);
+  const int most = static_cast<int>(c->smem > 32768 ? c->smem - 32768 : 0);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kClusterSize);
   cfg.blockDim = dim3(kClusterThreads);
@@ -2122,7 +2122,7 @@ int cg_init_device(xg_ctx* c, const double* b_dev, int zero_values, int pc) {
   h.pc = pc;
   h.guard = d->guard;
   XG_CUDA(c, cudaMemcpyAsync(d->scal, &h, sizeof(h), cudaMemcpyHostToDevice, s));
-  k_setup<<<pgrid<k_setup>(n), kBlock, 0, s>>>(n, d->soff, d->swidth, d->col, d->a, d->diagpos,
+  k_setup<<<pgrid<k_setup>(c, n), kBlock, 0, s>>>(n, d->soff, d->swidth, d->col, d->a, d->diagpos,
                                                d->x, d->b, d->r, d->d, d->z, d->p[0], d->d32,
                                                d->partial, d->scal);
   XG_CHECK_LAUNCH(c);
@@ -2199,17 +2199,7 @@ int xg_cg_setup(xg_ctx* c, int64_t nrow, const uint64_t* ia, const uint64_t* ja,
     }
     if (diagk[i] < 0) return fail(c, XG_ERR_ARG, "cg_setup: row without diagonal entry");
   }
-  if (g_nsm == 0) {
-    int dev = 0, nsm = 0;
-    XG_CUDA(c, cudaGetDevice(&dev));
-    XG_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    int smem = 0, coop = 0;
-    XG_CUDA(c, cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    XG_CUDA(c, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    g_smem = coop ? static_cast<size_t>(smem) : 0;
-    g_cluster = cluster_ok();
-    g_nsm = nsm > 0 ? nsm : 1;
-  }
+  if (c->cluster < 0) c->cluster = cluster_ok(c) ? 1 : 0;
   const int64_t nslice = (nrow + kSlice - 1) / kSlice;
   std::vector<int32_t> soff(nslice + 1), sw(nslice);
   int64_t tot = 0;
@@ -2323,7 +2313,7 @@ int xg_cg_setup(xg_ctx* c, int64_t nrow, const uint64_t* ia, const uint64_t* ja,
   d->nent = tot;
   d->use16 = fits16;
   d->wmax = *std::max_element(sw.begin(), sw.end());
-  d->maxgrid = int64_t(g_nsm) * (2048 / kBlock);
+  d->maxgrid = int64_t(c->nsm) * (2048 / kBlock);
   for (int pass = 0; pass < 2; ++pass) {
     Arena& A = d->arena;
     A.plan(d->soff, nslice + 1);
@@ -2355,7 +2345,7 @@ int xg_cg_setup(xg_ctx* c, int64_t nrow, const uint64_t* ia, const uint64_t* ja,
     A.plan(d->vt32, nrow);
     A.plan(d->partial, 3 * d->maxgrid);
     A.plan(d->scal, 1);
-    A.plan(d->lpart, size_t(6) * g_nsm);
+    A.plan(d->lpart, size_t(6) * c->nsm);
     A.plan(d->larrive, 1);
     A.plan(d->soffL, nslice + 1);
     A.plan(d->swL, nslice);
@@ -2440,7 +2430,7 @@ int xg_cg_mult(xg_ctx* c, const double* x, double* y) {
   if (!d) return fail(c, XG_ERR_STATE, "cg_mult before cg_setup");
   if (!x || !y) return fail(c, XG_ERR_ARG, "cg_mult: null vector");
   XG_CUDA(c, cudaMemcpyAsync(d->r, x, d->n * 8, cudaMemcpyHostToDevice, c->stream));
-  k_spmv<<<pgrid<k_spmv>(d->n), kBlock, 0, c->stream>>>(d->n, d->soff, d->swidth, d->col, d->a0,
+  k_spmv<<<pgrid<k_spmv>(c, d->n), kBlock, 0, c->stream>>>(d->n, d->soff, d->swidth, d->col, d->a0,
                                                         d->r, d->q);
   XG_CHECK_LAUNCH(c);
   XG_CUDA(c, cudaMemcpyAsync(y, d->q, d->n * 8, cudaMemcpyDeviceToHost, c->stream));
@@ -2508,7 +2498,7 @@ int xg_cg_init(xg_ctx* c, const double* x, const double* b, const double* neubc,
   h.pc = pc;
   h.guard = d->guard;
   XG_CUDA(c, cudaMemcpyAsync(d->scal, &h, sizeof(h), cudaMemcpyHostToDevice, s));
-  k_setup<<<pgrid<k_setup>(n), kBlock, 0, s>>>(n, d->soff, d->swidth, d->col, d->a, d->diagpos,
+  k_setup<<<pgrid<k_setup>(c, n), kBlock, 0, s>>>(n, d->soff, d->swidth, d->col, d->a, d->diagpos,
                                                d->x, d->b, d->r, d->d, d->z, d->p[0], d->d32,
                                                d->partial, d->scal);
   XG_CHECK_LAUNCH(c);

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <exception>
@@ -112,6 +113,8 @@ size_t bytes_kozcg(const KozCGDev*);
 struct xg_ctx {
   int device = 0;
   int nsm = 1;  // its multiprocessors
+  size_t smem = 0;  // shared memory a block may ask for there; 0: no cooperative launches
+  int cluster = -1;  // k_cg_cluster's clusters can be resident (1), cannot (0), not asked yet
   cudaStream_t stream = nullptr;
   std::string err;
   xg::RieCGDev* riecg = nullptr;
@@ -176,6 +179,21 @@ inline int node_block(const xg_ctx* c, int64_t n, int most) {
 // until the stream has been synchronised.
 inline cudaError_t upload(const xg_ctx* c, void* dst, const void* src, size_t bytes) {
   return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream) : cudaSuccess;
+}
+
+// Lets kernel K ask for `bytes` of dynamic shared memory on the context's device
+// (which is current): once per device, as attributes are the device's, and the
+// same `bytes` each time, as they are the process's: a value lowered for one
+// system would refuse another thread's launch.
+template <auto K>
+cudaError_t allow_smem(const xg_ctx* c, size_t bytes) {
+  static std::atomic<uint64_t> done{0};  // a bit per device; beyond 64 it is set each time
+  const uint64_t bit = c->device < 64 ? uint64_t(1) << c->device : 0;
+  if (done.load() & bit) return cudaSuccess;
+  const cudaError_t e =
+      cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  if (e == cudaSuccess) done.fetch_or(bit);
+  return e;
 }
 
 // Make the context's device current for the calling thread.

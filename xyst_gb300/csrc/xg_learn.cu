@@ -1134,15 +1134,8 @@ int ensure_work(xg_ctx* c, xg_lpc* m, int64_t n, int64_t nl, int64_t nu) {
 // at most (up to 128 TMEM columns and 64 KB of operand tiles each: four dense
 // CTAs fill the SM's 512 columns, two weight-gradient CTAs fit its partials).
 constexpr int kDensePerSm = 4, kWgradPerSm = 2;
-int umma_grid(int64_t n, int per_sm, int most) {
-  static int nsm = [] {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      v = 1;
-    return v < 1 ? 1 : v;
-  }();
-  const int64_t cap = std::min<int64_t>(most, int64_t(per_sm) * nsm);
+int umma_grid(const xg_ctx* c, int64_t n, int per_sm, int most) {
+  const int64_t cap = std::min<int64_t>(most, int64_t(per_sm) * c->nsm);
   return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((n + kUmmaM - 1) / kUmmaM, cap)));
 }
 
@@ -1150,10 +1143,8 @@ template <int KIN, int NOUT, bool FROM_W>
 int dense_umma(xg_ctx* c, xg_lpc* m, int64_t n, const float* X1, const float* X2, const float* W,
                const float* bias, int act, const float* maskY, float* Y1, float* Y2) {
   constexpr int smem = (kUmmaM * KIN + NOUT * KIN) * 2;
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_dense_umma<KIN, NOUT, FROM_W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  XG_CUDA(c, attr);
-  k_dense_umma<KIN, NOUT, FROM_W><<<umma_grid(n, kDensePerSm, INT_MAX), kUmmaThreads, smem, c->stream>>>(
+  XG_CUDA(c, (allow_smem<k_dense_umma<KIN, NOUT, FROM_W>>(c, smem)));
+  k_dense_umma<KIN, NOUT, FROM_W><<<umma_grid(c, n, kDensePerSm, INT_MAX), kUmmaThreads, smem, c->stream>>>(
       n, X1, X2, W, bias, act, maskY, Y1, Y2, m->uerr);
   XG_CHECK_LAUNCH(c);
   return XG_OK;
@@ -1164,10 +1155,8 @@ int wgrad_umma(xg_ctx* c, xg_lpc* m, int64_t n, const float* X1, const float* X2
                const float* dY1, const float* dY2, int64_t wofs, int64_t bofs) {
   constexpr int smem = (kUmmaM * kUmmaM + NOUT * kUmmaM) * 2;
   constexpr int NW = KIN * NOUT, NOUTP = NW + (BIAS ? NOUT : 0);
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_wgrad_umma<KIN, NOUT, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  XG_CUDA(c, attr);
-  const int grid = umma_grid(n, kWgradPerSm, kWgradBlocks);  // wpart holds kWgradBlocks rows
+  XG_CUDA(c, (allow_smem<k_wgrad_umma<KIN, NOUT, BIAS>>(c, smem)));
+  const int grid = umma_grid(c, n, kWgradPerSm, kWgradBlocks);  // wpart holds kWgradBlocks rows
   k_wgrad_umma<KIN, NOUT, BIAS><<<grid, kUmmaThreads, smem, c->stream>>>(n, X1, X2, dY1, dY2,
                                                                           m->wpart, m->uerr);
   k_reduce_parts<<<(NOUTP + 31) / 32, 32 * kRedRows, 0, c->stream>>>(m->wpart, grid, NOUTP, NW,
