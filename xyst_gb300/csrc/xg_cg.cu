@@ -1865,17 +1865,16 @@ bool loop_shape(const xg_ctx* c, int64_t n, LoopShape* out) {
 // The FP64 solve of a small system by k_cg_cluster launches; false where it
 // does not apply (rows, shared memory, or a device without such clusters).
 constexpr int64_t kClusterIts = 65536;
+constexpr size_t kClusterStatic = 32768;  // its static shared memory, rounded up
 bool cluster_shape(const xg_ctx* c, const CGDev* d, int* per, int* ents, size_t* smem) {
   if (d->n > kClusterRows || d->n < kClusterSize * kSlice || c->cluster != 1) return false;
   *per = static_cast<int>((d->n + kClusterSize * kSlice - 1) / (kClusterSize * kSlice)) * kSlice;
   *ents = d->wmax * *per;
   *smem = size_t(*per) * 5 * sizeof(double) + size_t(*ents) * (sizeof(double) + sizeof(uint32_t));
-  return *smem + 32768 <= c->smem;
+  return *smem + kClusterStatic <= c->smem;
 }
 int cluster_solve(xg_ctx* c, CGDev* d, int per, int ents, size_t smem, CGScalars* h) {
   cudaStream_t s = c->stream;
-  XG_CUDA(c, cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kClusterSize);
   cfg.blockDim = dim3(kClusterThreads);
@@ -1909,8 +1908,7 @@ constexpr int64_t kLoopIts = 8192;
 template <class CI>
 int loop_solve(xg_ctx* c, CGDev* d, const LoopShape& sh, CI ci, CGScalars* h) {
   cudaStream_t s = c->stream;
-  XG_CUDA(c, cudaFuncSetAttribute(k_cg_loop<CI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(sh.smem)));
+  XG_CUDA(c, allow_smem<k_cg_loop<CI>>(c, c->smem - kLoopStatic));
   int64_t n = d->n, its = kLoopIts;
   int per = sh.per;
   const double *a = d->a, *dd = d->d;
@@ -1982,10 +1980,9 @@ int mixed_loop(xg_ctx* c, CGDev* d, CI ca, CI cu, CI cl, CGScalars* h) {
                 d->rs32,  d->msrow, d->d32,  d->z32,    d->p32,
                 d->q32,   d->r32,   d->v32,  d->u32,    d->zp32,  d->vt32, d->e64,
                 d->lpart, d->larrive, d->scal};
-  const size_t smem = size_t(kMixThreads / 32) * SliceWalk<CI, float, kMixFull>::kBytes;
-  const auto kernel = k_mixed_loop<CI, FACTOR>;
-  XG_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
+  constexpr size_t smem = size_t(kMixThreads / 32) * SliceWalk<CI, float, kMixFull>::kBytes;
+  constexpr auto kernel = k_mixed_loop<CI, FACTOR>;
+  XG_CUDA(c, allow_smem<kernel>(c, smem));
   const int64_t ns = (d->n + kSlice - 1) / kSlice;
   const unsigned grid = static_cast<unsigned>(
       std::min<int64_t>(c->nsm, (ns + kMixMinSlices - 1) / kMixMinSlices));
@@ -2039,7 +2036,8 @@ bool cluster_ok(const xg_ctx* c) {
     (void)cudaGetLastError();
     return false;
   }
-  const int most = static_cast<int>(c->smem > 32768 ? c->smem - 32768 : 0);
+  if (c->smem <= kClusterStatic) return false;
+  const size_t most = c->smem - kClusterStatic;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kClusterSize);
   cfg.blockDim = dim3(kClusterThreads);
@@ -2052,8 +2050,7 @@ bool cluster_ok(const xg_ctx* c) {
   cfg.attrs = at;
   cfg.numAttrs = 1;
   int num = 0;
-  if (cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, most) !=
-          cudaSuccess ||
+  if (allow_smem<k_cg_cluster>(c, most) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&num, k_cg_cluster, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
     return false;
