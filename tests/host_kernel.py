@@ -19,6 +19,7 @@ SHIM = r"""
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <initializer_list>
 #define __device__
 #define __host__
 #define __global__
@@ -79,8 +80,8 @@ def cut(text, *names):
     """The definitions of the given functions, types and constants."""
     got = []
     for d in definitions(text):
-        head = re.split(r"[{;=]", re.sub(r"//.*", "", d), maxsplit=1)[0]
-        head = head.split("(")[0] if "__launch_bounds__" not in head else head
+        head = re.sub(r"__launch_bounds__\((?:[^()]|\([^()]*\))*\)", "", re.sub(r"//.*", "", d))
+        head = re.split(r"[({;=]", head, maxsplit=1)[0]
         if any(re.search(rf"\b{n}\b", head) for n in names):
             got.append(d)
     for n in names:

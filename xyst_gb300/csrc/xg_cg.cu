@@ -966,16 +966,21 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned b
       "l"(src), "r"(bytes), "r"(smem_at(mb)), "l"(once)
       : "memory");
 }
+// `bytes` will arrive at the barrier `mb` in its current phase.
+__device__ __forceinline__ void bulk_expect(uint64_t* mb, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_at(mb)), "r"(bytes)
+               : "memory");
+}
 // Waits for the phase `parity` of the barrier; false when it does not come
-// (each try waits for a system-dependent time, so this is seconds).
+// within about a second (a try is suspended for a microsecond at most).
 __device__ __forceinline__ bool bulk_wait(uint64_t* mb, unsigned parity) {
   for (int k = 0; k < kLoopSpin; ++k) {
     unsigned ok;
     asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
         "selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(ok)
-        : "r"(smem_at(mb)), "r"(parity)
+        : "r"(smem_at(mb)), "r"(parity), "r"(1000u)
         : "memory");
     if (ok) return true;
   }
@@ -997,6 +1002,12 @@ constexpr int kMixRound = 8;
 // slice two memory latencies, and the matrix is the larger part of the bytes.
 // The copies are bulk copies, two a slice: as 16-byte asynchronous copies of
 // every lane they held the load path (129^3: 132 us an iteration, 120 so).
+//
+// A warp's copies, in one word that its walks share: the phase of its barrier, a
+// copy under way, a copy that did not arrive.  After a lost copy the warp issues
+// no other and reads no stage; the kernel ends with an error, having waited for
+// that copy once more.
+constexpr unsigned kWalkPhase = 1, kWalkPending = 2, kWalkLost = 4;
 template <class CI, class V, int XM>
 struct SliceWalk {
   using E = typename CI::E;
@@ -1013,12 +1024,12 @@ struct SliceWalk {
   static constexpr int step = kMixThreads / 32;
 
   // (one lane) the slice's columns and values into the stage
-  __device__ __forceinline__ void copy() {
+  __device__ __forceinline__ void copy(unsigned& st) {
     const unsigned we = w < XM ? w : XM;
-    if ((threadIdx.x & 31) || !we) return;
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_at(mb)),
-                 "r"(we * unsigned(kSlice * (sizeof(E) + sizeof(V))))
-                 : "memory");
+    if (!we) return;
+    st |= kWalkPending;
+    if (threadIdx.x & 31) return;
+    bulk_expect(mb, we * unsigned(kSlice * (sizeof(E) + sizeof(V))));
     bulk_copy(stage, val + off, we * unsigned(kSlice * sizeof(V)), mb);
     bulk_copy(stage + XM * kSlice * sizeof(V), ci.c + off, we * unsigned(kSlice * sizeof(E)), mb);
   }
@@ -1035,28 +1046,27 @@ struct SliceWalk {
     }
     return f;
   }
-  // the first slice into the stage; whether a copy is under way
-  __device__ __forceinline__ bool start(int32_t first) {
-    s = first;
+  // the first slice into the stage
+  __device__ __forceinline__ void start(int32_t first, unsigned& st) {
+    s = st & kWalkLost ? end : first;
     asm volatile("" : "+r"(s));  // keeps the addresses of every pass out of the registers of the others
-    if (s >= end) return false;
+    if (s >= end) return;
     const int4 f = places[threadIdx.x >> 5];
     off = f.x;
     w = f.y;
     offn = f.z;
     wn = f.w;
     __syncwarp();
-    copy();
-    return w > 0;
+    copy(st);
   }
   // the stage has been read: the next slice into it
-  __device__ __forceinline__ void advance() {
+  __device__ __forceinline__ void advance(unsigned& st) {
     __syncwarp();
     s += step;
     if (s < end) {
       off = offn;
       w = wn;
-      copy();
+      copy(st);
       if (s + step < end) {
         offn = __ldg(soff + s + step);
         wn = __ldg(sw + s + step);
@@ -1098,23 +1108,25 @@ struct SliceWalk {
   // of the last staged round (loads of the next slice's own row go there).
   // The entries beyond XM of a wide slice are read one by one.
   template <class G, class O>
-  __device__ __forceinline__ float row(int32_t i, G g, O own, unsigned& parity) {
+  __device__ __forceinline__ float row(int32_t i, G g, O own, unsigned& st) {
     const int32_t o = off;
     int32_t r = w;
     if (r > 0) {
-      if (!__all_sync(0xffffffffu, bulk_wait(mb, parity))) {
-        *bad = 1;  // no entry is read, and the walk ends
+      if (__all_sync(0xffffffffu, bulk_wait(mb, st & kWalkPhase))) {
+        st = (st ^ kWalkPhase) & ~kWalkPending;
+      } else {  // no entry is read, and the walk ends
+        *bad = 1;
+        st |= kWalkLost;
         r = 0;
-        end = 0;
+        s = end;
       }
-      parity ^= 1u;
     }
     const int32_t rs = r < XM ? r : XM;
     float t = 0.0f;
     int k = 0;
     for (; rs - k > kMixRound; k += kMixRound) t = fixed<kMixRound>(k, t, i, g, [] {});
     t = pick<1>(rs - k, k, t, i, g, [&] {
-      advance();
+      advance(st);
       own();
     });
     for (k = XM; k < r; ++k) {
@@ -1210,7 +1222,7 @@ __global__ void __launch_bounds__(kMixThreads, 1)
     sh_beta = it == 0 ? 0.0 : sc->rho / sc->rho0;
   }
   for (int64_t i = r0 + threadIdx.x; i < r1; i += kMixThreads) A.zp[i] = make_float2(A.z[i], A.p[i]);
-  unsigned parity = 0;
+  unsigned st = 0;  // the warp's copies
   WalkA wa{A.soff, A.sw, A.ci, A.a, stage, 0, s1, 0, 0, 0, 0, sh_places[0], &sh_mb[wid], &sh_bad};
   WalkT wu{A.soffU, A.swU, A.cu, A.nvU, stage, 0, s1, 0, 0, 0, 0, sh_places[1], &sh_mb[wid], &sh_bad};
   WalkT wl{A.soffL, A.swL, A.cl, A.nvL, stage, 0, s1, 0, 0, 0, 0, sh_places[2], &sh_mb[wid], &sh_bad};
@@ -1225,7 +1237,7 @@ __global__ void __launch_bounds__(kMixThreads, 1)
     }
   }
   __syncwarp();
-  bool pending = wa.start(s0 + wid);
+  wa.start(s0 + wid, st);
   LoopSync sync{A.lpart, A.larrive, 0u, 0};
   const double none[1] = {0.0};
   bool ok = grid_sum<0>(none, 0, sync, sc, [](int, double) {});
@@ -1260,7 +1272,7 @@ __global__ void __launch_bounds__(kMixThreads, 1)
                               const float2 g = A.zp[c];
                               return (g.x + beta * g.y) - p;
                             },
-                            own, parity) +
+                            own, st) +
                         rp;
         if (k <= last) {
           A.p[row] = p;
@@ -1271,14 +1283,14 @@ __global__ void __launch_bounds__(kMixThreads, 1)
           dot[0] += p * q;
         }
       }
-      if (FACTOR) pending = wu.start(s0 + wid);
+      if (FACTOR) wu.start(s0 + wid, st);
       ok = grid_sum32<kMixThreads, 1>(dot, sync, sc, [&](int, double pq) {
         sh_pq = pq;
         sh_rho0 = sh_rho;
         sh_fin = fabs(pq) < DBL_MIN;
         sh_alpha = sh_fin ? 0.0 : sh_rho / pq;
       });
-      ok = ok && !sh_bad;
+      ok = __syncthreads_and(ok && !sh_bad);
       if (!ok) break;
     }
     alpha = float(sh_alpha);
@@ -1303,13 +1315,13 @@ __global__ void __launch_bounds__(kMixThreads, 1)
                 const float2 g = A.vt[c];
                 return g.x - alpha * g.y;
               },
-              own, parity);
+              own, st);
           if (k <= last) A.u[row] = vi + t;
         }
       }
-      pending = wl.start(s0 + wid);
+      wl.start(s0 + wid, st);
       ok = grid_sum<0>(none, 0, sync, sc, [](int, double) {});
-      ok = ok && !sh_bad;
+      ok = __syncthreads_and(ok && !sh_bad);
       if (!ok) break;
       {  // z = -S (I+N) u
         float vi = 0.0f, ui = 0.0f, si = 1.0f, pi = 0.0f;
@@ -1326,7 +1338,7 @@ __global__ void __launch_bounds__(kMixThreads, 1)
         while (wl.s < s1) {
           const int32_t k = wl.s * kSlice + lane, row = min(k, last);
           const float u = ui, p = pi, sr = si, r = vi * __frcp_rn(fabsf(sr));
-          const float acc = u + wl.row(row, [&](int32_t c) { return A.u[c]; }, own, parity);
+          const float acc = u + wl.row(row, [&](int32_t c) { return A.u[c]; }, own, st);
           const float zi = sr < 0.0f ? r : -sr * acc;
           if (k <= last) {
             A.zp[row] = make_float2(zi, p);
@@ -1345,7 +1357,7 @@ __global__ void __launch_bounds__(kMixThreads, 1)
         v[1] += r * r;
       }
     }
-    pending = wa.start(s0 + wid);
+    wa.start(s0 + wid, st);
     it += 1;
     ok = grid_sum32<kMixThreads, 2>(v, sync, sc, [&](int k, double sum) {
       if (k == 0) {
@@ -1356,10 +1368,10 @@ __global__ void __launch_bounds__(kMixThreads, 1)
         sh_end = sh_fin || sqrt(sum) < sh_lim || it >= sh_maxit;
       }
     });
-    ok = ok && !sh_bad;
+    ok = __syncthreads_and(ok && !sh_bad);
   }
   // the next pass's first slice may be on its way
-  if (pending) (void)bulk_wait(&sh_mb[wid], parity);
+  if (st & kWalkPending) (void)bulk_wait(&sh_mb[wid], st & kWalkPhase);
   if (!ok) {  // a wait ran out
     if (threadIdx.x == 0) atomicExch(&sc->err, 1);
     return;
@@ -1921,6 +1933,7 @@ int loop_solve(xg_ctx* c, CGDev* d, const LoopShape& sh, CI ci, CGScalars* h) {
     int rc = read_scal(c, d, h);
     if (rc) return rc;
     if (h->err) {
+      d->ready = false;  // the vectors are of no iteration: a new init is due
       h->err = 0;
       rc = write_scal(c, d, h);
       return rc ? rc : fail(c, XG_ERR_DEVICE, "cg_solve: a grid barrier timed out");
@@ -1994,6 +2007,7 @@ int mixed_loop(xg_ctx* c, CGDev* d, CI ca, CI cu, CI cl, CGScalars* h) {
     int rc = read_scal(c, d, h);
     if (rc) return rc;
     if (h->err) {
+      d->ready = false;  // the vectors are of no iteration: a new init is due
       h->err = 0;
       rc = write_scal(c, d, h);
       return rc ? rc : fail(c, XG_ERR_DEVICE, "cg_solve_mixed: a grid barrier timed out");
