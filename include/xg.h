@@ -187,7 +187,7 @@ int xg_riecg_kernel_times(xg_ctx* ctx, int cap, const char** names, double* ms,
  * and vol (npoin) are device pointers; dt (host) receives cfl * min over
  * nodes of cbrt(vol)/max(|u|+c, 1e-8) evaluated in FP64 arithmetic, or
  * const_dt when |const_dt| > eps.  That is xg_riecg_dt's result for an FP64
- * context up to rounding; an XG_FP32_FLUX context's xg_riecg_dt evaluates the same formula
+ * context; an XG_FP32_FLUX context's xg_riecg_dt evaluates the same formula
  * in FP32 arithmetic, which can differ in the low bits (about 1e-7
  * relative).  Work is issued on stream (a cudaStream_t, null for the
  * default stream) on the calling thread's current device, then synchronised.

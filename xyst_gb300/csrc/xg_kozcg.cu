@@ -132,19 +132,6 @@ __device__ __forceinline__ double dval(unsigned long long k) {
   return __longlong_as_double(b);
 }
 
-// A node's CFL time step before the CFL factor (KozCG.cpp:613-688), L =
-// cbrt(vol) formed at setup, with one quotient by the density: an FP64
-// division is about ten instructions, each of which holds an SM quarter's FP64
-// unit for 64 cycles on GB300.
-__device__ __forceinline__ double node_dt(const double u[5], double L, double g) {
-  const double ir = recip(u[0]);
-  const double uu = u[1] * ir, vv = u[2] * ir, ww = u[3] * ir;
-  const double k2 = uu * uu + vv * vv + ww * ww;
-  const double pr = (u[4] - 0.5 * u[0] * k2) * (g - 1.0);
-  const double c = xsqrt(g * fmax(pr, 0.0) * ir);
-  return L * recip(fmax(xsqrt(k2) + c, 1.0e-8));
-}
-
 __device__ __forceinline__ void block_min_atomic(double v, unsigned long long* dst) {
   __shared__ double red[32];
   unsigned long long bits = __double_as_longlong(v);

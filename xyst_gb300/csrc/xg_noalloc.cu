@@ -23,6 +23,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "xg_fp64.cuh"
 #include "xg_internal.hpp"
 
 namespace {
@@ -38,16 +39,6 @@ static __device__ __align__(256) unsigned long long g_dt_scratch[kNoallocMaxBloc
 unsigned long long* g_scratch_ptr[kNoallocMaxDevices] = {};
 std::once_flag g_scratch_once[kNoallocMaxDevices];
 cudaError_t g_scratch_err[kNoallocMaxDevices] = {};
-
-__device__ __forceinline__ double node_dt(const double u[5], double vol, double g) {
-  double r = u[0];
-  double uu = u[1] / r, vv = u[2] / r, ww = u[3] / r;
-  double pr = (u[4] - 0.5 * r * (uu * uu + vv * vv + ww * ww)) * (g - 1.0);
-  double c = sqrt(g * fmax(pr, 0.0) / r);
-  double L = cbrt(vol);
-  double vel = sqrt(uu * uu + vv * vv + ww * ww);
-  return L / fmax(vel + c, 1.0e-8);
-}
 
 __device__ __forceinline__ unsigned long long warp_min(unsigned long long b) {
 #pragma unroll
@@ -71,7 +62,7 @@ __global__ void __launch_bounds__(kNoallocBlock) k_dt_blocks(int64_t n,
     double u[5];
 #pragma unroll
     for (int c = 0; c < 5; ++c) u[c] = U[p * 5 + c];
-    dtp = node_dt(u, vol[p], gamma);
+    dtp = xg::node_dt(u, cbrt(vol[p]), gamma);
   }
   unsigned long long b = warp_min(__double_as_longlong(dtp));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = b;

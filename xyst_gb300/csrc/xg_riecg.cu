@@ -310,17 +310,6 @@ __device__ __forceinline__ void prim_record(const double u[5], F o[5]) {
   }
 }
 
-// Per-node CFL time step (src/Inciter/RieCG.cpp:827-838), before the CFL
-// factor, with L = cbrt(vol) formed at setup and one quotient by the density.
-__device__ __forceinline__ double node_dt(const double u[5], double L, double g) {
-  const double ir = recip(u[0]);
-  const double uu = u[1] * ir, vv = u[2] * ir, ww = u[3] * ir;
-  const double k2 = uu * uu + vv * vv + ww * ww;
-  const double pr = (u[4] - 0.5 * u[0] * k2) * (g - 1.0);
-  const double c = xsqrt(g * fmax(pr, 0.0) * ir);
-  return L * recip(fmax(xsqrt(k2) + c, 1.0e-8));
-}
-
 // Block-wide minimum of positive doubles folded into *dst with one atomic per
 // block.  Positive IEEE doubles order like their bit patterns.
 __device__ __forceinline__ void block_min_atomic(double v, unsigned long long* dst) {
