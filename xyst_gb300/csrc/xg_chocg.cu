@@ -24,9 +24,10 @@
 //                 plus |d| / |x_a - x_b| for the pressure damping
 //   bnode, park   boundary-node list and [nb][9] domain sums between passes
 // Each node owns its writes (no atomics except the scalar CFL minimum).  The
-// linear edge terms and the damp2 flux are evaluated from the node outwards
-// (they only change sign with the orientation); the damp4 reconstruction,
-// whose regularisation depends on it, in the edge's canonical orientation.
+// linear edge terms and the fluxes are evaluated from the node outwards; only
+// their sign changes with the orientation, to the last bit, so an edge makes no
+// volume or momentum.  The damp4 reconstruction, whose regularisation depends on
+// the orientation, is evaluated in the edge's canonical one.
 // On GB300 an FP64 instruction holds an SM quarter's FP64 unit for 64 cycles,
 // so these passes are written to their FP64 operation count, and signs are
 // flipped on the bits.  A node's neighbours are
@@ -616,7 +617,9 @@ __global__ void __launch_bounds__(kNode) k_crhs(int64_t n, ChoAdj adj, const dou
       const double dd[3] = {dx, dy, dz};
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        acc[c] += a[c] * va + b[c] * vb + pf * dd[c];
+        // a sum of two rounded products, as a fused one would round the two
+        // ends' products differently and the ends' terms would not cancel
+        acc[c] += __dadd_rn(__dmul_rn(a[c], va), __dmul_rn(b[c], vb)) + pf * dd[c];
         if (DAMP4)
           acc[c] -= aw * (b[c] - a[c]) - v * du[c];
         else
