@@ -437,6 +437,12 @@ int xg_cg_set_factor(xg_ctx* ctx, xg_lpc* model, double scale);
  * what ends the solve.  Applies from the next xg_cg_init. */
 int xg_cg_set_guard(xg_ctx* ctx, int guard);
 
+/* Iterations that one launch of a whole solve's kernel runs at most (no
+ * counterpart in the reference): a longer solve takes another launch, with the
+ * same iterates to the last bit.  0, the default after xg_cg_setup, is the
+ * kernels' own limit, which keeps a launch below some seconds. */
+int xg_cg_set_launch_limit(xg_ctx* ctx, int64_t its);
+
 /* z = M^-1 r with the preconditioner of the last xg_cg_init (host vectors). */
 int xg_cg_precondition(xg_ctx* ctx, const double* r, double* z);
 

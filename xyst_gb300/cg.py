@@ -93,6 +93,11 @@ class ConjugateGradients:
         self.ctx.check(self.lib.xg_cg_set_guard(self.ctx.h,
                                                 {"reference": 0, "underflow": 1}[guard]))
 
+    def set_launch_limit(self, its=0):
+        """Iterations per kernel launch of a whole solve (0: the library's
+        limit); the iterates do not depend on it."""
+        self.ctx.check(self.lib.xg_cg_set_launch_limit(self.ctx.h, its))
+
     def precondition(self, r):
         """z = M^-1 r with the preconditioner of the last init."""
         r = f64(r)

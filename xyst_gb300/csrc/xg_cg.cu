@@ -133,6 +133,7 @@ struct CGDev {
   bool factor_set = false;
   uint64_t bc_key = 0;  // hash of the Dirichlet mask the geometry was built for
   int guard = 0;        // breakdown guard of the FP64 solver (xg_cg_set_guard)
+  int64_t launch_its = 0;  // iterations per launch (xg_cg_set_launch_limit), 0: the kernels' own
   xg_lpc* factor_model = nullptr;  // network emitting N, or null: N = factor_c * e
   double factor_c = 1.0;
 };
@@ -1899,8 +1900,9 @@ int cluster_solve(xg_ctx* c, CGDev* d, int per, int ents, size_t smem, CGScalars
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  const int64_t its = d->launch_its ? d->launch_its : kClusterIts;
   for (;;) {
-    XG_CUDA(c, cudaLaunchKernelEx(&cfg, k_cg_cluster, d->n, per, ents, kClusterIts,
+    XG_CUDA(c, cudaLaunchKernelEx(&cfg, k_cg_cluster, d->n, per, ents, its,
                                   static_cast<const int32_t*>(d->soff),
                                   static_cast<const int32_t*>(d->swidth),
                                   static_cast<const int32_t*>(d->col),
@@ -1921,7 +1923,7 @@ template <class CI>
 int loop_solve(xg_ctx* c, CGDev* d, const LoopShape& sh, CI ci, CGScalars* h) {
   cudaStream_t s = c->stream;
   XG_CUDA(c, allow_smem<k_cg_loop<CI>>(c, c->smem - kLoopStatic));
-  int64_t n = d->n, its = kLoopIts;
+  int64_t n = d->n, its = d->launch_its ? d->launch_its : kLoopIts;
   int per = sh.per;
   const double *a = d->a, *dd = d->d;
   void* args[] = {&n,    &per,  &its,     &d->soff, &d->swidth, &ci,         &a,      &dd,
@@ -1988,7 +1990,8 @@ constexpr int kMixMinSlices = 4;  // slices per block at least: fewer blocks mee
 template <class CI, bool FACTOR>
 int mixed_loop(xg_ctx* c, CGDev* d, CI ca, CI cu, CI cl, CGScalars* h) {
   cudaStream_t s = c->stream;
-  MixArgs<CI> A{d->n,     kLoopIts, d->soff, d->swidth, d->soffU, d->swU,  d->soffL,
+  const int64_t its = d->launch_its ? d->launch_its : kLoopIts;
+  MixArgs<CI> A{d->n,     its,      d->soff, d->swidth, d->soffU, d->swU,  d->soffL,
                 d->swL,   ca,       cu,      cl,        d->a32,   d->hvU,  d->hvL,
                 d->rs32,  d->msrow, d->d32,  d->z32,    d->p32,
                 d->q32,   d->r32,   d->v32,  d->u32,    d->zp32,  d->vt32, d->e64,
@@ -2623,6 +2626,16 @@ int xg_cg_set_guard(xg_ctx* c, int guard) {
   if (!d) return fail(c, XG_ERR_STATE, "cg_set_guard before cg_setup");
   if (guard != 0 && guard != 1) return fail(c, XG_ERR_ARG, "cg_set_guard: guard is 0 or 1");
   d->guard = guard;
+  return XG_OK;
+}
+
+int xg_cg_set_launch_limit(xg_ctx* c, int64_t its) {
+  int rc = use(c);
+  if (rc) return rc;
+  CGDev* d = c->cg;
+  if (!d) return fail(c, XG_ERR_STATE, "cg_set_launch_limit before cg_setup");
+  if (its < 0) return fail(c, XG_ERR_ARG, "cg_set_launch_limit: negative");
+  d->launch_its = its;
   return XG_OK;
 }
 

@@ -106,6 +106,7 @@ SIGNATURES = {
     "xg_cg_set_factor": (_int, [_vp, _vp, _dbl]),
     "xg_cg_precondition": (_int, [_vp, _vp, _vp]),
     "xg_cg_set_guard": (_int, [_vp, _int]),
+    "xg_cg_set_launch_limit": (_int, [_vp, _i64]),
     "xg_lpc_nparams": (_i64, []),
     "xg_lpc_create": (_int, [_vp, _int, C.POINTER(_vp)]),
     "xg_lpc_destroy": (_int, [_vp]),
