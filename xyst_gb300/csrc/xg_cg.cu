@@ -18,7 +18,7 @@
 //
 // One PCG iteration (the reference's FP64 algorithm) runs inside k_cg_loop,
 // one cooperative launch for the whole solve, where the rows fit the SMs'
-// shared memory (about 960,000 rows) and no factor is applied.  Otherwise it
+// shared memory (924,160 rows on 152 of them) and no factor is applied.  Otherwise it
 // is three kernels:
 //   k_cg_p: p = z + beta p (beta = rho/rho0)
 //   k_cg_a: q = A p, partial (p, q)
@@ -47,7 +47,7 @@
 // restarting.
 //
 // Whole solves run in one launch: k_cg_cluster (FP64, systems that fit the
-// shared memory of 16 SMs), k_cg_loop (FP64, up to about 960,000 rows) and
+// shared memory of 16 SMs), k_cg_loop (FP64, up to 924,160 rows) and
 // k_mixed_loop (the FP32 iterations up to the next residual replacement); the
 // FP64 factored solve and larger FP64 systems take a launch per pass.
 
@@ -124,7 +124,8 @@ struct CGDev {
   int32_t *soffL = nullptr, *swL = nullptr, *colL = nullptr, *posL = nullptr, *tposU = nullptr;
   int32_t *soffU = nullptr, *swU = nullptr, *colU = nullptr;
   int16_t *colL16 = nullptr, *colU16 = nullptr;
-  float *nvL = nullptr, *nvU = nullptr, *srow = nullptr, *msrow = nullptr, *eL = nullptr, *eU = nullptr;
+  float *nvL = nullptr, *nvU = nullptr, *srow = nullptr, *msrow = nullptr;
+  float *eL = nullptr, *eU = nullptr;
   __half *hvL = nullptr, *hvU = nullptr;
   float* eF = nullptr;  // e_ij in the full layout (0 on the diagonal and at Dirichlet nodes)
   double *v = nullptr, *u = nullptr, *t = nullptr;  // S r, (I+N)^T S r; t: xg_cg_precondition
@@ -324,7 +325,8 @@ unsigned pgrid(const xg_ctx* c, int64_t n) {
     return v < 1 ? 1 : v;
   }();
   const int64_t want = (n + kBlock - 1) / kBlock;
-  return static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(per_sm) * c->nsm)));
+  return static_cast<unsigned>(
+      std::max<int64_t>(1, std::min<int64_t>(want, int64_t(per_sm) * c->nsm)));
 }
 
 #define XG_ROWS(i, n) \
@@ -705,7 +707,8 @@ struct LoopSync {
 // The second half of a barrier: warp k < K (at least warp 0) comes with the
 // block's sum of value k in lane 0 of `s`.
 template <int K, class F>
-__device__ __forceinline__ bool grid_meet(double s, LoopSync& sync, CGScalars* sc, int* okay, F fin) {
+__device__ __forceinline__ bool grid_meet(double s, LoopSync& sync, CGScalars* sc, int* okay,
+                                          F fin) {
   constexpr int KW = K > 0 ? K : 1;  // polling warps
   const int nb = gridDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   sync.target += unsigned(nb) * KW;
@@ -718,7 +721,10 @@ __device__ __forceinline__ bool grid_meet(double s, LoopSync& sync, CGScalars* s
       unsigned int seen = 0;
       int spin = 0;
       do {
-        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync.arrive) : "memory");
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
+                     : "=r"(seen)
+                     : "l"(sync.arrive)
+                     : "memory");
       } while (int(seen - sync.target) < 0 && ++spin < kLoopSpin);
       asm volatile("fence.acq_rel.gpu;" ::: "memory");
       if (spin >= kLoopSpin) {
@@ -802,7 +808,8 @@ __device__ __forceinline__ bool grid_sum(const double (&v)[K > 0 ? K : 1], int a
 // The barrier with sums of FP32 values: summed over each warp in FP32, the
 // warps' sums and the blocks' in FP64 (as block_partials sums them).
 template <int NT, int K, class F>
-__device__ __forceinline__ bool grid_sum32(const float (&v)[K], LoopSync& sync, CGScalars* sc, F fin) {
+__device__ __forceinline__ bool grid_sum32(const float (&v)[K], LoopSync& sync, CGScalars* sc,
+                                           F fin) {
   __shared__ float warps[K][32];
   __shared__ int okay;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -832,14 +839,11 @@ __device__ __forceinline__ bool grid_sum32(const float (&v)[K], LoopSync& sync, 
 // diagonal in shared memory; only the direction (gathered by other rows), x
 // and the matrix are in global memory.
 //
-// Three launches per iteration cost their drains, launch gaps and two
-// reduction tails (about 20 us an iteration however small the system), and
-// on GB300 the FP64 pipe is a bound beside memory: 22 FP64 operations a row
-// and iteration take 11 us at 65^3 and 38 us at 97^3 (530 G operations/s).
-// Here an iteration pays three grid barriers (grid_sum): 38 -> 21 us an
-// iteration at 65^3, 65 -> 48 us at 97^3, 17 -> 10 us at 17^3.  1024 threads with
-// rounds of 8 entries and 512 with rounds of 16 measured within 3 % of each
-// other.
+// The bounds are the FP64 pipe (22 operations a row: 11 us an iteration at 65^3,
+// 38 at 97^3, where it is 70 % busy) and three grid barriers (grid_sum), for
+// the drains, gaps and reduction tails of three launches: 38 -> 21 us an
+// iteration at 65^3, 65 -> 48 at 97^3, 17 -> 10 at 17^3.  1024 threads with
+// rounds of 8 entries and 512 with rounds of 16 are within 3 % of each other.
 template <class CI>
 __global__ void __launch_bounds__(kLoopThreads, 1)
     k_cg_loop(int64_t n, int per, int64_t maxits, const int32_t* __restrict__ soff,
@@ -957,19 +961,22 @@ __device__ __forceinline__ unsigned smem_at(const void* p) {
 // both), asynchronously, counted at the barrier `mb`.  The bytes are read once
 // a pass and leave L2 first: at 129^3 the vectors then stay there (A's pass
 // 46 -> 40 us, the lower triangle's 23.5 -> 21.5).
-__device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, uint64_t* mb) {
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes,
+                                          uint64_t* mb) {
   uint64_t once;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once));
   asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], "
-      "%4;" ::"r"(
-          smem_at(dst)),
-      "l"(src), "r"(bytes), "r"(smem_at(mb)), "l"(once)
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1], %2, [%3], %4;"
+      :
+      : "r"(smem_at(dst)), "l"(src), "r"(bytes), "r"(smem_at(mb)), "l"(once)
       : "memory");
 }
 // `bytes` will arrive at the barrier `mb` in its current phase.
 __device__ __forceinline__ void bulk_expect(uint64_t* mb, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_at(mb)), "r"(bytes)
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+               :
+               : "r"(smem_at(mb)), "r"(bytes)
                : "memory");
 }
 // Waits for the phase `parity` of the barrier; false when it does not come
@@ -1050,7 +1057,7 @@ struct SliceWalk {
   // the first slice into the stage
   __device__ __forceinline__ void start(int32_t first, unsigned& st) {
     s = st & kWalkLost ? end : first;
-    asm volatile("" : "+r"(s));  // keeps the addresses of every pass out of the registers of the others
+    asm volatile("" : "+r"(s));  // keeps a pass's addresses out of the others' registers
     if (s >= end) return;
     const int4 f = places[threadIdx.x >> 5];
     off = f.x;
@@ -1180,11 +1187,9 @@ constexpr int kMixFull = 16, kMixTri = 8;  // staged entries per row: whole rows
 // The bound is memory: 6 bytes an entry of A, 4 of each triangle and some 90
 // of vectors a row, 0.5 GB an iteration at 129^3; A's pass runs at 7.4 TB/s
 // there (part of the vectors stays in L2), the triangles' at 5, and the three
-// barriers with their sums take 2 to 5 us each.  A launch per pass (three an
-// iteration, every row waiting in turn for its columns, its values and its
-// gathers) took 145 us an iteration at 129^3 where this takes 106 (89 in the kernel), 35.5
-// against 27.9 at 65^3 and 27.1 against 24.3 at 17^3 (the whole solve's time
-// over its iterations).
+// barriers with their sums take 2 to 5 us each.  The whole solve's time over its
+// iterations, a launch per pass against this: 145 / 104 us at 129^3, 35.5 / 27.9
+// at 65^3, 27.1 / 24.3 at 17^3.
 template <class CI, bool FACTOR>
 __global__ void __launch_bounds__(kMixThreads, 1)
     k_mixed_loop(const __grid_constant__ MixArgs<CI> A) {
@@ -1222,12 +1227,15 @@ __global__ void __launch_bounds__(kMixThreads, 1)
     sh_bad = 0;
     sh_beta = it == 0 ? 0.0 : sc->rho / sc->rho0;
   }
-  for (int64_t i = r0 + threadIdx.x; i < r1; i += kMixThreads) A.zp[i] = make_float2(A.z[i], A.p[i]);
+  for (int64_t i = r0 + threadIdx.x; i < r1; i += kMixThreads)
+    A.zp[i] = make_float2(A.z[i], A.p[i]);
   unsigned st = 0;  // the warp's copies
-  WalkA wa{A.soff, A.sw, A.ci, A.a, stage, 0, s1, 0, 0, 0, 0, sh_places[0], &sh_mb[wid], &sh_bad};
-  WalkT wu{A.soffU, A.swU, A.cu, A.nvU, stage, 0, s1, 0, 0, 0, 0, sh_places[1], &sh_mb[wid], &sh_bad};
-  WalkT wl{A.soffL, A.swL, A.cl, A.nvL, stage, 0, s1, 0, 0, 0, 0, sh_places[2], &sh_mb[wid], &sh_bad};
-  if (lane == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_at(&sh_mb[wid])) : "memory");
+  uint64_t* mb = &sh_mb[wid];
+  WalkA wa{A.soff, A.sw, A.ci, A.a, stage, 0, s1, 0, 0, 0, 0, sh_places[0], mb, &sh_bad};
+  WalkT wu{A.soffU, A.swU, A.cu, A.nvU, stage, 0, s1, 0, 0, 0, 0, sh_places[1], mb, &sh_bad};
+  WalkT wl{A.soffL, A.swL, A.cl, A.nvL, stage, 0, s1, 0, 0, 0, 0, sh_places[2], mb, &sh_bad};
+  if (lane == 0)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_at(mb)) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncwarp();
   if (lane == 0) {
@@ -1859,7 +1867,8 @@ void factor_apply32(xg_ctx* c, CGDev* d, CI cu, CI cl) {
 // each of the SM's four FP64 units, which take as long for one warp as for
 // none beside it, and fewer blocks' sums to add.
 constexpr int64_t kLoopMinRows = 128;
-constexpr size_t kLoopStatic = 4 * (kLoopThreads + 128) * 8 + 1024;  // its static shared memory, rounded up
+// its static shared memory, rounded up
+constexpr size_t kLoopStatic = 4 * (kLoopThreads + 128) * 8 + 1024;
 struct LoopShape {
   int per = 0;
   unsigned grid = 0;

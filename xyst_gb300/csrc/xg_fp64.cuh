@@ -60,7 +60,7 @@ __device__ __forceinline__ double widen(float x, unsigned sign) {  // x > 0
 }
 // 1/d from the FP32 approximation x of 1/d (about 22 bits): with e = 1 - d x,
 // 1/d = x / (1 - e), taken to e^2 (the third-order Householder step; the rest
-// is e^3, below 1e-18): three FP64 instructions.
+// is e^3, below 1e-18): three FP64 instructions, within 1.1e-16 (one rounding).
 __device__ __forceinline__ double recip(double d) {
   if (!in_float(d)) return 1.0 / d;
   float a;
@@ -70,13 +70,13 @@ __device__ __forceinline__ double recip(double d) {
   return fma(x, fma(e, e, e), x);
 }
 __device__ __forceinline__ float recip(float d) { return 1.0f / d; }
-// a / b, in double as a times ib = recip(b)
+// a / b, in double as a times ib = recip(b), within 2.2e-16
 __device__ __forceinline__ double over(double a, double, double ib) { return a * ib; }
 __device__ __forceinline__ float over(float a, float b, float) { return a / b; }
 // sqrt: in double from the FP32 approximation y of 1/sqrt(x) (about 22 bits):
 // with s = x y and e = 1 - x y^2, sqrt(x) = s / sqrt(1 - e) =
-// s (1 + e/2 + 3 e^2/8 + ...), the rest below 1e-18: five FP64 instructions;
-// the library's root for negative x and outside FP32's range.
+// s (1 + e/2 + 3 e^2/8 + ...), the rest below 1e-18: five FP64 instructions,
+// within 1.7e-16; the library's root for negative x and outside FP32's range.
 __device__ __forceinline__ double xsqrt(double x) {
   if (!in_float(x) || __double2hiint(x) < 0) return sqrt(x);
   float a;

@@ -242,7 +242,8 @@ __device__ __forceinline__ void load10(const unsigned long long* p, unsigned lon
   }
 }
 __device__ __forceinline__ void load10(const unsigned int* p, unsigned int o[10]) {
-  const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+  const uint4 a = __ldg(reinterpret_cast<const uint4*>(p));
+  const uint4 b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
   const uint2 c = __ldg(reinterpret_cast<const uint2*>(p + 8));
   o[0] = a.x, o[1] = a.y, o[2] = a.z, o[3] = a.w;
   o[4] = b.x, o[5] = b.y, o[6] = b.z, o[7] = b.w;
@@ -469,15 +470,13 @@ __device__ __forceinline__ void elem_terms(int64_t n, int64_t ne, int64_t e,
 }
 
 // The FP32 residual pass is made of blocks of kFB elements (a slot 4 e + a of a
-// block fits a byte).  Atomics bound it: at about 200 G of 16 bytes a second,
-// four nodes of four each an element took 396 us at 97^3.  Consecutive elements
+// block fits a byte).  Atomics would bound it (about 200 G of 16 bytes a second:
+// 396 us at 97^3 with four nodes of four each an element).  Consecutive elements
 // share nodes (those of 64 hold 50 distinct ones of 256 with locality
-// numbering, 71 numbered at random), so a block leaves its elements'
-// contributions in shared memory, adds them per distinct node (lists made once
-// per mesh) and hands one record a node to the atomics: 262 us, with 14 blocks
-// an SM (12: 287).  The limiting pass, whose two atomics a node are not its
-// bound, gained nothing (227 against 223), nor did either pass from the nodes'
-// records staged in shared memory (308 and 269).
+// numbering, 71 numbered at random), so a block adds its elements' contributions
+// per distinct node in shared memory (lists made once per mesh) and hands one
+// record a node to the atomics: 262 us, with 14 blocks an SM (12: 287).  The
+// limiting pass, with two atomics a node, gains nothing so (227 against 223).
 constexpr int kFB = 64;
 constexpr int kFW = kFB / 32;
 constexpr int kNG = 6;  // nodes a warp adds together, a lane per component
@@ -590,7 +589,7 @@ __global__ void __launch_bounds__(kFB, 14) k_elem_rhs_aec32(int64_t n, int64_t n
 // builds its four in shared memory (kStW double2 per lane: 16-byte stores
 // of 8 lanes fall in distinct banks) and the warp moves the run to or from
 // global memory with contiguous 512-byte accesses.
-constexpr int kEB = 64;    // FP64 element-pass block: small, as an SM's FP64 units take its blocks in turn
+constexpr int kEB = 64;    // FP64 element-pass block: an SM's FP64 units take its blocks in turn
 constexpr int kStW = 21;   // staged double2 per lane
 constexpr int kRecD2 = 5;  // residual slot record, double2
 constexpr int kLimD2 = 3;  // limited slot record, double2

@@ -1144,7 +1144,8 @@ int dense_umma(xg_ctx* c, xg_lpc* m, int64_t n, const float* X1, const float* X2
                const float* bias, int act, const float* maskY, float* Y1, float* Y2) {
   constexpr int smem = (kUmmaM * KIN + NOUT * KIN) * 2;
   XG_CUDA(c, (allow_smem<k_dense_umma<KIN, NOUT, FROM_W>>(c, smem)));
-  k_dense_umma<KIN, NOUT, FROM_W><<<umma_grid(c, n, kDensePerSm, INT_MAX), kUmmaThreads, smem, c->stream>>>(
+  const int grid = umma_grid(c, n, kDensePerSm, INT_MAX);
+  k_dense_umma<KIN, NOUT, FROM_W><<<grid, kUmmaThreads, smem, c->stream>>>(
       n, X1, X2, W, bias, act, maskY, Y1, Y2, m->uerr);
   XG_CHECK_LAUNCH(c);
   return XG_OK;

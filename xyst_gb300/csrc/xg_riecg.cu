@@ -343,7 +343,8 @@ __device__ __forceinline__ void block_min_atomic(double v, unsigned long long* d
 // the same pair of numbers as 2|a|/(|a|+|b|), 2|b|/(|a|+|b|) for a b > 0 and
 // 0, 0 otherwise.  Both precisions reduce the limited reconstruction
 // algebraically (below): FP64 exactly, with one quotient per side and
-// component instead of the reference's four (the difference is rounding, a few 1e-16 of the increment); FP32 to the harmonic slope.
+// component instead of the reference's four (the difference is rounding, a few
+// 1e-16 of the increment); FP32 to the harmonic slope.
 template <class F>
 __device__ __forceinline__ void muscl(const F wl[5], const F wr[5], const F g1[5],
                                       const F g2[5], bool back, F l[5], F r[5]) {
@@ -363,7 +364,8 @@ __device__ __forceinline__ void muscl(const F wl[5], const F wr[5], const F g1[5
     // `back`: the ends are given as R, L, so every difference and slope has
     // the other sign; with eps negated as well every product, and so each end's
     // reconstruction, is the same number as with the ends in order.
-    constexpr F h1 = F(0.5e-9) * (F(1.0) - F(1.0) / F(3.0)), h2 = F(0.5e-9) * (F(1.0) + F(1.0) / F(3.0));
+    constexpr F h1 = F(0.5e-9) * (F(1.0) - F(1.0) / F(3.0));
+    constexpr F h2 = F(0.5e-9) * (F(1.0) + F(1.0) / F(3.0));
     constexpr F H = F(0.5) * h1 * h2;
     const F A0 = flip_if(F(0.5) * (F(1.0e-9) - h2), back), B0 = flip_if(F(1.0e-9) - h1, back);
     const F meps = flip_if(1.0e-9, !back);
@@ -780,11 +782,10 @@ struct NodeAux {
 // * After it, in a kernel of their own that adds the triangles to the domain
 //   sums: those were read coalesced, where boundary lanes reading the
 //   edges again take memory bandwidth.
-// A thread per node in the separate kernels was a serial chain on a handful of
-// SMs (in FP64 some 700 instructions of 64 cycles: 69 and 91 us a stage at any
-// size).  Also measured at 129^3, FP32, per stage (separate 297 us): beside
-// 322 us, beside with the boundary blocks spread over the grid 311 us, the
-// triangles by the domain blocks' own threads after a barrier 450 us.
+// Latency bounds it: one lane a node is a serial chain on a handful of SMs, in
+// FP64 some 700 instructions of 64 cycles (91 us a stage at any size; four lanes
+// 18 at 33^3).  At 129^3 in FP32 both passes take 297 us a stage separate, 322
+// beside, 450 with the triangles by the domain blocks' own threads.
 template <int BL>
 __device__ __forceinline__ bool bnd_lane(int64_t nbn, int64_t& bi, int& l) {
   const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
